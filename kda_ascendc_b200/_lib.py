@@ -132,5 +132,22 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host path of the public functions (csrc/kda_host.cpp), loaded once."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _kda_host
+        except ImportError as e:
+            raise RuntimeError("the native host module is missing or does not load (%s): build it with "
+                               "`python -m kda_ascendc_b200.build`" % e) from e
+        _host = _kda_host
+    return _host
+
+
 def last_error() -> str:
     return load().kda_last_error().decode("utf-8", "replace")

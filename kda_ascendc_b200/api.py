@@ -12,7 +12,9 @@ edits:
 Everything numeric happens in ``libkda_b200.so`` (two CUDA kernels, see
 ``include/kda_b200.h``).  This module validates, allocates outputs and the K1->K2
 workspace with ``torch.empty``, fills a ``KdaFwdArgs`` and launches on the current
-CUDA stream without synchronising.  Inputs that are not CUDA tensors are refused:
+CUDA stream without synchronising.  The plain calls are served by the native host module
+(``csrc/kda_host.cpp``), which accepts a call only when every check below would pass; what it
+leaves over -- wrong arguments, debug outputs, stage timing -- takes the Python path.  Inputs that are not CUDA tensors are refused:
 there is no CPU path.
 """
 from __future__ import annotations
@@ -256,6 +258,11 @@ def _varlen_tables(cu_seqlens, T: int, H: int, device):
     return n_seqs, n_chunks, dev_tab[:n_chunks], dev_tab[n_chunks:], host
 
 
+def _count_chunk() -> None:
+    _LAUNCH_COUNTS["kda_k1"] += 1
+    _LAUNCH_COUNTS["kda_k2"] += 1
+
+
 def _flags(use_gate, use_l2, use_beta_sigmoid) -> int:
     return ((_lib.FLAG_GATE if use_gate else 0) | (_lib.FLAG_L2NORM if use_l2 else 0) |
             (_lib.FLAG_BETA_SIGMOID if use_beta_sigmoid else 0))
@@ -306,8 +313,7 @@ def _forward(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_
                                  shape=(B, T, H), workspace_bytes=ws.numel())
         else:
             _check(lib.kda_fwd(ctypes.byref(args), stream))
-    _LAUNCH_COUNTS["kda_k1"] += 1
-    _LAUNCH_COUNTS["kda_k2"] += 1
+    _count_chunk()
     if return_intermediates:
         from .layout import unpack_records
         inter = unpack_records(ws, B, T, H)
@@ -332,6 +338,11 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_f
     the chunk path's bf16 rounding of the normalised q and k, so that a prefill by
     :func:`kda_bt16_fwd` followed by steps of this function continues the same sequence.
     """
+    res = _lib.host().recurrent(q, k, v, g, beta, scale, initial_state, output_final_state, lower_bound, A_log, dt_bias,
+                                inplace_state, state_v_first, RECURRENT_MAX_TOKENS, False)
+    if res is not None:
+        _LAUNCH_COUNTS["kda_recurrent"] += 1
+        return res
     _validate_kda_inputs(q, k, v, g, beta, initial_state, True, True, lower_bound, A_log, dt_bias, state_v_first,
                          require_contiguous=False)
     _require_cuda(q)
@@ -399,29 +410,17 @@ class ForwardPlan:
         if tables is not None:
             self._args.n_seqs, self._args.n_chunks = tables[0], tables[1]
             self._args.chunk_table, self._args.seq_table = _ptr(tables[2]), _ptr(tables[3])
-        self._ref = ctypes.byref(self._args)
-        self._fn = _lib.load().kda_fwd
+        self._run, self._addr, self._index = _lib.host().run_plan, ctypes.addressof(self._args), _device_index(q.device)
 
     def run(self, stream: Optional[int] = None):
         """One forward over the current contents of the input buffers; returns ``(o, final_state)``."""
-        if stream is None:
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-        rc = _call_on_device(self.device, self._fn, self._ref, ctypes.c_void_p(stream))
-        if rc != 0:
-            _check(rc)
-        _LAUNCH_COUNTS["kda_k1"] += 1
-        _LAUNCH_COUNTS["kda_k2"] += 1
+        self._run(self._addr, self._index, stream, False)
+        _count_chunk()
         return self.o, self.final_state
 
 
-def _call_on_device(device, fn, *args):
-    """Call a C entry point with ``device`` current.  The library sizes grids, caches kernel
-    attributes and resolves tensor maps for the CURRENT device, so a process that drives several
-    GPUs must not run a plan built for one of them while another is current."""
-    if torch.cuda.current_device() == device.index:
-        return fn(*args)
-    with torch.cuda.device(device):
-        return fn(*args)
+def _device_index(device) -> int:
+    return torch.cuda.current_device() if device.index is None else device.index
 
 
 class RecurrentPlan:
@@ -449,17 +448,12 @@ class RecurrentPlan:
         self._args = make_args(q, k, v, g, beta, scale=K ** -0.5 if scale is None else scale, lower_bound=lower_bound,
                                A_log=A_log, dt_bias=dt_bias, h0=state, o=self.o, ht=state, workspace=None,
                                flags=_flags(True, True, True) | (0 if state_v_first else _lib.FLAG_STATE_K_FIRST))
-        self._ref = ctypes.byref(self._args)
-        self._fn = _lib.load().kda_recurrent_fwd
+        self._run, self._addr, self._index = _lib.host().run_plan, ctypes.addressof(self._args), _device_index(q.device)
 
     def step(self, stream: Optional[int] = None):
         """Apply the tokens currently in the input buffers; returns ``o`` (the plan's own tensor).
         ``stream``: raw CUDA stream handle; default = the current torch stream of the plan's device."""
-        if stream is None:
-            stream = torch.cuda.current_stream(self.device).cuda_stream
-        rc = _call_on_device(self.device, self._fn, self._ref, ctypes.c_void_p(stream))
-        if rc != 0:
-            _check(rc)
+        self._run(self._addr, self._index, stream, True)
         _LAUNCH_COUNTS["kda_recurrent"] += 1
         return self.o
 
@@ -489,6 +483,13 @@ def kda_bt16_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_final_
     chunked from its own first token, ``initial_state`` / the returned state are
     ``[n_seqs, H, 128, 128]``.
     """
+    if not reuse_workspace:
+        res = _lib.host().chunk(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
+                                use_gate_in_kernel, use_beta_sigmoid_in_kernel, safe_gate, lower_bound, A_log, dt_bias,
+                                state_v_first, cu_seqlens, False)
+        if res is not None:
+            _count_chunk()
+            return res
     n_states = None
     if cu_seqlens is not None:
         if q.ndim == 4 and q.shape[0] != 1:

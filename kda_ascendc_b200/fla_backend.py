@@ -24,7 +24,7 @@ from typing import Optional
 
 import torch
 
-from . import api
+from . import _lib, api
 
 BACKEND_NAME = "kda_b200"
 
@@ -65,6 +65,14 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
     """FLA's ``chunk_kda`` keyword set on the B200 kernels (chunk size 16 inside; the result does
     not depend on the chunk size).  ``A_log`` / ``dt_bias`` come as keywords, as in FLA."""
     A_log, dt_bias = kwargs.get("A_log"), kwargs.get("dt_bias")
+    cu = cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens
+    if (use_qk_l2norm_in_kernel and use_gate_in_kernel and not return_intermediate_states and cp_context is None):
+        res = _lib.host().chunk(q, k, v, g, beta, scale, initial_state, output_final_state, True, True,
+                                use_beta_sigmoid_in_kernel, safe_gate, lower_bound, A_log, dt_bias,
+                                _v_first(kwargs, transpose_state_layout), cu, True)
+        if res is not None:
+            api._count_chunk()
+            return res
     ok, why = supports(q, k, v, g, beta, use_qk_l2norm_in_kernel=use_qk_l2norm_in_kernel,
                        use_gate_in_kernel=use_gate_in_kernel, use_beta_sigmoid_in_kernel=use_beta_sigmoid_in_kernel,
                        safe_gate=safe_gate, lower_bound=lower_bound, A_log=A_log,
@@ -73,7 +81,6 @@ def chunk_kda(q, k, v, g, beta, scale=None, initial_state=None, output_final_sta
         raise NotImplementedError(f"{BACKEND_NAME}: {why}")
     if dt_bias is not None:
         dt_bias = dt_bias.reshape(-1)
-    cu = cu_seqlens_cpu if cu_seqlens_cpu is not None else cu_seqlens
     return api.kda_bt16_fwd(q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous(), beta.float().contiguous(),
                             scale=scale, initial_state=initial_state, output_final_state=output_final_state,
                             use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True,
@@ -87,6 +94,12 @@ def fused_recurrent_kda(q, k, v, g, beta, A_log=None, dt_bias=None, scale=None, 
                         use_beta_sigmoid_in_kernel=False, lower_bound=None, cu_seqlens=None,
                         transpose_state_layout=None, **kwargs):
     """FLA's ``fused_recurrent_kda`` keyword set on the token-recurrence kernel (decode)."""
+    if use_qk_l2norm_in_kernel and use_gate_in_kernel and use_beta_sigmoid_in_kernel and cu_seqlens is None:
+        res = _lib.host().recurrent(q, k, v, g, beta, scale, initial_state, output_final_state, lower_bound, A_log, dt_bias,
+                                    False, _v_first(kwargs, transpose_state_layout), api.RECURRENT_MAX_TOKENS, True)
+        if res is not None:
+            api._LAUNCH_COUNTS["kda_recurrent"] += 1
+            return res
     ok, why = supports(q, k, v, g, beta, use_qk_l2norm_in_kernel=use_qk_l2norm_in_kernel,
                        use_gate_in_kernel=use_gate_in_kernel, use_beta_sigmoid_in_kernel=use_beta_sigmoid_in_kernel,
                        safe_gate=True, lower_bound=lower_bound, A_log=A_log)
