@@ -147,7 +147,63 @@ void pick_split(const KdaFwdArgs* a, bool state_only, int* vsplit, int* variant,
 int* status_ptr(const KdaFwdArgs* a) { return static_cast<int*>(a->workspace); }
 uint8_t* rec_ptr(const KdaFwdArgs* a) { return static_cast<uint8_t*>(a->workspace) + kda::WS_HEADER_BYTES; }
 
-int do_k1(const KdaFwdArgs* a, cudaStream_t st) {
+int device_sms() {
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+// Address range of a strided [B, T, heads, row] tensor (strides in elements, none negative).
+struct Span { uintptr_t lo, hi; };
+Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads, int row, int elem_bytes) {
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(ptr);
+  const int64_t last = (a->B - 1) * s[0] + (a->T - 1) * s[1] + (heads - 1) * s[2] + row;
+  return {lo, lo + static_cast<uintptr_t>(last) * elem_bytes};
+}
+
+// Chunks per window of a forward whose K2 runs beside its K1; 0 = K2 starts after K1.
+//
+// A K2 whose chains leave most of the chip idle runs on the SMs that K1 is still working on: K1 is held to
+// two CTAs per SM (that leaves a K2 CTA its shared memory and registers), walks the chunks of all chains in
+// time order and counts the finished items of every window of chunks; K2's producer warps wait for
+// the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA is
+// already running.  Where it pays, measured on B200 as the whole forward, K2 after K1 against beside it:
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T131072 H16 4,517 -> 4,268 us,
+//     B2 T4096 H8 153.3 -> 149.9, B1 T8192 H8 254.4 -> 250.5;
+//   tensor-memory form with one CTA per SM: T8192 H96 1,044 -> 970, T2048 H96 273 -> 255, T1024 H96 146 -> 135,
+//     but T4096 H128 602 -> 631 (no SM is left to K1 alone): up to three quarters of the SMs.
+// Not in the other forms: with four consumer warps per CTA K2 has no issue slots to spare, or (8-row form)
+// does not fit beside two K1 CTAs: T8192 H32 418 -> 515, T4096 H48 317 -> 379.
+int beside_window(const KdaFwdArgs* a) {
+  if (a->n_seqs > 0) return 0;
+  int vsplit = 0, variant = 0;
+  const int sms = device_sms();
+  pick_split(a, false, &vsplit, &variant, sms);
+  const long long chains = static_cast<long long>(a->B) * a->H, nt = (static_cast<long long>(a->T) + kda::BT - 1) / kda::BT;
+  if (!(variant == 1 && vsplit >= 8 && chains * vsplit <= sms) && !(variant == 4 && chains * 4 <= 3LL * sms)) return 0;
+  const long long round = 2LL * sms;   // items that K1 has in flight
+  if (chains * nt < 8 * round) return 0;   // K1 is over in a few rounds: nothing to run beside
+  // o is written while K1 still reads its inputs: they may not overlap (h0 and ht are safe: a chain's final
+  // state is written once every window, so every item of K1, is finished)
+  const int64_t* os = a->o_stride;
+  for (int i = 0; i < 3; ++i)
+    if (os[i] < 0 || a->beta_stride[i] < 0) return 0;
+  const int hq = a->Hq > 0 ? a->Hq : a->H;
+  const Span o = span_of(a->o, os, a, a->H, kda::D, 2);
+  const Span in[7] = {span_of(a->q, a->q_stride, a, hq, kda::D, 2), span_of(a->k, a->k_stride, a, hq, kda::D, 2),
+                      span_of(a->v, a->v_stride, a, a->H, kda::D, 2),
+                      span_of(a->g, a->g_stride, a, a->H, kda::D, a->g_dtype == KDA_G_BF16 ? 2 : 4),
+                      span_of(a->beta, a->beta_stride, a, a->H, 1, 4),
+                      {reinterpret_cast<uintptr_t>(a->A_log), reinterpret_cast<uintptr_t>(a->A_log + (a->A_log ? a->H : 0))},
+                      {reinterpret_cast<uintptr_t>(a->dt_bias),
+                       reinterpret_cast<uintptr_t>(a->dt_bias + (a->dt_bias ? static_cast<int64_t>(a->H) * kda::D : 0))}};
+  for (const Span& s : in)
+    if (o.lo < s.hi && s.lo < o.hi) return 0;
+  const long long by_count = (nt + kda::MAX_WINDOWS - 1) / kda::MAX_WINDOWS, by_round = (2 * round + chains - 1) / chains;
+  return static_cast<int>(by_count > by_round ? by_count : by_round);
+}
+
+int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
   kda::K1Params p;
   memset(&p, 0, sizeof(p));
   p.q = static_cast<const __nv_bfloat16*>(a->q);
@@ -177,6 +233,12 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st) {
   }
   p.Hq = a->Hq > 0 ? a->Hq : a->H;
   p.div_g.set(static_cast<uint32_t>(p.H / p.Hq));
+  if (win_chunks > 0) {
+    p.progress = status_ptr(a) + kda::HDR_PROGRESS;
+    p.ctas_per_sm = 2;   // with one, K1 becomes the longer of the two (T8192 H96 1,338 us); three do not fit beside K2
+    p.div_b.set(static_cast<uint32_t>(p.B));
+    p.div_win.set(static_cast<uint32_t>(win_chunks) * p.B * p.H);
+  }
   // 2^g may be factored as 2^(g-g_mid) * 2^(g_mid) only while no factor can underflow:
   // 16 tokens * |lower_bound| * RCP_LN2 must stay inside the fp32 exponent range.
   const bool fast_exp = (a->flags & KDA_FLAG_GATE_IN_KERNEL) && (16.0f * -a->lower_bound * kda::RCP_LN2 <= 120.0f);
@@ -217,7 +279,7 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st) {
 struct H0Flags { const int32_t* flags; int n, epoch; };
 
 int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, const KdaPeerPushArgs* push = nullptr,
-          const H0Flags* h0f = nullptr) {
+          const H0Flags* h0f = nullptr, bool after_k1 = false, int win_chunks = 0) {
   kda::K2Params p;
   memset(&p, 0, sizeof(p));
   p.rec = rec_ptr(a);
@@ -230,6 +292,10 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   p.scale = a->scale;
   p.zero_u = zero_u == 1;
   p.k_first = (a->flags & KDA_FLAG_STATE_K_FIRST) ? 1 : 0;
+  if (win_chunks > 0) {
+    p.progress = status_ptr(a) + kda::HDR_PROGRESS;
+    p.win_chunks = win_chunks;
+  }
   p.pair_mode = (state_only && zero_u == 2) ? 1 : 0;
   if (a->n_seqs > 0) {
     p.seq_table = reinterpret_cast<const int4*>(a->seq_table);
@@ -237,6 +303,18 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   }
   int vsplit = 4, variant = 3;
   pick_split(a, state_only, &vsplit, &variant);
+  if (after_k1) {
+    // Launched ahead of K1's end: K2's CTAs are set up (barriers, tensor memory, the initial state) on the SMs
+    // that K1 leaves.  Whole forward on B200, ordinary launch against this one: B1 T100 H32 17.0 -> 14.9 us, T512
+    // H32 35.6 -> 35.1, T1024 H8 41.3 -> 38.4, B8 T2048 H32 512 -> 507.  Not the 8-row form with four consumer
+    // warps per CTA on more than 32 chunks: in the order in which K1 leaves the SMs its CTAs step slower than
+    // in the order of an ordinary launch (T2048 H32 113.0 -> 115.2, T8192 H32 415 -> 420, H24 379 -> 386).
+    const long long steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : p.NT;
+    p.pdl = win_chunks > 0 || (variant != 5 && !(variant == 1 && vsplit == 4 && steps > 32));
+    const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
+    // without the bound on the CTAs per SM: T1024 H8 48.2 us
+    p.one_per_sm = p.pdl && win_chunks == 0 && chains * (variant == 4 ? 1 : vsplit) <= device_sms();
+  }
   if (p.pair_mode) {
     p.k_first = 0;   // the transforms are always written [chains][2][V][K]
     // Both transforms of a segment in one launch.  Few chains (two recurrences per chain still give
@@ -304,6 +382,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
       e = kda::launch_k2t(p, n_records, st);
       if (e == cudaSuccess) {
         ++g_launches;
+        p.pdl = p.one_per_sm = 0;   // behind the full waves, an ordinary launch
         p.chain0 = static_cast<int>(bh - tail);
         p.n_chains = static_cast<int>(tail);
         // the few-chain rule of pick_split applied to the tail alone
@@ -343,19 +422,19 @@ int kda_fwd(const KdaFwdArgs* a, void* stream) {
   if (int rc = check_k1(a)) return rc;
   if (int rc = check_k2(a, false)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
-  if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: status clear failed: %s", cudaGetErrorString(e));
-  if (int rc = do_k1(a, st)) return rc;
-  return do_k2(a, false, 0, st);
+  const int win = beside_window(a);
+  if (win > 0) {   // the window counters must be zero before either kernel starts
+    cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
+    if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));
+  }
+  if (int rc = do_k1(a, st, win)) return rc;
+  return do_k2(a, false, 0, st, nullptr, nullptr, true, win);
 }
 
 int kda_fwd_k1(const KdaFwdArgs* a, void* stream) {
   g_launches = 0;
   if (int rc = check_k1(a)) return rc;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
-  if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: status clear failed: %s", cudaGetErrorString(e));
-  return do_k1(a, st);
+  return do_k1(a, static_cast<cudaStream_t>(stream));
 }
 
 int kda_fwd_k2(const KdaFwdArgs* a, void* stream) {

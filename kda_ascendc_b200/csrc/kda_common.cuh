@@ -46,12 +46,17 @@ constexpr int REC_SHARED_BYTES = 17920;  // everything every V-slice needs
 constexpr int REC_U_TILE_BYTES = 512;    // one 8-column tile of u
 constexpr int REC_BYTES = 26112;
 constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the workspace
+// Header words: 0 = status, HDR_PROGRESS .. HDR_PROGRESS + MAX_WINDOWS - 1 = finished K1 items per window
+// of chunks, for a K2 that runs beside K1 (zeroed before K1 starts; unused otherwise)
+constexpr int HDR_PROGRESS = 4;
+constexpr int MAX_WINDOWS = WS_HEADER_BYTES / 4 - HDR_PROGRESS;
 
 // status codes written to workspace[0] by a kernel that gave up on a wait
 constexpr int ST_OK = 0;
 constexpr int ST_K1_LOAD_TIMEOUT = 1;
 constexpr int ST_K2_FULL_TIMEOUT = 2;
 constexpr int ST_K2_EMPTY_TIMEOUT = 3;
+constexpr int ST_K1_WINDOW_TIMEOUT = 8;   // K2 beside K1: a window of chunks was not finished in time
 constexpr int ST_PEER_TIMEOUT = 7;   // a flag from another GPU did not arrive in time (sequence-split exchange)
 
 constexpr float RCP_LN2 = 1.44269504089f;  // literal of tests/test_torch_reference.py:87
@@ -160,6 +165,37 @@ __device__ __forceinline__ bool flag_wait_bounded(const int* flag, int epoch) {
   }
 }
 
+// ---- K1 -> K2 hand-over on one GPU ------------------------------------------------
+// Programmatic dependent launch: K1 lets the next kernel of the stream start early, K2 waits for the
+// whole of K1 before it reads what K1 wrote.  Both are no-ops in an ordinary launch.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// fence between the generic and the async proxy for every state space (the plain form above covers
+// shared memory only): global memory written with plain stores and read by bulk copies, or the reverse
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void red_release_gpu(int* p, int v) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// A K2 that runs beside K1: waits until the K1 items of a window of chunks are all finished, then makes
+// their records readable by this thread's bulk copies.  Bounded; *abort_flag ends it early.
+__device__ __forceinline__ bool window_wait_bounded(const int* progress, int target, volatile int* abort_flag) {
+  const unsigned long long t0 = globaltimer_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 32; ++i) {
+      int v;
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(progress) : "memory");
+      if (v >= target) {
+        fence_proxy_async_all();
+        return true;
+      }
+      __nanosleep(64);
+    }
+    if (*abort_flag != 0 || globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
+  }
+}
+
 // ---- bulk (TMA, untiled) copies ---------------------------------------------
 // global -> shared, completion counted in bytes on an mbarrier.  Both addresses
 // 16-byte aligned, size a multiple of 16.
@@ -188,6 +224,7 @@ __device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src_smem, uint32_t 
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // ---- ldmatrix / mma ---------------------------------------------------------

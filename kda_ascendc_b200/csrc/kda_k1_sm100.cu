@@ -57,12 +57,16 @@ struct K1Smem {
 
 struct K1Item {   // one (batch, head, chunk) work item
   int b, h, hq, t0, nvalid;   // hq: the q/k head this (value) head reads
+  int win;                    // window the item counts towards (0 unless K2 runs beside K1)
   size_t rec_idx;
 };
 
 __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
-  // id -> (b, n, h) with h fastest: CTAs that run together read one contiguous span of tokens
+  // id -> (b, n, h) with h fastest: CTAs that run together read one contiguous span of tokens.
+  // With K2 beside K1 the order is (n, b, h): every chain's next chunk is finished before any chain's
+  // later one.
   K1Item w;
+  w.win = p.progress != nullptr ? static_cast<int>(p.div_win.div(id)) : 0;
   const int bn = static_cast<int>(p.div_h.div(id));
   w.h = id - bn * p.H;
   w.hq = static_cast<int>(p.div_g.div(w.h));
@@ -74,8 +78,14 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
     w.rec_idx = static_cast<size_t>(e.z) + static_cast<size_t>(w.h) * e.w;
     return w;
   }
-  w.b = static_cast<int>(p.div_nt.div(bn));
-  const int n = bn - w.b * p.NT;
+  int n;
+  if (p.progress != nullptr) {
+    n = static_cast<int>(p.div_b.div(bn));
+    w.b = bn - n * p.B;
+  } else {
+    w.b = static_cast<int>(p.div_nt.div(bn));
+    n = bn - w.b * p.NT;
+  }
   w.t0 = n * BT;
   w.nvalid = min(BT, p.T - w.t0);
   w.rec_idx = (static_cast<size_t>(w.b) * p.H + w.h) * p.NT + n;
@@ -103,6 +113,8 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   float* sGmid = reinterpret_cast<float*>(smem + SM::GMID);
   float* sTot1 = sTot + D;
   volatile int* sFlag = reinterpret_cast<volatile int*>(smem + SM::FLAG);
+  grid_dep_launch();   // K2 may be set up, or run, beside this kernel
+  if (p.progress == nullptr && blockIdx.x == 0 && tid == 0) *p.status = ST_OK;
 
   const bool use_gate = (p.flags & 1u) != 0;
   const bool use_l2 = (p.flags & 2u) != 0;
@@ -209,6 +221,21 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     publish_params(par, cur.nvalid, 0);
   }
 
+  // K2 beside K1: the items finished in the current window, and the window (and count) whose records
+  // have been handed to the copy engine but not yet reported
+  int done = 0, rep_win = 0, rep_done = 0;
+  // thread 0, once per item and two phases after the stores were issued: the tiles may be rewritten
+  // (their bulk stores have read them); with a window to report, the stores have also arrived
+  auto drain_stores = [&]() {
+    if (rep_done != 0) {
+      bulk_wait_all();
+      fence_proxy_async_all();
+      red_release_gpu(p.progress + rep_win, rep_done);
+    } else {
+      bulk_wait_read_all();
+    }
+  };
+
   for (int it = 0; id < n_items; ++it, id += gridDim.x) {
     const int b = cur.b, h = cur.h, t0 = cur.t0, nvalid = cur.nvalid;
     uint8_t* rec = p.rec + cur.rec_idx * REC_BYTES;
@@ -286,7 +313,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
         if (!FAST_EXP && rh == (mid >> 3)) *reinterpret_cast<float2*>(sGmid + c0) = gm;
         // the previous item's bulk stores must have read the qg / kg / Aqk / dec tiles before the
         // operand loop below rewrites them; by now they have had two phases to do so
-        if (tid == 0) bulk_wait_read_all();
+        if (tid == 0) drain_stores();
         __syncthreads();
         const float2 t0 = *reinterpret_cast<const float2*>(sTot + c0);
         const float2 t1 = *reinterpret_cast<const float2*>(sTot1 + c0);
@@ -306,7 +333,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
         for (int i = 0; i < 8; ++i) gv[i] = ld_g(min(r0 + i, nvalid - 1));
         gmid = ld_g(min(BT / 2, nvalid - 1));
         glast = ld_g(nvalid - 1);
-        if (tid == 0) bulk_wait_read_all();   // as above
+        if (tid == 0) drain_stores();   // as above
         __syncthreads();
       }
       dec2 = make_float2(ex2f(glast.x), ex2f(glast.y));
@@ -525,6 +552,15 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     // w leaves as one more bulk store (4-byte stores of a swizzled tile straight to global memory
     // would cost eight sectors per instruction)
     fence_proxy_async();
+    ++done;
+    rep_done = 0;
+    if (p.progress != nullptr && (!has_next || nxt.win != cur.win)) {
+      // the window's last item of this CTA: thread 0 reports it once its stores have arrived
+      rep_win = cur.win;
+      rep_done = done;
+      done = 0;
+      fence_proxy_async_all();   // u left by plain stores, K2 reads it with bulk copies
+    }
     __syncthreads();   // also orders phase E's reads of X / KB / VB before the next item rewrites them
     if (tid == 0) {
       bulk_s2g(rec + REC_W, sbase + S_WST, TILE_BYTES);
@@ -534,13 +570,13 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     par = par_next;
     pre_normalised = pre_next;
   }
-  if (tid == 0) bulk_wait_read_all();
+  if (tid == 0) drain_stores();
 }
 
 template <bool G_BF16, bool FAST_EXP>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
-  static int grid_cap[64] = {};
+  static int grid_cap[64] = {}, n_sms[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return cudaErrorInvalidDevice;
@@ -557,9 +593,12 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem_bytes);
     if (e != cudaSuccess) return e;
     grid_cap[dev] = sms * (per_sm > 0 ? per_sm : 1);   // persistent: one CTA per resident slot
+    n_sms[dev] = sms;
   }
   const long long n_items = (p.chunk_table != nullptr ? static_cast<long long>(p.n_chunks) : static_cast<long long>(p.B) * p.NT) * p.H;
-  const int grid = static_cast<int>(n_items < grid_cap[dev] ? n_items : grid_cap[dev]);
+  int cap = grid_cap[dev];
+  if (p.ctas_per_sm > 0 && p.ctas_per_sm * n_sms[dev] < cap) cap = p.ctas_per_sm * n_sms[dev];
+  const int grid = static_cast<int>(n_items < cap ? n_items : cap);
   kda_k1_kernel<G_BF16, FAST_EXP><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();
 }

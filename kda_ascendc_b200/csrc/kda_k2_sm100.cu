@@ -108,8 +108,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
   if (warp == CW) {
     // ------------------------------ producer -------------------------------
     if (lane == 0) {
+      if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
         const int s = n % K2_STAGES;
+        if (p.progress != nullptr && n == gate) {
+          if (!window_wait_bounded(p.progress + n / p.win_chunks, min(p.win_chunks, NT - n) * p.B * p.H, sAbort)) {
+            if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K1_WINDOW_TIMEOUT); }
+            break;
+          }
+          gate += p.win_chunks;
+        }
         if (n >= K2_STAGES) {
           if (!mbar_wait_bounded(empty0 + s * 8, ((n / K2_STAGES) - 1) & 1, sAbort)) {
             if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_EMPTY_TIMEOUT); }
@@ -399,6 +408,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     for (int n = max(0, issued - K2_STAGES); n < issued; ++n)
       mbar_wait_bounded(full0 + (n % K2_STAGES) * 8, (n / K2_STAGES) & 1, nullptr);
   }
+  if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
 }
 
 template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false>
@@ -410,13 +420,17 @@ static cudaError_t launch_k2_t(const K2Params& p, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem_bytes > ONE_CTA_SMEM ? smem_bytes : ONE_CTA_SMEM);
+    if (e != cudaSuccess) return e;
+    // the carve-out of K1, so that an SM can hold CTAs of both
+    e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (D / (CW * RT * 8));
-  kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR><<<nblocks, (CW + 1) * 32, smem_bytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dep(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
 }
 
 cudaError_t launch_k2n(const K2Params& p, int vsplit, int ntile, bool state_only, cudaStream_t stream) {

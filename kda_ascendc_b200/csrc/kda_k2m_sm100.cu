@@ -84,6 +84,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   if (warp == CW) {
     // ------------------------------ producer -------------------------------
     if (lane == 0) {
+      grid_dep_wait();   // K1's records; everything above ran under K1's tail
       for (int n = 0; n < NT; ++n) {
         const int s = n % K2M_STAGES;
         if (n >= K2M_STAGES) {
@@ -364,17 +365,15 @@ static cudaError_t launch_k2m_t(const K2Params& p, int nblocks, cudaStream_t str
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
     cudaError_t e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem_bytes);
+                                         smem_bytes > ONE_CTA_SMEM ? smem_bytes : ONE_CTA_SMEM);
     if (e != cudaSuccess) return e;
-    if (MINB > 1) {
-      e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                               cudaSharedmemCarveoutMaxShared);
-      if (e != cudaSuccess) return e;
-    }
+    // K1's carve-out: CTAs of this kernel move onto an SM while K1 still leaves it (and two of them fit)
+    e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  kda_k2m_kernel<CW, STATE_ONLY, MINB><<<nblocks, (CW + 1) * 32, smem_bytes, stream>>>(p);
-  return cudaGetLastError();
+  return launch_dep(kda_k2m_kernel<CW, STATE_ONLY, MINB>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
 }
 
 template <int CW, bool STATE_ONLY>

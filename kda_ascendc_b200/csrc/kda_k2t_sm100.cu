@@ -228,8 +228,17 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   if (warp == KT_EPI_WARPS) {
     // ------------------------------ producer -------------------------------
     if (lane == 0) {
+      if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
         const int s = n % KT_STAGES;
+        if (p.progress != nullptr && n == gate) {
+          if (!window_wait_bounded(p.progress + n / p.win_chunks, min(p.win_chunks, NT - n) * p.B * p.H, sAbort)) {
+            if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K1_WINDOW_TIMEOUT); }
+            break;
+          }
+          gate += p.win_chunks;
+        }
         if (n >= KT_STAGES && !mbar_wait_bounded(empty(s), ((n / KT_STAGES) - 1) & 1, sAbort)) { give_up(); break; }
         const int rec_i = static_cast<int>(rec_first) + n;
         const uint8_t* rec = p.rec + (rec_first + n) * REC_BYTES;
@@ -516,6 +525,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   __syncthreads();
   if (warp == KT_EPI_WARPS + 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(C_TOTAL) : "memory");
+  if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -554,15 +564,15 @@ cudaError_t launch_k2t(const K2Params& p, long long n_records, cudaStream_t stre
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kda_k2t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T_TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(kda_k2t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         T_TOTAL > ONE_CTA_SMEM ? T_TOTAL : ONE_CTA_SMEM);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(kda_k2t_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int nblocks = p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H;
-  kda_k2t_kernel<<<nblocks, KT_THREADS, T_TOTAL, stream>>>(pp);
-  return cudaGetLastError();
+  return launch_dep(kda_k2t_kernel, nblocks, KT_THREADS, k2_smem(p, T_TOTAL), stream, p.pdl, pp);
 }
 
 }  // namespace kda

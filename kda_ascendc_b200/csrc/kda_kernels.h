@@ -49,6 +49,11 @@ struct K1Params {
   // grouped value heads: q and k have Hq heads, head h of everything else reads q/k head h / (H/Hq)
   int Hq;
   FastDiv div_g;   // divides by H / Hq
+  // K2 beside K1 (null = K2 starts after K1): items run time-major, and the finished items of every
+  // window of chunks (all chains) are counted in progress[window]
+  int* progress;
+  int ctas_per_sm;         // cap on the resident K1 CTAs per SM (0 = as many as fit)
+  FastDiv div_b, div_win;  // divide by B and by the items of a window
 };
 
 constexpr int MAX_PEERS = 16;   // = KDA_MAX_PEERS of the public header
@@ -88,7 +93,34 @@ struct K2Params {
   // status code 7), while the producer warp already streams the first records in.
   const int* h0_flags;
   int h0_n_flags, h0_epoch;
+  // Launched with programmatic stream serialization behind K1 (pdl).  With progress the kernel runs
+  // beside K1: record n is read once progress[n / win_chunks] counts all items of that window.
+  int pdl;
+  const int* progress;
+  int win_chunks;
+  int one_per_sm;    // no SM may take two CTAs of the launch (there are enough SMs, but K1 leaves them one by one)
 };
+
+// Two CTAs with this much shared memory do not fit an SM.  A K2 launched ahead of K1's end is placed on
+// the SMs that K1 leaves first; without the bound several CTAs of a one-per-SM grid land on one of them.
+constexpr int ONE_CTA_SMEM = 116 * 1024;
+inline int k2_smem(const K2Params& p, int need) { return p.one_per_sm && need < ONE_CTA_SMEM ? ONE_CTA_SMEM : need; }
+
+// One launch, with or without the programmatic stream serialization attribute.
+template <typename Kernel, typename Params>
+cudaError_t launch_dep(Kernel kernel, int grid, int block, int smem_bytes, cudaStream_t stream, int pdl, const Params& p) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(grid));
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, p);
+}
 
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream);
 // Fills the four tensor maps of p from its pointers, sizes and strides (host, no device work).

@@ -1,0 +1,91 @@
+"""The forward whose K2 runs beside its K1 against the same two kernels one after the other: the same bits."""
+import ctypes
+
+import pytest
+import torch
+
+import kda_ascendc_b200 as K
+from kda_ascendc_b200 import _lib, api
+from oracle import kda_oracle as O
+from tests.conftest import to_device
+
+pytestmark = pytest.mark.gpu
+
+
+def _args(d, o, ht, ws, prepared=False):
+    return api.make_args(d["q"], d["k"], d["v"], d["g"], d["beta"], scale=d["scale"], lower_bound=d["lower_bound"],
+                         A_log=d["A_log"], dt_bias=d["dt_bias"], h0=d["initial_state"], o=o, ht=ht, workspace=ws,
+                         flags=0 if prepared else api._flags(True, True, True))
+
+
+def _buffers(B, T, H, dev):
+    return (torch.full((B, T, H, 128), float("nan"), dtype=torch.bfloat16, device=dev),
+            torch.full((B, H, 128, 128), float("nan"), dtype=torch.float32, device=dev),
+            torch.full((K.workspace_bytes(B, T, H),), 0xFF, dtype=torch.uint8, device=dev))
+
+
+def _after(d, B, T, H, dev, **kw):
+    o, ht, ws = _buffers(B, T, H, dev)
+    a, lib, st = _args(d, o, ht, ws, **kw), _lib.load(), api._stream_handle()
+    api._check(lib.kda_fwd_k1(ctypes.byref(a), st))
+    api._check(lib.kda_fwd_k2(ctypes.byref(a), st))
+    assert api.check_device_status(ws) == 0
+    return o, ht
+
+
+def _whole(d, B, T, H, dev, **kw):
+    o, ht, ws = _buffers(B, T, H, dev)
+    a = _args(d, o, ht, ws, **kw)
+    api._check(_lib.load().kda_fwd(ctypes.byref(a), api._stream_handle()))
+    assert api.check_device_status(ws) == 0
+    return o, ht
+
+
+# 8-row form (chains x 8 <= SMs) and tensor-memory form (up to three quarters of the SMs), on both sides of the
+# rule's line of 16 items per SM and of its line in chains; whole and partial last windows and chunks
+@pytest.mark.parametrize("B,T,H,lower_bound,prepared", [
+    (1, 4736, 8, -5.0, False), (1, 4720, 8, -5.0, False), (2, 2353, 8, -5.0, False), (1, 40001, 1, -5.0, False),
+    (3, 9000, 6, -5.0, False), (2, 2400, 8, -8.0, False), (2, 2400, 8, -5.0, True), (1, 16 * 121 + 5, 18, -5.0, False),
+    (1, 531, 75, -5.0, False), (1, 1024, 96, -5.0, False), (3, 1003, 37, -5.0, False), (1, 530, 112, -5.0, False),
+    (1, 20, 96, -5.0, False)])
+def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
+    d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.05), cuda_device)
+    d["lower_bound"] = lower_bound
+    if prepared:   # what a caller that normalises and sums the gate itself hands over
+        d["q"], d["k"] = (torch.nn.functional.normalize(d[n].float(), dim=-1).bfloat16() for n in ("q", "k"))
+        d["g"] = -d["g"].float().abs() * 0.1
+        d["beta"] = d["beta"].sigmoid()
+    ref = _after(d, B, T, H, cuda_device, prepared=prepared)
+    for _ in range(3):
+        got = _whole(d, B, T, H, cuda_device, prepared=prepared)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+def test_output_over_an_input(cuda_device):
+    """o over v: K2 may not write outputs before K1 has read the values."""
+    B, T, H = 2, 2400, 8
+    d = to_device(O.make_inputs(B, T, H, seed0=5, h0_std=0.05), cuda_device)
+    ref = _after(d, B, T, H, cuda_device)
+    _, ht, ws = _buffers(B, T, H, cuda_device)
+    a = _args(d, d["v"], ht, ws)
+    api._check(_lib.load().kda_fwd(ctypes.byref(a), api._stream_handle()))
+    assert torch.equal(d["v"], ref[0]) and torch.equal(ht, ref[1])
+
+
+@pytest.mark.parametrize("B,T,H", [(2, 2400, 8), (1, 600, 96), (1, 100, 32)])
+def test_captured_forward_follows_its_inputs(cuda_device, B, T, H):
+    """Both kernels in a CUDA graph, replayed back to back on changing inputs."""
+    d = to_device(O.make_inputs(B, T, H, seed0=9, h0_std=0.05), cuda_device)
+    plan = K.ForwardPlan(d["q"], d["k"], d["v"], d["g"], d["beta"], scale=d["scale"], initial_state=d["initial_state"],
+                         lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"])
+    plan.run()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.run()
+    for _ in range(3):
+        d["v"].mul_(-0.5)
+        graph.replay()
+        got = plan.o.clone(), plan.final_state.clone()
+        ref = _after(d, B, T, H, cuda_device)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
