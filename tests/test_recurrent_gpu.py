@@ -199,3 +199,40 @@ def test_long_calls_run_on_the_chunk_kernels_and_keep_the_in_place_contract():
     o_g, ht_g = O.run_recurrent_gold(inp)
     assert (o_ref.float().cpu() - o_g.float()).abs().max().item() <= 1e-3 * max(1.0, o_g.abs().max().item() / 0.06)
     assert (ht_ref.cpu() - ht_g.float()).abs().max().item() <= 2e-3 * max(1.0, ht_g.abs().max().item())
+
+
+# heads on both sides of the rule's lines (2, 4 and 8 rows per warp; the K-first kernels), tokens around the
+# groups of four that are prepared together, grouped q/k heads, both gate types
+@pytest.mark.parametrize("B,H", [(1, 3), (2, 20), (3, 26)])
+@pytest.mark.parametrize("T", [1, 2, 4, 5, 8, 9])
+@pytest.mark.parametrize("k_first,g_dtype,group", [(False, torch.bfloat16, 1), (False, torch.float32, 2), (True, torch.float32, 1),
+                                                   (True, torch.bfloat16, 2)])
+def test_token_groups_match_the_recurrence_in_64_bits(B, H, T, k_first, g_dtype, group):
+    import kda_ascendc_b200 as K
+    if H % group:
+        group = 1
+    inp = O.make_inputs(B, T, H, seed0=T, regime="carry", h0_std=0.3, g_dtype=g_dtype)
+    for n in ("q", "k"):   # value head h reads q/k head h // group
+        inp[n] = inp[n][:, :, ::group].repeat_interleave(group, dim=2).contiguous()
+    d = _dev(inp)
+    q, k = (d[n][:, :, ::group].contiguous() for n in ("q", "k"))
+    h0 = d["initial_state"].transpose(-1, -2).contiguous() if k_first else d["initial_state"].clone()   # updated in place
+    # the plan stays on the token kernels at any length (the function hands more than four tokens to the chunk kernels)
+    plan = K.RecurrentPlan(q, k, d["v"], d["g"], d["beta"], h0, state_v_first=not k_first, **_kw(d))
+    o, ht = plan.step(), plan.state
+    ht = ht.transpose(-1, -2) if k_first else ht
+    # the recurrence in 64 bits, with the kernels' rounding of the normalised q and k to bf16
+    x = {n: (v.double() if torch.is_tensor(v) else v) for n, v in d.items()}
+    x["q"], x["k"] = (torch.nn.functional.normalize(x[n], dim=-1, eps=0).bfloat16().double() for n in ("q", "k"))
+    gate = x["lower_bound"] * torch.sigmoid(x["A_log"].exp()[:, None] * (x["g"] + x["dt_bias"].view(H, 128)))
+    s, beta, outs = x["initial_state"], x["beta"].sigmoid(), []
+    for t in range(T):
+        s = s * gate[:, t].exp()[..., None, :]
+        pred = torch.einsum("bhvk,bhk->bhv", s, x["k"][:, t])
+        s = s + (beta[:, t, :, None] * (x["v"][:, t] - pred))[..., None] * x["k"][:, t][..., None, :]
+        outs.append(x["scale"] * torch.einsum("bhvk,bhk->bhv", s, x["q"][:, t]))
+    rel = lambda a, b: ((a.double() - b).norm() / b.norm()).item()
+    # state: fp32 sums (1e-6), and the few q, k whose rounding to bf16 falls the other way in 32 bits (about one in
+    # 3e4 by 2^-8: 2e-5); output: rounded to bf16, at most 2^-9 of each value
+    assert rel(ht, s) <= 1e-4
+    assert rel(o, torch.stack(outs, 1)) <= 2.0 ** -9 + 1e-4
