@@ -196,6 +196,24 @@ __device__ __forceinline__ bool window_wait_bounded(const int* progress, int tar
   }
 }
 
+// Chains of packed sequences in order of length, longest sequence first (ties by index): the chain
+// (sequence * H + head) at place `place`.  Called by every thread of the CTA.
+constexpr int MAX_SORTED_SEQS = 256;
+__device__ __forceinline__ int chain_by_length(const int4* seq_table, int n_seqs, int H, int place) {
+  __shared__ int lens[MAX_SORTED_SEQS + 1];
+  const int pos = place / H;
+  for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) lens[i] = __ldg(seq_table + i).y;
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) {
+    const int len = lens[i];
+    int rank = 0;
+    for (int j = 0; j < n_seqs; ++j) rank += (lens[j] > len || (lens[j] == len && j < i)) ? 1 : 0;
+    if (rank == pos) lens[MAX_SORTED_SEQS] = i;
+  }
+  __syncthreads();
+  return lens[MAX_SORTED_SEQS] * H + place % H;
+}
+
 // ---- bulk (TMA, untiled) copies ---------------------------------------------
 // global -> shared, completion counted in bytes on an mbarrier.  Both addresses
 // 16-byte aligned, size a multiple of 16.

@@ -38,7 +38,8 @@ struct K2mSmem {
 // MINB = CTAs that must fit on one SM.  With 2 (register cap 168) eight consumer warps share an
 // SM; that pays as soon as there are more CTAs than SMs (measured: B1 T8192 H96 765 -> 677 us),
 // while a grid that fits in one wave is faster with the uncapped registers.
-template <int CW, bool STATE_ONLY, int MINB>
+// ORD: packed sequences, longest first
+template <int CW, bool STATE_ONLY, int MINB, bool ORD = false>
 __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K2mSmem<CW>;
@@ -46,7 +47,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int warp = tid >> 5;
-  const int chain = blockIdx.x / NV + p.chain0;
+  const int chain = ORD ? chain_by_length(p.seq_table, p.n_seqs, p.H, blockIdx.x / NV + p.chain0) : blockIdx.x / NV + p.chain0;
   const bool pair = STATE_ONLY && p.pair_mode != 0;
   const int bh = pair ? (chain >> 1) : chain;      // the (batch, head) whose records are walked
   const int plane = pair ? (chain & 1) : 1;        // pair mode: 0 = transition matrix, 1 = offset
@@ -357,23 +358,23 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   }
 }
 
-template <int CW, bool STATE_ONLY, int MINB>
+template <int CW, bool STATE_ONLY, int MINB, bool ORD = false>
 static cudaError_t launch_k2m_t(const K2Params& p, int nblocks, cudaStream_t stream) {
   constexpr int smem_bytes = K2mSmem<CW>::TOTAL;
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes > ONE_CTA_SMEM ? smem_bytes : ONE_CTA_SMEM);
     if (e != cudaSuccess) return e;
     // K1's carve-out: CTAs of this kernel move onto an SM while K1 still leaves it (and two of them fit)
-    e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_dep(kda_k2m_kernel<CW, STATE_ONLY, MINB>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
+  return launch_dep(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
 }
 
 template <int CW, bool STATE_ONLY>
@@ -388,6 +389,8 @@ static cudaError_t launch_k2m_c(const K2Params& p, cudaStream_t stream) {
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (8 / CW);
   if (CW == 4 && nblocks > sms[dev]) return launch_k2m_t<CW, STATE_ONLY, 2>(p, nblocks, stream);
+  if constexpr (CW == 4 && !STATE_ONLY)   // the tail of a tensor-memory launch
+    if (p.by_length) return launch_k2m_t<4, false, 1, true>(p, nblocks, stream);
   return launch_k2m_t<CW, STATE_ONLY, 1>(p, nblocks, stream);
 }
 

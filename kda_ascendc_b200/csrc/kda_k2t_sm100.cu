@@ -175,7 +175,8 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   extern __shared__ __align__(1024) uint8_t smem[];
   const K2Params& p = pp.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int bh = blockIdx.x + p.chain0;
+  int bh = blockIdx.x + p.chain0;
+  if (p.by_length) bh = chain_by_length(p.seq_table, p.n_seqs, p.H, bh);
   int b = bh / p.H;
   const int h = bh % p.H;
   int NT = p.NT, Tlen = p.T, tok0 = 0;

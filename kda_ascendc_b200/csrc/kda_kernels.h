@@ -77,6 +77,7 @@ struct K2Params {
   // length); the grid then runs over (sequence, head); null for a fixed-length batch
   const int4* seq_table;
   int n_seqs;
+  int by_length;     // packed: chains are taken longest sequence first (n_seqs <= MAX_SORTED_SEQS)
   // a launch may cover a sub-range of the (batch, head) chains: first chain and count (0 = all)
   int chain0, n_chains;
   // Transform-pair pass of a sequence split over peer memory (the 8-row pair form only): the (M, Q) tiles

@@ -100,3 +100,23 @@ def test_tail_wave_with_packed_sequences():
     o_r, ht_r = O.run_chunk_reference_varlen(inp, cu)
     assert (o - o_r.float()).abs().max().item() <= 1e-3
     assert (ht - ht_r).abs().max().item() <= 2e-3
+
+
+# chains are taken longest sequence first, up to 256 sequences: ties, one-token sequences, and the line itself
+@pytest.mark.parametrize("lengths,H", [([65] * 10, 16), ([1, 300, 17, 300, 16, 64, 1, 299, 33, 128], 16), ([5, 700] * 11, 15),
+                                       ([70 + i % 9 for i in range(256)], 1), ([70 + i % 9 for i in range(257)], 1)])
+def test_longest_sequence_first(lengths, H):
+    T = sum(lengths)
+    inp = O.make_inputs(1, T, H, seed0=41, h0_std=None)
+    g = torch.Generator().manual_seed(8)
+    inp["initial_state"] = torch.randn(len(lengths), H, 128, 128, generator=g) * 0.05
+    cu = [0]
+    for L in lengths:
+        cu.append(cu[-1] + L)
+    o, ht = _run(inp, 0, cu=cu)
+    o4, ht4 = _run(inp, 4, cu=cu)
+    o3, ht3 = _run(inp, 3, cu=cu)
+    for a, b in ((o, o3), (o4, o3)):
+        assert (a - b).abs().max().item() <= 2.5e-4
+    for a, b in ((ht, ht3), (ht4, ht3)):
+        assert (a - b).abs().max().item() <= 2e-5
