@@ -61,12 +61,13 @@ struct K1Item {   // one (batch, head, chunk) work item
   size_t rec_idx;
 };
 
+template <bool BESIDE>
 __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
   // id -> (b, n, h) with h fastest: CTAs that run together read one contiguous span of tokens.
   // With K2 beside K1 the order is (n, b, h): every chain's next chunk is finished before any chain's
   // later one.
   K1Item w;
-  w.win = p.progress != nullptr ? static_cast<int>(p.div_win.div(id)) : 0;
+  w.win = BESIDE ? static_cast<int>(p.div_win.div(id)) : 0;
   const int bn = static_cast<int>(p.div_h.div(id));
   w.h = id - bn * p.H;
   w.hq = static_cast<int>(p.div_g.div(w.h));
@@ -79,7 +80,7 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
     return w;
   }
   int n;
-  if (p.progress != nullptr) {
+  if (BESIDE) {
     n = static_cast<int>(p.div_b.div(bn));
     w.b = bn - n * p.B;
   } else {
@@ -92,7 +93,8 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
   return w;
 }
 
-template <bool G_BF16, bool FAST_EXP>
+// BESIDE: K2 runs beside this kernel (time-major items, finished items counted per window)
+template <bool G_BF16, bool FAST_EXP, bool BESIDE>
 __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K1Smem<G_BF16, FAST_EXP>;
@@ -114,7 +116,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   float* sTot1 = sTot + D;
   volatile int* sFlag = reinterpret_cast<volatile int*>(smem + SM::FLAG);
   grid_dep_launch();   // K2 may be set up, or run, beside this kernel
-  if (p.progress == nullptr && blockIdx.x == 0 && tid == 0) *p.status = ST_OK;
+  if (!BESIDE && blockIdx.x == 0 && tid == 0) *p.status = ST_OK;
 
   const bool use_gate = (p.flags & 1u) != 0;
   const bool use_l2 = (p.flags & 2u) != 0;
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   K1Item cur{}, nxt{};
   Par par{}, par_next{};
   if (id < n_items) {
-    cur = k1_item(p, id);
+    cur = k1_item<BESIDE>(p, id);
     issue_loads(cur);
     par = load_params(cur);
     publish_params(par, cur.nvalid, 0);
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   // thread 0, once per item and two phases after the stores were issued: the tiles may be rewritten
   // (their bulk stores have read them); with a window to report, the stores have also arrived
   auto drain_stores = [&]() {
-    if (rep_done != 0) {
+    if (BESIDE && rep_done != 0) {
       bulk_wait_all();
       fence_proxy_async_all();
       red_release_gpu(p.progress + rep_win, rep_done);
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     uint8_t* rec = p.rec + cur.rec_idx * REC_BYTES;
     const bool has_next = id + static_cast<int>(gridDim.x) < n_items;
     if (has_next) {
-      nxt = k1_item(p, id + gridDim.x);
+      nxt = k1_item<BESIDE>(p, id + gridDim.x);
       par_next = load_params(nxt);
     }
     const float bias0 = par.bias0, bias1 = par.bias1;
@@ -554,7 +556,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     fence_proxy_async();
     ++done;
     rep_done = 0;
-    if (p.progress != nullptr && (!has_next || nxt.win != cur.win)) {
+    if (BESIDE && (!has_next || nxt.win != cur.win)) {
       // the window's last item of this CTA: thread 0 reports it once its stores have arrived
       rep_win = cur.win;
       rep_done = done;
@@ -573,7 +575,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   if (tid == 0) drain_stores();
 }
 
-template <bool G_BF16, bool FAST_EXP>
+template <bool G_BF16, bool FAST_EXP, bool BESIDE>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
   static int grid_cap[64] = {}, n_sms[64] = {};
@@ -581,7 +583,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   cudaGetDevice(&dev);
   if (dev >= 64) return cudaErrorInvalidDevice;
   if (grid_cap[dev] == 0) {
-    auto kern = kda_k1_kernel<G_BF16, FAST_EXP>;
+    auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;
     // ask for the full shared-memory carve-out so that four CTAs are resident per SM
@@ -599,7 +601,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   int cap = grid_cap[dev];
   if (p.ctas_per_sm > 0 && p.ctas_per_sm * n_sms[dev] < cap) cap = p.ctas_per_sm * n_sms[dev];
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
-  kda_k1_kernel<G_BF16, FAST_EXP><<<grid, 128, smem_bytes, stream>>>(p);
+  kda_k1_kernel<G_BF16, FAST_EXP, BESIDE><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();
 }
 
@@ -649,9 +651,14 @@ cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what) {
   return cudaSuccess;
 }
 
+template <bool BESIDE>
+static cudaError_t launch_k1_b(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream) {
+  if (g_bf16) return fast_exp ? launch_k1_t<true, true, BESIDE>(p, stream) : launch_k1_t<true, false, BESIDE>(p, stream);
+  return fast_exp ? launch_k1_t<false, true, BESIDE>(p, stream) : launch_k1_t<false, false, BESIDE>(p, stream);
+}
+
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream) {
-  if (g_bf16) return fast_exp ? launch_k1_t<true, true>(p, stream) : launch_k1_t<true, false>(p, stream);
-  return fast_exp ? launch_k1_t<false, true>(p, stream) : launch_k1_t<false, false>(p, stream);
+  return p.progress != nullptr ? launch_k1_b<true>(p, g_bf16, fast_exp, stream) : launch_k1_b<false>(p, g_bf16, fast_exp, stream);
 }
 
 }  // namespace kda
