@@ -168,9 +168,9 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // time order and counts the finished items of every window of chunks; K2's producer warps wait for
 // the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA is
 // already running.  Where it pays, measured on B200 as the whole forward, K2 after K1 against beside it:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T131072 H16 4,517 -> 4,268 us,
-//     B2 T4096 H8 153.3 -> 149.9, B1 T8192 H8 254.4 -> 250.5;
-//   tensor-memory form with one CTA per SM: T8192 H96 1,044 -> 970, T2048 H96 273 -> 255, T1024 H96 146 -> 135,
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T131072 H16 4,527 -> 4,321 us,
+//     B2 T4096 H8 154.3 -> 150.1, B1 T8192 H8 254.4 -> 250.5;
+//   tensor-memory form with one CTA per SM: T8192 H96 1,044 -> 976, T2048 H96 273 -> 255, T1024 H96 146 -> 135,
 //     but T4096 H128 602 -> 631 (no SM is left to K1 alone): up to three quarters of the SMs.
 // Not in the other forms: with four consumer warps per CTA K2 has no issue slots to spare, or (8-row form)
 // does not fit beside two K1 CTAs: T8192 H32 418 -> 515, T4096 H48 317 -> 379.
@@ -378,7 +378,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     const long long tail = bh % (2LL * sms);
     // Packed sequences of unequal length: the CTAs come in waves, so the longest chains go first (a long one
     // that starts in the last wave runs on alone while the rest of the chip is idle): 24 sequences of 16,411
-    // tokens, H32, whole forward 752 -> 640 us.  The order is worked out by every CTA, hence the bound on n_seqs.
+    // tokens, H32, whole forward 747 -> 616 us.  The order is worked out by every CTA, hence the bound on n_seqs.
     p.by_length = a->n_seqs > 1 && a->n_seqs <= kda::MAX_SORTED_SEQS && bh > sms;
     if (a->k2_variant == 0 && bh > 2LL * sms && tail > 0 && tail * 2 <= sms) {
       p.chain0 = 0;
