@@ -116,14 +116,22 @@ const at::Tensor* bias_tensor(PyObject* o, const Inputs& in, bool fla) {
   return side_tensor(o, in, {in.H * kD});
 }
 
-// The C calls run without the interpreter lock (a launch can wait for room in the stream's queue).
+// The C calls run without the interpreter lock (a launch can wait for room in the stream's queue).  The
+// destructor takes the lock back, also when `f` throws.
+class ReleasedLock {
+ public:
+  ReleasedLock() : state_(PyEval_SaveThread()) {}
+  ~ReleasedLock() { PyEval_RestoreThread(state_); }
+  ReleasedLock(const ReleasedLock&) = delete;
+  ReleasedLock& operator=(const ReleasedLock&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
 template <class F>
 int unlocked(F f) {
-  int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = f();
-  Py_END_ALLOW_THREADS
-  return rc;
+  const ReleasedLock released;
+  return f();
 }
 
 // cu_seqlens as 32-bit host values: a list or tuple of integers, or a 1-D integer tensor on any device (one
