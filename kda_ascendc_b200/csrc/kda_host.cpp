@@ -13,12 +13,14 @@
 
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <vector>
 
 #include <ATen/ATen.h>
 #include <ATen/core/grad_mode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/kda_b200.h"
@@ -173,6 +175,13 @@ PyObject* raise_for(int rc) {
   return nullptr;
 }
 
+// The C++ exception being handled, as the Python exception that PyTorch's own bindings raise for it (out of memory
+// keeps its type; an error raised in Python under an ATen call is that error).
+PyObject* raise_current() {
+  torch::translate_exception_to_python(std::current_exception());
+  return nullptr;
+}
+
 PyObject* result(at::Tensor o, PyObject* ht) {   // steals ht
   PyObject* out = PyTuple_New(2);
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(o)));
@@ -247,9 +256,8 @@ PyObject* chunk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   } catch (const Miss&) {
     PyErr_Clear();
     Py_RETURN_NONE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  } catch (...) {
+    return raise_current();
   }
 }
 
@@ -304,9 +312,8 @@ PyObject* recurrent(PyObject*, PyObject* const* a, Py_ssize_t n) {
   } catch (const Miss&) {
     PyErr_Clear();
     Py_RETURN_NONE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  } catch (...) {
+    return raise_current();
   }
 }
 
@@ -332,9 +339,8 @@ PyObject* run_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const bool rec = a[3] == Py_True;
     const int rc = unlocked([&] { return rec ? kda_recurrent_fwd(args, stream) : kda_fwd(args, stream); });
     if (rc != KDA_OK) return raise_for(rc);
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  } catch (...) {
+    return raise_current();
   }
   Py_RETURN_NONE;
 }

@@ -51,3 +51,17 @@ def test_an_exception_outside_the_interpreter_lock_reaches_the_caller():
             else:
                 raise SystemExit("no exception")
     """)
+
+
+@pytest.mark.parametrize("error", ["RuntimeError('an operation ran')", "torch.OutOfMemoryError('no room')", "KeyError(7)"])
+def test_exceptions_keep_their_type_and_message(error):
+    """What PyTorch raises under the native call arrives as it would from the Python path."""
+    run(f"""
+        OnCuda.error = {error}
+        try:
+            _lib.host().chunk(*chunk_args(cu_seqlens=OnCuda(3, dtype=torch.int32)))
+        except Exception as e:
+            assert type(e) is type(OnCuda.error) and str(e) == str(OnCuda.error), repr(e)
+        else:
+            raise SystemExit("no exception")
+    """)

@@ -47,3 +47,18 @@ def test_recurrent_call_takes_strided_views(cuda_device, T, inplace):
     st = d["initial_state"].clone()
     o, ht = K.kda_recurrent_fwd(*args, initial_state=st, inplace_state=inplace, **kw)
     assert torch.equal(o, want[0]) and torch.equal(ht, want[1]) and (ht is st) == inplace
+
+
+def test_out_of_memory_keeps_its_type(cuda_device):
+    d = to_device(O.make_inputs(1, 1, 32, seed0=5, h0_std=None), cuda_device)
+    args = tuple(d[n].expand(2048, *d[n].shape[1:]).contiguous() for n in ("q", "k", "v", "g", "beta"))
+    kw = dict(lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"])
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(0.02)     # 3.6 GB of 180; the returned state alone takes 4.3
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            K.kda_recurrent_fwd(*args, **kw)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    o, ht = K.kda_recurrent_fwd(*(a[:2] for a in args), **kw)
+    assert torch.equal(o[0], o[1]) and torch.equal(ht[0], ht[1]) and ht.abs().sum().item() > 0
