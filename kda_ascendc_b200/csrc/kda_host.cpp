@@ -44,7 +44,10 @@ bool truth(PyObject* o) {
 }
 double number(PyObject* o) {
   if (PyFloat_CheckExact(o)) return PyFloat_AS_DOUBLE(o);
-  if (PyLong_CheckExact(o)) return PyLong_AsDouble(o);
+  if (PyLong_CheckExact(o)) {
+    const double x = PyLong_AsDouble(o);
+    if (x != -1.0 || PyErr_Occurred() == nullptr) return x;   // else beyond a double: the handler of Miss clears the error
+  }
   throw Miss();
 }
 void need(bool ok) {

@@ -6,8 +6,6 @@ import sys
 import textwrap
 from pathlib import Path
 
-import pytest
-
 ROOT = Path(__file__).resolve().parents[1]
 
 PRELUDE = """
@@ -53,15 +51,22 @@ def test_an_exception_outside_the_interpreter_lock_reaches_the_caller():
     """)
 
 
-@pytest.mark.parametrize("error", ["RuntimeError('an operation ran')", "torch.OutOfMemoryError('no room')", "KeyError(7)"])
-def test_exceptions_keep_their_type_and_message(error):
+def test_exceptions_keep_their_type_and_message():
     """What PyTorch raises under the native call arrives as it would from the Python path."""
-    run(f"""
-        OnCuda.error = {error}
-        try:
-            _lib.host().chunk(*chunk_args(cu_seqlens=OnCuda(3, dtype=torch.int32)))
-        except Exception as e:
-            assert type(e) is type(OnCuda.error) and str(e) == str(OnCuda.error), repr(e)
-        else:
-            raise SystemExit("no exception")
+    run("""
+        for OnCuda.error in (RuntimeError("an operation ran"), torch.OutOfMemoryError("no room"), KeyError(7)):
+            try:
+                _lib.host().chunk(*chunk_args(cu_seqlens=OnCuda(3, dtype=torch.int32)))
+            except Exception as e:
+                assert type(e) is type(OnCuda.error) and str(e) == str(OnCuda.error), repr(e)
+            else:
+                raise SystemExit("no exception")
+    """)
+
+
+def test_a_number_that_does_not_fit_is_left_to_the_python_path():
+    """No launch with a value that is not the caller's, and no exception left pending."""
+    run("""
+        for bad in (dict(scale=10**400), dict(lower_bound=-10**400), dict(lower_bound=10**400)):
+            assert _lib.host().chunk(*chunk_args(**bad)) is None, bad
     """)
