@@ -177,7 +177,7 @@ kda_state_fold_kernel(const FoldParams p) {
 template <int ROWS>
 static cudaError_t launch_fold_t(const FoldParams& p, cudaStream_t stream) {
   constexpr int smem_bytes = FoldSmem<ROWS>::TOTAL;
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {

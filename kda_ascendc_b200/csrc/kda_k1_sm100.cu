@@ -578,28 +578,31 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
 template <bool G_BF16, bool FAST_EXP, bool BESIDE>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
-  static int grid_cap[64] = {}, n_sms[64] = {};
+  // per device: SMs << 8 | resident CTAs per SM, 0 = not looked up yet.  One word, published after the attributes
+  // are set: another thread's first call sees all of it or nothing.
+  static std::atomic<int> residency[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 64) return cudaErrorInvalidDevice;
-  if (grid_cap[dev] == 0) {
+  int res = residency[dev].load(std::memory_order_acquire);
+  if (res == 0) {
     auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;
     // ask for the full shared-memory carve-out so that four CTAs are resident per SM
     e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
-    int sms = 0, per_sm = 0;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int n_sms = 0, per_sm = 0;
+    e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem_bytes);
     if (e != cudaSuccess) return e;
-    grid_cap[dev] = sms * (per_sm > 0 ? per_sm : 1);   // persistent: one CTA per resident slot
-    n_sms[dev] = sms;
+    res = n_sms << 8 | (per_sm > 0 ? per_sm : 1);
+    residency[dev].store(res, std::memory_order_release);
   }
   const long long n_items = (p.chunk_table != nullptr ? static_cast<long long>(p.n_chunks) : static_cast<long long>(p.B) * p.NT) * p.H;
-  int cap = grid_cap[dev];
-  if (p.ctas_per_sm > 0 && p.ctas_per_sm * n_sms[dev] < cap) cap = p.ctas_per_sm * n_sms[dev];
+  const int sms = res >> 8, fit = res & 255;
+  const int cap = sms * (p.ctas_per_sm > 0 && p.ctas_per_sm < fit ? p.ctas_per_sm : fit);   // persistent: one CTA per slot
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
   kda_k1_kernel<G_BF16, FAST_EXP, BESIDE><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();

@@ -417,7 +417,7 @@ template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false>
 static cudaError_t launch_k2_t(const K2Params& p, cudaStream_t stream) {
   constexpr int RT = PAIR ? 1 : NVT;
   constexpr int smem_bytes = K2Smem<CW, RT>::TOTAL;
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {

@@ -462,7 +462,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
 template <int CW, bool STATE_ONLY>
 static cudaError_t launch_k2la_t(const K2Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K2LSmem<CW>::TOTAL;
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {

@@ -361,7 +361,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 template <int CW, bool STATE_ONLY, int MINB, bool ORD = false>
 static cudaError_t launch_k2m_t(const K2Params& p, int nblocks, cudaStream_t stream) {
   constexpr int smem_bytes = K2mSmem<CW>::TOTAL;
-  static bool configured[64] = {};
+  static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {

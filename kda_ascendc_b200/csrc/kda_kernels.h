@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace kda {
 
 // division by a runtime constant as multiply-high + shift (n < 2^31): q = n / d

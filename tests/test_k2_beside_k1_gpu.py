@@ -1,5 +1,8 @@
 """The forward whose K2 runs beside its K1 against the same two kernels one after the other: the same bits."""
 import ctypes
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -89,3 +92,39 @@ def test_captured_forward_follows_its_inputs(cuda_device, B, T, H):
         got = plan.o.clone(), plan.final_state.clone()
         ref = _after(d, B, T, H, cuda_device)
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+def test_first_use_from_several_threads():
+    """The first calls of a process, from eight threads at once on streams of their own: what a launch looks up once per
+    device must be complete when another thread sees it."""
+    body = """
+import threading, torch
+import kda_ascendc_b200 as K
+from oracle import kda_oracle as O
+from tests.conftest import to_device
+dev = torch.device("cuda:0")
+d = [to_device(O.make_inputs(B, T, H, seed0=7, h0_std=0.05), dev) for B, T, H in ((2, 2400, 8), (1, 600, 96)) * 4]
+plans = [K.ForwardPlan(x["q"], x["k"], x["v"], x["g"], x["beta"], scale=x["scale"], initial_state=x["initial_state"],
+                       lower_bound=x["lower_bound"], A_log=x["A_log"], dt_bias=x["dt_bias"]) for x in d]
+streams = [torch.cuda.Stream() for _ in plans]
+torch.cuda.synchronize()
+start, errors = threading.Barrier(len(plans)), []
+def work(i):
+    try:
+        start.wait()
+        plans[i].run(streams[i].cuda_stream)
+    except Exception as e:
+        errors.append(repr(e))
+threads = [threading.Thread(target=work, args=(i,)) for i in range(len(plans))]
+[t.start() for t in threads]
+[t.join() for t in threads]
+torch.cuda.synchronize()
+assert not errors, errors
+got = [(p.o.clone(), p.final_state.clone()) for p in plans]
+for p, (o, ht) in zip(plans, got):
+    p.run()
+    assert torch.equal(p.o, o) and torch.equal(p.final_state, ht)
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
