@@ -435,6 +435,18 @@ int kda_fwd(const KdaFwdArgs* a, void* stream) {
   return do_k2(a, false, 0, st, nullptr, nullptr, true, win);
 }
 
+int kda_selftest_window_wait(const KdaFwdArgs* a, void* stream) {
+  g_launches = 0;
+  if (int rc = check_k1(a)) return rc;
+  if (int rc = check_k2(a, false)) return rc;
+  const int win = beside_window(a);
+  if (win == 0) return fail(KDA_ERR_INVALID_ARG, "kda: K2 does not run beside K1 for this problem%s", "");
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(status_ptr(a) + kda::HDR_PROGRESS, 0, kda::MAX_WINDOWS * sizeof(int), st);
+  if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));
+  return do_k2(a, false, 0, st, nullptr, nullptr, false, win);
+}
+
 int kda_fwd_k1(const KdaFwdArgs* a, void* stream) {
   g_launches = 0;
   if (int rc = check_k1(a)) return rc;
@@ -790,6 +802,13 @@ int kda_fwd_status(const void* workspace, void* stream, int32_t* status_out) {
   cudaError_t e = cudaMemcpyAsync(&v, workspace, sizeof(v), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: status read failed: %s", cudaGetErrorString(e));
+  if (v != 0) {   // a K1 that gave up is the cause of what its K2 reported after it
+    int32_t k1 = 0;
+    e = cudaMemcpyAsync(&k1, static_cast<const int32_t*>(workspace) + kda::HDR_K1_STATUS, sizeof(k1), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: status read failed: %s", cudaGetErrorString(e));
+    if (k1 == kda::ST_K1_LOAD_TIMEOUT) v = k1;
+  }
   *status_out = v;
   if (v != 0) return fail(KDA_ERR_DEVICE_STATUS, "kda: a bounded device-side wait gave up%s (status %lld)", "", v);
   return KDA_OK;

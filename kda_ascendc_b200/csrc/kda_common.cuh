@@ -46,8 +46,11 @@ constexpr int REC_SHARED_BYTES = 17920;  // everything every V-slice needs
 constexpr int REC_U_TILE_BYTES = 512;    // one 8-column tile of u
 constexpr int REC_BYTES = 26112;
 constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the workspace
-// Header words: 0 = status, HDR_PROGRESS .. HDR_PROGRESS + MAX_WINDOWS - 1 = finished K1 items per window
-// of chunks, for a K2 that runs beside K1 (zeroed before K1 starts; unused otherwise)
+// Header words: 0 = status; HDR_K1_STATUS = K1's own code, which no later kernel overwrites (K2 waits for K1, so a K1
+// that gave up makes K2's waits run out after it; a first-one-wins exchange in K2 instead costs its 8-row form 0.7 %:
+// T8192 H32 411.7 -> 414.5 us); HDR_PROGRESS .. HDR_PROGRESS + MAX_WINDOWS - 1 = finished K1 items per window of
+// chunks, for a K2 that runs beside K1 (zeroed before K1 starts; unused otherwise)
+constexpr int HDR_K1_STATUS = 1;
 constexpr int HDR_PROGRESS = 4;
 constexpr int MAX_WINDOWS = WS_HEADER_BYTES / 4 - HDR_PROGRESS;
 

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
   float* sTot1 = sTot + D;
   volatile int* sFlag = reinterpret_cast<volatile int*>(smem + SM::FLAG);
   grid_dep_launch();   // K2 may be set up, or run, beside this kernel
-  if (!BESIDE && blockIdx.x == 0 && tid == 0) *p.status = ST_OK;
+  if (!BESIDE && blockIdx.x == 0 && tid == 0) *reinterpret_cast<int2*>(p.status) = make_int2(ST_OK, ST_OK);
 
   const bool use_gate = (p.flags & 1u) != 0;
   const bool use_l2 = (p.flags & 2u) != 0;
@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
       // a copy never completed: report, give in-flight copies one more bounded wait, leave
       if (tid == 0) {
         atomicExch(p.status, ST_K1_LOAD_TIMEOUT);
+        p.status[HDR_K1_STATUS] = ST_K1_LOAD_TIMEOUT;
         mbar_wait_bounded(mbar, it & 1, nullptr);
       }
       __syncthreads();

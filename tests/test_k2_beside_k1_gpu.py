@@ -94,6 +94,46 @@ def test_captured_forward_follows_its_inputs(cuda_device, B, T, H):
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
 
 
+# the 8-row form (full barrier: 2) and the tensor-memory form (any of its waits: 4)
+@pytest.mark.parametrize("B,T,H,own", [(1, 4736, 8, 2), (1, 600, 96, 4)])
+@pytest.mark.parametrize("k1_status", [0, 1])
+def test_window_wait_runs_out(cuda_device, B, T, H, own, k1_status):
+    """K2 on window counters that nothing counts up: it gives up after its limit, the outputs are left alone and the
+    next forward works.  After a K1 that gave up (its word of the header), that is what the status names."""
+    d = to_device(O.make_inputs(B, T, H, seed0=11, h0_std=0.05), cuda_device)
+    o, ht, ws = _buffers(B, T, H, cuda_device)
+    header = ws[:8].view(torch.int32)
+    header.copy_(torch.tensor([0, k1_status]))
+    a = _args(d, o, ht, ws)
+    api._check(_lib.load().kda_selftest_window_wait(ctypes.byref(a), api._stream_handle()))
+    torch.cuda.synchronize()
+    assert int(header[0]) in (8, own) and int(header[1]) == k1_status
+    assert o.isnan().all() and ht.isnan().all()
+    status = ctypes.c_int32(-1)
+    assert _lib.load().kda_fwd_status(api._ptr(ws), api._stream_handle(), ctypes.byref(status)) == -3
+    assert status.value == (k1_status or int(header[0]))
+    api._check(_lib.load().kda_fwd(ctypes.byref(a), api._stream_handle()))
+    assert api.check_device_status(ws) == 0
+    ref = _after(d, B, T, H, cuda_device)
+    assert torch.equal(o, ref[0]) and torch.equal(ht, ref[1])
+
+
+def test_k1_clears_both_status_words(cuda_device):
+    B, T, H = 1, 100, 3
+    d = to_device(O.make_inputs(B, T, H, seed0=11, h0_std=0.05), cuda_device)
+    o, ht, ws = _buffers(B, T, H, cuda_device)
+    a = _args(d, o, ht, ws)
+    api._check(_lib.load().kda_fwd_k1(ctypes.byref(a), api._stream_handle()))
+    assert ws[:8].view(torch.int32).tolist() == [0, 0]
+
+
+def test_window_wait_selftest_refuses_other_forwards(cuda_device):
+    d = to_device(O.make_inputs(1, 100, 32, seed0=11, h0_std=0.05), cuda_device)
+    a = _args(d, *_buffers(1, 100, 32, cuda_device))
+    assert _lib.load().kda_selftest_window_wait(ctypes.byref(a), api._stream_handle()) == -1
+    assert "beside" in _lib.last_error()
+
+
 def test_first_use_from_several_threads():
     """The first calls of a process, from eight threads at once on streams of their own: what a launch looks up once per
     device must be complete when another thread sees it."""
