@@ -1,12 +1,16 @@
 """The native host path (csrc/kda_host.cpp) launches what the Python path launches: bit-equal results for the
 options that change its argument block, and refusals that end in the Python path's own errors."""
+import subprocess
+import sys
+from pathlib import Path
+
 import numpy as np
 import pytest
 import torch
 
 import kda_ascendc_b200 as K
 from conftest import to_device
-from kda_ascendc_b200 import _lib, api
+from kda_ascendc_b200 import _lib, api, fla_backend
 from oracle import kda_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +66,73 @@ def test_out_of_memory_keeps_its_type(cuda_device):
         torch.cuda.set_per_process_memory_fraction(1.0)
     o, ht = K.kda_recurrent_fwd(*(a[:2] for a in args), **kw)
     assert torch.equal(o[0], o[1]) and torch.equal(ht[0], ht[1]) and ht.abs().sum().item() > 0
+
+
+def _chunk_kw(d):
+    return dict(initial_state=d["initial_state"], output_final_state=True, use_qk_l2norm_in_kernel=True,
+                use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True, lower_bound=d["lower_bound"], A_log=d["A_log"])
+
+
+def test_calls_follow_the_current_stream(cuda_device):
+    d = to_device(O.make_inputs(1, 100, 4, seed0=6, h0_std=0.1), cuda_device)
+    rest = (d["g"], d["beta"])
+    rec = dict(lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"], initial_state=d["initial_state"])
+    v2 = d["v"] * -0.5
+    want = K.kda_bt16_fwd(d["q"], d["k"], v2, *rest, dt_bias=d["dt_bias"], **_chunk_kw(d))
+    one = lambda v: tuple(x[:, :1] for x in (d["q"], d["k"], v, *rest))
+    want1 = K.kda_recurrent_fwd(*one(v2), **rec)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)            # about 10 ms: a launch on another stream would read v unchanged
+        d["v"].mul_(-0.5)
+        got = K.kda_bt16_fwd(d["q"], d["k"], d["v"], *rest, dt_bias=d["dt_bias"], **_chunk_kw(d))
+        got1 = K.kda_recurrent_fwd(*one(d["v"]), **rec)
+    side.synchronize()
+    for a, b in zip((*got, *got1), (*want, *want1)):
+        assert torch.equal(a, b)
+
+
+def test_adapter_takes_the_bias_per_head(cuda_device):
+    d = to_device(O.make_inputs(1, 50, 4, seed0=7, h0_std=0.1), cuda_device)
+    args, kw = (d["q"], d["k"], d["v"], d["g"], d["beta"]), _chunk_kw(d)
+    bias = d["dt_bias"].view(4, 128)
+    assert bias.abs().max().item() > 0
+    want = K.kda_bt16_fwd(*args, dt_bias=d["dt_bias"], scale=d["scale"], **kw)
+    got = fla_backend.chunk_kda(*args, dt_bias=bias, scale=d["scale"], safe_gate=True, transpose_state_layout=True, **kw)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    one = tuple(a[:, :1] for a in args)
+    want = K.kda_recurrent_fwd(*one, initial_state=d["initial_state"], lower_bound=d["lower_bound"], A_log=d["A_log"],
+                               dt_bias=d["dt_bias"], scale=d["scale"])
+    got = fla_backend.fused_recurrent_kda(*one, dt_bias=bias, scale=d["scale"], transpose_state_layout=True, **kw)
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+def test_offsets_on_the_gpu_under_capture_are_an_ordinary_error():
+    """Reading them back is not allowed while the stream is captured; the process goes on."""
+    body = """
+import torch
+import kda_ascendc_b200 as K
+from oracle import kda_oracle as O
+from tests.conftest import to_device
+d = to_device(O.make_inputs(1, 40, 2, seed0=8, h0_std=None), torch.device("cuda:0"))
+cu = torch.tensor([0, 17, 40], dtype=torch.int32, device="cuda:0")
+call = lambda: K.kda_bt16_fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], cu_seqlens=cu, output_final_state=True,
+                              use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True,
+                              lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"])
+want = call()
+torch.cuda.synchronize()
+try:
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        call()
+except RuntimeError as e:
+    assert "captur" in str(e), e
+else:
+    raise SystemExit("no error")
+got = call()
+torch.cuda.synchronize()
+assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+"""
+    r = subprocess.run([sys.executable, "-c", body], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-3000:]
