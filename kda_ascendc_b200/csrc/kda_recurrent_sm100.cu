@@ -340,10 +340,13 @@ __global__ void __launch_bounds__(128, 7) kda_recurrent_kfirst_kernel(const Recu
 
 // One token: every warp prepares it for itself, so that nothing stands between the state's loads and the first
 // product; two reductions through shared memory (one for both takes more registers: B64 H32 51.0 us against
-// 46.6).  The state's traffic bounds it: B64 H32 49.2 -> 45.3 us, B8 10.7 -> 8.2 with the evict-first hint and
-// seven CTAs per SM.
+// 46.6).  The state's traffic bounds it, and the CTAs per SM that cover its latency.  Every bound on the registers below 96
+// (five CTAs) spills a few of a thread's own inputs: seven CTAs (72 registers) 68 bytes with a bf16 gate, 84 with an fp32
+// gate, six (80 registers) 56 and 64.  Steps in a graph, H32, states beyond L2, B8 / B64 / B256, no hint and no bound first:
+//   bf16 gate 10.9 / 49.8 / 179 us; now 8.4 / 45.8 / 169 with seven, 9.3 / 48.3 / 193 with six, 9.1 / 46.0 / 173 with five;
+//   fp32 gate 10.9 / 50.5 / 181 us; now 8.9 / 49.2 / 191 with seven, 8.8 / 45.9 / 172-178 with six, 9.1 / 46.0 / 174 with five.
 template <bool G_BF16>
-__global__ void __launch_bounds__(128, 7) kda_recurrent_kfirst_one_kernel(const RecurrentParams p) {
+__global__ void __launch_bounds__(128, G_BF16 ? 7 : 6) kda_recurrent_kfirst_one_kernel(const RecurrentParams p) {
   __shared__ float4 red[2][4][8];   // [prediction | output][warp][v quad]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int vq = tid & 7, kg = tid >> 3;
