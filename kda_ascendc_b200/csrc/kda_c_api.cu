@@ -378,8 +378,12 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     const long long tail = bh % (2LL * sms);
     // Packed sequences of unequal length: the CTAs come in waves, so the longest chains go first (a long one
     // that starts in the last wave runs on alone while the rest of the chip is idle): 24 sequences of 16,411
-    // tokens, H32, whole forward 747 -> 616 us.  The order is worked out by every CTA, hence the bound on n_seqs.
-    p.by_length = a->n_seqs > 1 && a->n_seqs <= kda::MAX_SORTED_SEQS && bh > sms;
+    // tokens, H32, whole forward 747 -> 616 us.  Every CTA works its chain out, which costs about 0.4 us per wave: up to
+    // 2 % where the chains are of equal length and four chunks short.  Hence the bound on n_seqs (eight lengths per
+    // lane), and none of it where many waves of short chains leave little at the end (256 sequences of about 4
+    // chunks, H16: 420 us in their own order, 435 by length; of 8 to 13 chunks 701 and 709, of 29 1,240 and 1,040).
+    const long long mean_steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : 0;
+    p.by_length = a->n_seqs > 1 && a->n_seqs <= kda::MAX_SORTED_SEQS && bh > sms && bh <= 4LL * sms * mean_steps;
     if (a->k2_variant == 0 && bh > 2LL * sms && tail > 0 && tail * 2 <= sms) {
       p.chain0 = 0;
       p.n_chains = static_cast<int>(bh - tail);

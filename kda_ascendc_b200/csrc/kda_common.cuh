@@ -200,21 +200,41 @@ __device__ __forceinline__ bool window_wait_bounded(const int* progress, int tar
 }
 
 // Chains of packed sequences in order of length, longest sequence first (ties by index): the chain
-// (sequence * H + head) at place `place`.  Called by every thread of the CTA.
+// (sequence * H + head) at place `place`.  Called by every thread of the CTA; one warp works it out, bit by bit: the
+// length at a place is the largest that more than `place` sequences reach.
 constexpr int MAX_SORTED_SEQS = 256;
 __device__ __forceinline__ int chain_by_length(const int4* seq_table, int n_seqs, int H, int place) {
-  __shared__ int lens[MAX_SORTED_SEQS + 1];
-  const int pos = place / H;
-  for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) lens[i] = __ldg(seq_table + i).y;
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_seqs; i += blockDim.x) {
-    const int len = lens[i];
-    int rank = 0;
-    for (int j = 0; j < n_seqs; ++j) rank += (lens[j] > len || (lens[j] == len && j < i)) ? 1 : 0;
-    if (rank == pos) lens[MAX_SORTED_SEQS] = i;
+  __shared__ int chosen;
+  if (threadIdx.x < 32) {
+    constexpr int PER_LANE = MAX_SORTED_SEQS / 32;
+    const int lane = threadIdx.x, pos = place / H;
+    int len[PER_LANE], longest = 0;
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      len[j] = j * 32 + lane < n_seqs ? __ldg(&seq_table[j * 32 + lane].y) : 0;   // every sequence has a chunk
+      longest = max(longest, len[j]);
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    int at = 0, above = 0;
+    for (int bit = 31 - __clz(longest); bit >= 0; --bit) {
+      const int t = at | (1 << bit);
+      int n = 0;
+#pragma unroll
+      for (int j = 0; j < PER_LANE; ++j) n += len[j] >= t ? 1 : 0;
+      if (__reduce_add_sync(0xffffffffu, n) > pos) at = t;
+    }
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) above += len[j] > at ? 1 : 0;
+    int k = pos - __reduce_add_sync(0xffffffffu, above);   // place among the sequences of this length
+#pragma unroll
+    for (int j = 0; j < PER_LANE; ++j) {
+      const unsigned same = __ballot_sync(0xffffffffu, len[j] == at);
+      if (len[j] == at && __popc(same & ((1u << lane) - 1)) == k) chosen = j * 32 + lane;
+      k -= __popc(same);
+    }
   }
   __syncthreads();
-  return lens[MAX_SORTED_SEQS] * H + place % H;
+  return chosen * H + place % H;
 }
 
 // ---- bulk (TMA, untiled) copies ---------------------------------------------

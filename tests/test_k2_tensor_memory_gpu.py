@@ -120,3 +120,20 @@ def test_longest_sequence_first(lengths, H):
         assert (a - b).abs().max().item() <= 2.5e-4
     for a, b in ((ht, ht3), (ht4, ht3)):
         assert (a - b).abs().max().item() <= 2e-5
+
+
+# the chain at a place is picked bit by bit: lengths of one to seven bits with many ties, eight lengths per lane; and
+# both sides of the line in chains (4 x SMs x mean chunks), above which the chains keep their own order
+@pytest.mark.parametrize("n,lo,hi,H", [(2, 1, 600, 150), (33, 1, 1500, 9), (255, 1, 64, 2), (256, 20, 40, 4), (256, 20, 40, 5)])
+def test_any_lengths_longest_first(n, lo, hi, H):
+    g = torch.Generator().manual_seed(n + H)
+    lengths = torch.randint(lo, hi + 1, (n,), generator=g).tolist()
+    inp = O.make_inputs(1, sum(lengths), H, seed0=43, h0_std=None)
+    inp["initial_state"] = torch.randn(n, H, 128, 128, generator=g) * 0.05
+    cu = [0]
+    for L in lengths:
+        cu.append(cu[-1] + L)
+    o, ht = _run(inp, 4, cu=cu)
+    o3, ht3 = _run(inp, 3, cu=cu)
+    assert (o - o3).abs().max().item() <= 2.5e-4       # one bf16 step of |o| <= 0.06, as above
+    assert (ht - ht3).abs().max().item() <= 2e-5
