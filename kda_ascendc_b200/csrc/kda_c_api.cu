@@ -310,8 +310,13 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     // warps per CTA on more than 32 chunks: in the order in which K1 leaves the SMs its CTAs step slower than
     // in the order of an ordinary launch (T2048 H32 113.0 -> 115.2, T8192 H32 415 -> 420, H24 379 -> 386).
     const long long steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : p.NT;
-    p.pdl = win_chunks > 0 || (variant != 5 && !(variant == 1 && vsplit == 4 && steps > 32));
+    // Nor packed sequences of more than eight chunks in the mean in the 16-row form on more CTAs than SMs: the long
+    // chains of unequal lengths then run on beside others of the launch.  3 to 64 sequences of log-normal lengths
+    // (sigma 1), 75 to 148 chains, whole forward: up to three chunks in the mean 0.92 of the ordinary launch's time, four to
+    // eight 0.97, nine to 16 1.03, more 1.04 and up to 1.31 (16 sequences, H8, the longest 264 chunks of 460: 285 -> 372 us).
     const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
+    const bool uneven = a->n_seqs > 0 && variant == 3 && chains * vsplit > device_sms() && steps > 8;
+    p.pdl = win_chunks > 0 || (variant != 5 && !(variant == 1 && vsplit == 4 && steps > 32) && !uneven);
     // without the bound on the CTAs per SM: T1024 H8 48.2 us
     p.one_per_sm = p.pdl && win_chunks == 0 && chains * (variant == 4 ? 1 : vsplit) <= device_sms();
   }

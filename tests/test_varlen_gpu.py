@@ -53,6 +53,26 @@ def test_varlen_matches_oracle_and_fixed_length_calls(lengths, H, h0_std):
         assert (ht[i:i + 1] - ht_i).abs().max().item() <= 2e-5, i
 
 
+# 80 chains on 160 CTAs of the 16-row form, eight and ten chunks per sequence in the mean: both sides of the line beyond
+# which K2 is not launched ahead of K1's end
+@pytest.mark.parametrize("longest", [400, 700])
+def test_varlen_launch_forms(longest):
+    import kda_ascendc_b200 as K
+    lengths, H = [64] + [100] * 4 + [longest] + [100] * 4, 8
+    n_chunks = sum((n + 15) // 16 for n in lengths)
+    assert K.api.k2_choice(1, sum(lengths), H, n_seqs=10, n_chunks=n_chunks) == ("m16", 2)
+    assert (n_chunks // 10 > 8) == (longest == 700)
+    inp, d, cu, kw = _setup(lengths, H, 31, 0.05)
+    call = lambda a, b, h0, **extra: K.kda_bt16_fwd(*(d[n][:, a:b].contiguous() for n in ("q", "k", "v", "g", "beta")),
+                                                    initial_state=h0, **FLAGS, **kw, **extra)
+    for _ in range(2):
+        o, ht = call(0, cu[-1], d["initial_state"], cu_seqlens=cu)
+    for i in range(len(lengths)):
+        o_i, ht_i = call(cu[i], cu[i + 1], d["initial_state"][i:i + 1])
+        assert (o[:, cu[i]:cu[i + 1]].float() - o_i.float()).abs().max().item() <= 2.5e-4, i   # as above
+        assert (ht[i:i + 1] - ht_i).abs().max().item() <= 2e-5, i
+
+
 def test_varlen_single_sequence_equals_fixed_length():
     import kda_ascendc_b200 as K
     inp, d, cu, kw = _setup([333], 4, 4, 0.1)
