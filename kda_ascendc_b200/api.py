@@ -365,7 +365,7 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_f
     # 279 us against 107 us); each K2 CTA reads its rows of the state before it writes them, so the in-place
     # update carries over.
     chunked = T > RECURRENT_MAX_TOKENS
-    ws = _get_workspace(dev, B, T, H, True) if chunked else None
+    ws = _get_workspace(dev, B, T, H, False) if chunked else None   # calls on several streams share no scratch
     args = make_args(q, k, v, g, beta, scale=scale, lower_bound=lower_bound, A_log=A_log, dt_bias=dt_bias,
                      h0=initial_state, o=o, ht=ht, workspace=ws,
                      flags=_flags(True, True, True) | (0 if state_v_first else _lib.FLAG_STATE_K_FIRST))

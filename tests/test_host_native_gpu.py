@@ -136,3 +136,16 @@ assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     r = subprocess.run([sys.executable, "-c", body], cwd=Path(__file__).resolve().parents[1], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stderr[-3000:]
+
+
+def test_long_recurrent_call_shares_no_scratch(cuda_device):
+    """A call that takes the Python path and the chunk kernels: calls of one shape on two streams may overlap."""
+    T = api.RECURRENT_MAX_TOKENS + 1
+    d = to_device(O.make_inputs(1, T, 3, seed0=9, h0_std=0.1), cuda_device)
+    args = tuple(d[n] for n in ("q", "k", "v", "g", "beta"))
+    kw = dict(lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"], initial_state=d["initial_state"])
+    kept = dict(api._WORKSPACE_CACHE)
+    o, ht = K.kda_recurrent_fwd(*args, scale=np.float64(d["scale"]), **kw)
+    assert api._WORKSPACE_CACHE.keys() == kept.keys()
+    want = K.kda_recurrent_fwd(*args, scale=d["scale"], **kw)
+    assert torch.equal(o, want[0]) and torch.equal(ht, want[1])
