@@ -329,7 +329,7 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_f
 
     Same tensors as :func:`kda_bt16_fwd` with the in-kernel gate, l2-norm and beta sigmoid
     (``g`` raw, ``beta`` logits, ``A_log`` required), any ``T >= 1`` (calls of more than
-    ``RECURRENT_MAX_TOKENS`` tokens run on the chunk kernels, which are faster from there on), fp32
+    ``RECURRENT_MAX_TOKENS`` tokens run on the chunk kernels), fp32
     state ``[B, H, V, K]`` or, with ``state_v_first=False``, ``[B, H, K, V]`` (read and written in
     that layout by the kernels, no transpose).  Returns ``(o, state)``; with
     ``inplace_state=True`` the new state overwrites ``initial_state`` (which is returned).
@@ -360,10 +360,14 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_f
         ht = initial_state
     else:
         ht = torch.empty((B, H, HEAD_DIM, HEAD_DIM), dtype=torch.float32, device=dev) if output_final_state else None
-    # Beyond RECURRENT_MAX_TOKENS tokens per call the chunk kernels are faster (measured on B200, B64 H32:
-    # 4 tokens 88 us token by token against 104 us as one chunk, 8 tokens 151 us against 105 us, 16 tokens
-    # 279 us against 107 us); each K2 CTA reads its rows of the state before it writes them, so the in-place
-    # update carries over.
+    # Beyond RECURRENT_MAX_TOKENS tokens a call runs on the chunk kernels, whose time hardly depends on T up to a chunk;
+    # each K2 CTA reads its rows of the state before it writes them, so the in-place update carries over.  Measured on
+    # B200 (H32, V-first; K-first within 10 % from B4 on), token by token / as one chunk, us:
+    #   B1  T4 4.9 / 7.3, T5 6.2 / 7.4, T6 6.5 / 7.4, T8 7.2 / 7.3, T12 9.5 / 7.4
+    #   B16 T4 20.4 / 29.8, T5 25.3 / 30.1, T6 27.5 / 30.2, T8 31.7 / 30.2, T12 43.7 / 30.7
+    #   B64 T4 64.0 / 103, T5 81.4 / 103, T6 89.7 / 104, T8 107 / 104, T12 150 / 105
+    # The line was drawn for an earlier token kernel; with this one calls of five and six tokens would be faster
+    # token by token as well (K-first B1 T6: 8.0 / 7.8).
     chunked = T > RECURRENT_MAX_TOKENS
     ws = _get_workspace(dev, B, T, H, False) if chunked else None   # calls on several streams share no scratch
     args = make_args(q, k, v, g, beta, scale=scale, lower_bound=lower_bound, A_log=A_log, dt_bias=dt_bias,

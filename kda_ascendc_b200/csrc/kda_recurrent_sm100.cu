@@ -8,14 +8,17 @@
 //   v'  =  beta * (v - h khat)
 //   h   <- h + v' (x) khat
 //   o   =  scale * h qhat
+// The output is taken from the decayed state before the update, o = scale * (h qhat + v' (khat . qhat)), so that both
+// products of a token with the state go through one reduction.
 // Every state row v is independent, so a warp owns ROWS rows of one (batch, head) state and keeps
 // them in registers over all T tokens: lane l holds columns 4l..4l+3 of each row (one 16-byte
-// load per row), the two dot products per row and token are warp reductions.  The kernel moves
+// load per row), and the 2 x ROWS dot products of a token are reduced over the warp together.  The kernel moves
 // 64 KiB of state in and out per (batch, head) and a few hundred bytes per token: HBM bound; the
 // grid is (batch x head) x (128 / rows per CTA) CTAs.  A K-first state h[K][V] (the layout
 // flash-linear-attention keeps) is read and written in place: for one column k the warp's ROWS
 // rows are ROWS consecutive floats, so the lane moves them as 16- or 8-byte pieces (full 32-byte
-// sectors at 8 rows per warp) into the same registers.
+// sectors at 8 rows per warp) into the same registers; with enough heads two kernels with the lanes along v take
+// over (below).
 #include "kda_common.cuh"
 #include "kda_kernels.h"
 

@@ -18,8 +18,9 @@
 //   * All calls on a device share the one array.  Two calls whose kernels can overlap on the
 //     GPU (different streams without an ordering between them) corrupt each other; calls on
 //     one stream, or otherwise ordered, are fine.  What a call left behind stays in the array:
-//     the status block at its start is cleared by every call, and the chunk records are always
-//     written by K1 before K2 reads them, so stale contents are never consumed.
+//     every call clears the status words of the header at its start (and the counters of the header
+//     if it uses them), and the chunk records are always written by K1 before K2 reads them, so
+//     stale contents are never consumed.
 //   * A bounded device-side wait that gave up leaves its code in the status word at the start of
 //     the array; since the array's address never leaves the library, kda_fwd_static_scratch_status
 //     reads that word for the current device (kda_fwd_status needs a caller-owned workspace).
@@ -116,7 +117,7 @@ extern "C" int kda_fwd_static_scratch(const KdaFwdArgs* args, void* stream) {
   if (scratch == nullptr) return rc;
   KdaFwdArgs local = *args;          // the caller's block is left untouched
   local.workspace = scratch;         // whatever the caller put there is ignored
-  return kda_fwd(&local, stream);    // clears the status block, then K1 and K2
+  return kda_fwd(&local, stream);    // K1 (clears the status words) and K2
 }
 
 extern "C" int kda_fwd_static_scratch_status(void* stream, int32_t* status_out) {
