@@ -240,11 +240,11 @@ bool output_over_v(const KdaFwdArgs* a) {
 //   few chains, cut into segments: T131072 H16 4,316 -> 2,831, T4096 H16 150 -> 140, T8192 H32 412 -> 393.
 // Not where the 16-token K2 has enough chains to fill the chip (B8 T2048 H32 498 -> 524: K1 is the longer part) and
 // not where sequences are short (T2048 H32 112 -> 131, B2 T1024 H4 39 -> 52).
-// Gate sums made by the caller take the same lines (their K1 checks the range, 294 -> 333 us at B8 T2037 H32); a lower
-// bound below -5.03 does not (its Grams need 16-token blocks: K1 571 us there).
+// Not a lower bound below -5.03 (its Grams need 16-token blocks: K1 571 us at B8 T2037 H32 against 294), and not yet gate
+// sums made by the caller or packed sequences, which the kernels take but which have not been compared on the GPU.
 bool wide_records(const KdaFwdArgs* a) {
   if (a->k2_variant != 0 || a->k2_vsplit != 0 || a->g_out != nullptr || a->ainv_out != nullptr || a->v == nullptr) return false;
-  if ((a->flags & KDA_FLAG_GATE_IN_KERNEL) && !(16.0f * -a->lower_bound * kda::RCP_LN2 <= 116.0f)) return false;
+  if (a->n_seqs > 0 || !(a->flags & KDA_FLAG_GATE_IN_KERNEL) || !(16.0f * -a->lower_bound * kda::RCP_LN2 <= 116.0f)) return false;
   const int sms = device_sms();
   const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
   // wide chunks of a chain (the mean, for packed sequences: at least 1,024 tokens, which also keeps their records, one
