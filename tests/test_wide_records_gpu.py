@@ -72,54 +72,6 @@ def test_wide_forward_carries_the_state(cuda_device, B, T, H, regime):
     assert (ht[:, heads].cpu() - ht_r).abs().max().item() <= 2e-2 * ht_r.abs().max().item()
 
 
-def _prepared(inp, spread):
-    """What a caller that normalises, activates and sums the gate over every 16 tokens itself hands over."""
-    p = dict(inp)
-    p["q"], p["k"] = (torch.nn.functional.normalize(inp[n].float(), dim=-1).bfloat16() for n in ("q", "k"))
-    p["beta"] = inp["beta"].sigmoid()
-    B, T, H, D = inp["g"].shape
-    gate = -(inp["g"].float().abs().clamp(max=3.0) / 3.0) * spread
-    gate = torch.nn.functional.pad(gate, (0, 0, 0, 0, 0, -T % 16)).view(B, -1, 16, H, D).cumsum(2)
-    p["g"] = gate.view(B, -1, H, D)[:, :T].contiguous()
-    return p
-
-
-# within the range of 32-token blocks, beyond it (the second K1 launch redoes all records), and one column beyond it
-@pytest.mark.parametrize("spread,one", [(7.0, False), (15.0, False), (2.0, True)])
-def test_gate_sums_made_by_the_caller(cuda_device, spread, one):
-    inp = O.make_inputs(2, 2037, 64, seed0=11, h0_std=0.05)
-    p = _prepared(inp, spread)
-    if one:   # 16 tokens of one column at 9 each
-        p["g"][1, 1024:1040, 5, 77] = -9.0 * torch.arange(1, 17)
-    d = to_device(p, cuda_device)
-    o, ht = _forward(d, flags=(False, False, False))
-    o3, ht3 = _forward(d, variant=3, flags=(False, False, False))
-    assert o.isfinite().all() and ht.isfinite().all()
-    assert (o.float() - o3.float()).abs().max().item() <= 7.5e-4
-    assert (ht - ht3).abs().max().item() <= 2e-4
-
-
-def test_packed_sequences_do_not_see_each_other(cuda_device):
-    """Ragged sequences in one batch against each on its own; the first tokens of the next sequence, which a chunk of 64
-    reads past a sequence's end, hold infinities and NaN."""
-    lengths, H = [2000, 65, 1640, 4050, 129, 1, 700], 16
-    inp = O.make_inputs(1, sum(lengths), H, seed0=29, h0_std=None)
-    inp["initial_state"] = torch.randn(len(lengths), H, 128, 128, generator=torch.Generator().manual_seed(5)) * 0.05
-    cu = [0]
-    for n in lengths:
-        cu.append(cu[-1] + n)
-    o, ht = _forward(to_device(inp, cuda_device), cu=cu)
-    o_r, ht_r = O.run_chunk_reference_varlen(_heads(inp, [3, 15]), cu)
-    assert (o[:, :, [3, 15]].float().cpu() - o_r.float()).abs().max().item() <= 1e-3
-    assert (ht[:, [3, 15]].cpu() - ht_r).abs().max().item() <= 2e-3
-    bad = {k: (v.clone() if torch.is_tensor(v) else v) for k, v in inp.items()}
-    for n, x in (("q", float("inf")), ("k", float("nan")), ("v", float("nan")), ("g", float("nan"))):
-        bad[n][:, cu[3]:cu[4]] = x
-    o2, ht2 = _forward(to_device(bad, cuda_device), cu=cu)
-    for i in (0, 1, 2, 4, 5, 6):
-        assert torch.equal(o2[:, cu[i]:cu[i + 1]], o[:, cu[i]:cu[i + 1]]) and torch.equal(ht2[i], ht[i])
-
-
 def _stage_args(d, B, T, H, dev, **kw):
     o = torch.full((B, T, H, 128), float("nan"), dtype=torch.bfloat16, device=dev)
     ht = torch.full((B, H, 128, 128), float("nan"), device=dev)
