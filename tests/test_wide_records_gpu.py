@@ -128,7 +128,7 @@ def test_workspace_that_was_sized_for_16_token_records_is_enough(cuda_device):
     """Nothing is written behind kda_fwd_workspace_bytes."""
     for B, T, H in ((1, 8192, 32), (1, 40000, 8), (2, 1500, 60)):
         d = to_device(O.make_inputs(B, T, H, seed0=3, h0_std=0.05), cuda_device)
-        a, _, _, ws = _stage_args(d, B, T, H, cuda_device)
+        a, o, ht, ws = _stage_args(d, B, T, H, cuda_device)     # o and ht live on: a freed o could become `guarded`
         n = ws.numel()
         guarded = torch.full((n + 4096,), 0x5A, dtype=torch.uint8, device=cuda_device)
         a.workspace = guarded.data_ptr()
