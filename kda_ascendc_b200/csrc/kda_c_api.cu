@@ -11,7 +11,6 @@
 #include "../../include/kda_b200.h"
 #include "kda_common.cuh"
 #include "kda_kernels.h"
-#include "kda_wide.cuh"
 
 static_assert(sizeof(KdaFwdArgs) == 312 && offsetof(KdaFwdArgs, chunk_table) == 288 && offsetof(KdaFwdArgs, Hq) == 308,
               "KdaFwdArgs layout is part of the ABI (bindings mirror it field by field)");
@@ -204,103 +203,13 @@ int beside_window(const KdaFwdArgs* a) {
   return static_cast<int>(by_count > by_round ? by_count : by_round);
 }
 
-// Segments a chain of nt wide chunks is cut into when its K2 runs as a walk over segments (do_k2w); 1 = not cut.
-// The first of the two passes has 2 n - 3 CTAs per chain, and one per SM is what pays: two on an SM take twice as
-// long a step (T8192 H32: 3 segments 211 us, 4 239, 5 216; H16 T4096: 5 segments 88, 6 88, 9 101; T131072 H16 6
-// segments 1,488, 9 1,554).  The walk costs about a step and a half per segment, hence n^2 <= 2 nt.
-int split_segments(long long chains, int nt, int sms) {
-  long long n = (sms / chains + 3) / 2;
-  while (n > 1 && n * n > 2LL * nt) --n;
-  // transforms and entry states lie in the part of the workspace that wide records leave free
-  const long long spare = nt * (4LL * kda::REC_BYTES - kda::WREC_BYTES) - 3LL * kda::REC_BYTES;
-  while (n > 1 && (3 * n - 5) * kda::D * kda::D * 4 > spare) --n;
-  return n >= 3 ? static_cast<int>(n) : 1;
-}
-
-// v is read by the K2 of wide records, chunk by chunk ahead of the outputs: o may lie exactly over it, but o and ht may
-// not overlap it in another way.
-bool output_over_v(const KdaFwdArgs* a) {
-  const Span v = span_of(a->v, a->v_stride, a, a->H, kda::D, 2);
-  const uintptr_t ht = reinterpret_cast<uintptr_t>(a->ht);
-  const uintptr_t states = static_cast<uintptr_t>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H * kda::D * kda::D * sizeof(float);
-  if (ht != 0 && ht < v.hi && v.lo < ht + states) return true;
-  if (a->o == nullptr) return false;
-  for (int i = 0; i < 3; ++i)
-    if (a->o_stride[i] < 0) return true;
-  const Span o = span_of(a->o, a->o_stride, a, a->H, kda::D, 2);
-  if (o.hi <= v.lo || v.hi <= o.lo) return false;
-  return !(a->o == a->v && memcmp(a->o_stride, a->v_stride, sizeof(a->v_stride)) == 0);
-}
-
-// Whether K1 writes, and K2 reads, wide records (kda_wide.cuh).  A function of the arguments alone, so that the stage
-// entry points agree with each other and with kda_fwd.
-//
-// Whole forward on B200, 16-token records against wide ones:
-//   from half as many chains as SMs up to the SMs, one CTA per chain: T8192 H96 945 -> 791 us, T1024 H96 135 -> 122;
-//   few chains, cut into segments: T131072 H16 4,316 -> 2,831, T4096 H16 150 -> 140, T8192 H32 412 -> 393.
-// Not where the 16-token K2 has enough chains to fill the chip (B8 T2048 H32 498 -> 524: K1 is the longer part) and
-// not where sequences are short (T2048 H32 112 -> 131, B2 T1024 H4 39 -> 52).
-// Not a lower bound below -5.03 (its Grams need 16-token blocks: K1 571 us at B8 T2037 H32 against 294), and not yet gate
-// sums made by the caller or packed sequences, which the kernels take but which have not been compared on the GPU.
-bool wide_records(const KdaFwdArgs* a) {
-  if (a->k2_variant != 0 || a->k2_vsplit != 0 || a->g_out != nullptr || a->ainv_out != nullptr || a->v == nullptr) return false;
-  if (a->n_seqs > 0 || !(a->flags & KDA_FLAG_GATE_IN_KERNEL) || !(16.0f * -a->lower_bound * kda::RCP_LN2 <= 116.0f)) return false;
-  const int sms = device_sms();
-  const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
-  // wide chunks of a chain (the mean, for packed sequences: at least 1,024 tokens, which also keeps their records, one
-  // partial chunk a sequence included, within the workspace)
-  const int nt = a->n_seqs > 0 ? a->n_chunks / a->n_seqs / 4 : (a->T + kda::WT - 1) / kda::WT;
-  const bool whole = chains * 2 > sms && chains <= sms && nt >= 16;
-  const bool cut = a->n_seqs == 0 && chains * 4 <= sms && nt >= (chains * 8 <= sms ? 64 : 128) && split_segments(chains, nt, sms) > 1;
-  return (whole || cut) && a->n_seqs <= kda::WIDE_MAX_SEQS && !output_over_v(a);
-}
-
-// The tensor maps of q, k, v, g with boxes of `rows` tokens.  They depend only on the input pointers, sizes and
-// strides: a loop that calls with the same buffers (a serving loop, a benchmark) re-uses the maps of its previous call.
-int tensor_maps(const KdaFwdArgs* a, kda::K1Params& p, int rows) {
+int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
+  kda::K1Params p;
+  memset(&p, 0, sizeof(p));
   p.q = static_cast<const __nv_bfloat16*>(a->q);
   p.k = static_cast<const __nv_bfloat16*>(a->k);
   p.v = static_cast<const __nv_bfloat16*>(a->v);
   p.g = a->g;
-  p.B = a->B; p.T = a->T; p.H = a->H;
-  p.Hq = a->Hq > 0 ? a->Hq : a->H;
-  for (int i = 0; i < 3; ++i) {
-    p.q_s[i] = a->q_stride[i]; p.k_s[i] = a->k_stride[i]; p.v_s[i] = a->v_stride[i];
-    p.g_s[i] = a->g_stride[i]; p.beta_s[i] = a->beta_stride[i];
-  }
-  struct MapKey {
-    const void *q, *k, *v, *g;
-    int32_t B, T, H, Hq, g_dtype, rows;
-    int64_t s[12];
-  };
-  thread_local MapKey last_key;
-  thread_local CUtensorMap last_maps[4];
-  thread_local bool have_maps = false;
-  MapKey key;
-  memset(&key, 0, sizeof(key));
-  key.q = a->q; key.k = a->k; key.v = a->v; key.g = a->g;
-  key.B = a->B; key.T = a->T; key.H = a->H; key.Hq = p.Hq; key.g_dtype = a->g_dtype; key.rows = rows;
-  for (int i = 0; i < 3; ++i) {
-    key.s[i] = a->q_stride[i]; key.s[3 + i] = a->k_stride[i]; key.s[6 + i] = a->v_stride[i]; key.s[9 + i] = a->g_stride[i];
-  }
-  if (have_maps && memcmp(&key, &last_key, sizeof(key)) == 0) {
-    p.tm_q = last_maps[0]; p.tm_k = last_maps[1]; p.tm_v = last_maps[2]; p.tm_g = last_maps[3];
-    return KDA_OK;
-  }
-  const char* what = "";
-  if (kda::k1_encode_tensor_maps(p, a->g_dtype == KDA_G_BF16, rows, &what) != cudaSuccess)
-    return fail(KDA_ERR_CUDA, "kda: building the TMA descriptor failed for: %s", what);
-  last_key = key;
-  last_maps[0] = p.tm_q; last_maps[1] = p.tm_k; last_maps[2] = p.tm_v; last_maps[3] = p.tm_g;
-  have_maps = true;
-  return KDA_OK;
-}
-
-int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
-  const bool wide = win_chunks == 0 && wide_records(a);
-  const int rows = wide ? kda::WT : kda::BT;
-  kda::K1Params p;
-  memset(&p, 0, sizeof(p));
   p.beta = a->beta;
   p.A_log = a->A_log;
   p.dt_bias = a->dt_bias;
@@ -308,19 +217,21 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
   p.status = status_ptr(a);
   p.g_out = a->g_out;
   p.ainv_out = a->ainv_out;
-  if (int rc = tensor_maps(a, p, rows)) return rc;
-  p.NT = (a->T + rows - 1) / rows;
+  p.B = a->B; p.T = a->T; p.H = a->H; p.NT = (a->T + kda::BT - 1) / kda::BT;
   p.div_h.set(static_cast<uint32_t>(p.H));
   p.div_nt.set(static_cast<uint32_t>(p.NT));
+  for (int i = 0; i < 3; ++i) {
+    p.q_s[i] = a->q_stride[i]; p.k_s[i] = a->k_stride[i]; p.v_s[i] = a->v_stride[i];
+    p.g_s[i] = a->g_stride[i]; p.beta_s[i] = a->beta_stride[i];
+  }
   p.scale = a->scale;
   p.lower_bound = a->lower_bound;
   p.flags = a->flags;
   if (a->n_seqs > 0) {
     p.chunk_table = reinterpret_cast<const int4*>(a->chunk_table);
     p.n_chunks = a->n_chunks;
-    p.seq_table = reinterpret_cast<const int4*>(a->seq_table);
-    p.n_seqs = a->n_seqs;
   }
+  p.Hq = a->Hq > 0 ? a->Hq : a->H;
   p.div_g.set(static_cast<uint32_t>(p.H / p.Hq));
   if (win_chunks > 0) {
     p.progress = status_ptr(a) + kda::HDR_PROGRESS;
@@ -330,22 +241,36 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
   }
   // 2^g may be factored as 2^(g-g_mid) * 2^(g_mid) only while no factor can underflow:
   // 16 tokens * |lower_bound| * RCP_LN2 must stay inside the fp32 exponent range.
-  const bool gate = (a->flags & KDA_FLAG_GATE_IN_KERNEL) != 0, g_bf16 = a->g_dtype == KDA_G_BF16;
-  const float span = 16.0f * -a->lower_bound * kda::RCP_LN2;
-  cudaError_t e;
-  if (!wide) {
-    e = kda::launch_k1(p, g_bf16, gate && span <= 120.0f, st);
-  } else if (gate) {
-    e = kda::launch_k1w(p, g_bf16, span <= 116.0f, st);
-  } else {
-    p.check_range = 1;
-    e = cudaMemsetAsync(status_ptr(a) + kda::HDR_RANGE, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = kda::launch_k1w(p, g_bf16, true, st);
-    p.check_range = 0;
-    p.redo = 1;
-    if (e == cudaSuccess) e = kda::launch_k1w(p, g_bf16, false, st);
-    ++g_launches;
+  const bool fast_exp = (a->flags & KDA_FLAG_GATE_IN_KERNEL) && (16.0f * -a->lower_bound * kda::RCP_LN2 <= 120.0f);
+  // The four tensor maps depend only on the input pointers, sizes and strides: a loop that calls with
+  // the same buffers (a serving loop, a benchmark) re-uses the maps of its previous call.
+  struct MapKey {
+    const void *q, *k, *v, *g;
+    int32_t B, T, H, Hq, g_dtype;
+    int64_t s[12];
+  };
+  thread_local MapKey last_key;
+  thread_local CUtensorMap last_maps[4];
+  thread_local bool have_maps = false;
+  MapKey key;
+  memset(&key, 0, sizeof(key));
+  key.q = a->q; key.k = a->k; key.v = a->v; key.g = a->g;
+  key.B = a->B; key.T = a->T; key.H = a->H; key.Hq = p.Hq; key.g_dtype = a->g_dtype;
+  for (int i = 0; i < 3; ++i) {
+    key.s[i] = a->q_stride[i]; key.s[3 + i] = a->k_stride[i]; key.s[6 + i] = a->v_stride[i]; key.s[9 + i] = a->g_stride[i];
   }
+  cudaError_t e = cudaSuccess;
+  if (have_maps && memcmp(&key, &last_key, sizeof(key)) == 0) {
+    p.tm_q = last_maps[0]; p.tm_k = last_maps[1]; p.tm_v = last_maps[2]; p.tm_g = last_maps[3];
+  } else {
+    const char* what = "";
+    e = kda::k1_encode_tensor_maps(p, a->g_dtype == KDA_G_BF16, &what);
+    if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: building the TMA descriptor failed for: %s", what);
+    last_key = key;
+    last_maps[0] = p.tm_q; last_maps[1] = p.tm_k; last_maps[2] = p.tm_v; last_maps[3] = p.tm_g;
+    have_maps = true;
+  }
+  e = kda::launch_k1(p, a->g_dtype == KDA_G_BF16, fast_exp, st);
   if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: K1 launch failed: %s", cudaGetErrorString(e));
   ++g_launches;
   return KDA_OK;
@@ -353,92 +278,8 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
 
 struct H0Flags { const int32_t* flags; int n, epoch; };
 
-// K2 over wide records; the arguments mean what they mean to do_k2.
-int do_k2w(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, const KdaPeerPushArgs* push = nullptr,
-           const H0Flags* h0f = nullptr, bool after_k1 = false) {
-  kda::K1Params maps;
-  memset(&maps, 0, sizeof(maps));
-  if (int rc = tensor_maps(a, maps, kda::WT)) return rc;
-  kda::K2wParams p;
-  memset(&p, 0, sizeof(p));
-  p.tm_v = maps.tm_v;
-  p.rec = rec_ptr(a);
-  p.h0 = a->h0;
-  p.o = static_cast<__nv_bfloat16*>(a->o);
-  p.ht = a->ht;
-  p.status = status_ptr(a);
-  p.B = a->B; p.T = a->T; p.H = a->H; p.NT = (a->T + kda::WT - 1) / kda::WT;
-  for (int i = 0; i < 3; ++i) p.o_s[i] = a->o_stride[i];
-  p.k_first = (a->flags & KDA_FLAG_STATE_K_FIRST) ? 1 : 0;
-  const int sms = device_sms();
-  const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
-  if (a->n_seqs > 0) {
-    p.seq_table = reinterpret_cast<const int4*>(a->seq_table);
-    p.n_seqs = a->n_seqs;
-  }
-  p.pdl = after_k1;
-  p.n_chains = static_cast<int>(chains);
-  p.n_seg = a->n_seqs > 0 || state_only || h0f != nullptr ? 1 : split_segments(chains, p.NT, sms);
-  auto launch = [&](int job, long long jobs) -> int {
-    p.job = job;
-    const cudaError_t e = kda::launch_k2w(p, static_cast<int>(jobs), jobs <= sms, st);
-    if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: K2 launch failed: %s", cudaGetErrorString(e));
-    ++g_launches;
-    p.pdl = 0;
-    return KDA_OK;
-  };
-  if (state_only && zero_u == 2) {
-    if (2 * chains > 0x3fffffffLL) return fail(KDA_ERR_INVALID_ARG, "kda: too many chains%s", "");
-    if (push != nullptr) {
-      const long long hp = push->slice_floats / (2LL * kda::D * kda::D);
-      if (hp <= 0 || hp * push->world != chains || push->slice_floats % (2LL * kda::D * kda::D) != 0)
-        return fail(KDA_ERR_INVALID_ARG, "kda: slice_floats must be chains / world whole (M, Q) pairs%s (chains %lld)", "", chains);
-      p.push_on = 1;
-      p.push_hp = static_cast<int>(hp);
-      p.push_epoch = push->epoch;
-      p.push_dst_offset = push->dst_offset_floats;
-      p.push_counter = push->counter;
-      for (int d = 0; d < push->world; ++d) { p.push_dst[d] = push->dst[d]; p.push_flag[d] = push->flag[d]; }
-    }
-    return launch(kda::W2_STATE_PAIR, 2 * chains);
-  }
-  if (state_only) {
-    p.zero_u = zero_u == 1;
-    return launch(kda::W2_STATE, chains);
-  }
-  if (h0f != nullptr) { p.h0_flags = h0f->flags; p.h0_n_flags = h0f->n; p.h0_epoch = h0f->epoch; }
-  if (p.n_seg <= 2) return launch(kda::W2_FORWARD, chains);
-  // the sequence in segments: transforms of the middle ones beside the first one's own pass, a walk over them, the
-  // other segments from their entry states.  The buffers lie in the part of the workspace that wide records leave free.
-  const size_t state = static_cast<size_t>(kda::D) * kda::D;
-  p.seg = (p.NT + p.n_seg - 1) / p.n_seg;
-  p.n_seg = (p.NT + p.seg - 1) / p.seg;
-  p.entry = reinterpret_cast<float*>(rec_ptr(a) + static_cast<size_t>(chains) * p.NT * kda::WREC_BYTES);
-  p.mq = p.entry + static_cast<size_t>(p.n_seg - 1) * chains * state;
-  if (int rc = launch(kda::W2_SPLIT_FIRST, chains * (2 * p.n_seg - 3))) return rc;
-  if (p.n_seg > 2) {
-    kda::FoldParams f;
-    memset(&f, 0, sizeof(f));
-    f.mq = p.mq;
-    f.seg_stride = 2 * state;
-    f.chain_stride = static_cast<long long>(p.n_seg - 2) * 2 * state;
-    f.h0 = p.entry;
-    f.h0_stride = state;
-    f.s_in = p.entry;
-    f.n_chains = static_cast<int>(chains);
-    f.n_seg = p.n_seg - 2;
-    f.use_q = 1;
-    f.status = status_ptr(a);
-    const cudaError_t e = kda::launch_state_fold(f, st);
-    if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: fold launch failed: %s", cudaGetErrorString(e));
-    ++g_launches;
-  }
-  return launch(kda::W2_SPLIT_LAST, chains * (p.n_seg - 1));
-}
-
 int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, const KdaPeerPushArgs* push = nullptr,
           const H0Flags* h0f = nullptr, bool after_k1 = false, int win_chunks = 0) {
-  if (win_chunks == 0 && wide_records(a)) return do_k2w(a, state_only, zero_u, st, push, h0f, after_k1);
   kda::K2Params p;
   memset(&p, 0, sizeof(p));
   p.rec = rec_ptr(a);
@@ -594,7 +435,7 @@ int kda_fwd(const KdaFwdArgs* a, void* stream) {
   if (int rc = check_k1(a)) return rc;
   if (int rc = check_k2(a, false)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int win = wide_records(a) ? 0 : beside_window(a);
+  const int win = beside_window(a);
   if (win > 0) {   // the window counters must be zero before either kernel starts
     cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
     if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));

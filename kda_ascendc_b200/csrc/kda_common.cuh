@@ -51,7 +51,6 @@ constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the wor
 // T8192 H32 411.7 -> 414.5 us); HDR_PROGRESS .. HDR_PROGRESS + MAX_WINDOWS - 1 = finished K1 items per window of
 // chunks, for a K2 that runs beside K1 (zeroed before K1 starts; unused otherwise)
 constexpr int HDR_K1_STATUS = 1;
-constexpr int HDR_RANGE = 2;       // wide K1: a sum made by the caller was out of the range of its 32-token blocks
 constexpr int HDR_PROGRESS = 4;
 constexpr int MAX_WINDOWS = WS_HEADER_BYTES / 4 - HDR_PROGRESS;
 
@@ -132,26 +131,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
 #pragma unroll 1
     for (int i = 0; i < 32; ++i)
       if (mbar_try_wait(bar, parity)) return true;
-    if (abort_flag != nullptr && *abort_flag != 0) return false;
-    if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
-  }
-}
-
-// The same for waits of many warps beside working ones: the thread is parked until the phase completes or 20 us have
-// passed, instead of polling (sixteen warps of polling threads slow the shared-memory path of the others several times).
-__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  for (;;) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(20000u)
-        : "memory");
-    if (ok != 0) return true;
     if (abort_flag != nullptr && *abort_flag != 0) return false;
     if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) return false;
   }

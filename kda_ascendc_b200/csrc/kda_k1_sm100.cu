@@ -626,7 +626,7 @@ EncodeTiledFn get_encode_fn() {
 }
 }  // namespace
 
-cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, int rows, const char** what) {
+cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) { *what = "cuTensorMapEncodeTiled is not available from this driver"; return cudaErrorNotSupported; }
   struct T { CUtensorMap* m; const void* ptr; const int64_t* s; CUtensorMapDataType dt; int es; const char* name; };
@@ -646,7 +646,7 @@ cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, int rows, const char
                              static_cast<cuuint64_t>(t.s[0]) * t.es};
     for (int i = 0; i < 3; ++i)
       if (dims[i + 1] == 1) strides[i] = static_cast<cuuint64_t>(D) * t.es;
-    const cuuint32_t box[4] = {static_cast<cuuint32_t>(D), 1, static_cast<cuuint32_t>(rows), 1};
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(D), 1, static_cast<cuuint32_t>(BT), 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = enc(t.m, t.dt, 4, const_cast<void*>(t.ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

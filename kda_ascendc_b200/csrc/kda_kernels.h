@@ -48,13 +48,6 @@ struct K1Params {
   // chunks of its sequence), B == 1; null for a fixed-length batch
   const int4* chunk_table;
   int n_chunks;
-  // wide records: the packed sequences themselves (first token, chunks of 16, first record, length); NT and div_nt count
-  // the wide chunks of a fixed-length batch
-  const int4* seq_table;
-  int n_seqs;
-  // wide records, gate sums made by the caller: they are checked against the range of 32-token blocks as they are read, and
-  // a second launch (redo) does all of it over 16-token blocks if one was outside
-  int check_range, redo;
   // grouped value heads: q and k have Hq heads, head h of everything else reads q/k head h / (H/Hq)
   int Hq;
   FastDiv div_g;   // divides by H / Hq
@@ -133,11 +126,8 @@ cudaError_t launch_dep(Kernel kernel, int grid, int block, int smem_bytes, cudaS
 }
 
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream);
-// The same for wide records (kda_wide.cuh): NT and div_nt count chunks of 64 tokens.  two_blocks: the Gram exponents are
-// centred over 32 tokens instead of 16, finite while 16 |lower_bound| log2 e <= 116.
-cudaError_t launch_k1w(const K1Params& p, bool g_bf16, bool two_blocks, cudaStream_t stream);
-// Fills the four tensor maps of p from its pointers, sizes and strides (host, no device work); boxes of `rows` tokens.
-cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, int rows, const char** what);
+// Fills the four tensor maps of p from its pointers, sizes and strides (host, no device work).
+cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what);
 // Two organisations of K2 (same arithmetic, bit-identical results within one organisation):
 //   "n8":       state rows on the MMA N dimension, ntile = 1 tile of 8 rows per warp,
 //               16 / vsplit in {1, 2, 4} consumer warps per CTA                 (kda_k2_sm100.cu)
@@ -158,44 +148,6 @@ cudaError_t launch_k2n_pair(const K2Params& p, int vsplit, cudaStream_t stream);
 //   "tc":       the whole 128-row state of a head in tensor memory, tcgen05 MMAs, one CTA per
 //               (batch, head), two CTAs per SM; outputs + final state only              (kda_k2t_sm100.cu)
 cudaError_t launch_k2t(const K2Params& p, long long n_records, cudaStream_t stream);
-
-// K2 of wide records (kda_k2w_sm100.cu).  What a launch does with every chain:
-enum W2Job {
-  W2_FORWARD,       // all its chunks: outputs and final state                                       1 CTA per chain
-  W2_SPLIT_FIRST,   // the chain in n_seg segments: outputs of the first one and its final state (entry[0]); M and Q of
-                    // the segments 1 .. n_seg - 2 (mq)                                              2 n_seg - 3
-  W2_SPLIT_LAST,    // the segments 1 .. n_seg - 1 from entry[0 ..]: outputs, and ht from the last     n_seg - 1
-  W2_STATE,         // final state only, without v if zero_u                                         1
-  W2_STATE_PAIR,    // M and Q of the whole chain, ht [chains][2][128][128]                             2
-};
-struct K2wParams {
-  CUtensorMap tm_v;   // (d, head, token, batch), boxes of 64 tokens
-  const uint8_t* rec;
-  const float* h0;
-  __nv_bfloat16* o;
-  float* ht;
-  int* status;
-  int B, T, H, NT;    // NT: wide chunks of a sequence
-  int64_t o_s[3];
-  int k_first;
-  const int4* seq_table;
-  int n_seqs;
-  int pdl;
-  int job, zero_u;
-  int n_chains, n_seg, seg;   // split: segments of seg wide chunks (the last may be shorter)
-  float* mq;                  // [n_chains][n_seg - 2][2][128][128]
-  float* entry;               // [n_seg - 1][n_chains][128][128]: the states before segments 1 ..
-  // W2_STATE_PAIR into peers' receive buffers, and W2_FORWARD from an entry state that peers store (as in K2Params)
-  int push_on, push_hp, push_epoch;
-  long long push_dst_offset;
-  float* push_dst[MAX_PEERS];
-  int* push_flag[MAX_PEERS];
-  int* push_counter;
-  const int* h0_flags;
-  int h0_n_flags, h0_epoch;
-};
-// jobs = CTAs; one_per_sm: two stages of operands, else one stage and two CTAs per SM
-cudaError_t launch_k2w(const K2wParams& p, int jobs, bool one_per_sm, cudaStream_t stream);
 
 // Walk of the per-segment affine state transforms of a sequence split (kda_fold_sm100.cu).
 struct FoldParams {

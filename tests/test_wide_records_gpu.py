@@ -1,9 +1,10 @@
-"""The forward on 64-token records (kda_k1w_sm100.cu, kda_k2w_sm100.cu) against the CPU oracle, against the 16-token
-kernels, and against itself through the stage entry points.
+"""The forward of long sequences, and of about as many chains as SMs, against the CPU oracle, against the 16-row K2, and
+against itself through the stage entry points.  These are the shapes that a record of 64 tokens was once written for;
+its bounds stay, whatever form runs them.
 
 Bounds: the absolute ones of the 16-token path on benchmark-distributed inputs (o 1e-3, state 2e-3), the reference's
-relative 2e-2 of the largest value where states are O(1); against the 16-token kernels one more rounding step of each
-side (|o| <= 0.06 has bf16 steps of 2.5e-4)."""
+relative 2e-2 of the largest value where states are O(1); against the 16-row K2 one more rounding step of each side
+(|o| <= 0.06 has bf16 steps of 2.5e-4)."""
 import ctypes
 
 import pytest
@@ -39,8 +40,7 @@ def _heads(inp, heads):
     return s
 
 
-# whole and ragged last chunks of 64 (1, 63, 17, 56 tokens), whole chains and segments, both sides of the line in the lower
-# bound (-5.03), fp32 gates
+# last chunks of 16, 1, 15 and 8 tokens, few and many chains, lower bounds around -5.03, fp32 gates
 @pytest.mark.parametrize("B,T,H,lower_bound,g_dtype", [
     (1, 8192, 32, -5.0, torch.bfloat16), (1, 4097, 16, -5.0, torch.float32), (1, 1087, 96, -5.0, torch.bfloat16),
     (4, 1041, 37, -5.0, torch.bfloat16), (1, 3000, 75, -5.02, torch.float32), (1, 3000, 96, -5.04, torch.bfloat16)])
@@ -60,7 +60,7 @@ def test_wide_forward_matches_oracle(cuda_device, B, T, H, lower_bound, g_dtype)
     assert torch.equal(o, ok) and torch.equal(ht, htk)
 
 
-# states that persist: every hand-over between chunks, and between the segments of a long sequence on few heads, shows
+# states that persist: every hand-over between chunks shows
 @pytest.mark.parametrize("B,T,H,regime", [(1, 16384, 16, "carry"), (1, 16421, 13, "carry"), (2, 2100, 60, "carry"),
                                           (1, 8200, 32, "long_memory"), (1, 4100, 1, "carry")])
 def test_wide_forward_carries_the_state(cuda_device, B, T, H, regime):
