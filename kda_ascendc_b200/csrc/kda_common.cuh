@@ -82,6 +82,15 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// One lane of a converged warp, chosen by the hardware.  The compiler knows that a branch on it is taken by one
+// thread; behind `lane == 0` it does not, and wraps every tcgen05 instruction in a loop over the lanes that may be
+// there (eight tcgen05.mma M128 N32 issue in 37 cycles behind elect.sync, in 402 behind lane == 0).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

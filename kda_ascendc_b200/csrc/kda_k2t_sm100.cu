@@ -174,7 +174,7 @@ struct K2tParams {
 __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_constant__ K2tParams pp) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const K2Params& p = pp.k;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler
   int bh = blockIdx.x + p.chain0;
   if (p.by_length) bh = chain_by_length(p.seq_table, p.n_seqs, p.H, bh);
   int b = bh / p.H;
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tbase = *slot;
+  const uint32_t tbase = __shfl_sync(0xffffffffu, *slot, 0);
 
   auto give_up = [&]() {
     if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2T_TIMEOUT); }
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
 
   if (warp == KT_EPI_WARPS) {
     // ------------------------------ producer -------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
       int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     __syncwarp();
   } else if (warp == KT_EPI_WARPS + 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t ID_P1 = instr_desc(128, 32, 0), ID_P2 = instr_desc(128, 128, 1), ID_P3 = instr_desc(128, 16, 0);
       int s = 0;
       for (int n = 0; n < NT; ++n, s = (s + 1 == KT_STAGES) ? 0 : s + 1) {
