@@ -20,7 +20,7 @@ HOST_PATH = PKG_DIR / "_kda_host.so"
 HOST_SOURCE = "kda_host.cpp"
 SOURCES = ["kda_c_api.cu", "kda_k1_sm100.cu", "kda_k2_sm100.cu", "kda_k2la_sm100.cu", "kda_k2m_sm100.cu", "kda_k2t_sm100.cu", "kda_recurrent_sm100.cu", "kda_fold_sm100.cu", "kda_peer_sm100.cu",
            "kda_selftest.cu", "kda_static_scratch.cu"]
-HEADERS = ["kda_common.cuh", "kda_kernels.h", "../../include/kda_b200.h"]
+HEADERS = ["kda_common.cuh", "kda_tc.cuh", "kda_kernels.h", "../../include/kda_b200.h"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-shared", "-Xcompiler", "-fPIC",

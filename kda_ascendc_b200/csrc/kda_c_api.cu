@@ -370,8 +370,6 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   }
   cudaError_t e;
   if (variant == 4) {
-    const long long n_records = a->n_seqs > 0 ? static_cast<long long>(a->n_chunks) * a->H
-                                              : static_cast<long long>(a->B) * a->H * p.NT;
     // Tail wave.  The tensor-memory form holds two chains per SM at once; when the chains left over
     // after the full waves are at most half as many as SMs, they run faster in an mma.sync form
     // (16-row: two CTAs per chain, one per SM, 0.8 us per step; 8-row for at most SMs/4 chains,
@@ -392,7 +390,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     if (a->k2_variant == 0 && bh > 2LL * sms && tail > 0 && tail * 2 <= sms) {
       p.chain0 = 0;
       p.n_chains = static_cast<int>(bh - tail);
-      e = kda::launch_k2t(p, n_records, st);
+      e = kda::launch_k2t(p, st);
       if (e == cudaSuccess) {
         ++g_launches;
         p.pdl = p.one_per_sm = 0;   // behind the full waves, an ordinary launch
@@ -403,7 +401,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
         else e = kda::launch_k2m(p, 2, false, st);
       }
     } else {
-      e = kda::launch_k2t(p, n_records, st);
+      e = kda::launch_k2t(p, st);
     }
   } else {
     e = (variant == 3) ? kda::launch_k2m(p, vsplit, state_only, st)

@@ -8,22 +8,22 @@
 // stage is one bulk (TMA) copy.
 //
 //   offset  bytes  contents
-//   0       4096   w    bf16 [16 tok][128 k]   swizzled tile (see swz_off)
-//   4096    4096   qg   bf16 [16][128]  = bf16(qhat * 2^g)
-//   8192    4096   kg_h bf16 [16][128]  \ hi/lo split of khat * 2^(g_last - g)
-//   12288   4096   kg_l bf16 [16][128]  /
-//   16384   512    Aqk_h bf16 [16 i][16 j] row-major \ hi/lo split of the scaled lower
-//   16896   512    Aqk_l bf16 [16][16]               / triangle (incl. diagonal)
-//   17408   512    dec  fp32 [128]      = 2^(g_last)
-//   17920   8192   u    fp32, accumulator-fragment order [16 column tile][32 lane][4]:
-//                       lane (g = lane/4, t = lane%4) holds u[tok g][v], u[tok g][v+1],
-//                       u[tok g+8][v], u[tok g+8][v+1] with v = 8*tile + 2t
+//   0       8192   w, qg     bf16, two halves of 64 k: [half][w, qg][16 tok][64 k], the eight 16-byte units of a
+//                            128-byte row XOR-permuted by the row index (wq_off)
+//   8192    4096   kg_h      bf16 [2 token halves][128 k][8 tok] \ hi/lo split of khat * 2^(g_last - g),
+//   12288   4096   kg_l      bf16 [2][128][8]                    / transposed (kg_off)
+//   16384   1024   Aqk       bf16 [2 column halves][hi, lo][16 i][8 j]: hi/lo split of the scaled lower triangle
+//                            incl. diagonal (aq_off)
+//   17408   512    dec       fp32 [128]      = 2^(g_last)
+//   17920   8192   u         fp32, accumulator-fragment order [16 column tile][32 lane][4]:
+//                            lane (g = lane/4, t = lane%4) holds u[tok g][v], u[tok g][v+1],
+//                            u[tok g+8][v], u[tok g+8][v+1] with v = 8*tile + 2t
 //
-// Swizzled bf16 tile: element (r, c) of a [16][128] tile lives at byte
-//   r*256 + ((((c>>3) ^ (r&7)) << 4) | ((c&7) << 1))
-// i.e. the eight 16-byte units of each 128-byte half-row are XOR-permuted by the
-// row index, which makes every ldmatrix (8 rows, same column unit) bank-conflict
-// free after a straight, unpadded bulk copy.
+// with qg = bf16(qhat * 2^g).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
+// operand as it stands: [w; qg] is a 32-row K-major operand in the 128-byte swizzle of tcgen05 (8-row groups 1024
+// bytes apart), kg^T and Aqk are 8x8 core matrices of 128 contiguous bytes (K-major without swizzle).  tcgen05.mma
+// reads them by descriptor, tcgen05.cp moves 32 rows x 16 bytes of them into tensor memory, and every 8x8 matrix of an
+// ldmatrix is free of bank conflicts.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -34,12 +34,13 @@ namespace kda {
 constexpr int BT = 16;
 constexpr int D = 128;
 constexpr int TILE_BYTES = BT * D * 2;  // 4096
-constexpr int REC_W = 0;
-constexpr int REC_QG = 4096;
+constexpr int REC_W = 0;         // w of half hf at REC_W + hf * REC_HALF, qg at REC_QG + hf * REC_HALF
+constexpr int REC_QG = 2048;
+constexpr int REC_HALF = 4096;
 constexpr int REC_KGH = 8192;
 constexpr int REC_KGL = 12288;
-constexpr int REC_AQK = 16384;
-constexpr int REC_AQL = 16896;
+constexpr int REC_AQK = 16384;   // hi; lo at REC_AQL
+constexpr int REC_AQL = 16640;
 constexpr int REC_DEC = 17408;
 constexpr int REC_U = 17920;
 constexpr int REC_SHARED_BYTES = 17920;  // everything every V-slice needs
@@ -72,8 +73,21 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// Swizzled bf16 tile of K1: element (r, c) of a [16][128] tile, the eight 16-byte units of each 128-byte half row
+// XOR-permuted by the row index, so that every ldmatrix (8 rows, same column unit) is free of bank conflicts.
 __device__ __forceinline__ uint32_t swz_off(int r, int c) {
   return static_cast<uint32_t>(r * 256 + ((((c >> 3) ^ (r & 7)) << 4) | ((c & 7) << 1)));
+}
+
+// the record's tiles: element offsets in bytes (w / qg relative to their part of half 0, see above)
+__device__ __forceinline__ uint32_t wq_off(int r, int c) {
+  return static_cast<uint32_t>((c >> 6) * REC_HALF + r * 128 + (((((c >> 3) & 7) ^ (r & 7)) << 4) | ((c & 7) << 1)));
+}
+__device__ __forceinline__ uint32_t kg_off(int tok, int k) {
+  return static_cast<uint32_t>((tok >> 3) * 2048 + k * 16 + (tok & 7) * 2);
+}
+__device__ __forceinline__ uint32_t aq_off(int i, int j) {
+  return static_cast<uint32_t>((j >> 3) * 512 + i * 16 + (j & 7) * 2);
 }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -296,6 +310,9 @@ __device__ __forceinline__ uint32_t movmatrix_t(uint32_t a) {
 }
 __device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x2_t(uint32_t addr, uint32_t& r0, uint32_t& r1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
 // D(16x8,f32) += A(16x16,bf16,row) * B(16x8,bf16,col)
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

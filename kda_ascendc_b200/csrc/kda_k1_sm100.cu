@@ -30,8 +30,9 @@
 namespace kda {
 
 // shared-memory map (bytes): four CTAs of the production variant (bf16 gate, FAST_EXP) per SM
-constexpr int S_QG = 0, S_KGH = 4096, S_KGL = 8192;   // -> record[4096, 16384)
-constexpr int S_AQK = 12288, S_AQL = 12800, S_DEC = 13312;   // -> record[16384, 17920)
+constexpr int S_QG = 0;                               // two halves of 2048 bytes -> the record's qg parts
+constexpr int S_KGH = 4096, S_KGL = 8192;             // -> record[8192, 16384)
+constexpr int S_AQK = 12288, S_AQL = S_AQK + (REC_AQL - REC_AQK), S_DEC = 13312;   // -> record[16384, 17920)
 constexpr int S_L = 13824;                            // fp32 [16][16], -Akk
 constexpr int S_XH = 14848, S_XL = 15360;             // bf16 [16][16] hi / lo of (I+Akk)^-1
 constexpr int S_GRAM = 15872;
@@ -39,7 +40,12 @@ constexpr int S_QGH = S_GRAM, S_QGL = S_GRAM + 4096, S_KQH = S_GRAM + 8192, S_KQ
               S_KNH = S_GRAM + 16384, S_KNL = S_GRAM + 20480;   // KN tiles only without FAST_EXP
 // once the Grams are done their A tiles hold the B operands of w and u
 constexpr int S_KBH = S_GRAM, S_VBH = S_GRAM + 4096, S_VBL = S_GRAM + 8192;
-constexpr int S_WST = S_GRAM + 12288;   // staging tile of w (the fourth Gram tile slot), -> record[0, 4096)
+constexpr int S_WST = S_GRAM + 12288;   // staging tile of w (the fourth Gram tile slot), -> the record's w parts
+
+// element (r, c) of a staged w or qg tile: the record's layout with the two halves back to back
+__device__ __forceinline__ uint32_t stage_off(int r, int c) {
+  return wq_off(r, c) - static_cast<uint32_t>((c >> 6) * (REC_HALF - TILE_BYTES / 2));
+}
 
 template <bool G_BF16, bool FAST_EXP>
 struct K1Smem {
@@ -93,9 +99,12 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
   return w;
 }
 
-// BESIDE: K2 runs beside this kernel (time-major items, finished items counted per window)
+// BESIDE: K2 runs beside this kernel (time-major items, finished items counted per window).  Registers: four CTAs per
+// SM need 128 a thread or fewer.  Beside K2, two CTAs share every SM sub-partition's 16,384 registers with up to three
+// warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
+// start before K1 ends (T8192 H96, whole forward: 1,254 us with 128 registers, 883 with 112).
 template <bool G_BF16, bool FAST_EXP, bool BESIDE>
-__global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ K1Params p) {
+__global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K1Smem<G_BF16, FAST_EXP>;
   constexpr int S_Q = SM::Q, S_K = SM::K, S_V = SM::V, S_G = SM::G;
@@ -351,46 +360,66 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
 
       const float2 centre = FAST_EXP ? glast : gmid;
       const float2 ncentre = make_float2(-centre.x, -centre.y);
+      // kg (and kn) go out transposed, eight tokens of a column per 16-byte store: pairs of rows are packed
+      uint32_t kgh[2][4], kgl[2][4], knh[2][4], knl[2][4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int r = r0 + i;
-        const uint32_t off = swz_off(r, c0);
-        const uint32_t qp = *reinterpret_cast<const uint32_t*>(smem + S_Q + (r * D + c0) * 2);
-        const uint32_t kp = *reinterpret_cast<const uint32_t*>(smem + S_K + (r * D + c0) * 2);
-        const uint32_t vp = *reinterpret_cast<const uint32_t*>(smem + S_V + (r * D + c0) * 2);
-        const float2 qn = make_float2(bf16_lo_to_f32(qp), bf16_hi_to_f32(qp));   // already normalised
-        const float2 kn = make_float2(bf16_lo_to_f32(kp), bf16_hi_to_f32(kp));
-        const float br = sBeta[r];
-        const float2 d = __fadd2_rn(gv[i], ncentre);                  // g - centre
-        const float2 e = make_float2(ex2f(d.x), ex2f(d.y));           // 2^(g - centre)
-        const float2 en = make_float2(ex2f(-d.x), ex2f(-d.y));        // 2^(centre - g)
-        float2 eg, ekg;                                               // 2^g, 2^(g_last - g)
-        if (FAST_EXP) { eg = __fmul2_rn(e, dec2); ekg = en; }
-        else {
-          eg = make_float2(ex2f(gv[i].x), ex2f(gv[i].y));
-          ekg = make_float2(ex2f(glast.x - gv[i].x), ex2f(glast.y - gv[i].y));
+      for (int i2 = 0; i2 < 4; ++i2) {
+        float2 kg2[2], kn2[2];
+#pragma unroll
+        for (int ii = 0; ii < 2; ++ii) {
+          const int i = i2 * 2 + ii, r = r0 + i;
+          const uint32_t off = swz_off(r, c0);
+          const uint32_t qp = *reinterpret_cast<const uint32_t*>(smem + S_Q + (r * D + c0) * 2);
+          const uint32_t kp = *reinterpret_cast<const uint32_t*>(smem + S_K + (r * D + c0) * 2);
+          const uint32_t vp = *reinterpret_cast<const uint32_t*>(smem + S_V + (r * D + c0) * 2);
+          const float2 qn = make_float2(bf16_lo_to_f32(qp), bf16_hi_to_f32(qp));   // already normalised
+          const float2 kn = make_float2(bf16_lo_to_f32(kp), bf16_hi_to_f32(kp));
+          const float br = sBeta[r];
+          const float2 d = __fadd2_rn(gv[i], ncentre);                  // g - centre
+          const float2 e = make_float2(ex2f(d.x), ex2f(d.y));           // 2^(g - centre)
+          const float2 en = make_float2(ex2f(-d.x), ex2f(-d.y));        // 2^(centre - g)
+          float2 eg, ekg;                                               // 2^g, 2^(g_last - g)
+          if (FAST_EXP) { eg = __fmul2_rn(e, dec2); ekg = en; }
+          else {
+            eg = make_float2(ex2f(gv[i].x), ex2f(gv[i].y));
+            ekg = make_float2(ex2f(glast.x - gv[i].x), ex2f(glast.y - gv[i].y));
+          }
+          uint32_t hi, lo;
+          split_pack2(__fmul2_rn(qn, e), hi, lo);
+          *reinterpret_cast<uint32_t*>(smem + S_QGH + off) = hi;
+          *reinterpret_cast<uint32_t*>(smem + S_QGL + off) = lo;
+          split_pack2(__fmul2_rn(kn, e), hi, lo);
+          *reinterpret_cast<uint32_t*>(smem + S_KQH + off) = hi;
+          *reinterpret_cast<uint32_t*>(smem + S_KQL + off) = lo;
+          if (!FAST_EXP) kn2[ii] = __fmul2_rn(kn, en);
+          kg2[ii] = __fmul2_rn(kn, ekg);
+          const float2 qgo = __fmul2_rn(qn, eg);
+          *reinterpret_cast<uint32_t*>(smem + S_QG + stage_off(r, c0)) = pack_bf16(qgo.x, qgo.y);
+          const float2 kbv = __fmul2_rn(__fmul2_rn(kn, make_float2(br, br)), eg);
+          kbh[i] = pack_bf16(kbv.x, kbv.y);
+          split_pack2(__fmul2_rn(make_float2(bf16_lo_to_f32(vp), bf16_hi_to_f32(vp)), make_float2(br, br)), vbh[i], vbl[i]);
         }
-        uint32_t hi, lo;
-        split_pack2(__fmul2_rn(qn, e), hi, lo);
-        *reinterpret_cast<uint32_t*>(smem + S_QGH + off) = hi;
-        *reinterpret_cast<uint32_t*>(smem + S_QGL + off) = lo;
-        split_pack2(__fmul2_rn(kn, e), hi, lo);
-        *reinterpret_cast<uint32_t*>(smem + S_KQH + off) = hi;
-        *reinterpret_cast<uint32_t*>(smem + S_KQL + off) = lo;
+        split_pack(kg2[0].x, kg2[1].x, kgh[0][i2], kgl[0][i2]);
+        split_pack(kg2[0].y, kg2[1].y, kgh[1][i2], kgl[1][i2]);
         if (!FAST_EXP) {
-          split_pack2(__fmul2_rn(kn, en), hi, lo);
-          *reinterpret_cast<uint32_t*>(smem + S_KNH + off) = hi;
-          *reinterpret_cast<uint32_t*>(smem + S_KNL + off) = lo;
+          split_pack(kn2[0].x, kn2[1].x, knh[0][i2], knl[0][i2]);
+          split_pack(kn2[0].y, kn2[1].y, knh[1][i2], knl[1][i2]);
         }
-        split_pack2(__fmul2_rn(kn, ekg), hi, lo);
-        *reinterpret_cast<uint32_t*>(smem + S_KGH + off) = hi;
-        *reinterpret_cast<uint32_t*>(smem + S_KGL + off) = lo;
-        const float2 qgo = __fmul2_rn(qn, eg);
-        *reinterpret_cast<uint32_t*>(smem + S_QG + off) = pack_bf16(qgo.x, qgo.y);
-        const float2 kbv = __fmul2_rn(__fmul2_rn(kn, make_float2(br, br)), eg);
-        kbh[i] = pack_bf16(kbv.x, kbv.y);
-        split_pack2(__fmul2_rn(make_float2(bf16_lo_to_f32(vp), bf16_hi_to_f32(vp)), make_float2(br, br)), vbh[i], vbl[i]);
       }
+      // a lane's two columns are neighbours: half of the lanes store the odd one first, so that the eight lanes of a
+      // shared-memory pass cover 128 different bytes
+      const bool odd_first = (lane & 4) != 0;
+      auto put = [&](int base, const uint32_t (&t)[2][4]) {
+        uint32_t x[4], y[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) { x[w] = odd_first ? t[1][w] : t[0][w]; y[w] = odd_first ? t[0][w] : t[1][w]; }
+        const uint32_t off = base + kg_off(r0, c0);
+        *reinterpret_cast<uint4*>(smem + off + (odd_first ? 16 : 0)) = make_uint4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<uint4*>(smem + off + (odd_first ? 0 : 16)) = make_uint4(y[0], y[1], y[2], y[3]);
+      };
+      put(S_KGH, kgh);
+      put(S_KGL, kgl);
+      if (!FAST_EXP) { put(S_KNH, knh); put(S_KNL, knl); }
     }
     __syncthreads();  // every thread has read its q/k/v/g elements: the input tiles are free
 
@@ -405,23 +434,28 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
       const int mt = warp >> 1;  // 0: Aqk, 1: Akk
       const int nt = warp & 1;   // column block j in [8nt, 8nt+8)
       const int arow = (lane & 7) + ((lane >> 3) & 1) * 8, acol = (lane >> 4) * 8;
-      const int brow = nt * 8 + (lane & 7), bcol = ((lane >> 3) & 1) * 8;
       // swizzled address of k-step ks = (256-byte aligned tile base + lane part) ^ (ks << 5)
       const uint32_t a_hi = sbase + (mt == 0 ? S_QGH : S_KQH) + swz_off(arow, acol);
-      const uint32_t b_hi = sbase + (FAST_EXP ? S_KGH : S_KNH) + swz_off(brow, bcol);
+      // B operand out of the transposed tile (rows k, columns tok): k-step ks is 256 bytes further
+      const uint32_t b_hi = sbase + (FAST_EXP ? S_KGH : S_KNH) + kg_off(nt * 8, lane);
       constexpr uint32_t A_LO = S_QGL - S_QGH, B_LO = FAST_EXP ? S_KGL - S_KGH : S_KNL - S_KNH;
       static_assert(S_KQL - S_KQH == S_QGL - S_QGH && S_GRAM % 256 == 0, "tile layout");
       float acc0[4] = {0, 0, 0, 0}, acc1[4] = {0, 0, 0, 0}, acc2[4] = {0, 0, 0, 0};
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        uint32_t ah[4], al[4], bh0, bh1, bl0, bl1;
-        ldsm_x4(a_hi ^ (ks << 5), ah[0], ah[1], ah[2], ah[3]);
-        ldsm_x4((a_hi ^ (ks << 5)) + A_LO, al[0], al[1], al[2], al[3]);
-        ldsm_x2(b_hi ^ (ks << 5), bh0, bh1);
-        ldsm_x2((b_hi ^ (ks << 5)) + B_LO, bl0, bl1);
-        mma_bf16(acc0, ah, bh0, bh1);
-        mma_bf16(acc1, ah, bl0, bl1);
-        mma_bf16(acc2, al, bh0, bh1);
+      for (int kp = 0; kp < 4; ++kp) {
+        uint32_t bh[4], bl[4];   // two k-steps
+        ldsm_x4_t(b_hi + kp * 512, bh[0], bh[1], bh[2], bh[3]);
+        ldsm_x4_t(b_hi + kp * 512 + B_LO, bl[0], bl[1], bl[2], bl[3]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int ks = kp * 2 + j;
+          uint32_t ah[4], al[4];
+          ldsm_x4(a_hi ^ (ks << 5), ah[0], ah[1], ah[2], ah[3]);
+          ldsm_x4((a_hi ^ (ks << 5)) + A_LO, al[0], al[1], al[2], al[3]);
+          mma_bf16(acc0, ah, bh[2 * j], bh[2 * j + 1]);
+          mma_bf16(acc1, ah, bl[2 * j], bl[2 * j + 1]);
+          mma_bf16(acc2, al, bh[2 * j], bh[2 * j + 1]);
+        }
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc0[e] += acc1[e] + acc2[e];
@@ -434,8 +468,8 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
           const float v1 = (i >= j0 + 1) ? acc0[hrow * 2 + 1] * p.scale : 0.f;
           uint32_t hi2, lo2;
           split_pack(v0, v1, hi2, lo2);
-          *reinterpret_cast<uint32_t*>(smem + S_AQK + (i * 16 + j0) * 2) = hi2;
-          *reinterpret_cast<uint32_t*>(smem + S_AQL + (i * 16 + j0) * 2) = lo2;
+          *reinterpret_cast<uint32_t*>(smem + S_AQK + aq_off(i, j0)) = hi2;
+          *reinterpret_cast<uint32_t*>(smem + S_AQL + aq_off(i, j0)) = lo2;
         }
       } else {
 #pragma unroll
@@ -507,8 +541,9 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
 
     // the finished tiles leave while phase E runs
     if (tid == 0) {
-      bulk_s2g(rec + REC_QG, sbase + S_QG, REC_AQK - REC_QG);
-      bulk_s2g(rec + REC_AQK, sbase + S_AQK, REC_U - REC_AQK);
+      bulk_s2g(rec + REC_QG, sbase + S_QG, TILE_BYTES / 2);
+      bulk_s2g(rec + REC_QG + REC_HALF, sbase + S_QG + TILE_BYTES / 2, TILE_BYTES / 2);
+      bulk_s2g(rec + REC_KGH, sbase + S_KGH, REC_U - REC_KGH);
       bulk_commit();
     }
 
@@ -547,8 +582,8 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
           mma_bf16(accw, xah, bk[2 * j], bk[2 * j + 1]);
           mma_bf16(accw, xal, bk[2 * j], bk[2 * j + 1]);
           const int kc = n0 + j * 8 + tq * 2;
-          *reinterpret_cast<uint32_t*>(smem + S_WST + swz_off(gq, kc)) = pack_bf16(accw[0], accw[1]);
-          *reinterpret_cast<uint32_t*>(smem + S_WST + swz_off(gq + 8, kc)) = pack_bf16(accw[2], accw[3]);
+          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq, kc)) = pack_bf16(accw[0], accw[1]);
+          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq + 8, kc)) = pack_bf16(accw[2], accw[3]);
         }
       }
     }
@@ -566,7 +601,8 @@ __global__ void __launch_bounds__(128, 4) kda_k1_kernel(const __grid_constant__ 
     }
     __syncthreads();   // also orders phase E's reads of X / KB / VB before the next item rewrites them
     if (tid == 0) {
-      bulk_s2g(rec + REC_W, sbase + S_WST, TILE_BYTES);
+      bulk_s2g(rec + REC_W, sbase + S_WST, TILE_BYTES / 2);
+      bulk_s2g(rec + REC_W + REC_HALF, sbase + S_WST + TILE_BYTES / 2, TILE_BYTES / 2);
       bulk_commit();
     }
     cur = nxt;

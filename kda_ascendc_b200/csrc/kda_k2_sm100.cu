@@ -183,16 +183,15 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         for (int nv = 0; nv < NVT; ++nv) hT[m][nv][0] = hT[m][nv][1] = hT[m][nv][2] = hT[m][nv][3] = 0.f;
     }
 
-    // per-lane ldmatrix address components (constant across steps)
-    const int a1_row = (lane & 7) + ((lane >> 3) & 1) * 8, a1_col = (lane >> 4) * 8;   // [w;qg]: rows tok, cols k
-    const int a2_row = (lane & 7) + (lane >> 4) * 8, a2_col = ((lane >> 3) & 1) * 8;   // kg^T via .trans
-    const uint32_t a3_off = REC_AQK + (a1_row * 16 + a1_col) * 2;                      // Aqk: rows i, cols j
-    // Swizzled tile address of k-step ks = (256-byte aligned tile base + lane part) ^ (ks << 5): the
-    // k-step only moves bits 5..7 of the address, which the tile base leaves clear (stages and tile
-    // offsets are multiples of 256 bytes), so one XOR with an immediate replaces the index arithmetic.
-    static_assert(SM::STAGE % 256 == 0 && REC_W % 256 == 0 && REC_QG % 256 == 0 && REC_KGH % 256 == 0 && REC_KGL % 256 == 0,
-                  "tile bases must keep address bits 5..7 clear");
-    const uint32_t a1_lane = swz_off(a1_row, a1_col), a2_lane = swz_off(a2_row, a2_col);
+    // per-lane ldmatrix address components (constant across steps): mi = the 8x8 matrix of an x4 load, r8 = its row.
+    // Within a half of w / qg the k-step only moves bits 5 and 6 of the address, which the tile bases leave clear.
+    static_assert(SM::STAGE % 128 == 0 && REC_W % 128 == 0 && REC_QG % 128 == 0 && REC_HALF % 128 == 0,
+                  "tile bases must keep address bits 5 and 6 clear");
+    const int mi = lane >> 3, r8 = lane & 7;
+    const uint32_t a1_lane = wq_off(r8 + (mi & 1) * 8, (mi >> 1) * 8);                 // [w;qg]: rows tok, cols k
+    const uint32_t a2_lane = kg_off((mi >> 1) * 8, (mi & 1) * 8 + r8);                 // kg^T: rows k, cols tok
+    const uint32_t a3_off = REC_AQK + aq_off(r8 + (mi & 1) * 8, (mi >> 1) * 8);        // Aqk: rows i, cols j
+    auto wq_at = [](uint32_t base, int ks) { return (base ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF; };
     const uint32_t u_off = REC_SHARED_BYTES + warp * (RT * REC_U_TILE_BYTES) + lane * 16;
     __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + v0 + tq * 2;
     const bool use_u = PAIR || (pair_rt ? plane == 1 : !(STATE_ONLY && p.zero_u));
@@ -212,9 +211,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     } else {
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        ldsm_x4(((sbase + a1_lane) ^ (ks << 5)) + REC_W, aw[ks][0], aw[ks][1], aw[ks][2], aw[ks][3]);
+        ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_W, aw[ks][0], aw[ks][1], aw[ks][2], aw[ks][3]);
         if (!STATE_ONLY)
-          ldsm_x4(((sbase + a1_lane) ^ (ks << 5)) + REC_QG, aq[ks][0], aq[ks][1], aq[ks][2], aq[ks][3]);
+          ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_QG, aq[ks][0], aq[ks][1], aq[ks][2], aq[ks][3]);
         dk[ks][0] = *reinterpret_cast<const float*>(smem + REC_DEC + (ks * 16 + gq) * 4);
         dk[ks][1] = *reinterpret_cast<const float*>(smem + REC_DEC + (ks * 16 + gq + 8) * 4);
       }
@@ -260,7 +259,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
           if (ks < 2) mma_bf16_z(pw[ks & 1][nv], aw[ks], bh[ks][nv][0], bh[ks][nv][1]);
           else mma_bf16_v(pw[ks & 1][nv], aw[ks], bh[ks][nv][0], bh[ks][nv][1]);
         }
-        ldsm_x4_t((t2 ^ (ks << 5)) + REC_KGH, kgh[ks][0], kgh[ks][1], kgh[ks][2], kgh[ks][3]);
+        ldsm_x4(t2 + ks * 256 + REC_KGH, kgh[ks][0], kgh[ks][1], kgh[ks][2], kgh[ks][3]);
         if (!STATE_ONLY) {
 #pragma unroll
           for (int nv = 0; nv < NVT; ++nv) {
@@ -268,7 +267,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
             else mma_bf16_v(pq[ks & 1][nv], aq[ks], bh[ks][nv][0], bh[ks][nv][1]);
           }
         }
-        ldsm_x4_t((t2 ^ (ks << 5)) + REC_KGL, kgl[ks][0], kgl[ks][1], kgl[ks][2], kgl[ks][3]);
+        ldsm_x4(t2 + ks * 256 + REC_KGL, kgl[ks][0], kgl[ks][1], kgl[ks][2], kgl[ks][3]);
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) {
           const float2 lo = __fmul2_rn(make_float2(hT[ks][nv][0], hT[ks][nv][1]), make_float2(dk[ks][0], dk[ks][0]));
@@ -324,7 +323,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvh[nv][0], bvh[nv][1]);
-        if (more) ldsm_x4((t1n ^ (m << 5)) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
+        if (more) ldsm_x4(wq_at(t1n, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
@@ -340,7 +339,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgl[m], bvh[nv][0], bvh[nv][1]);
         if (!STATE_ONLY && more)
-          ldsm_x4((t1n ^ (m << 5)) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
+          ldsm_x4(wq_at(t1n, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
       }
 
       // P3: o = scale * (qg hT) + Aqk v_new

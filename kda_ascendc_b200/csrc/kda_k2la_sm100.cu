@@ -151,15 +151,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
       for (int m = 0; m < 8; ++m) hT[m][0] = hT[m][1] = hT[m][2] = hT[m][3] = 0.f;
     }
 
-    // per-lane ldmatrix address components (constant across steps).  A swizzled tile address of
-    // k-step ks is (256-byte aligned tile base + lane part) ^ (ks << 5): the k-step only moves bits
-    // 5..7, which the tile bases leave clear.
-    static_assert(SM::STAGE % 256 == 0 && REC_W % 256 == 0 && REC_QG % 256 == 0 && REC_KGH % 256 == 0 && REC_KGL % 256 == 0,
-                  "tile bases must keep address bits 5..7 clear");
-    const int a1_row = (lane & 7) + ((lane >> 3) & 1) * 8, a1_col = (lane >> 4) * 8;   // [w;qg]: rows tok, cols k
-    const int a2_row = (lane & 7) + (lane >> 4) * 8, a2_col = ((lane >> 3) & 1) * 8;   // kg^T via .trans
-    const uint32_t a1_lane = swz_off(a1_row, a1_col), a2_lane = swz_off(a2_row, a2_col);
-    const uint32_t a3_off = (a1_row * 16 + a1_col) * 2;                                // 16x16 tiles: rows i, cols j
+    // per-lane ldmatrix address components (constant across steps): mi = the 8x8 matrix of an x4 load, r8 = its row.
+    // Within a half of w / qg the k-step only moves bits 5 and 6 of the address, which the tile bases leave clear.
+    static_assert(SM::STAGE % 128 == 0 && REC_W % 128 == 0 && REC_QG % 128 == 0 && REC_HALF % 128 == 0,
+                  "tile bases must keep address bits 5 and 6 clear");
+    const int mi = lane >> 3, r8 = lane & 7;
+    const int a1_row = r8 + (mi & 1) * 8, a1_col = (mi >> 1) * 8;                      // [w;qg]: rows tok, cols k
+    const uint32_t a1_lane = wq_off(a1_row, a1_col);
+    const uint32_t a2_lane = kg_off((mi >> 1) * 8, (mi & 1) * 8 + r8);                 // kg^T: rows k, cols tok
+    const uint32_t aq_lane = aq_off(a1_row, a1_col);                                   // Aqk: rows i, cols j
+    const uint32_t a3_off = (a1_row * 16 + a1_col) * 2;                                // exchange tiles: rows i, cols j
+    auto wq_at = [](uint32_t base, int ks) { return (base ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF; };
     const uint32_t u_off = REC_SHARED_BYTES + warp * REC_U_TILE_BYTES + lane * 16;
     // this warp's cross-Gram tiles: tile t -> part (0 = w -> C, 1 = qg -> A'), half of the 16 kg rows
     const int tile0 = warp * TPW;
@@ -169,7 +171,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
     for (int t = 0; t < TPW; ++t) {
       const int tile = (tile0 + t) % NTILES, part = tile >> 1, half = tile & 1;
       g_aoff[t] = part ? REC_QG : REC_W;
-      g_blane[t] = swz_off(8 * half + (lane & 7), ((lane >> 3) & 1) * 8) + REC_KGH;
+      g_blane[t] = kg_off(8 * half, lane & 15) + REC_KGH;   // through .trans: rows k, cols tok
       g_xoff[t] = SM::XG + part * 512 + (gq * 16 + 8 * half + 2 * tq) * 2;
     }
     __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + v0 + tq * 2;
@@ -193,8 +195,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           uint32_t a[4], b0, b1;
-          ldsm_x4(((spa + a1_lane) ^ (ks << 5)) + g_aoff[t], a[0], a[1], a[2], a[3]);
-          ldsm_x2(((spb + g_blane[t]) ^ (ks << 5)), b0, b1);
+          ldsm_x4(wq_at(spa + a1_lane, ks) + g_aoff[t], a[0], a[1], a[2], a[3]);
+          ldsm_x2_t(spb + g_blane[t] + ks * 256, b0, b1);
           if (ks < 2) mma_bf16_z(acc[ks & 1], a, b0, b1);
           else mma_bf16_v(acc[ks & 1], a, b0, b1);
         }
@@ -218,10 +220,10 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
         for (int ks = 0; ks < 8; ++ks) {
           uint32_t a[4];
           const uint32_t b0 = movmatrix_t(pack_bf16(hT[ks][0], hT[ks][1])), b1 = movmatrix_t(pack_bf16(hT[ks][2], hT[ks][3]));
-          ldsm_x4(((sbase + a1_lane) ^ (ks << 5)) + REC_W, a[0], a[1], a[2], a[3]);
+          ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_W, a[0], a[1], a[2], a[3]);
           mma_bf16_v(pw[ks & 1], a, b0, b1);
           if (!STATE_ONLY) {
-            ldsm_x4(((sbase + a1_lane) ^ (ks << 5)) + REC_QG, a[0], a[1], a[2], a[3]);
+            ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_QG, a[0], a[1], a[2], a[3]);
             mma_bf16_v(pq2[ks & 1], a, b0, b1);
           }
         }
@@ -275,16 +277,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
 #pragma unroll
         for (int m = m0; m < m0 + 2; ++m) {
           if (MORE) {
-            ldsm_x4((t1a ^ (m << 5)) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
-            if (!STATE_ONLY) ldsm_x4((t1a ^ (m << 5)) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
+            ldsm_x4(wq_at(t1a, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
+            if (!STATE_ONLY) ldsm_x4(wq_at(t1a, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
           }
-          ldsm_x4_t((t0k ^ (m << 5)) + REC_KGH, kgh[m][0], kgh[m][1], kgh[m][2], kgh[m][3]);
-          ldsm_x4_t((t0k ^ (m << 5)) + REC_KGL, kgl[m][0], kgl[m][1], kgl[m][2], kgl[m][3]);
+          ldsm_x4(t0k + REC_KGH + m * 256, kgh[m][0], kgh[m][1], kgh[m][2], kgh[m][3]);
+          ldsm_x4(t0k + REC_KGL + m * 256, kgl[m][0], kgl[m][1], kgl[m][2], kgl[m][3]);
           if (MORE2 && has_tile) {
 #pragma unroll
             for (int t = 0; t < TPW; ++t) {
-              ldsm_x4((t2a ^ (m << 5)) + g_aoff[t], ga[t][m][0], ga[t][m][1], ga[t][m][2], ga[t][m][3]);
-              ldsm_x2(((sp1 + g_blane[t]) ^ (m << 5)), gb[t][m][0], gb[t][m][1]);
+              ldsm_x4(wq_at(t2a, m) + g_aoff[t], ga[t][m][0], ga[t][m][1], ga[t][m][2], ga[t][m][3]);
+              ldsm_x2_t(sp1 + g_blane[t] + m * 256, gb[t][m][0], gb[t][m][1]);
             }
           }
         }
@@ -296,8 +298,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
       float4 un = make_float4(0, 0, 0, 0);
       uint32_t ah3[4], al3[4], cfw[4], cfq[4];
       if (!STATE_ONLY) {
-        ldsm_x4(sp0 + REC_AQK + a3_off, ah3[0], ah3[1], ah3[2], ah3[3]);
-        ldsm_x4(sp0 + REC_AQL + a3_off, al3[0], al3[1], al3[2], al3[3]);
+        ldsm_x4(sp0 + REC_AQK + aq_lane, ah3[0], ah3[1], ah3[2], ah3[3]);
+        ldsm_x4(sp0 + REC_AQL + aq_lane, al3[0], al3[1], al3[2], al3[3]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) oa[e] = p.scale * pq[e];
       }

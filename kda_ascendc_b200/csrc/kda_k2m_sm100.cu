@@ -142,11 +142,11 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     }
 
     // per-lane ldmatrix address components (constant across steps)
-    const int b1_row = (lane & 7) + (lane >> 4) * 8, b1_col = ((lane >> 3) & 1) * 8;   // w, qg: [N=tok][K=k]
-    const int b2_row = (lane & 7) + ((lane >> 3) & 1) * 8, b2_col = (lane >> 4) * 8;   // kg: [K=tok][N=k], .trans
-    // swizzled address of k-step ks = (256-byte aligned tile base + lane part) ^ (ks << 5)
-    const uint32_t b1_lane = swz_off(b1_row, b1_col), b2_lane = swz_off(b2_row, b2_col);
-    const uint32_t b3_off = REC_AQK + (((lane & 7) + (lane >> 4) * 8) * 16 + ((lane >> 3) & 1) * 8) * 2;
+    const int mi = lane >> 3, r8 = lane & 7;   // the 8x8 matrix of an x4 load, and its row, that this lane addresses
+    // w, qg: [N=tok][K=k]; within a half the k-step moves bits 5 and 6 of the address, which the tile bases leave clear
+    const uint32_t b1_lane = wq_off(r8 + (mi >> 1) * 8, (mi & 1) * 8);
+    const uint32_t b2_lane = kg_off((mi & 1) * 8, (mi >> 1) * 8 + r8);               // kg: [N=k][K=tok]
+    const uint32_t b3_off = REC_AQK + aq_off((mi >> 1) * 8 + r8, (mi & 1) * 8);      // Aqk: [N=i][K=j]
     // u^T fragment of this warp out of the record's [8-column tile][lane][4] blocks (see kda_common.cuh):
     // element (v = vrow0 + gq + 8a, tok = 2tq + j + 8c)  ->  tile 2*warp + a, lane (2tq+j)*4 + gq/2, slot 2c + gq%2
     const uint32_t u_off = REC_SHARED_BYTES + (warp * 2) * REC_U_TILE_BYTES + ((tq * 2) * 4 + (gq >> 1)) * 16 + (gq & 1) * 4;
@@ -174,9 +174,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       for (int nt = nt0; nt < nt1; ++nt) dec[nt] = *reinterpret_cast<const float2*>(spg + REC_DEC + (nt * 8 + tq * 2) * 4);
     };
     auto load_b1 = [&](uint32_t sp, int ks, int slot) {
-      ldsm_x4(((sp + b1_lane) ^ (ks << 5)) + REC_W, bw[slot][0], bw[slot][1], bw[slot][2], bw[slot][3]);
-      if (!STATE_ONLY)
-        ldsm_x4(((sp + b1_lane) ^ (ks << 5)) + REC_QG, bq[slot][0], bq[slot][1], bq[slot][2], bq[slot][3]);
+      const uint32_t at = ((sp + b1_lane) ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF;
+      ldsm_x4(at + REC_W, bw[slot][0], bw[slot][1], bw[slot][2], bw[slot][3]);
+      if (!STATE_ONLY) ldsm_x4(at + REC_QG, bq[slot][0], bq[slot][1], bq[slot][2], bq[slot][3]);
     };
 
     bool failed = false;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
           mma_bf16_v(pq[1], ah, bq[sl][2], bq[sl][3]);
         }
         if (ks + 2 < 8) load_b1(sp, ks + 2, sl);
-        ldsm_x4_t(((sp + b2_lane) ^ (ks << 5)) + REC_KGH, kgh[ks][0], kgh[ks][1], kgh[ks][2], kgh[ks][3]);
+        ldsm_x4(sp + b2_lane + REC_KGH + ks * 256, kgh[ks][0], kgh[ks][1], kgh[ks][2], kgh[ks][3]);
         {
           const float2 d0 = dec[2 * ks], d1 = dec[2 * ks + 1];
 #pragma unroll
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       for (int np = 0; np < 8; ++np) {
         mma_bf16_v(hs[2 * np], avh, kgh[np][0], kgh[np][1]);
         mma_bf16_v(hs[2 * np + 1], avh, kgh[np][2], kgh[np][3]);
-        ldsm_x4_t(((sp + b2_lane) ^ (np << 5)) + REC_KGL, kgl[np][0], kgl[np][1], kgl[np][2], kgl[np][3]);
+        ldsm_x4(sp + b2_lane + REC_KGL + np * 256, kgl[np][0], kgl[np][1], kgl[np][2], kgl[np][3]);
       }
       uint32_t ba[4], bl[4];
       if (!STATE_ONLY) {

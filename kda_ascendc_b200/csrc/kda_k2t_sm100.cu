@@ -11,9 +11,8 @@
 //   P2  h[v][:]   += v_new^T[v][:] . kg                   3 x M128 N128 K16 (hi.hi, lo.hi, hi.lo)
 //   P3  D3[v][16]  = v_new^T[v][:] . Aqk^T                3 x M128 N16 K16
 //   E2  read h, write bf16(h) (next P1's A operand) and h * dec(next chunk); o = scale D1[:, 16:32] + D3
-// The record tiles become tensor-core operands without a second pass over them: a 5-D tiled TMA
-// map over the record array lands every [16 tok][128 k] tile as two 64-column atoms in the
-// canonical 128-byte-swizzled layout (the records are already XOR-swizzled per 128-byte half row).
+// The record's tiles are tensor-core operands as they stand (kda_common.cuh): one bulk copy per chunk, no second
+// pass over them.
 //
 // A commit -> mbarrier -> waiting-thread round trip costs ~430 cycles on this part and a step needs
 // two of them, so ONE chain per SM is slower than the mma.sync kernels (~2,200 against ~1,100
@@ -22,10 +21,9 @@
 //
 // Warp roles: 0-7 element-wise work (warp w: TMEM lanes 32 (w%4).., column / token half w/4),
 // 8 = producer (TMA), 9 = MMA issuer and TMEM owner.  Every wait is bounded.
-#include <cuda.h>
-
 #include "kda_common.cuh"
 #include "kda_kernels.h"
+#include "kda_tc.cuh"
 
 namespace kda {
 
@@ -34,14 +32,7 @@ namespace {
 constexpr int KT_STAGES = 3;
 constexpr int KT_EPI_WARPS = 8;
 constexpr int KT_THREADS = (KT_EPI_WARPS + 2) * 32;
-// stage layout (1024-byte aligned base: the swizzled atoms need it)
-constexpr int T_WQ = 0;        // [2 atoms][32 rows: w 0..15, qg 16..31][128 B]
-constexpr int T_KGH = 8192;    // [2 atoms][16 tok][128 B]
-constexpr int T_KGL = 12288;
-constexpr int T_U = 16384;     // fp32 u, fragment order (8192 B)
-constexpr int T_AQ = 24576;    // Aqk hi, Aqk lo, dec as in the record (1536 B)
-constexpr int T_AQF = 26112;   // Aqk hi / lo re-laid as 8x8 core matrices (2 x 512 B)
-constexpr int T_STAGE = 27648;
+constexpr int T_STAGE = (REC_BYTES + 1023) / 1024 * 1024;   // a record as it is (1024-byte aligned: the swizzled atoms need it)
 constexpr int T_BARS = KT_STAGES * T_STAGE;
 // The state snapshot reaches the MMA thread in KT_PG column groups, so that the first k-steps of the
 // next P1 are issued while the element-wise warps still convert the rest of the state.
@@ -58,122 +49,8 @@ constexpr uint32_t C_S = 0, C_D1 = 128, C_D3 = 160, C_AS = 176, C_VH = 240, C_VL
 
 constexpr int ST_K2T_TIMEOUT = 4;
 
-// ---- tcgen05 wrappers ------------------------------------------------------------------------
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem descriptor]
-__device__ __forceinline__ void umma_ts(uint32_t d, uint32_t a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d),
-      "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t a, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(a));
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t a, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(a));
-}
-// The registers of a tcgen05.ld are valid only after tcgen05.wait::ld; the compiler sees the wait
-// as an unrelated statement, so after it the registers are passed through an empty asm that pins
-// every later use behind the wait.
-__device__ __forceinline__ void pin8(uint32_t (&r)[8]) {
-  asm volatile("" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])::"memory");
-}
-__device__ __forceinline__ void pin16(uint32_t (&r)[16]) {
-  asm volatile(""
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
-                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
-}
-__device__ __forceinline__ void tmem_st4(uint32_t a, const uint32_t (&r)[4]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t a, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(a), "r"(r[0]), "r"(r[1]),
-               "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st16(uint32_t a, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(a),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-// 16-lane shapes: thread (g = lane / 4, t = lane % 4) of the warp holds, per repeat n, the fp32 pairs
-// (row g, columns 8n + 2t, 8n + 2t + 1) and (row g + 8, same columns) -- the mma.sync accumulator layout,
-// whose rows are 32-byte pieces of memory rows: the state moves between global memory and TMEM with
-// fully used sectors.  The 128-bit shape is the same with one 32-bit column per thread and repeat.
-__device__ __forceinline__ void tmem_st_16x256b_x8(uint32_t a, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x256b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(a),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
-      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
-      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t a, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(a));
-}
-__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t a, const uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(a),
-      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_5d(uint32_t dst_smem, const void* tmap, int c0, int c1, int c2, int c3, int c4,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::
-          "r"(dst_smem), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
-      : "memory");
-}
-
-// shared-memory matrix descriptor (sm_100 format): start address, leading / stride byte offsets in
-// 16-byte units, descriptor version 1, layout type (0 = no swizzle, 2 = 128-byte swizzle)
-__host__ __device__ constexpr uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes, uint32_t layout) {
-  return static_cast<uint64_t>((saddr >> 4) & 0x3FFF) | (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFF) << 16) |
-         (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFF) << 32) | (static_cast<uint64_t>(1) << 46) |
-         (static_cast<uint64_t>(layout) << 61);
-}
-// instruction descriptor: fp32 accumulate, bf16 x bf16, A K-major, B K-major (0) or MN-major (1)
-__host__ __device__ constexpr uint32_t instr_desc(int M, int N, int b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(b_mn_major) << 16) |
-         (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
-}
-
-struct K2tParams {
-  K2Params k;
-  CUtensorMap tm_rec;   // 5-D view of the record array: (64 bf16, 2 halves, 16 rows, 4 tiles, records)
-};
-
-__global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_constant__ K2tParams pp) {
+__global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_constant__ K2Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const K2Params& p = pp.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // warp-uniform for the compiler
   int bh = blockIdx.x + p.chain0;
   if (p.by_length) bh = chain_by_length(p.seq_table, p.n_seqs, p.H, bh);
@@ -210,11 +87,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     *sIssued = 0;
     fence_mbar_init();
   }
-  if (warp == KT_EPI_WARPS + 1) {   // the MMA warp owns the tensor memory of the CTA
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(C_TOTAL)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
+  if (warp == KT_EPI_WARPS + 1) tmem_alloc(smem_u32(slot), C_TOTAL);   // the MMA warp owns the tensor memory of the CTA
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -239,78 +112,75 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
           gate += p.win_chunks;
         }
         if (n >= KT_STAGES && !mbar_wait_bounded(empty(s), ((n / KT_STAGES) - 1) & 1, sAbort)) { give_up(); break; }
-        const int rec_i = static_cast<int>(rec_first) + n;
-        const uint8_t* rec = p.rec + (rec_first + n) * REC_BYTES;
-        const uint32_t dst = sbase + s * T_STAGE;
-        mbar_arrive_expect_tx(full(s), 4 * TILE_BYTES + (REC_U - REC_AQK) + (REC_BYTES - REC_U));
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tma_load_5d(dst + T_WQ + half * 4096, &pp.tm_rec, 0, half, 0, 0, rec_i, full(s));          // w
-          tma_load_5d(dst + T_WQ + half * 4096 + 2048, &pp.tm_rec, 0, half, 0, 1, rec_i, full(s));   // qg
-          tma_load_5d(dst + T_KGH + half * 2048, &pp.tm_rec, 0, half, 0, 2, rec_i, full(s));         // kg hi
-          tma_load_5d(dst + T_KGL + half * 2048, &pp.tm_rec, 0, half, 0, 3, rec_i, full(s));         // kg lo
-        }
-        bulk_g2s(dst + T_AQ, rec + REC_AQK, REC_U - REC_AQK, full(s));
-        bulk_g2s(dst + T_U, rec + REC_U, REC_BYTES - REC_U, full(s));
+        mbar_arrive_expect_tx(full(s), REC_BYTES);
+        bulk_g2s(sbase + s * T_STAGE, p.rec + (rec_first + n) * REC_BYTES, REC_BYTES, full(s));
         *sIssued = n + 1;
       }
     }
     __syncwarp();
   } else if (warp == KT_EPI_WARPS + 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (elect_one()) {
-      constexpr uint32_t ID_P1 = instr_desc(128, 32, 0), ID_P2 = instr_desc(128, 128, 1), ID_P3 = instr_desc(128, 16, 0);
-      int s = 0;
-      for (int n = 0; n < NT; ++n, s = (s + 1 == KT_STAGES) ? 0 : s + 1) {
-        const uint32_t st = sbase + s * T_STAGE;
-        if (!mbar_wait_bounded(full(s), (n / KT_STAGES) & 1, sAbort)) { give_up(); break; }
-        const uint64_t dwq = smem_desc(st + T_WQ, 16, 1024, 2);   // k-step ks: start address + atom * 4096 + (ks % 4) * 32 bytes
-        bool ready = true;
+    // The whole warp walks the loop, so that the descriptors stay in uniform registers; one lane issues.
+    constexpr uint32_t ID_P1 = instr_desc(128, 32), ID_P2 = instr_desc(128, 128), ID_P3 = instr_desc(128, 16);
+    auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, sAbort)) != 0; };
+    int s = 0;
+    uint32_t ph = 0;
+    for (int n = 0; n < NT; ++n) {
+      const uint32_t st = sbase + s * T_STAGE;
+      if (!wait(full(s), ph)) { give_up(); break; }
+      const uint64_t dwq = smem_desc(st + REC_W, 16, 1024, 2);   // k-step ks: start address + (ks / 4) * 4096 + (ks % 4) * 32 bytes
+      bool ready = true;
 #pragma unroll
-        for (int q = 0; q < KT_PG; ++q) {
-          // column group q of both halves of bf16(h) is in TMEM (with the last group: the decayed h too)
-          if (!mbar_wait_bounded(bar_s(q), n & 1, sAbort)) { ready = false; break; }
+      for (int q = 0; q < KT_PG; ++q) {
+        // column group q of both halves of bf16(h) is in TMEM (with the last group: the decayed h too)
+        if (ready && !wait(bar_s(q), n & 1)) ready = false;
+        if (ready) {
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int cc = q * (4 / KT_PG); cc < (q + 1) * (4 / KT_PG); ++cc)
+            for (int cc = q * (4 / KT_PG); cc < (q + 1) * (4 / KT_PG); ++cc)
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              const int ks = hf * 4 + cc;
-              umma_ts(tbase + C_D1, tbase + C_AS + ks * 8, dwq + static_cast<uint64_t>((hf * 4096 + cc * 32) >> 4), ID_P1,
-                      !(cc == 0 && hf == 0));
-            }
+              for (int hf = 0; hf < 2; ++hf) {
+                const int ks = hf * 4 + cc;
+                umma_ts(tbase + C_D1, tbase + C_AS + ks * 8, dwq + static_cast<uint64_t>((hf * REC_HALF + cc * 32) >> 4), ID_P1,
+                        !(cc == 0 && hf == 0));
+              }
+            if (q == KT_PG - 1) umma_commit(bar_p1);
+          }
+          __syncwarp();
         }
-        if (!ready) { give_up(); break; }
-        umma_commit(bar_p1);
-        if (!mbar_wait_bounded(bar_v, n & 1, sAbort)) { give_up(); break; }     // v_new hi/lo are in TMEM
-        tc_fence_after();
-        const uint64_t dkh = smem_desc(st + T_KGH, 2048, 1024, 2), dkl = smem_desc(st + T_KGL, 2048, 1024, 2);
+      }
+      if (!ready || !wait(bar_v, n & 1)) { give_up(); break; }     // v_new hi/lo are in TMEM
+      tc_fence_after();
+      if (elect_one()) {
+        const uint64_t dkh = smem_desc(st + REC_KGH, 2048, 128, 0), dkl = smem_desc(st + REC_KGL, 2048, 128, 0);
         umma_ts(tbase + C_S, tbase + C_VH, dkh, ID_P2, 1);
         umma_ts(tbase + C_S, tbase + C_VL, dkh, ID_P2, 1);
         umma_ts(tbase + C_S, tbase + C_VH, dkl, ID_P2, 1);
         umma_commit(bar_p2);   // the state pass of the element-wise warps starts while P3 runs
-        const uint64_t dah = smem_desc(st + T_AQF, 128, 256, 0), dal = smem_desc(st + T_AQF + 512, 128, 256, 0);
+        const uint64_t dah = smem_desc(st + REC_AQK, 512, 128, 0), dal = smem_desc(st + REC_AQL, 512, 128, 0);
         umma_ts(tbase + C_D3, tbase + C_VH, dah, ID_P3, 0);
         umma_ts(tbase + C_D3, tbase + C_VL, dah, ID_P3, 1);
         umma_ts(tbase + C_D3, tbase + C_VH, dal, ID_P3, 1);
         umma_commit(bar_p3);
       }
+      __syncwarp();
+      if (++s == KT_STAGES) { s = 0; ph ^= 1; }
     }
-    __syncwarp();
   } else {
     // ------------------------------ element-wise warps ----------------------
     const int quad = warp & 3, half = warp >> 2;
     const int v = quad * 32 + lane;                       // state row = TMEM lane
     const uint32_t tl = tbase + (static_cast<uint32_t>(quad * 32) << 16);
     // u[tok = 8 half + j][v] in the record's fragment order
-    const uint32_t u_off = T_U + (v >> 3) * 512 + ((v & 7) >> 1) * 16 + (half * 2 + (v & 1)) * 4;
+    const uint32_t u_off = REC_U + (v >> 3) * 512 + ((v & 7) >> 1) * 16 + (half * 2 + (v & 1)) * 4;
     bool ok = true;
 
     // initial state: TMEM <- h0 * dec(chunk 0); bf16(h0) as the first A operand
     ok = mbar_wait_bounded(full(0), 0, sAbort);
     if (ok) {
       // this warp's 32 rows x 64 columns in two 16-row halves, through the 16-lane access shapes
-      const float* dec0 = reinterpret_cast<const float*>(smem + T_AQ + (REC_DEC - REC_AQK)) + half * 64;
+      const float* dec0 = reinterpret_cast<const float*>(smem + REC_DEC) + half * 64;
       const int g4 = lane >> 2, t4 = lane & 3;
 #pragma unroll 1
       for (int hh = 0; hh < 2; ++hh) {
@@ -357,20 +227,11 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     uint32_t aq[8];
     __nv_bfloat16* const orow = p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2];
 
-    // State-independent operands of chunk n1: this thread's eight u values and, by warp 0, Aqk hi / lo
-    // re-laid as 8x8 core matrices (the B operand of P3).  Runs while the tensor core works.
+    // State-independent operands of chunk n1: this thread's eight u values.  Runs while the tensor core works.
     auto prepare = [&](int n1) -> bool {
       const int s1 = n1 % KT_STAGES;
       if (!mbar_wait_bounded(full(s1), (n1 / KT_STAGES) & 1, sAbort)) return false;
       const uint8_t* stg = smem + s1 * T_STAGE;
-      if (warp == 0) {
-        const int mat = lane >> 4, i = lane & 15;
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-          *reinterpret_cast<uint4*>(smem + s1 * T_STAGE + T_AQF + mat * 512 + (i >> 3) * 256 + c * 128 + (i & 7) * 16) =
-              *reinterpret_cast<const uint4*>(stg + T_AQ + mat * 512 + i * 32 + c * 16);
-        fence_proxy_async();
-      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) uv[j] = *reinterpret_cast<const float*>(stg + u_off + j * 64);
       return true;
@@ -428,7 +289,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
       if (!mbar_wait_bounded(bar_p2, n & 1, sAbort)) { ok = false; break; }
       tc_fence_after();
       // dec of the next chunk (its stage was waited for in prepare)
-      const float* decn = reinterpret_cast<const float*>(smem + ((n + 1) % KT_STAGES) * T_STAGE + T_AQ + (REC_DEC - REC_AQK)) + half * 64;
+      const float* decn = reinterpret_cast<const float*>(smem + ((n + 1) % KT_STAGES) * T_STAGE + REC_DEC) + half * 64;
       // the TMEM loads of the state are issued one 16-column step ahead of their use
       uint32_t sr[2][16];
       tmem_ld16(tl + C_S + half * 64, sr[0]);
@@ -522,42 +383,13 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   }
   __syncthreads();
   if (warp == KT_EPI_WARPS + 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(C_TOTAL) : "memory");
+    tmem_dealloc(tbase, C_TOTAL);
   if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
 }
 
 }  // namespace
 
-// n_records: chunk records in the workspace (the tensor map must cover every record the grid reads)
-cudaError_t launch_k2t(const K2Params& p, long long n_records, cudaStream_t stream) {
-  EncodeTiledFn enc = encode_fn();
-  if (enc == nullptr) return cudaErrorNotSupported;
-  K2tParams pp;
-  pp.k = p;
-  // (64 bf16 = one 128-byte half row, 2 halves, 16 rows, 4 tiles, records); strides in bytes for dims 1..4
-  const cuuint64_t dims[5] = {64, 2, 16, 4, static_cast<cuuint64_t>(n_records)};
-  const cuuint64_t strides[4] = {128, 256, 4096, static_cast<cuuint64_t>(REC_BYTES)};
-  const cuuint32_t box[5] = {64, 1, 16, 1, 1};
-  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-  CUresult r = enc(&pp.tm_rec, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<uint8_t*>(p.rec), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+cudaError_t launch_k2t(const K2Params& p, cudaStream_t stream) {
   static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
@@ -570,7 +402,7 @@ cudaError_t launch_k2t(const K2Params& p, long long n_records, cudaStream_t stre
     configured[dev] = true;
   }
   const int nblocks = p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H;
-  return launch_dep(kda_k2t_kernel, nblocks, KT_THREADS, k2_smem(p, T_TOTAL), stream, p.pdl, pp);
+  return launch_dep(kda_k2t_kernel, nblocks, KT_THREADS, k2_smem(p, T_TOTAL), stream, p.pdl, p);
 }
 
 }  // namespace kda

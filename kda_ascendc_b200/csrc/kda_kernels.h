@@ -147,7 +147,7 @@ cudaError_t launch_k2la(const K2Params& p, int vsplit, bool state_only, cudaStre
 cudaError_t launch_k2n_pair(const K2Params& p, int vsplit, cudaStream_t stream);
 //   "tc":       the whole 128-row state of a head in tensor memory, tcgen05 MMAs, one CTA per
 //               (batch, head), two CTAs per SM; outputs + final state only              (kda_k2t_sm100.cu)
-cudaError_t launch_k2t(const K2Params& p, long long n_records, cudaStream_t stream);
+cudaError_t launch_k2t(const K2Params& p, cudaStream_t stream);
 
 // Walk of the per-segment affine state transforms of a sequence split (kda_fold_sm100.cu).
 struct FoldParams {

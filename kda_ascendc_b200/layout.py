@@ -14,7 +14,8 @@ CHUNK = 16
 D = 128
 REC_BYTES = 26112
 WS_HEADER_BYTES = 256
-REC_W, REC_QG, REC_KGH, REC_KGL, REC_AQK, REC_AQL, REC_DEC, REC_U = 0, 4096, 8192, 12288, 16384, 16896, 17408, 17920
+REC_W, REC_QG, REC_KGH, REC_KGL, REC_AQK, REC_AQL, REC_DEC, REC_U = 0, 2048, 8192, 12288, 16384, 16640, 17408, 17920
+REC_HALF = 4096   # from a 64-column half of w / qg to the other
 
 
 def pack_tokens(x: torch.Tensor, chunk: int = CHUNK) -> torch.Tensor:
@@ -34,10 +35,30 @@ def unpack_tokens(x: torch.Tensor, b: int, t: int, h: int, chunk: int = CHUNK) -
 
 
 def _swizzle_index(device) -> torch.Tensor:
-    """Position (in bf16 elements) of element (r, c) inside a swizzled [16][128] tile."""
+    """Position (in bf16 elements) of element (r, c) inside a w or qg tile, its two 64-column halves back to back."""
     r = torch.arange(CHUNK, device=device)[:, None]
     c = torch.arange(D, device=device)[None, :]
-    return (r * D + ((((c >> 3) ^ (r & 7)) << 3) | (c & 7))).reshape(-1)
+    return ((c >> 6) * 1024 + r * 64 + ((((c >> 3) & 7) ^ (r & 7)) << 3) + (c & 7)).reshape(-1)
+
+
+def _wq_index(device) -> torch.Tensor:
+    """Byte offset of element (r, c) of w or qg inside a record, relative to its part of the first half."""
+    at = 2 * _swizzle_index(device).view(CHUNK, D)
+    return at + (at >= 2048) * (REC_HALF - 2048)
+
+
+def _kg_index(device) -> torch.Tensor:
+    """Byte offset of element (token, k) inside a transposed kg tile."""
+    t = torch.arange(CHUNK, device=device)[:, None]
+    k = torch.arange(D, device=device)[None, :]
+    return (t >> 3) * 2048 + k * 16 + ((t & 7) << 1)
+
+
+def _aq_index(device) -> torch.Tensor:
+    """Byte offset of element (i, j) of Aqk's hi (or lo) part."""
+    i = torch.arange(CHUNK, device=device)[:, None]
+    j = torch.arange(CHUNK, device=device)[None, :]
+    return (j >> 3) * 512 + i * 16 + ((j & 7) << 1)
 
 
 def _u_index(device) -> torch.Tensor:
@@ -60,11 +81,10 @@ def unpack_records(workspace: torch.Tensor, B: int, T: int, H: int) -> dict:
     c = B * H * nt
     rec = workspace[WS_HEADER_BYTES:WS_HEADER_BYTES + c * REC_BYTES].view(c, REC_BYTES)
     dev = workspace.device
-    sw = _swizzle_index(dev)
+    half_words = rec.view(torch.bfloat16)   # [c, REC_BYTES / 2]
 
-    def tile(off):
-        t = rec[:, off:off + 4096].contiguous().view(torch.bfloat16)  # [c, 2048]
-        return t[:, sw].view(c, CHUNK, D)
+    def elements(off, index):
+        return half_words[:, ((off + index) >> 1).reshape(-1)].view(c, *index.shape)
 
     def to_public(x):  # [c, 16, n] -> [B, T, H, n]
         n = x.shape[-1]
@@ -72,9 +92,9 @@ def unpack_records(workspace: torch.Tensor, B: int, T: int, H: int) -> dict:
         return y[:, :T].contiguous()
 
     uT = rec[:, REC_U:REC_U + 8192].contiguous().view(torch.float32)[:, _u_index(dev)].view(c, CHUNK, D)
-    aqk = (rec[:, REC_AQK:REC_AQK + 512].contiguous().view(torch.bfloat16).float() +
-           rec[:, REC_AQL:REC_AQL + 512].contiguous().view(torch.bfloat16).float()).view(c, CHUNK, CHUNK)
+    wq, kg, aq = _wq_index(dev), _kg_index(dev), _aq_index(dev)
+    aqk = elements(REC_AQK, aq).float() + elements(REC_AQL, aq).float()
     dec = rec[:, REC_DEC:REC_DEC + 512].contiguous().view(torch.float32).view(B, H, nt, D)
-    return dict(w=to_public(tile(REC_W)), qg=to_public(tile(REC_QG)),
-                kg=to_public(tile(REC_KGH).float() + tile(REC_KGL).float()),
+    return dict(w=to_public(elements(REC_W, wq)), qg=to_public(elements(REC_QG, wq)),
+                kg=to_public(elements(REC_KGH, kg).float() + elements(REC_KGL, kg).float()),
                 u=to_public(uT), Aqk=to_public(aqk), dec=dec)
