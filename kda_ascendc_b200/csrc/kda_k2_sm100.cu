@@ -29,8 +29,7 @@
 // sub-partition issues meanwhile), so a step costs about 8 cycles per MMA plus 2 per other
 // instruction and what matters is the instruction count.  Loads are still interleaved with the
 // MMA sequences so that their latency is covered: P1 carries this step's kg fragment loads and
-// the decay of hT; P2 carries the next step's [w;qg] / decay / u loads; the previous step's output
-// tile is stored at the start of the next step.
+// the decay of hT; P2 carries the next step's [w;qg] / decay / u loads, and P3 runs inside it.
 //
 // A CTA = CW consumer warps (CW*NVT*8 state rows of one (batch, head)) plus one producer warp
 // that streams the chunk records through a ring of shared-memory stages with bulk (TMA)
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     uint32_t aw[8][4], aq[8][4];     // A fragments of w and qg (one per 16-wide k-step)
     float dk[8][2];                  // decay of the rows k = 16m+gq and 16m+gq+8
     float4 u[NVT];
-    float oa[NVT][4];                // output tile of the previous step, stored one step late
+    float oa[NVT][4];                // output tile
 
     bool failed = false;
     if (!h0_ok) {
@@ -223,20 +222,20 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
                                               : make_float4(0, 0, 0, 0);
     }
 
+    // A step is two straight runs of instructions around one branch (the slow path of the wait for the next record),
+    // which is what the compiler schedules well: the loads for the next step are made in the last step too, the output
+    // stores are predicated and the shared-memory loads are pinned.  With conditions around them, K2 alone (us), before
+    // and now: T8192 H32 257 -> 250, B2 T4096 H8 107 -> 97; state-only 220 -> 199 and 101 -> 87.
+    __nv_bfloat16* o_at = STATE_ONLY ? nullptr : ob + static_cast<int64_t>(gq) * p.o_s[1];
+    const int64_t o_step = BT * p.o_s[1], o_8 = 8 * p.o_s[1];
+    int left = Tlen;
     for (int n = 0; n < NT && !failed; ++n) {
       const int s = n % K2_STAGES;
       const uint32_t sp = sbase + s * SM::STAGE;
       const uint32_t t2 = sp + a2_lane;
-
-      // the previous step's output tile (always a full chunk)
-      if (!STATE_ONLY && n > 0) {
-        __nv_bfloat16* op = ob + static_cast<int64_t>((n - 1) * BT + gq) * p.o_s[1];
-#pragma unroll
-        for (int nv = 0; nv < NVT; ++nv) {
-          *reinterpret_cast<uint32_t*>(op + nv * 8) = pack_bf16(oa[nv][0], oa[nv][1]);
-          *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1] + nv * 8) = pack_bf16(oa[nv][2], oa[nv][3]);
-        }
-      }
+      const int s1 = (n + 1) % K2_STAGES;
+      const uint32_t sp1 = sbase + s1 * SM::STAGE;
+      const uint32_t t1n = sp1 + a1_lane;
 
       // B fragments of bf16(hT) (pre-chunk state): accumulator fragment -> pack -> 8x8 transpose
       uint32_t bh[8][NVT][2];
@@ -275,6 +274,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
           hT[ks][nv][0] = lo.x; hT[ks][nv][1] = lo.y; hT[ks][nv][2] = hi.x; hT[ks][nv][3] = hi.y;
         }
       }
+      // probed here and looked at when the answer is needed: a probe and the vote on it take 126 cycles
+      const bool next_ready = mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1) || n + 1 >= NT;
       uint32_t ah3[4], al3[4];
       if (!STATE_ONLY) {
         ldsm_x4(sp + a3_off, ah3[0], ah3[1], ah3[2], ah3[3]);
@@ -304,12 +305,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + s * 8);
-      const bool more = n + 1 < NT;
-      const int s1 = (n + 1) % K2_STAGES;
-      const uint32_t sp1 = sbase + s1 * SM::STAGE;
-      const uint8_t* spg1 = smem + s1 * SM::STAGE;
-      const uint32_t t1n = sp1 + a1_lane;
-      if (more) {
+      if (!__all_sync(0xffffffffu, next_ready)) {
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1, sAbort))) {
           if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_FULL_TIMEOUT); }
           failed = true;
@@ -318,58 +314,53 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       }
 
       // P2: hT += kg^T v_new  (hi*hi, then hi*lo(v), then lo(kg)*hi: three passes over independent
-      // tiles), carrying the next step's operand loads
+      // tiles), carrying the next step's operand loads (of the last step: never used), and P3: o = scale * (qg hT) +
+      // Aqk v_new
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvh[nv][0], bvh[nv][1]);
-        if (more) ldsm_x4(wq_at(t1n, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
+        ldsm_x4(wq_at(t1n, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvl[nv][0], bvl[nv][1]);
-        if (more) {
-          dk[m][0] = *reinterpret_cast<const float*>(spg1 + REC_DEC + (m * 16 + gq) * 4);
-          dk[m][1] = *reinterpret_cast<const float*>(spg1 + REC_DEC + (m * 16 + gq + 8) * 4);
-        }
+        dk[m][0] = lds_f32(sp1 + REC_DEC + (m * 16 + gq) * 4);
+        dk[m][1] = lds_f32(sp1 + REC_DEC + (m * 16 + gq + 8) * 4);
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgl[m], bvh[nv][0], bvh[nv][1]);
-        if (!STATE_ONLY && more)
-          ldsm_x4(wq_at(t1n, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
-      }
-
-      // P3: o = scale * (qg hT) + Aqk v_new
-      if (!STATE_ONLY) {
+        if (!STATE_ONLY) ldsm_x4(wq_at(t1n, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
+        if (!STATE_ONLY && (m == 0 || m == 3 || m == 6)) {
 #pragma unroll
-        for (int nv = 0; nv < NVT; ++nv) {
+          for (int nv = 0; nv < NVT; ++nv) {
+            if (m == 0) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) oa[nv][e] = p.scale * (pq[0][nv][e] + pq[1][nv][e]);
-          mma_bf16_v(oa[nv], ah3, bvh[nv][0], bvh[nv][1]);
-          mma_bf16_v(oa[nv], ah3, bvl[nv][0], bvl[nv][1]);
-          mma_bf16_v(oa[nv], al3, bvh[nv][0], bvh[nv][1]);
+              for (int e = 0; e < 4; ++e) oa[nv][e] = p.scale * (pq[0][nv][e] + pq[1][nv][e]);
+              mma_bf16_v(oa[nv], ah3, bvh[nv][0], bvh[nv][1]);
+            }
+            if (m == 3) mma_bf16_v(oa[nv], ah3, bvl[nv][0], bvl[nv][1]);
+            if (m == 6) mma_bf16_v(oa[nv], al3, bvh[nv][0], bvh[nv][1]);
+          }
         }
       }
-      if (more) {
-#pragma unroll
-        for (int nv = 0; nv < NVT; ++nv)
-          u[nv] = (use_u && !(PAIR && nv == 0)) ? *reinterpret_cast<const float4*>(spg1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
-                                                : make_float4(0, 0, 0, 0);
-      }
-    }
 
-    // the last chunk's output tile (it may be a partial chunk)
-    if (!STATE_ONLY && !failed) {
-      const int tok = (NT - 1) * BT + gq;
-      __nv_bfloat16* op = ob + static_cast<int64_t>(tok) * p.o_s[1];
+      if (!STATE_ONLY) {   // rows past the end of a partial last chunk stay as they are
 #pragma unroll
-      for (int nv = 0; nv < NVT; ++nv) {
-        if (tok < Tlen) *reinterpret_cast<uint32_t*>(op + nv * 8) = pack_bf16(oa[nv][0], oa[nv][1]);
-        if (tok + 8 < Tlen) *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1] + nv * 8) = pack_bf16(oa[nv][2], oa[nv][3]);
+        for (int nv = 0; nv < NVT; ++nv) {
+          stg_u32_if(o_at + nv * 8, pack_bf16(oa[nv][0], oa[nv][1]), gq < left);
+          stg_u32_if(o_at + o_8 + nv * 8, pack_bf16(oa[nv][2], oa[nv][3]), gq + 8 < left);
+        }
+        o_at += o_step;
+        left -= BT;
       }
+#pragma unroll
+      for (int nv = 0; nv < NVT; ++nv)
+        u[nv] = (use_u && !(PAIR && nv == 0)) ? lds_f32x4(sp1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
+                                              : make_float4(0, 0, 0, 0);
     }
 
     if (!failed && (p.ht != nullptr || (PAIR && p.push_on))) {
