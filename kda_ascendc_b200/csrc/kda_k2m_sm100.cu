@@ -159,19 +159,19 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     uint32_t o_st[2][2];        // previous step's output tile, already transposed and packed
     float2 dec[16];             // decay of the columns k = 8nt + 2tq, +1 (loaded one step ahead)
 
-    auto load_u = [&](const uint8_t* spg) {
+    auto load_u = [&](uint32_t spg) {
 #pragma unroll
       for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
           for (int j = 0; j < 2; ++j)
-            ut[c][a * 2 + j] = use_u ? *reinterpret_cast<const float*>(spg + u_off + a * REC_U_TILE_BYTES + j * 64 + c * 8)
+            ut[c][a * 2 + j] = use_u ? lds_f32(spg + u_off + a * REC_U_TILE_BYTES + j * 64 + c * 8)
                                      : 0.f;
     };
-    auto load_dec = [&](const uint8_t* spg, int nt0, int nt1) {
+    auto load_dec = [&](uint32_t spg, int nt0, int nt1) {
 #pragma unroll
-      for (int nt = nt0; nt < nt1; ++nt) dec[nt] = *reinterpret_cast<const float2*>(spg + REC_DEC + (nt * 8 + tq * 2) * 4);
+      for (int nt = nt0; nt < nt1; ++nt) dec[nt] = lds_f32x2(spg + REC_DEC + (nt * 8 + tq * 2) * 4);
     };
     auto load_b1 = [&](uint32_t sp, int ks, int slot) {
       const uint32_t at = ((sp + b1_lane) ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF;
@@ -189,14 +189,15 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     } else {
       load_b1(sbase, 0, 0);
       load_b1(sbase, 1, 1);
-      load_u(smem);
-      load_dec(smem, 0, 16);
+      load_u(sbase);
+      load_dec(sbase, 0, 16);
     }
 
     for (int n = 0; n < NT && !failed; ++n) {
       const int s = n % K2M_STAGES;
       const uint32_t sp = sbase + s * SM::STAGE;
-      const uint8_t* spg = smem + s * SM::STAGE;
+      const int s1 = (n + 1) % K2M_STAGES;
+      const uint32_t sp1 = sbase + s1 * SM::STAGE;
 
       // the previous step's output tile (always a full chunk): rows tok gq / gq+8, 2 value columns
       if (!STATE_ONLY && n > 0) {
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         ldsm_x4(sp + b3_off, ba[0], ba[1], ba[2], ba[3]);
         ldsm_x4(sp + b3_off + (REC_AQL - REC_AQK), bl[0], bl[1], bl[2], bl[3]);
       }
+      const bool next_ready = mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2M_STAGES) & 1) || n + 1 >= NT;
       // P2 pass 2 (lo(v) * hi)
 #pragma unroll
       for (int np = 0; np < 8; ++np) {
@@ -267,10 +269,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
       // every shared-memory operand of this stage has been requested; once the loads have landed
       // (they are consumed below) the stage is released and the next one checked
-      const bool more = n + 1 < NT;
-      const int s1 = (n + 1) % K2M_STAGES;
-      const uint32_t sp1 = sbase + s1 * SM::STAGE;
-      const uint8_t* spg1 = smem + s1 * SM::STAGE;
 
       // P2 pass 3 (hi * lo(kg)), with P3 and the next step's first operands in its gaps
       float oa[2][4];
@@ -298,17 +296,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
           asm volatile("" ::"r"(landed) : "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(empty0 + s * 8);
-          if (more) {
+          if (!__all_sync(0xffffffffu, next_ready)) {
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + s1 * 8, ((n + 1) / K2M_STAGES) & 1, sAbort))) {
               if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_FULL_TIMEOUT); }
               failed = true;
             }
           }
         }
-        if (more && !failed) {
-          if (np == 4) { load_b1(sp1, 0, 0); load_dec(spg1, 0, 6); }
-          if (np == 5) { load_b1(sp1, 1, 1); load_dec(spg1, 6, 12); }
-          if (np == 6) { load_u(spg1); load_dec(spg1, 12, 16); }
+        {
+          if (np == 4) { load_b1(sp1, 0, 0); load_dec(sp1, 0, 6); }
+          if (np == 5) { load_b1(sp1, 1, 1); load_dec(sp1, 6, 12); }
+          if (np == 6) { load_u(sp1); load_dec(sp1, 12, 16); }
         }
       }
 
