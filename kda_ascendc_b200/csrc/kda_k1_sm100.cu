@@ -103,7 +103,9 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // SM need 128 a thread or fewer.  Beside K2, two CTAs share every SM sub-partition's 16,384 registers with up to three
 // warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
 // start before K1 ends (T8192 H96, whole forward: 1,254 us with 128 registers, 883 with 112).
-template <bool G_BF16, bool FAST_EXP, bool BESIDE>
+// PLAIN: gate, l2-norm and beta sigmoid all in the kernel and no debug outputs, known when it is compiled: without the
+// conditions between its loops, T8192 H32 154.2 -> 149.9 us, H96 447 -> 433 (beside K2 the whole forward 887 -> 847).
+template <bool G_BF16, bool FAST_EXP, bool BESIDE, bool PLAIN>
 __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K1Smem<G_BF16, FAST_EXP>;
@@ -127,8 +129,8 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   grid_dep_launch();   // K2 may be set up, or run, beside this kernel
   if (!BESIDE && blockIdx.x == 0 && tid == 0) *reinterpret_cast<int2*>(p.status) = make_int2(ST_OK, ST_OK);
 
-  const bool use_gate = (p.flags & 1u) != 0;
-  const bool use_l2 = (p.flags & 2u) != 0;
+  const bool use_gate = PLAIN || (p.flags & 1u) != 0;
+  const bool use_l2 = PLAIN || (p.flags & 2u) != 0;
   const int cp = tid & 63, rh = tid >> 6;   // phase-B mapping: column pair, row half
   const int c0 = cp * 2, r0 = rh * 8;
 
@@ -173,7 +175,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   auto publish_params = [&](const Par& q, int nvalid_, int slot) {
     if (tid >= 32 && tid < 48) {
       float bv = q.beta;
-      if (tid - 32 < nvalid_) { if (p.flags & 4u) bv = 1.0f / (1.0f + __expf(-bv)); } else bv = 0.f;
+      if (tid - 32 < nvalid_) { if (PLAIN || (p.flags & 4u)) bv = 1.0f / (1.0f + __expf(-bv)); } else bv = 0.f;
       sBetaAll[slot * 16 + tid - 32] = bv;
     }
     if (tid == 48) sBetaAll[32 + slot] = use_gate ? expf(q.a_log) : 1.f;
@@ -351,7 +353,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       dec2 = make_float2(ex2f(glast.x), ex2f(glast.y));
       if (rh == 1) *reinterpret_cast<float2*>(smem + S_DEC + c0 * 4) = dec2;
 
-      if (p.g_out != nullptr) {
+      if (!PLAIN && p.g_out != nullptr) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           if (r0 + i < nvalid)
@@ -529,7 +531,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         *reinterpret_cast<unsigned short*>(smem + S_XH + (i * 16 + lane) * 2) = bf16_bits(hi);
         *reinterpret_cast<unsigned short*>(smem + S_XL + (i * 16 + lane) * 2) = bf16_bits(x[i] - hi);
       }
-      if (p.ainv_out != nullptr) {
+      if (!PLAIN && p.ainv_out != nullptr) {
 #pragma unroll
         for (int i = 0; i < BT; ++i)
           if (i < nvalid) p.ainv_out[((static_cast<size_t>(b) * p.T + t0 + i) * p.H + h) * BT + lane] = x[i];
@@ -612,7 +614,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   if (tid == 0) drain_stores();
 }
 
-template <bool G_BF16, bool FAST_EXP, bool BESIDE>
+template <bool G_BF16, bool FAST_EXP, bool BESIDE, bool PLAIN>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
   // per device: SMs << 8 | resident CTAs per SM, 0 = not looked up yet.  One word, published after the attributes
@@ -623,7 +625,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   if (dev >= 64) return cudaErrorInvalidDevice;
   int res = residency[dev].load(std::memory_order_acquire);
   if (res == 0) {
-    auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE>;
+    auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, PLAIN>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;
     // ask for the full shared-memory carve-out so that four CTAs are resident per SM
@@ -641,7 +643,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   const int sms = res >> 8, fit = res & 255;
   const int cap = sms * (p.ctas_per_sm > 0 && p.ctas_per_sm < fit ? p.ctas_per_sm : fit);   // persistent: one CTA per slot
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
-  kda_k1_kernel<G_BF16, FAST_EXP, BESIDE><<<grid, 128, smem_bytes, stream>>>(p);
+  kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, PLAIN><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();
 }
 
@@ -691,14 +693,17 @@ cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what) {
   return cudaSuccess;
 }
 
-template <bool BESIDE>
-static cudaError_t launch_k1_b(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream) {
-  if (g_bf16) return fast_exp ? launch_k1_t<true, true, BESIDE>(p, stream) : launch_k1_t<true, false, BESIDE>(p, stream);
-  return fast_exp ? launch_k1_t<false, true, BESIDE>(p, stream) : launch_k1_t<false, false, BESIDE>(p, stream);
+template <bool G_BF16, bool BESIDE>
+static cudaError_t launch_k1_b(const K1Params& p, bool fast_exp, cudaStream_t stream) {
+  if (!fast_exp) return launch_k1_t<G_BF16, false, BESIDE, false>(p, stream);
+  return (p.flags & 7u) == 7u && p.g_out == nullptr && p.ainv_out == nullptr
+             ? launch_k1_t<G_BF16, true, BESIDE, true>(p, stream)
+             : launch_k1_t<G_BF16, true, BESIDE, false>(p, stream);
 }
 
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream) {
-  return p.progress != nullptr ? launch_k1_b<true>(p, g_bf16, fast_exp, stream) : launch_k1_b<false>(p, g_bf16, fast_exp, stream);
+  if (g_bf16) return p.progress != nullptr ? launch_k1_b<true, true>(p, fast_exp, stream) : launch_k1_b<true, false>(p, fast_exp, stream);
+  return p.progress != nullptr ? launch_k1_b<false, true>(p, fast_exp, stream) : launch_k1_b<false, false>(p, fast_exp, stream);
 }
 
 }  // namespace kda
