@@ -103,9 +103,12 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // SM need 128 a thread or fewer.  Beside K2, two CTAs share every SM sub-partition's 16,384 registers with up to three
 // warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
 // start before K1 ends (T8192 H96, whole forward: 1,254 us with 128 registers, 883 with 112).
-// PLAIN: gate, l2-norm and beta sigmoid all in the kernel and no debug outputs, known when it is compiled: without the
-// conditions between its loops, T8192 H32 154.2 -> 149.9 us, H96 447 -> 433 (beside K2 the whole forward 887 -> 847).
-template <bool G_BF16, bool FAST_EXP, bool BESIDE, bool PLAIN>
+// FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel; FORM_NONE: all
+// three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags decide.  Without the
+// conditions between its loops K1 takes, T8192 H32 154.2 -> 149.9 us, H96 447 -> 433 (beside K2 the whole forward
+// 887 -> 847); inputs prepared by the caller, B8 T2037 H32 with 8 q/k heads, 297 -> 274.
+enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
+template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K1Smem<G_BF16, FAST_EXP>;
@@ -129,8 +132,9 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   grid_dep_launch();   // K2 may be set up, or run, beside this kernel
   if (!BESIDE && blockIdx.x == 0 && tid == 0) *reinterpret_cast<int2*>(p.status) = make_int2(ST_OK, ST_OK);
 
-  const bool use_gate = PLAIN || (p.flags & 1u) != 0;
-  const bool use_l2 = PLAIN || (p.flags & 2u) != 0;
+  const bool use_gate = FORM == FORM_ANY ? (p.flags & 1u) != 0 : FORM == FORM_ALL;
+  const bool use_l2 = FORM == FORM_ANY ? (p.flags & 2u) != 0 : FORM == FORM_ALL;
+  const bool use_sigmoid = FORM == FORM_ANY ? (p.flags & 4u) != 0 : FORM == FORM_ALL;
   const int cp = tid & 63, rh = tid >> 6;   // phase-B mapping: column pair, row half
   const int c0 = cp * 2, r0 = rh * 8;
 
@@ -175,7 +179,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   auto publish_params = [&](const Par& q, int nvalid_, int slot) {
     if (tid >= 32 && tid < 48) {
       float bv = q.beta;
-      if (tid - 32 < nvalid_) { if (PLAIN || (p.flags & 4u)) bv = 1.0f / (1.0f + __expf(-bv)); } else bv = 0.f;
+      if (tid - 32 < nvalid_) { if (use_sigmoid) bv = 1.0f / (1.0f + __expf(-bv)); } else bv = 0.f;
       sBetaAll[slot * 16 + tid - 32] = bv;
     }
     if (tid == 48) sBetaAll[32 + slot] = use_gate ? expf(q.a_log) : 1.f;
@@ -353,7 +357,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       dec2 = make_float2(ex2f(glast.x), ex2f(glast.y));
       if (rh == 1) *reinterpret_cast<float2*>(smem + S_DEC + c0 * 4) = dec2;
 
-      if (!PLAIN && p.g_out != nullptr) {
+      if (FORM == FORM_ANY && p.g_out != nullptr) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           if (r0 + i < nvalid)
@@ -362,11 +366,11 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
 
       const float2 centre = FAST_EXP ? glast : gmid;
       const float2 ncentre = make_float2(-centre.x, -centre.y);
-      // kg (and kn) go out transposed, eight tokens of a column per 16-byte store: pairs of rows are packed
-      uint32_t kgh[2][4], kgl[2][4], knh[2][4], knl[2][4];
+      // kg goes out transposed, eight tokens of a column per 16-byte store: pairs of rows are packed
+      uint32_t kgh[2][4], kgl[2][4];
 #pragma unroll
       for (int i2 = 0; i2 < 4; ++i2) {
-        float2 kg2[2], kn2[2];
+        float2 kg2[2];
 #pragma unroll
         for (int ii = 0; ii < 2; ++ii) {
           const int i = i2 * 2 + ii, r = r0 + i;
@@ -393,7 +397,11 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
           split_pack2(__fmul2_rn(kn, e), hi, lo);
           *reinterpret_cast<uint32_t*>(smem + S_KQH + off) = hi;
           *reinterpret_cast<uint32_t*>(smem + S_KQL + off) = lo;
-          if (!FAST_EXP) kn2[ii] = __fmul2_rn(kn, en);
+          if (!FAST_EXP) {
+            split_pack2(__fmul2_rn(kn, en), hi, lo);
+            *reinterpret_cast<uint32_t*>(smem + S_KNH + off) = hi;
+            *reinterpret_cast<uint32_t*>(smem + S_KNL + off) = lo;
+          }
           kg2[ii] = __fmul2_rn(kn, ekg);
           const float2 qgo = __fmul2_rn(qn, eg);
           *reinterpret_cast<uint32_t*>(smem + S_QG + stage_off(r, c0)) = pack_bf16(qgo.x, qgo.y);
@@ -403,10 +411,6 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         }
         split_pack(kg2[0].x, kg2[1].x, kgh[0][i2], kgl[0][i2]);
         split_pack(kg2[0].y, kg2[1].y, kgh[1][i2], kgl[1][i2]);
-        if (!FAST_EXP) {
-          split_pack(kn2[0].x, kn2[1].x, knh[0][i2], knl[0][i2]);
-          split_pack(kn2[0].y, kn2[1].y, knh[1][i2], knl[1][i2]);
-        }
       }
       // a lane's two columns are neighbours: half of the lanes store the odd one first, so that the eight lanes of a
       // shared-memory pass cover 128 different bytes
@@ -421,7 +425,6 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       };
       put(S_KGH, kgh);
       put(S_KGL, kgl);
-      if (!FAST_EXP) { put(S_KNH, knh); put(S_KNL, knl); }
     }
     __syncthreads();  // every thread has read its q/k/v/g elements: the input tiles are free
 
@@ -438,16 +441,22 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       const int arow = (lane & 7) + ((lane >> 3) & 1) * 8, acol = (lane >> 4) * 8;
       // swizzled address of k-step ks = (256-byte aligned tile base + lane part) ^ (ks << 5)
       const uint32_t a_hi = sbase + (mt == 0 ? S_QGH : S_KQH) + swz_off(arow, acol);
-      // B operand out of the transposed tile (rows k, columns tok): k-step ks is 256 bytes further
-      const uint32_t b_hi = sbase + (FAST_EXP ? S_KGH : S_KNH) + kg_off(nt * 8, lane);
+      // B operand: out of the transposed kg tile (rows k, columns tok; a k-step is 256 bytes), or with the general
+      // centring out of the swizzled kn tile (rows tok, columns k)
+      const uint32_t b_hi = sbase + (FAST_EXP ? S_KGH + kg_off(nt * 8, lane) : S_KNH + swz_off(nt * 8 + (lane & 7), (lane >> 3) * 8));
       constexpr uint32_t A_LO = S_QGL - S_QGH, B_LO = FAST_EXP ? S_KGL - S_KGH : S_KNL - S_KNH;
       static_assert(S_KQL - S_KQH == S_QGL - S_QGH && S_GRAM % 256 == 0, "tile layout");
       float acc0[4] = {0, 0, 0, 0}, acc1[4] = {0, 0, 0, 0}, acc2[4] = {0, 0, 0, 0};
 #pragma unroll
       for (int kp = 0; kp < 4; ++kp) {
         uint32_t bh[4], bl[4];   // two k-steps
-        ldsm_x4_t(b_hi + kp * 512, bh[0], bh[1], bh[2], bh[3]);
-        ldsm_x4_t(b_hi + kp * 512 + B_LO, bl[0], bl[1], bl[2], bl[3]);
+        if (FAST_EXP) {
+          ldsm_x4_t(b_hi + kp * 512, bh[0], bh[1], bh[2], bh[3]);
+          ldsm_x4_t(b_hi + kp * 512 + B_LO, bl[0], bl[1], bl[2], bl[3]);
+        } else {
+          ldsm_x4(b_hi ^ (kp << 6), bh[0], bh[1], bh[2], bh[3]);
+          ldsm_x4((b_hi ^ (kp << 6)) + B_LO, bl[0], bl[1], bl[2], bl[3]);
+        }
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int ks = kp * 2 + j;
@@ -531,7 +540,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         *reinterpret_cast<unsigned short*>(smem + S_XH + (i * 16 + lane) * 2) = bf16_bits(hi);
         *reinterpret_cast<unsigned short*>(smem + S_XL + (i * 16 + lane) * 2) = bf16_bits(x[i] - hi);
       }
-      if (!PLAIN && p.ainv_out != nullptr) {
+      if (FORM == FORM_ANY && p.ainv_out != nullptr) {
 #pragma unroll
         for (int i = 0; i < BT; ++i)
           if (i < nvalid) p.ainv_out[((static_cast<size_t>(b) * p.T + t0 + i) * p.H + h) * BT + lane] = x[i];
@@ -614,7 +623,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   if (tid == 0) drain_stores();
 }
 
-template <bool G_BF16, bool FAST_EXP, bool BESIDE, bool PLAIN>
+template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
   // per device: SMs << 8 | resident CTAs per SM, 0 = not looked up yet.  One word, published after the attributes
@@ -625,7 +634,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   if (dev >= 64) return cudaErrorInvalidDevice;
   int res = residency[dev].load(std::memory_order_acquire);
   if (res == 0) {
-    auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, PLAIN>;
+    auto kern = kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, FORM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e != cudaSuccess) return e;
     // ask for the full shared-memory carve-out so that four CTAs are resident per SM
@@ -643,7 +652,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   const int sms = res >> 8, fit = res & 255;
   const int cap = sms * (p.ctas_per_sm > 0 && p.ctas_per_sm < fit ? p.ctas_per_sm : fit);   // persistent: one CTA per slot
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
-  kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, PLAIN><<<grid, 128, smem_bytes, stream>>>(p);
+  kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, FORM><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();
 }
 
@@ -695,10 +704,14 @@ cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what) {
 
 template <bool G_BF16, bool BESIDE>
 static cudaError_t launch_k1_b(const K1Params& p, bool fast_exp, cudaStream_t stream) {
-  if (!fast_exp) return launch_k1_t<G_BF16, false, BESIDE, false>(p, stream);
-  return (p.flags & 7u) == 7u && p.g_out == nullptr && p.ainv_out == nullptr
-             ? launch_k1_t<G_BF16, true, BESIDE, true>(p, stream)
-             : launch_k1_t<G_BF16, true, BESIDE, false>(p, stream);
+  const uint32_t in_kernel = p.flags & 7u;
+  const bool debug = p.g_out != nullptr || p.ainv_out != nullptr;
+  if (fast_exp)
+    return in_kernel == 7u && !debug ? launch_k1_t<G_BF16, true, BESIDE, FORM_ALL>(p, stream)
+                                     : launch_k1_t<G_BF16, true, BESIDE, FORM_ANY>(p, stream);
+  if (in_kernel == 7u && !debug) return launch_k1_t<G_BF16, false, BESIDE, FORM_ALL>(p, stream);
+  if (in_kernel == 0u && !debug) return launch_k1_t<G_BF16, false, BESIDE, FORM_NONE>(p, stream);
+  return launch_k1_t<G_BF16, false, BESIDE, FORM_ANY>(p, stream);
 }
 
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream) {
