@@ -111,12 +111,12 @@ int check_k2(const KdaFwdArgs* a, bool state_only) {
 // warps per CTA, which reads half the shared-memory bytes per MMA.  With more chains than SMs the
 // tensor-memory form (one CTA per chain, two per SM, tcgen05) is 10-35 % faster still once the
 // chains are a few chunks long: its set-up (TMEM allocation, the state in and out through
-// registers) costs about as much as two steps.  2,048 chains x 1 chunk: 81 us against 80 us,
-// x 4: 126 against 134, x 16: 243 against 343; 1,024 chains x 64: 404 against 601; 256 chains
-// x 4: 17 against 21 -- hence from four chunks per chain on.  Between half as many chains as SMs and as many
-// (where the 16-row form needs two CTAs per chain and so more than one CTA per SM) it wins from
-// about 32 chunks per chain: 96 chains x 64 chunks 85 us against 92, x 16 equal.  It has no
-// state-only variant.
+// registers) costs about as much as two steps.  K2 alone against the 16-row form: 160 chains x 2 chunks 14.6 us
+// against 13.2, x 4 16.7 against 16.8; 296 chains x 1 12.8 against 13.9, x 4 17.4 against 21.1; 592 chains x 2 36.5
+// against 35.2; 160 chains x 64 95 against 136 -- hence from four chunks per chain on.  Between half as many chains as
+// SMs and as many (where the 16-row form needs two CTAs per chain and so more than one CTA per SM): 96 chains x 8 chunks
+// equal, x 16 23 against 27, x 32 41 against 47, x 64 68 against 85, x 256 232 against 311; up to half as many chains as
+// SMs the 16-row form wins at every length (74 chains x 256 chunks 175 against 229).  It has no state-only variant.
 void pick_split(const KdaFwdArgs* a, bool state_only, int* vsplit, int* variant, int sms = 0, int chain_mult = 1) {
   if (sms <= 0) {   // the current device's SM count
     int dev = 0;
@@ -168,9 +168,10 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // time order and counts the finished items of every window of chunks; K2's producer warps wait for
 // the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA is
 // already running.  Where it pays, measured on B200 as the whole forward, K2 after K1 against beside it:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T131072 H16 4,527 -> 4,321 us,
-//     B2 T4096 H8 154.3 -> 150.1, B1 T8192 H8 254.4 -> 250.5;
-//   tensor-memory form with one CTA per SM: T8192 H96 1,044 -> 976, T2048 H96 273 -> 255, T1024 H96 146 -> 135,
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T32768 H16 1,036 -> 994 us,
+//     B2 T4096 H8 138.6 -> 137.0, B1 T8192 H16 267.0 -> 259.5;
+//   tensor-memory form with one CTA per SM: T8192 H96 889 -> 883, T2048 H80 220 -> 207, T1024 H96 129 -> 126 (with a K1
+//     of 112 registers, beside which it fits: see there),
 //     but T4096 H128 602 -> 631 (no SM is left to K1 alone): up to three quarters of the SMs.
 // Not in the other forms: with four consumer warps per CTA K2 has no issue slots to spare, or (8-row form)
 // does not fit beside two K1 CTAs: T8192 H32 418 -> 515, T4096 H48 317 -> 379.

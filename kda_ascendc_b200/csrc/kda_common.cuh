@@ -22,8 +22,8 @@
 // with qg = bf16(qhat * 2^g).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
 // operand as it stands: [w; qg] is a 32-row K-major operand in the 128-byte swizzle of tcgen05 (8-row groups 1024
 // bytes apart), kg^T and Aqk are 8x8 core matrices of 128 contiguous bytes (K-major without swizzle).  tcgen05.mma
-// reads them by descriptor, tcgen05.cp moves 32 rows x 16 bytes of them into tensor memory, and every 8x8 matrix of an
-// ldmatrix is free of bank conflicts.
+// reads them by descriptor, and every 8x8 matrix of an ldmatrix is free of bank conflicts, most of them at
+// an immediate offset.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -24,12 +24,12 @@
 // with v_new and Aqk (the intra-chunk term dominates o); P1 uses plain bf16 operands.
 // The result does not depend on how the rows are distributed over warps and CTAs.
 //
-// One warp executes its chain in program order.  Measured on B200: an mma.sync holds the
-// sub-partition's issue port for its 8 cycles (neither this warp nor another one on the same
-// sub-partition issues meanwhile), so a step costs about 8 cycles per MMA plus 2 per other
-// instruction and what matters is the instruction count.  Loads are still interleaved with the
-// MMA sequences so that their latency is covered: P1 carries this step's kg fragment loads and
-// the decay of hT; P2 carries the next step's [w;qg] / decay / u loads, and P3 runs inside it.
+// One warp executes its chain in program order: 43 MMAs of 8 cycles, 20 movmatrix of 5.5, 34 ldmatrix, and the waits
+// between the dependent parts.  Loads are interleaved with the MMA sequences so that their latency is covered: P1
+// carries this step's kg fragment loads and the decay of hT; P2 carries the next step's [w;qg] / decay / u loads and P3.
+// A step takes 0.38 us with one or two consumer warps per CTA and 0.49 with four (T8192 H32 K2 250 us), where the operand
+// fragments of four warps keep the SM's shared-memory pipe busy.  Measured without gain: the fragments copied into
+// tensor memory once per SM (tcgen05.cp) and read by tcgen05.ld, 0.79 us: a copy stalls the SM's mma.sync while it runs.
 //
 // A CTA = CW consumer warps (CW*NVT*8 state rows of one (batch, head)) plus one producer warp
 // that streams the chunk records through a ring of shared-memory stages with bulk (TMA)
