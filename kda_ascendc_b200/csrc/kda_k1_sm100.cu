@@ -264,6 +264,22 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     const bool ok = mbar_wait_bounded(mbar, it & 1, sFlag);
     if (!ok) *sFlag = 1;
 
+    // packed sequences: behind the last token of a sequence the copies have brought the first tokens of the next one.  They
+    // must not enter this chunk, not even times zero (they may not be finite): zeros, as behind the end of a batch row.
+    // (Calls that do only some of gate, norms and sigmoid here, bf16 gate: T4096 H32 76.3 -> 77.4 us; the others the same.)
+    if (!BESIDE && p.chunk_table != nullptr && nvalid < BT) {
+#pragma unroll 1
+      for (int i = nvalid * 16 + tid; ok && i < BT * 16; i += 128) {   // 16-byte units of a bf16 tile
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4*>(smem + S_Q + i * 16) = z;
+        *reinterpret_cast<uint4*>(smem + S_K + i * 16) = z;
+        *reinterpret_cast<uint4*>(smem + S_V + i * 16) = z;
+        *reinterpret_cast<uint4*>(smem + S_G + i * (G_BF16 ? 16 : 32)) = z;
+        if (!G_BF16) *reinterpret_cast<uint4*>(smem + S_G + i * 32 + 16) = z;
+      }
+      __syncthreads();
+    }
+
     // ---- phase A: l2-normalise q and k in place.  (Not earlier, by the warps that do not solve under the previous
     //      item's solve: the inputs have rarely arrived by then; T8192 H32 149.5 us with a probe for them, 147.1 without.) ----
     if (use_l2 && ok) l2_normalise();

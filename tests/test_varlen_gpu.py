@@ -96,3 +96,26 @@ def test_varlen_argument_errors():
     with pytest.raises(ValueError):
         K.kda_bt16_fwd(q2, q2, q2, torch.cat([d["g"], d["g"]]), torch.cat([d["beta"], d["beta"]]), cu_seqlens=[0, 50],
                        **FLAGS, **kw)
+
+
+@pytest.mark.parametrize("prepared,g32", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("what", ["q", "k", "v", "g", "beta"])
+def test_values_that_are_not_finite_stay_in_their_sequence(what, prepared, g32):
+    """A sequence of NaNs between two others, which end and begin inside a 16-token tile of the packed batch: their bits."""
+    import kda_ascendc_b200 as K
+    inp, d, cu, kw = _setup([40, 37, 60], 3, 41, 0.05)
+    flags = FLAGS
+    if prepared:
+        flags = dict(FLAGS, use_qk_l2norm_in_kernel=False, use_gate_in_kernel=False, use_beta_sigmoid_in_kernel=False)
+        d["q"], d["k"] = (torch.nn.functional.normalize(d[n].float(), dim=-1).bfloat16() for n in ("q", "k"))
+        d["g"], d["beta"] = -d["g"].float().abs() * 0.1, d["beta"].sigmoid()
+    if g32:
+        d["g"] = d["g"].float()
+    run = lambda: K.kda_bt16_fwd(d["q"], d["k"], d["v"], d["g"], d["beta"], initial_state=d["initial_state"], cu_seqlens=cu,
+                                 **flags, **kw)
+    o, ht = run()
+    d[what][:, cu[1]:cu[2]] = float("nan")
+    o_n, ht_n = run()
+    assert o_n[:, cu[1]:cu[2]].isnan().any()
+    for s in (0, 2):
+        assert torch.equal(o_n[:, cu[s]:cu[s + 1]], o[:, cu[s]:cu[s + 1]]) and torch.equal(ht_n[s], ht[s])
