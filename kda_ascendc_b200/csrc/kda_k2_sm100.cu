@@ -34,6 +34,8 @@
 // A CTA = CW consumer warps (CW*NVT*8 state rows of one (batch, head)) plus one producer warp
 // that streams the chunk records through a ring of shared-memory stages with bulk (TMA)
 // copies: full/empty mbarriers, every wait bounded.
+#include <type_traits>
+
 #include "kda_common.cuh"
 #include "kda_kernels.h"
 
@@ -223,13 +225,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     }
 
     // A step is two straight runs of instructions around one branch (the slow path of the wait for the next record),
-    // which is what the compiler schedules well: the loads for the next step are made in the last step too, the output
-    // stores are predicated and the shared-memory loads are pinned.  With conditions around them, K2 alone (us), before
-    // and now: T8192 H32 257 -> 250, B2 T4096 H8 107 -> 97; state-only 220 -> 199 and 101 -> 87.
+    // which is what the compiler schedules well: the last step, which has no next record to wait for and to load from, is an
+    // instantiation of its own, the output stores are predicated and the shared-memory loads are pinned.  K2 alone (us), with
+    // conditions around them, with the loads made in the last step too (out of a stage that no copy has filled), and now:
+    // T8192 H32 262, 249.5, 249; T4096 H8 -, 98.8, 94.6; T16 H32 4.7, 4.9, 4.2 (whole forward 9.3, 10.3, 9.3); state-only
+    // T8192 H32 203, 198, 184; T4096 H8 -, 84.4, 71.2; transform pairs T8192 H32 278, 254.5, 257.5.
     __nv_bfloat16* o_at = STATE_ONLY ? nullptr : ob + static_cast<int64_t>(gq) * p.o_s[1];
     const int64_t o_step = BT * p.o_s[1], o_8 = 8 * p.o_s[1];
     int left = Tlen;
-    for (int n = 0; n < NT && !failed; ++n) {
+    auto step = [&](auto more_c, int n) {
+      constexpr bool MORE = decltype(more_c)::value;   // chunk n + 1 exists
       const int s = n % K2_STAGES;
       const uint32_t sp = sbase + s * SM::STAGE;
       const uint32_t t2 = sp + a2_lane;
@@ -275,7 +280,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         }
       }
       // probed here and looked at when the answer is needed: a probe and the vote on it take 126 cycles
-      const bool next_ready = mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1) || n + 1 >= NT;
+      const bool next_ready = MORE ? mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1) : true;
       uint32_t ah3[4], al3[4];
       if (!STATE_ONLY) {
         ldsm_x4(sp + a3_off, ah3[0], ah3[1], ah3[2], ah3[3]);
@@ -305,35 +310,37 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + s * 8);
-      if (!__all_sync(0xffffffffu, next_ready)) {
+      if (MORE && !__all_sync(0xffffffffu, next_ready)) {
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1, sAbort))) {
           if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_FULL_TIMEOUT); }
           failed = true;
-          break;
+          return;
         }
       }
 
       // P2: hT += kg^T v_new  (hi*hi, then hi*lo(v), then lo(kg)*hi: three passes over independent
-      // tiles), carrying the next step's operand loads (of the last step: never used), and P3: o = scale * (qg hT) +
+      // tiles), carrying the next step's operand loads, and P3: o = scale * (qg hT) +
       // Aqk v_new
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvh[nv][0], bvh[nv][1]);
-        ldsm_x4(wq_at(t1n, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
+        if (MORE) ldsm_x4(wq_at(t1n, m) + REC_W, aw[m][0], aw[m][1], aw[m][2], aw[m][3]);
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvl[nv][0], bvl[nv][1]);
-        dk[m][0] = lds_f32(sp1 + REC_DEC + (m * 16 + gq) * 4);
-        dk[m][1] = lds_f32(sp1 + REC_DEC + (m * 16 + gq + 8) * 4);
+        if (MORE) {
+          dk[m][0] = lds_f32(sp1 + REC_DEC + (m * 16 + gq) * 4);
+          dk[m][1] = lds_f32(sp1 + REC_DEC + (m * 16 + gq + 8) * 4);
+        }
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgl[m], bvh[nv][0], bvh[nv][1]);
-        if (!STATE_ONLY) ldsm_x4(wq_at(t1n, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
+        if (MORE && !STATE_ONLY) ldsm_x4(wq_at(t1n, m) + REC_QG, aq[m][0], aq[m][1], aq[m][2], aq[m][3]);
         if (!STATE_ONLY && (m == 0 || m == 3 || m == 6)) {
 #pragma unroll
           for (int nv = 0; nv < NVT; ++nv) {
@@ -357,10 +364,39 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         o_at += o_step;
         left -= BT;
       }
+      if (MORE) {
 #pragma unroll
-      for (int nv = 0; nv < NVT; ++nv)
-        u[nv] = (use_u && !(PAIR && nv == 0)) ? lds_f32x4(sp1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
-                                              : make_float4(0, 0, 0, 0);
+        for (int nv = 0; nv < NVT; ++nv)
+          u[nv] = (use_u && !(PAIR && nv == 0)) ? lds_f32x4(sp1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
+                                                : make_float4(0, 0, 0, 0);
+      }
+    };
+    // The same walk in three spellings, because the compiler's schedule of a step hangs on the loop around it.  T4096, us per
+    // CTA split in 4 / 8 / 16, in the spelling of pairs, of states, of outputs: outputs 127.7 / 98.9 / 97.0, 128.7 / 96.8 /
+    // 94.8, 127.5 / 96.8 / 94.8; states 108 / 91.3 / 84.6, 94.7 / 78.3 / 72.2, 107.8 / 90.9 / 85.0; pairs 132 / 115 / 119,
+    // 137 / 115 / 122, 134 / 120 / 117.  With `&& !failed` as the loop's condition: outputs 144 / 113 / 109.
+    if (!failed) {
+      if constexpr (PAIR) {
+        int n = 0;
+        for (int todo = NT - 1; todo > 0; --todo, ++n) {
+          step(std::true_type{}, n);
+          if (failed) break;
+        }
+        if (!failed) step(std::false_type{}, NT - 1);
+      } else if constexpr (STATE_ONLY) {
+        int n = 0;
+        for (; n + 1 < NT; ++n) {
+          step(std::true_type{}, n);
+          if (failed) break;
+        }
+        if (n + 1 >= NT) step(std::false_type{}, n);
+      } else {
+        for (int n = 0; n + 1 < NT; ++n) {
+          step(std::true_type{}, n);
+          if (failed) break;
+        }
+        if (!failed) step(std::false_type{}, NT - 1);
+      }
     }
 
     if (!failed && (p.ht != nullptr || (PAIR && p.push_on))) {
