@@ -19,9 +19,12 @@
 // instructions): P1 carries its own rolling B-fragment loads,
 // the decay row and the kg(hi) fragments; P2's first two passes carry kg(lo), its last pass the
 // next step's first fragments; the output tile is transposed in-warp (movmatrix) and stored one
-// step late.  The loads for the next step are made in the last step too and the next record's barrier is probed a pass
-// ahead, so that one branch (the slow path of that wait) cuts the step: K2 alone T4096 H64 201.5 -> 176.8 us,
-// state-only 156 -> 133.  Producer warp, stage ring, bounded waits: as in kda_k2_sm100.cu.
+// step late.  The last step, which has no next record, is an instantiation of its own, and the next record's barrier is
+// probed a pass ahead, so that one condition (the slow path of that wait) cuts a step behind the store of the previous
+// output.  K2 alone with conditions around the loads and now: T4096 H64 201 -> 172 us, T2048 H32 CTA-split in four 90 -> 79,
+// state-only T4096 H64 157 -> 130; one chunk, H32 in four 4.8 -> 4.4.  Producer warp, stage ring, bounded waits: as in kda_k2_sm100.cu.
+#include <type_traits>
+
 #include "kda_common.cuh"
 #include "kda_kernels.h"
 
@@ -195,7 +198,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       load_dec(sbase, 0, 16);
     }
 
-    for (int n = 0; n < NT && !failed; ++n) {
+    auto step = [&](auto more_c, int n) {
+      constexpr bool MORE = decltype(more_c)::value;   // chunk n + 1 exists
       const int s = n % K2M_STAGES;
       const uint32_t sp = sbase + s * SM::STAGE;
       const int s1 = (n + 1) % K2M_STAGES;
@@ -261,7 +265,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         ldsm_x4(sp + b3_off, ba[0], ba[1], ba[2], ba[3]);
         ldsm_x4(sp + b3_off + (REC_AQL - REC_AQK), bl[0], bl[1], bl[2], bl[3]);
       }
-      const bool next_ready = mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2M_STAGES) & 1) || n + 1 >= NT;
+      const bool next_ready = MORE ? mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2M_STAGES) & 1) : true;
       // P2 pass 2 (lo(v) * hi)
 #pragma unroll
       for (int np = 0; np < 8; ++np) {
@@ -298,14 +302,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
           asm volatile("" ::"r"(landed) : "memory");
           __syncwarp();
           if (lane == 0) mbar_arrive(empty0 + s * 8);
-          if (!__all_sync(0xffffffffu, next_ready)) {
+          if (MORE && !__all_sync(0xffffffffu, next_ready)) {
             if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + s1 * 8, ((n + 1) / K2M_STAGES) & 1, sAbort))) {
+              // the loads below are made all the same, out of a stage that a copy may still be writing: nothing of them
+              // is used, neither this step's output nor the state is stored
               if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_FULL_TIMEOUT); }
               failed = true;
             }
           }
         }
-        {
+        if (MORE) {
           if (np == 4) { load_b1(sp1, 0, 0); load_dec(sp1, 0, 6); }
           if (np == 5) { load_b1(sp1, 1, 1); load_dec(sp1, 6, 12); }
           if (np == 6) { load_u(sp1); load_dec(sp1, 12, 16); }
@@ -319,7 +325,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         o_st[1][0] = movmatrix_t(pack_bf16(oa[1][0], oa[1][1]));   // tokens 8..15
         o_st[1][1] = movmatrix_t(pack_bf16(oa[1][2], oa[1][3]));
       }
-    }
+    };
+    for (int n = 0; n + 1 < NT && !failed; ++n) step(std::true_type{}, n);
+    if (!failed) step(std::false_type{}, NT - 1);
 
     // the last chunk's output tile (it may be a partial chunk)
     if (!STATE_ONLY && !failed) {
