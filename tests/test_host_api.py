@@ -149,7 +149,7 @@ def test_record_index_maps_are_permutations():
     ui = layout._u_index("cpu")
     assert sorted(ui.tolist()) == list(range(16 * 128))
     # ldmatrix reads 8 rows at one 16-byte column unit: all eight must hit different units
-    units = sw.view(16, 128)[:8, 0] % 128 // 8
+    units = sw.view(16, 128)[:8, 0] % 64 // 8
     assert len(set(units.tolist())) == 8
 
 
