@@ -15,10 +15,12 @@ from tests.conftest import to_device
 pytestmark = pytest.mark.gpu
 
 
-def _args(d, o, ht, ws, prepared=False):
+def _args(d, o, ht, ws, prepared=False, flags=None, g_out=None):
+    if flags is None:
+        flags = 0 if prepared else api._flags(True, True, True)
     return api.make_args(d["q"], d["k"], d["v"], d["g"], d["beta"], scale=d["scale"], lower_bound=d["lower_bound"],
                          A_log=d["A_log"], dt_bias=d["dt_bias"], h0=d["initial_state"], o=o, ht=ht, workspace=ws,
-                         flags=0 if prepared else api._flags(True, True, True))
+                         flags=flags, g_out=g_out)
 
 
 def _buffers(B, T, H, dev):
@@ -62,6 +64,31 @@ def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
     for _ in range(3):
         got = _whole(d, B, T, H, cuda_device, prepared=prepared)
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+# K1 beside K2 is compiled for either gate type and centring, with all three of gate, l2-norm and sigmoid in the kernel, with
+# none of them (general centring only), and with the flags deciding (some of them, or debug outputs): all ten instances, in
+# front of either form of K2
+@pytest.mark.parametrize("B,T,H", [(2, 2400, 8), (1, 531, 75)])
+@pytest.mark.parametrize("g32", [False, True])
+@pytest.mark.parametrize("flags,lower_bound,debug", [(7, -5.0, False), (7, -8.0, False), (0, -5.0, False), (2, -5.0, False),
+                                                     (5, -5.0, False), (5, -8.0, False), (7, -5.0, True), (7, -8.0, True)])
+def test_beside_equals_after_in_every_instance_of_k1(cuda_device, B, T, H, g32, flags, lower_bound, debug):
+    d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.05), cuda_device)
+    d["lower_bound"] = lower_bound
+    if not flags & _lib.FLAG_GATE:
+        d["g"] = -d["g"].float().abs() * 0.1
+    if not flags & _lib.FLAG_L2NORM:
+        d["q"], d["k"] = (torch.nn.functional.normalize(d[n].float(), dim=-1).bfloat16() for n in ("q", "k"))
+    if not flags & _lib.FLAG_BETA_SIGMOID:
+        d["beta"] = d["beta"].sigmoid()
+    d["g"] = d["g"].float() if g32 else d["g"].bfloat16()
+    g_out = [torch.full((B, T, H, 128), float("nan"), device=cuda_device) if debug else None for _ in range(2)]
+    ref = _after(d, B, T, H, cuda_device, flags=flags, g_out=g_out[0])
+    got = _whole(d, B, T, H, cuda_device, flags=flags, g_out=g_out[1])
+    assert got[0].isfinite().all() and got[1].isfinite().all()
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+    assert not debug or torch.equal(g_out[0], g_out[1])
 
 
 def test_output_over_an_input(cuda_device):
