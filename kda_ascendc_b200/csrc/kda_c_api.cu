@@ -105,18 +105,22 @@ int check_k2(const KdaFwdArgs* a, bool state_only) {
 // How one head's 128x128 state is spread over warps.  The recurrence is a serial chain per head;
 // a warp alone on an SM sub-partition cannot overlap its own MMA issue with its other
 // instructions, so a step costs about 8 cycles per MMA plus its non-MMA instructions, and every
-// warp re-reads the shared operand tiles from shared memory.  Measured on B200 (T = 8192):
-// up to ~37 (batch x head) chains the 8-rows-per-warp "n8" form wins (two warps per SM while
-// chains x 8 CTAs fit the SMs, else four); beyond that the 16-rows-per-warp "m16" form with four
-// warps per CTA, which reads half the shared-memory bytes per MMA.  With more chains than SMs the
-// tensor-memory form (one CTA per chain, two per SM, tcgen05) is 10-35 % faster still once the
-// chains are a few chunks long: its set-up (TMEM allocation, the state in and out through
-// registers) costs about as much as two steps.  K2 alone against the 16-row form: 160 chains x 2 chunks 14.6 us
-// against 13.2, x 4 16.7 against 16.8; 296 chains x 1 12.8 against 13.9, x 4 17.4 against 21.1; 592 chains x 2 36.5
-// against 35.2; 160 chains x 64 95 against 136 -- hence from four chunks per chain on.  Between half as many chains as
-// SMs and as many (where the 16-row form needs two CTAs per chain and so more than one CTA per SM): 96 chains x 8 chunks
-// equal, x 16 23 against 27, x 32 41 against 47, x 64 68 against 85, x 256 232 against 311; up to half as many chains as
-// SMs the 16-row form wins at every length (74 chains x 256 chunks 175 against 229).  It has no state-only variant.
+// warp re-reads the shared operand tiles from shared memory.  Measured on B200, kda_fwd in us, chains x chunks:
+//   up to SMs/4 chains the 8-rows-per-warp "n8" form (two warps per SM while chains x 8 CTAs fit the SMs, else four), from
+//     there on the 16-rows-per-warp "m16" form with four warps per CTA, which reads half the shared-memory bytes per MMA:
+//     n8 / m16  37 x 8 14.4 / 16.3, 37 x 128 115 / 124, 37 x 512 418 / 465;  38 x 8 19.6 / 16.5, 38 x 128 177 / 137,
+//     38 x 512 669 / 521.
+//   more chains than SMs: the tensor-memory form (one CTA per chain, two per SM, tcgen05) from four chunks per chain on; its
+//     set-up (TMEM allocation, the state in and out through registers) costs about as much as two steps:
+//     m16 / tc  160 x 2 17.6 / 18.8, 160 x 4 24.7 / 24.7, 160 x 8 38.9 / 37.0;  296 x 2 22.6 / 22.6, 296 x 4 34.9 / 32.8;
+//     400 x 4 49.6 / 52.2, 400 x 6 64.4 / 64.1;  592 x 4 68.1 / 64.1.
+//   between half as many chains as SMs and as many (where m16 needs two CTAs per chain and so more than one per SM) from 32
+//     chunks on.  K2 alone tc is ahead from 12 chunks, but the forward follows late and less the more chains there are:
+//     m16 / tc  80 x 8 24.7 / 24.7, 80 x 16 39.4 / 37.8, 80 x 24 55.8 / 52.4, 80 x 32 71.1 / 63.1;  112 x 16 45.6 / 44.3,
+//     112 x 24 63.9 / 61.3, 112 x 32 80.5 / 78.6;  148 x 16 51.7 / 50.4, 148 x 24 71.9 / 73.8, 148 x 32 90.8 / 91.3,
+//     148 x 48 129.7 / 126.2.  The line is safe for all of them; below it 75 to 130 chains of 16 to 31 chunks give up 2 to 6 %.
+//   up to half as many chains as SMs m16 wins at every length (K2 alone, 74 chains x 256 chunks 175 / 229).
+// The tensor-memory form has no state-only variant.
 void pick_split(const KdaFwdArgs* a, bool state_only, int* vsplit, int* variant, int sms = 0, int chain_mult = 1) {
   if (sms <= 0) {   // the current device's SM count
     int dev = 0;
@@ -168,13 +172,14 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // time order and counts the finished items of every window of chunks; K2's producer warps wait for
 // the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA is
 // already running.  Where it pays, measured on B200 as the whole forward, K2 after K1 against beside it:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T32768 H16 1,036 -> 994 us,
-//     B2 T4096 H8 138.6 -> 137.0, B1 T8192 H16 267.0 -> 259.5;
-//   tensor-memory form with one CTA per SM: T8192 H96 889 -> 883, T2048 H80 220 -> 207, T1024 H96 129 -> 126 (with a K1
-//     of 112 registers, beside which it fits: see there),
-//     but T4096 H128 602 -> 631 (no SM is left to K1 alone): up to three quarters of the SMs.
-// Not in the other forms: with four consumer warps per CTA K2 has no issue slots to spare, or (8-row form)
-// does not fit beside two K1 CTAs: T8192 H32 418 -> 515, T4096 H48 317 -> 379.
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T32768 H16 1,028 -> 987 us,
+//     B1 T131072 H16 4,077 -> 3,856, B1 T8192 H16 266.5 -> 259.1, H8 236 -> 226, B2 T4096 H8 142.7 -> 142.5;
+//   tensor-memory form with one CTA per SM (and a K1 of 112 registers, beside which it fits: see there): T8192 H96
+//     878 -> 854, T2048 H80 214 -> 202, T1024 H96 126.8 -> 123.7, up to three quarters of the SMs.  There it no longer
+//     pays (T2048 H111 252 -> 254, T4096 H111 484 -> 494), and with a K2 CTA on almost every SM it costs (T4096 H128
+//     527 -> 556).
+// Not with four consumer warps per CTA in the 8-row form, which does not fit beside two K1 CTAs: T8192 H32 397 -> 490,
+// H24 361 -> 432, T4096 H37 216 -> 273.  The 16-row form cannot wait for windows.
 int beside_window(const KdaFwdArgs* a) {
   if (a->n_seqs > 0) return 0;
   int vsplit = 0, variant = 0;
@@ -373,9 +378,12 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   if (variant == 4) {
     // Tail wave.  The tensor-memory form holds two chains per SM at once; when the chains left over
     // after the full waves are at most half as many as SMs, they run faster in an mma.sync form
-    // (16-row: two CTAs per chain, one per SM, 0.8 us per step; 8-row for at most SMs/4 chains,
-    // 0.55 us per step; against 1.3 us for a lone tensor-memory CTA), launched behind the full
-    // waves.  Only for the automatic choice.
+    // (8-row for at most SMs/4 chains, 0.49 us per step; 16-row: two CTAs per chain, one per SM, 0.65 us
+    // per step; against 0.9 for a lone tensor-memory CTA), launched behind the full waves, at every length that the
+    // tensor-memory form is chosen for.  kda_fwd in us, no tail / 16-row / 8-row, 296 chains and so many more x chunks:
+    // 9 x 4 45.5 / 43.4 / 41.3, 9 x 64 335 / 325 / 306; 37 x 4 47.3 / 45.0 / 45.2, 37 x 64 353 / 342 / 331; 38 x 4 47.9 /
+    // 45.3 / 47.4, 38 x 64 353 / 343 / 363; 74 x 4 49.7 / 47.7 / 50.5, 74 x 64 374 / 365 / 389; 75 x 4 50.7 / 52.6,
+    // 75 x 64 375 / 400.  Only for the automatic choice.
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const long long bh = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;

@@ -96,9 +96,8 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// One lane of a converged warp, chosen by the hardware.  The compiler knows that a branch on it is taken by one
-// thread; behind `lane == 0` it does not, and wraps every tcgen05 instruction in a loop over the lanes that may be
-// there (eight tcgen05.mma M128 N32 issue in 37 cycles behind elect.sync, in 402 behind lane == 0).
+// One lane of a converged warp, chosen by the hardware.  Measured: eight tcgen05.mma M128 N32 issue in 37 cycles behind
+// elect.sync and in 402 behind `lane == 0`, presumably because only the former tells the compiler that one thread is there.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
@@ -331,9 +330,6 @@ __device__ __forceinline__ uint32_t movmatrix_t(uint32_t a) {
   uint32_t d;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
   return d;
-}
-__device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t& r0, uint32_t& r1) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
 __device__ __forceinline__ void ldsm_x2_t(uint32_t addr, uint32_t& r0, uint32_t& r1) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));

@@ -102,11 +102,12 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // BESIDE: K2 runs beside this kernel (time-major items, finished items counted per window).  Registers: four CTAs per
 // SM need 128 a thread or fewer.  Beside K2, two CTAs share every SM sub-partition's 16,384 registers with up to three
 // warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
-// start before K1 ends (T8192 H96, whole forward: 1,254 us with 128 registers, 883 with 112).
+// start before K1 ends.  kda_fwd, with 128 registers and with 112: T8192 H96 1,223 and 849 us, T2048 H80 303 and 201;
+// beside the 8-row form both fit (T32768 H16 988 and 990, B2 T4096 H8 135.1 and 135.6).
 // FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel; FORM_NONE: all
-// three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags decide.  Without the
-// conditions between its loops K1 takes, T8192 H32 154.2 -> 149.9 us, H96 447 -> 433 (beside K2 the whole forward
-// 887 -> 847); inputs prepared by the caller, B8 T2037 H32 with 8 q/k heads, 297 -> 274.
+// three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags decide.  Against
+// FORM_ANY for the same call: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs prepared by the caller (B8 T2037
+// H32 with 8 q/k heads) 294 -> 274; kda_fwd T8192 H96 881 -> 849, the prepared batch 474 -> 454.
 enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
 template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {

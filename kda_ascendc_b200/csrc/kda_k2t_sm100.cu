@@ -15,11 +15,11 @@
 // pass over them.
 //
 // A step is a chain of hand-overs: eight MMAs, commit and wait about 190 cycles, P2 300, a TMEM load 140, the state pass
-// 600.  One CTA alone on its SM takes 0.88 us per step (the 8-row mma.sync form 0.38 to 0.49), two resident ones 1.55
+// 600.  One CTA alone on its SM takes 0.88 us per step (the 8-row mma.sync form 0.37 to 0.49), two resident ones 1.55
 // together (256 of the 512 TMEM columns, 88 KB of shared memory each): the form pays once there are enough chains.
-// Every tcgen05 instruction is issued behind elect.sync by a warp that walks the loop as a whole; behind lane == 0 the
-// compiler wraps it in a loop over the lanes.  K2 alone with that and records loaded by tiled copies, and now:
-// T8192 H96 605 -> 447 us, B8 T1024 H32 111 -> 98.
+// Every tcgen05 instruction is issued behind elect.sync (see elect_one) by a warp that walks the loop as a whole.  K2
+// alone with the instructions behind lane == 0 and records loaded by tiled copies, and now: T8192 H96 606 -> 447 us,
+// B8 T1024 H32 110.5 -> 98.6.
 //
 // Warp roles: 0-7 element-wise work (warp w: TMEM lanes 32 (w%4).., column / token half w/4),
 // 8 = producer (TMA), 9 = MMA issuer and TMEM owner.  Every wait is bounded.
