@@ -67,8 +67,10 @@ K2_FLOPS_PER_CHUNK = 1638400.0
 # dram__bytes_read.sum + dram__bytes_write.sum of ONE launch of each kernel on the headline shape, from
 # an ncu capture (profiles/kda_k1_k2_B1_T8192_H32.md, which names the commit it was taken at).  It is
 # reported only for that shape and only while the record layout it was captured with is current.
-NCU_TRAFFIC = dict(shape=(1, 8192, 32), record_bytes=26112, source="profiles/kda_k1_k2_B1_T8192_H32.md",
-                   bytes={"kda_k1": 642.14e6, "kda_k2": 489.44e6})
+NCU_TRAFFIC = dict(shape=(1, 8192, 32), source="profiles/kda_k1_k2_B1_T8192_H32.md",
+                   record=dict(REC_W=0, REC_QG=2048, REC_HALF=4096, REC_KGH=8192, REC_KGL=12288, REC_AQK=16384, REC_AQL=16640,
+                               REC_DEC=17408, REC_U=17920, REC_BYTES=26112),
+                   bytes={"kda_k1": 642.58e6, "kda_k2": 488.83e6})
 
 
 def merge_exchange_marks(names, values):
@@ -304,7 +306,7 @@ def _view_args(api, d, sl_h, o, ht, ws, h0):
 
 def run_gpu_arm(steps, warmup, n_gpus, kernels_only=False):
     import kda_ascendc_b200 as K
-    from kda_ascendc_b200 import _lib, api, shard
+    from kda_ascendc_b200 import _lib, api, layout, shard
 
     rank = int(os.environ.get("RANK", "0"))
     local_rank = int(os.environ.get("LOCAL_RANK", "0"))
@@ -609,7 +611,7 @@ def run_gpu_arm(steps, warmup, n_gpus, kernels_only=False):
                               tensor_frac=tf / tc_tflops)
         dom = "kda_k2" if k2_avg >= k1_avg else "kda_k1"
         traffic = None
-        if NCU_TRAFFIC["shape"] == (B, T, H) and NCU_TRAFFIC["record_bytes"] * chunks + 256 == K.workspace_bytes(B, T, H):
+        if NCU_TRAFFIC["shape"] == (B, T, H) and all(getattr(layout, n) == at for n, at in NCU_TRAFFIC["record"].items()):
             traffic = NCU_TRAFFIC["bytes"].get(dom)
         roofline = dict(kernel=dom, bound="hbm", achieved=kern[dom]["algorithmic_GBps"], peak=hbm_gbs, unit="GB/s",
                         frac=kern[dom]["hbm_frac"], traffic=traffic,
