@@ -165,35 +165,62 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
   return {lo, lo + static_cast<uintptr_t>(last) * elem_bytes};
 }
 
-// Chunks per window of a forward whose K2 runs beside its K1; 0 = K2 starts after K1.
+// A forward whose K2 runs beside its K1, on part of the chip.
 //
-// A K2 whose chains leave most of the chip idle runs on the SMs that K1 is still working on: K1 is held to
-// two CTAs per SM (that leaves a K2 CTA its shared memory and registers), walks the chunks of all chains in
-// time order and counts the finished items of every window of chunks; K2's producer warps wait for
-// the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA is
-// already running.  Where it pays, measured on B200 as the whole forward, K2 after K1 against beside it:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs): B1 T32768 H16 1,028 -> 987 us,
-//     B1 T131072 H16 4,077 -> 3,856, B1 T8192 H16 266.5 -> 259.1, H8 236 -> 226, B2 T4096 H8 142.7 -> 142.5;
-//   tensor-memory form with one CTA per SM (and a K1 of 112 registers, beside which it fits: see there): T8192 H96
-//     878 -> 854, T2048 H80 214 -> 202, T1024 H96 126.8 -> 123.7, up to three quarters of the SMs.  There it no longer
-//     pays (T2048 H111 252 -> 254, T4096 H111 484 -> 494), and with a K2 CTA on almost every SM it costs (T4096 H128
-//     527 -> 556).
-// Not with four consumer warps per CTA in the 8-row form, which does not fit beside two K1 CTAs: T8192 H32 397 -> 490,
-// H24 361 -> 432, T4096 H37 216 -> 273.  The 16-row form cannot wait for windows.
-int beside_window(const KdaFwdArgs* a) {
-  if (a->n_seqs > 0) return 0;
-  int vsplit = 0, variant = 0;
-  const int sms = device_sms();
-  pick_split(a, false, &vsplit, &variant, sms);
+// K1 walks the chunks of all chains in time order and counts the finished items of every window of chunks; K2's producer
+// warps wait for the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA
+// is already running.  On k2_sms of the SMs only k2_sm_ctas of K1's CTAs stay (k1_stays), and K2's CTAs fit nowhere else.
+// Which of it pays, measured on B200 as the whole forward in us, K2 after K1 against beside it unless said otherwise:
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on K2's SMs: B1 T32768 H16 1,028 /
+//     987, T8192 H16 266.5 / 259.1, H8 236 / 226.  With one K1 CTA there K1 is the longer part (T32768 H16 1,329).
+//   Up to 23 of 148 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H19 337 / 296, H22
+//     351 / 293, T2500 H19 113 / 110, H23 117 / 115.  Beyond, K1 has too few SMs left: T8192 H24 360 / 363, T2500 H25 121 / 134.
+//   From there to 42 of 148 chains: the 16-row form, whose bits are the same, on SMs of its own (2 per chain), at chunk counts
+//     that make up for its longer step: T8192 H24 360 / 352, H32 397 / 355, H37 418 / 393, H38 511 / 410, H40 519 / 447; T4096
+//     H23 184 / 189, H25 189 / 189, H28 195 / 189, H34 208 / 192, H38 256 / 209, H42 265 / 248; T2048 H32 109 / 109, H40 137 /
+//     126, H42 138 / 136; T2500 H25 121 / 126, H30 127 / 129; T1600 H38 109 / 97, H42 112 / 112, H43 113 / 117; T1100 H37 67 /
+//     74, H40 80 / 78, H42 81 / 83.  With a K1 CTA beside K2's: T8192 H32 403.
+//   Tensor-memory form with one CTA per SM and two K1 CTAs there (a K1 of 112 registers: see there), four on the other SMs,
+//     against two everywhere up to 111 chains and after K1 beyond: T8192 H96 850 / 721, T4096 H75 371 / 337, H111 493 / 442, T1024
+//     H75 105 / 104, H96 123 / 115, H111 134 / 124; T1024 H120 142 / 135, T4096 H120 504 / 493, H128 524 / 521, H136 545 / 560.
+//   The same form, two CTAs per SM on SMs of their own, where its step for two (1.36 us) and K1 on the others take the same
+//     time, and long chains: against the line above T8192 H88 689 / 690, H96 721 / 701, H104 782 / 780, H111 839 / 857, T2048
+//     H96 198 / 199, T512 H96 68.6 / 75.4.
+struct Beside {
+  int win;                       // chunks per window; 0 = K2 starts after K1
+  int variant, vsplit;           // K2's form: pick_split's, or one with the same bits
+  int sms, k2_sms, k2_sm_ctas;   // see K1Params
+};
+
+Beside beside_plan(const KdaFwdArgs* a) {
+  Beside r = {};
+  if (a->n_seqs > 0) return r;
+  r.sms = device_sms();
+  pick_split(a, false, &r.vsplit, &r.variant, r.sms);
   const long long chains = static_cast<long long>(a->B) * a->H, nt = (static_cast<long long>(a->T) + kda::BT - 1) / kda::BT;
-  if (!(variant == 1 && vsplit >= 8 && chains * vsplit <= sms) && !(variant == 4 && chains * 4 <= 3LL * sms)) return 0;
-  const long long round = 2LL * sms;   // items that K1 has in flight
-  if (chains * nt < 8 * round) return 0;   // K1 is over in a few rounds: nothing to run beside
+  const bool automatic = a->k2_variant == 0 && a->k2_vsplit == 0;
+  long long k2_sms = 0;
+  if (r.variant == 1 && r.vsplit >= 8 && chains * r.vsplit <= r.sms) {
+    k2_sms = chains * r.vsplit; r.k2_sm_ctas = 2;
+  } else if (automatic && r.variant == 1 && chains * 32 <= 5LL * r.sms) {
+    k2_sms = chains * 4;
+  } else if (automatic && ((r.variant == 1 && chains * nt >= 6400) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 96))) {
+    k2_sms = chains * 2; r.variant = 3; r.vsplit = 2;
+  } else if (r.variant == 4 && chains * 5 > 3LL * r.sms && chains * 10 <= 7LL * r.sms && nt >= 512) {
+    k2_sms = (chains + 1) / 2;
+  } else if (r.variant == 4 && chains * 6 <= 5LL * r.sms) {
+    k2_sms = chains; r.k2_sm_ctas = 2;
+  } else {
+    return r;
+  }
+  r.k2_sms = static_cast<int>(k2_sms);
+  const long long round = 2LL * r.sms;   // items that K1 has in flight
+  if (chains * nt < 8 * round) return r;   // K1 is over in a few rounds: nothing to run beside
   // o is written while K1 still reads its inputs: they may not overlap (h0 and ht are safe: a chain's final
   // state is written once every window, so every item of K1, is finished)
   const int64_t* os = a->o_stride;
   for (int i = 0; i < 3; ++i)
-    if (os[i] < 0 || a->beta_stride[i] < 0) return 0;
+    if (os[i] < 0 || a->beta_stride[i] < 0) return r;
   const int hq = a->Hq > 0 ? a->Hq : a->H;
   const Span o = span_of(a->o, os, a, a->H, kda::D, 2);
   const Span in[7] = {span_of(a->q, a->q_stride, a, hq, kda::D, 2), span_of(a->k, a->k_stride, a, hq, kda::D, 2),
@@ -204,12 +231,15 @@ int beside_window(const KdaFwdArgs* a) {
                       {reinterpret_cast<uintptr_t>(a->dt_bias),
                        reinterpret_cast<uintptr_t>(a->dt_bias + (a->dt_bias ? static_cast<int64_t>(a->H) * kda::D : 0))}};
   for (const Span& s : in)
-    if (o.lo < s.hi && s.lo < o.hi) return 0;
-  const long long by_count = (nt + kda::MAX_WINDOWS - 1) / kda::MAX_WINDOWS, by_round = (2 * round + chains - 1) / chains;
-  return static_cast<int>(by_count > by_round ? by_count : by_round);
+    if (o.lo < s.hi && s.lo < o.hi) return r;
+  // windows of two rounds of K1, where it has most SMs to itself of one: T8192 H32 359 -> 355, but B2 T4096 H8 138 -> 145
+  const long long by_count = (nt + kda::MAX_WINDOWS - 1) / kda::MAX_WINDOWS;
+  const long long by_round = ((r.k2_sm_ctas == 0 ? 1 : 2) * round + chains - 1) / chains;
+  r.win = static_cast<int>(by_count > by_round ? by_count : by_round);
+  return r;
 }
 
-int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
+int do_k1(const KdaFwdArgs* a, cudaStream_t st, const Beside& side = Beside{}) {
   kda::K1Params p;
   memset(&p, 0, sizeof(p));
   p.q = static_cast<const __nv_bfloat16*>(a->q);
@@ -239,11 +269,11 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
   }
   p.Hq = a->Hq > 0 ? a->Hq : a->H;
   p.div_g.set(static_cast<uint32_t>(p.H / p.Hq));
-  if (win_chunks > 0) {
+  if (side.win > 0) {
     p.progress = status_ptr(a) + kda::HDR_PROGRESS;
-    p.ctas_per_sm = 2;   // with one, K1 becomes the longer of the two (T8192 H96 1,338 us); three do not fit beside K2
+    p.n_sms = side.sms; p.k2_sms = side.k2_sms; p.k2_sm_ctas = side.k2_sm_ctas;
     p.div_b.set(static_cast<uint32_t>(p.B));
-    p.div_win.set(static_cast<uint32_t>(win_chunks) * p.B * p.H);
+    p.div_win.set(static_cast<uint32_t>(side.win) * p.B * p.H);
   }
   // 2^g may be factored as 2^(g-g_mid) * 2^(g_mid) only while no factor can underflow:
   // 16 tokens * |lower_bound| * RCP_LN2 must stay inside the fp32 exponent range.
@@ -285,7 +315,7 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, int win_chunks = 0) {
 struct H0Flags { const int32_t* flags; int n, epoch; };
 
 int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, const KdaPeerPushArgs* push = nullptr,
-          const H0Flags* h0f = nullptr, bool after_k1 = false, int win_chunks = 0) {
+          const H0Flags* h0f = nullptr, bool after_k1 = false, const Beside& side = Beside{}) {
   kda::K2Params p;
   memset(&p, 0, sizeof(p));
   p.rec = rec_ptr(a);
@@ -298,9 +328,9 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   p.scale = a->scale;
   p.zero_u = zero_u == 1;
   p.k_first = (a->flags & KDA_FLAG_STATE_K_FIRST) ? 1 : 0;
-  if (win_chunks > 0) {
+  if (side.win > 0) {
     p.progress = status_ptr(a) + kda::HDR_PROGRESS;
-    p.win_chunks = win_chunks;
+    p.win_chunks = side.win;
   }
   p.pair_mode = (state_only && zero_u == 2) ? 1 : 0;
   if (a->n_seqs > 0) {
@@ -309,6 +339,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   }
   int vsplit = 4, variant = 3;
   pick_split(a, state_only, &vsplit, &variant);
+  if (side.win > 0) { vsplit = side.vsplit; variant = side.variant; }
   if (after_k1) {
     // Launched ahead of K1's end: K2's CTAs are set up (barriers, tensor memory, the initial state) on the SMs
     // that K1 leaves.  Whole forward on B200, ordinary launch against this one: B1 T100 H32 17.0 -> 14.9 us, T512
@@ -322,9 +353,10 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     // eight 0.97, nine to 16 1.03, more 1.04 and up to 1.31 (16 sequences, H8, the longest 264 chunks of 460: 285 -> 372 us).
     const long long chains = static_cast<long long>(a->n_seqs > 0 ? a->n_seqs : a->B) * a->H;
     const bool uneven = a->n_seqs > 0 && variant == 3 && chains * vsplit > device_sms() && steps > 8;
-    p.pdl = win_chunks > 0 || (variant != 5 && !(variant == 1 && vsplit == 4 && steps > 32) && !uneven);
+    p.pdl = side.win > 0 || (variant != 5 && !(variant == 1 && vsplit == 4 && steps > 32) && !uneven);
     // without the bound on the CTAs per SM: T1024 H8 48.2 us
-    p.one_per_sm = p.pdl && win_chunks == 0 && chains * (variant == 4 ? 1 : vsplit) <= device_sms();
+    p.one_per_sm = p.pdl && (side.win > 0 ? side.k2_sm_ctas == 0 && chains * (variant == 4 ? 1 : vsplit) <= side.k2_sms
+                                         : chains * (variant == 4 ? 1 : vsplit) <= device_sms());
   }
   if (p.pair_mode) {
     p.k_first = 0;   // the transforms are always written [chains][2][V][K]
@@ -442,25 +474,25 @@ int kda_fwd(const KdaFwdArgs* a, void* stream) {
   if (int rc = check_k1(a)) return rc;
   if (int rc = check_k2(a, false)) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int win = beside_window(a);
-  if (win > 0) {   // the window counters must be zero before either kernel starts
+  const Beside side = beside_plan(a);
+  if (side.win > 0) {   // the window counters must be zero before either kernel starts
     cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
     if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));
   }
-  if (int rc = do_k1(a, st, win)) return rc;
-  return do_k2(a, false, 0, st, nullptr, nullptr, true, win);
+  if (int rc = do_k1(a, st, side)) return rc;
+  return do_k2(a, false, 0, st, nullptr, nullptr, true, side);
 }
 
 int kda_selftest_window_wait(const KdaFwdArgs* a, void* stream) {
   g_launches = 0;
   if (int rc = check_k1(a)) return rc;
   if (int rc = check_k2(a, false)) return rc;
-  const int win = beside_window(a);
-  if (win == 0) return fail(KDA_ERR_INVALID_ARG, "kda: K2 does not run beside K1 for this problem%s", "");
+  const Beside side = beside_plan(a);
+  if (side.win == 0) return fail(KDA_ERR_INVALID_ARG, "kda: K2 does not run beside K1 for this problem%s", "");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(status_ptr(a) + kda::HDR_PROGRESS, 0, kda::MAX_WINDOWS * sizeof(int), st);
   if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));
-  return do_k2(a, false, 0, st, nullptr, nullptr, false, win);
+  return do_k2(a, false, 0, st, nullptr, nullptr, false, side);
 }
 
 int kda_fwd_k1(const KdaFwdArgs* a, void* stream) {

@@ -49,9 +49,12 @@ constexpr int REC_BYTES = 26112;
 constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the workspace
 // Header words: 0 = status; HDR_K1_STATUS = K1's own code, which no later kernel overwrites (K2 waits for K1, so a K1
 // that gave up makes K2's waits run out after it; a first-one-wins exchange in K2 instead costs its 8-row form 0.7 %:
-// T8192 H32 411.7 -> 414.5 us); HDR_PROGRESS .. HDR_PROGRESS + MAX_WINDOWS - 1 = finished K1 items per window of
-// chunks, for a K2 that runs beside K1 (zeroed before K1 starts; unused otherwise)
+// T8192 H32 411.7 -> 414.5 us); for a K2 that runs beside K1 (zeroed before K1 starts; unused
+// otherwise) HDR_TICKET = K1 items handed out, HDR_ARRIVED = K1 CTAs that have started, HDR_PROGRESS .. = finished K1 items
+// per window of chunks
 constexpr int HDR_K1_STATUS = 1;
+constexpr int HDR_TICKET = 2;
+constexpr int HDR_ARRIVED = 3;
 constexpr int HDR_PROGRESS = 4;
 constexpr int MAX_WINDOWS = WS_HEADER_BYTES / 4 - HDR_PROGRESS;
 
@@ -307,6 +310,12 @@ __device__ __forceinline__ float4 lds_f32x4(uint32_t addr) {
   return v;
 }
 
+__device__ __forceinline__ uint4 lds_u32x4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 // a 4-byte global store by the lanes for which c holds, without a branch
 __device__ __forceinline__ void stg_u32_if(void* p, uint32_t v, bool c) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.global.u32 [%0], %1;\n\t}" ::"l"(p), "r"(v),
@@ -324,6 +333,12 @@ __device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t& r0, uint32_t&
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
                : "r"(addr));
+}
+// four 8x8 b16 matrices in fragment layout, transposed: lane 8 i + r gives the address of row r of matrix i^T
+__device__ __forceinline__ void stsm_x4_t(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2),
+               "r"(r3)
+               : "memory");
 }
 // transpose an 8x8 b16 matrix held as one register per lane (fragment layout) inside the warp
 __device__ __forceinline__ uint32_t movmatrix_t(uint32_t a) {
@@ -393,6 +408,11 @@ __device__ __forceinline__ void split_pack2(float2 x, uint32_t& hi, uint32_t& lo
   hi = pack_bf16(x.x, x.y);
   const float2 r = __ffma2_rn(make_float2(bf16_lo_to_f32(hi), bf16_hi_to_f32(hi)), make_float2(-1.f, -1.f), x);
   lo = pack_bf16(r.x, r.y);
+}
+// u - (a + b) of two neighbours of an accumulator fragment, as a hi/lo pair
+__device__ __forceinline__ void split_pack_diff(float2 u, const float* a, const float* b, uint32_t& hi, uint32_t& lo) {
+  const float2 s = __fadd2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
+  split_pack2(__fadd2_rn(u, make_float2(-s.x, -s.y)), hi, lo);
 }
 __device__ __forceinline__ float rcpf(float x) {
   float y;

@@ -57,7 +57,7 @@ struct K1Smem {
   static constexpr int TOT = BETA + 144;      // fp32 [2][128]: column sums of the gate over rows 0..7 and rows 8..15
   static constexpr int GMID = TOT + 1024;     // fp32 [128] g[mid] (not needed with FAST_EXP)
   static constexpr int MBAR = GMID + (FAST_EXP ? 0 : 512);
-  static constexpr int FLAG = MBAR + 8;
+  static constexpr int FLAG = MBAR + 8;   // a wait gave up; the item after the next one (beside K2)
   static constexpr int TOTAL = FLAG + 8;
 };
 
@@ -109,6 +109,33 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // FORM_ANY for the same call: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs prepared by the caller (B8 T2037
 // H32 with 8 q/k heads) 294 -> 274; kda_fwd T8192 H96 881 -> 849, the prepared batch 474 -> 454.
 enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
+//
+// Beside K2 the work is handed out item by item, and not every SM does the same share of it: on k2_sms of the SMs (spread
+// evenly) only the first k2_sm_ctas CTAs of this kernel stay, and K2's CTAs, which find no room on the others, are placed
+// there.  The first ones, by the warp slots they run in, so that the registers and the shared memory that become free lie together:
+// with two other CTAs staying (as they came) a tensor-memory K2 found no room on some SMs until K1 ended (T8192 H96
+// 720 -> 1,200 us).  Those that leave wait until the whole grid has started, so that no later CTA takes their place,
+// and until somebody stays.  Where that takes longer than 20 us they stay too: all this decides about speed only, whoever
+// stays takes items until none is left.
+__device__ __forceinline__ bool k1_stays(const K1Params& p) {
+  uint32_t sm, slot;
+  asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+  asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+  int* arrived = p.progress - HDR_PROGRESS + HDR_ARRIVED;
+  const bool stays = sm >= static_cast<uint32_t>(p.n_sms) || (sm * p.k2_sms) % p.n_sms >= static_cast<uint32_t>(p.k2_sms) ||
+                     slot < static_cast<uint32_t>(4 * p.k2_sm_ctas);
+  constexpr int STAYS = 1 << 16;   // started CTAs in the lower half of the word (a grid is below 65,536), staying ones above
+  atomicAdd(arrived, stays ? STAYS + 1 : 1);
+  if (stays) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  do {
+    int n;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
+    if ((n & (STAYS - 1)) == static_cast<int>(gridDim.x) && n >= STAYS) return false;
+  } while (globaltimer_ns() - t0 < 20000ull);
+  return true;
+}
+
 template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -143,6 +170,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     mbar_init(mbar, 1);
     sFlag[0] = 0;   // a wait gave up
     fence_mbar_init();
+    if (BESIDE) sFlag[1] = k1_stays(p) ? atomicAdd(p.progress - HDR_PROGRESS + HDR_TICKET, 2) : n_items;
   }
   __syncthreads();
 
@@ -224,7 +252,9 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     }
   };
 
-  int id = blockIdx.x;
+  int id = BESIDE ? sFlag[1] : blockIdx.x;
+  int id_next = BESIDE ? id + 1 : id + static_cast<int>(gridDim.x);
+  if (BESIDE) __syncthreads();   // read by everyone before thread 0 puts the next one there
   K1Item cur{}, nxt{};
   Par par{}, par_next{};
   if (id < n_items) {
@@ -249,12 +279,14 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     }
   };
 
-  for (int it = 0; id < n_items; ++it, id += gridDim.x) {
+  for (int it = 0; id < n_items; ++it, id = id_next, id_next = BESIDE ? sFlag[1] : id_next + static_cast<int>(gridDim.x)) {
     const int b = cur.b, h = cur.h, t0 = cur.t0, nvalid = cur.nvalid;
     uint8_t* rec = p.rec + cur.rec_idx * REC_BYTES;
-    const bool has_next = id + static_cast<int>(gridDim.x) < n_items;
+    const bool has_next = id_next < n_items;
+    int ticket = n_items;   // thread 0: the item after the next one, on its way while this one is worked on
     if (has_next) {
-      nxt = k1_item<BESIDE>(p, id + gridDim.x);
+      if (BESIDE && tid == 0) ticket = atomicAdd(p.progress - HDR_PROGRESS + HDR_TICKET, 1);
+      nxt = k1_item<BESIDE>(p, id_next);
       par_next = load_params(nxt);
     }
     const float bias0 = par.bias0, bias1 = par.bias1;
@@ -612,6 +644,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       done = 0;
       fence_proxy_async_all();   // u left by plain stores, K2 reads it with bulk copies
     }
+    if (BESIDE && tid == 0) sFlag[1] = ticket;
     __syncthreads();   // also orders phase E's reads of X / KB / VB before the next item rewrites them
     if (tid == 0) {
       bulk_s2g(rec + REC_W, sbase + S_WST, TILE_BYTES / 2);
@@ -650,8 +683,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
     residency[dev].store(res, std::memory_order_release);
   }
   const long long n_items = (p.chunk_table != nullptr ? static_cast<long long>(p.n_chunks) : static_cast<long long>(p.B) * p.NT) * p.H;
-  const int sms = res >> 8, fit = res & 255;
-  const int cap = sms * (p.ctas_per_sm > 0 && p.ctas_per_sm < fit ? p.ctas_per_sm : fit);   // persistent: one CTA per slot
+  const int cap = (res >> 8) * (res & 255);   // persistent: one CTA per slot
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
   kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, FORM><<<grid, 128, smem_bytes, stream>>>(p);
   return cudaGetLastError();

@@ -291,11 +291,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       uint32_t bvh[NVT][2], bvl[NVT][2];
 #pragma unroll
       for (int nv = 0; nv < NVT; ++nv) {
-        const float x0 = u[nv].x - (pw[0][nv][0] + pw[1][nv][0]), x1 = u[nv].y - (pw[0][nv][1] + pw[1][nv][1]);
-        const float x2 = u[nv].z - (pw[0][nv][2] + pw[1][nv][2]), x3 = u[nv].w - (pw[0][nv][3] + pw[1][nv][3]);
         uint32_t h01, l01, h23, l23;
-        split_pack(x0, x1, h01, l01);
-        split_pack(x2, x3, h23, l23);
+        split_pack_diff(make_float2(u[nv].x, u[nv].y), &pw[0][nv][0], &pw[1][nv][0], h01, l01);
+        split_pack_diff(make_float2(u[nv].z, u[nv].w), &pw[0][nv][2], &pw[1][nv][2], h23, l23);
         bvh[nv][0] = movmatrix_t(h01); bvh[nv][1] = movmatrix_t(h23);
         bvl[nv][0] = movmatrix_t(l01); bvl[nv][1] = movmatrix_t(l23);
       }
@@ -346,7 +344,11 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
           for (int nv = 0; nv < NVT; ++nv) {
             if (m == 0) {
 #pragma unroll
-              for (int e = 0; e < 4; ++e) oa[nv][e] = p.scale * (pq[0][nv][e] + pq[1][nv][e]);
+              for (int e = 0; e < 4; e += 2) {
+                const float2 x = __fmul2_rn(make_float2(p.scale, p.scale), __fadd2_rn(make_float2(pq[0][nv][e], pq[0][nv][e + 1]),
+                                                                                      make_float2(pq[1][nv][e], pq[1][nv][e + 1])));
+                oa[nv][e] = x.x; oa[nv][e + 1] = x.y;
+              }
               mma_bf16_v(oa[nv], ah3, bvh[nv][0], bvh[nv][1]);
             }
             if (m == 3) mma_bf16_v(oa[nv], ah3, bvl[nv][0], bvl[nv][1]);

@@ -18,10 +18,12 @@
 // holds the sub-partition's issue port for 8 cycles; the step time is 8 x MMAs + 2 x the other
 // instructions): P1 carries its own rolling B-fragment loads,
 // the decay row and the kg(hi) fragments; P2's first two passes carry kg(lo), its last pass the
-// next step's first fragments; the output tile is transposed in-warp (movmatrix) and stored one
-// step late.  The last step, which has no next record, is an instantiation of its own, and the next record's barrier is
+// next step's first fragments; the output tile is transposed through 512 bytes of a warp's own
+// (stmatrix) and leaves one step late, 16 bytes a lane, as whole 32-byte sectors (four 4-byte stores behind movmatrix before:
+// K2 alone T4096 H64 172 -> 167 us, the forward T8192 H32 with K2 on SMs of its own 381 -> 363).  The last step, which has no next record, is an instantiation of its own, and the next record's barrier is
 // probed a pass ahead, so that one condition (the slow path of that wait) cuts a step behind the store of the previous
-// output.  K2 alone with conditions around the loads and now: T4096 H64 201 -> 172 us, T2048 H32 CTA-split in four 90 -> 79,
+// output.  P1's sums run over even and odd k-steps apart, as in the 8-row form, so that both forms give the same bits (T8192
+// H32 298 -> 303 us).  K2 alone with conditions around the loads and now: T4096 H64 201 -> 172 us, T2048 H32 CTA-split in four 90 -> 79,
 // state-only T4096 H64 157 -> 130; one chunk, H32 in four 4.8 -> 4.4.  Producer warp, stage ring, bounded waits: as in kda_k2_sm100.cu.
 #include <type_traits>
 
@@ -30,24 +32,25 @@
 
 namespace kda {
 
-constexpr int K2M_STAGES = 4;
-
-template <int CW>
+// STAGES: 8 on an SM of its own beside K1, which holds up the records now and then (T8192 H32 363 -> 355 us); else 4
+template <int CW, int STAGES>
 struct K2mSmem {
   static constexpr int STAGE = REC_SHARED_BYTES + CW * 2 * REC_U_TILE_BYTES;   // 16 rows = two 8-column u tiles
-  static constexpr int BARS = K2M_STAGES * STAGE;
-  static constexpr int FLAG = BARS + 2 * K2M_STAGES * 8;
-  static constexpr int TOTAL = FLAG + 16;
+  static constexpr int BARS = STAGES * STAGE;
+  static constexpr int FLAG = BARS + 2 * STAGES * 8;
+  static constexpr int OST = FLAG + 16;              // a warp's output tile: [16 tok][16 v] bf16
+  static constexpr int TOTAL = OST + CW * 512;
+  static_assert(OST % 16 == 0, "the output tile is written and read 16 bytes at a time");
 };
 
 // MINB = CTAs that must fit on one SM.  With 2 (register cap 168) eight consumer warps share an
 // SM; that pays as soon as there are more CTAs than SMs (measured: B1 T8192 H96 765 -> 677 us),
 // while a grid that fits in one wave is faster with the uncapped registers.
 // ORD: packed sequences, longest first
-template <int CW, bool STATE_ONLY, int MINB, bool ORD = false>
+template <int CW, bool STATE_ONLY, int MINB, bool ORD = false, int K2M_STAGES = 4>
 __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  using SM = K2mSmem<CW>;
+  using SM = K2mSmem<CW, K2M_STAGES>;
   constexpr int NV = 8 / CW;            // CTAs per (batch, head)
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -90,9 +93,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   if (warp == CW) {
     // ------------------------------ producer -------------------------------
     if (lane == 0) {
-      grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
         const int s = n % K2M_STAGES;
+        if (p.progress != nullptr && n == gate) {
+          if (!window_wait_bounded(p.progress + n / p.win_chunks, min(p.win_chunks, NT - n) * p.B * p.H, sAbort)) {
+            if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K1_WINDOW_TIMEOUT); }
+            break;
+          }
+          gate += p.win_chunks;
+        }
         if (n >= K2M_STAGES) {
           if (!mbar_wait_bounded(empty0 + s * 8, ((n / K2M_STAGES) - 1) & 1, sAbort)) {
             if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_EMPTY_TIMEOUT); }
@@ -155,13 +166,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     // u^T fragment of this warp out of the record's [8-column tile][lane][4] blocks (see kda_common.cuh):
     // element (v = vrow0 + gq + 8a, tok = 2tq + j + 8c)  ->  tile 2*warp + a, lane (2tq+j)*4 + gq/2, slot 2c + gq%2
     const uint32_t u_off = REC_SHARED_BYTES + (warp * 2) * REC_U_TILE_BYTES + ((tq * 2) * 4 + (gq >> 1)) * 16 + (gq & 1) * 4;
-    __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + vrow0 + tq * 2;
+    // the output tile: the 16-byte units of tokens 4..7 and 12..15 swapped, so that eight rows of either unit lie in different banks
+    auto ost_at = [&](int tok, int unit) { return sbase + SM::OST + warp * 512 + tok * 32 + ((unit ^ ((tok >> 2) & 1)) << 4); };
+    const uint32_t ost_put = ost_at((mi >> 1) * 8 + r8, mi & 1), ost_get = ost_at(lane >> 1, lane & 1);
+    __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + vrow0 +
+                                                     (lane >> 1) * p.o_s[1] + (lane & 1) * 8;
     const bool use_u = pair ? (plane == 1) : !(STATE_ONLY && p.zero_u);
 
     // rolling B fragments of P1: two k-steps ahead
     uint32_t bw[2][4], bq[2][4];
     float ut[2][4];             // u^T fragment: [token tile c][e]: e = 2a + j
-    uint32_t o_st[2][2];        // previous step's output tile, already transposed and packed
     float2 dec[16];             // decay of the columns k = 8nt + 2tq, +1 (loaded one step ahead)
 
     auto load_u = [&](uint32_t spg) {
@@ -205,18 +219,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       const int s1 = (n + 1) % K2M_STAGES;
       const uint32_t sp1 = sbase + s1 * SM::STAGE;
 
-      // the previous step's output tile (always a full chunk): rows tok gq / gq+8, 2 value columns
-      if (!STATE_ONLY && n > 0) {
-        __nv_bfloat16* op = ob + static_cast<int64_t>((n - 1) * BT + gq) * p.o_s[1];
-        *reinterpret_cast<uint32_t*>(op) = o_st[0][0];
-        *reinterpret_cast<uint32_t*>(op + 8) = o_st[0][1];
-        *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1]) = o_st[1][0];
-        *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1] + 8) = o_st[1][1];
-      }
+      // the previous step's output tile (always a full chunk): 16 bytes of a token row per lane
+      if (!STATE_ONLY && n > 0)
+        *reinterpret_cast<uint4*>(ob + static_cast<int64_t>((n - 1) * BT) * p.o_s[1]) = lds_u32x4(ost_get);
 
       // P1 with the A fragments of bf16(h) packed on the fly; carries the decay of the fp32 state,
       // its own rolling B loads and the kg(hi) fragments of this step
-      float pw[2][4] = {}, pq[2][4] = {};
+      float pw[2][2][4], pq[2][2][4];   // [k-step parity][token tile]: summed as in the 8-row form, so that the bits are the same
       uint32_t kgh[8][4], kgl[8][4];
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
@@ -226,11 +235,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         ah[2] = pack_bf16(hs[2 * ks + 1][0], hs[2 * ks + 1][1]);
         ah[3] = pack_bf16(hs[2 * ks + 1][2], hs[2 * ks + 1][3]);
         const int sl = ks & 1;
-        mma_bf16_v(pw[0], ah, bw[sl][0], bw[sl][1]);
-        mma_bf16_v(pw[1], ah, bw[sl][2], bw[sl][3]);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (ks < 2) mma_bf16_z(pw[sl][c], ah, bw[sl][2 * c], bw[sl][2 * c + 1]);
+          else mma_bf16_v(pw[sl][c], ah, bw[sl][2 * c], bw[sl][2 * c + 1]);
+        }
         if (!STATE_ONLY) {
-          mma_bf16_v(pq[0], ah, bq[sl][0], bq[sl][1]);
-          mma_bf16_v(pq[1], ah, bq[sl][2], bq[sl][3]);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            if (ks < 2) mma_bf16_z(pq[sl][c], ah, bq[sl][2 * c], bq[sl][2 * c + 1]);
+            else mma_bf16_v(pq[sl][c], ah, bq[sl][2 * c], bq[sl][2 * c + 1]);
+          }
         }
         if (ks + 2 < 8) load_b1(sp, ks + 2, sl);
         ldsm_x4(sp + b2_lane + REC_KGH + ks * 256, kgh[ks][0], kgh[ks][1], kgh[ks][2], kgh[ks][3]);
@@ -248,10 +263,11 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
       // v_new^T (fp32, accumulator layout: rows v, cols tok) and its hi/lo A fragments
       uint32_t avh[4], avl[4];
-      split_pack(ut[0][0] - pw[0][0], ut[0][1] - pw[0][1], avh[0], avl[0]);
-      split_pack(ut[0][2] - pw[0][2], ut[0][3] - pw[0][3], avh[1], avl[1]);
-      split_pack(ut[1][0] - pw[1][0], ut[1][1] - pw[1][1], avh[2], avl[2]);
-      split_pack(ut[1][2] - pw[1][2], ut[1][3] - pw[1][3], avh[3], avl[3]);
+      auto vn = [&](int c, int e) { return ut[c][e] - (pw[0][c][e] + pw[1][c][e]); };
+      split_pack(vn(0, 0), vn(0, 1), avh[0], avl[0]);
+      split_pack(vn(0, 2), vn(0, 3), avh[1], avl[1]);
+      split_pack(vn(1, 0), vn(1, 1), avh[2], avl[2]);
+      split_pack(vn(1, 2), vn(1, 3), avh[3], avl[3]);
 
       // P2 pass 1 (hi * hi), carrying the kg(lo) fragments
 #pragma unroll
@@ -282,7 +298,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) oa[j][e] = p.scale * pq[j][e];
+          for (int e = 0; e < 4; ++e) oa[j][e] = p.scale * (pq[0][j][e] + pq[1][j][e]);
       }
 #pragma unroll
       for (int np = 0; np < 8; ++np) {
@@ -318,12 +334,12 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         }
       }
 
-      // output tile: o^T fragments (rows v, cols tok) -> in-warp transpose -> (rows tok, 2 value columns)
+      // output tile: o^T fragments (rows v, cols tok) leave transposed: [tok][16 v]
       if (!STATE_ONLY) {
-        o_st[0][0] = movmatrix_t(pack_bf16(oa[0][0], oa[0][1]));   // tokens 0..7,  v = vrow0 + 2tq
-        o_st[0][1] = movmatrix_t(pack_bf16(oa[0][2], oa[0][3]));   // tokens 0..7,  v = vrow0 + 8 + 2tq
-        o_st[1][0] = movmatrix_t(pack_bf16(oa[1][0], oa[1][1]));   // tokens 8..15
-        o_st[1][1] = movmatrix_t(pack_bf16(oa[1][2], oa[1][3]));
+        __syncwarp();   // the previous tile has been read
+        stsm_x4_t(ost_put, pack_bf16(oa[0][0], oa[0][1]), pack_bf16(oa[0][2], oa[0][3]), pack_bf16(oa[1][0], oa[1][1]),
+                  pack_bf16(oa[1][2], oa[1][3]));
+        __syncwarp();
       }
     };
     for (int n = 0; n + 1 < NT && !failed; ++n) step(std::true_type{}, n);
@@ -331,16 +347,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
     // the last chunk's output tile (it may be a partial chunk)
     if (!STATE_ONLY && !failed) {
-      const int tok = (NT - 1) * BT + gq;
-      __nv_bfloat16* op = ob + static_cast<int64_t>(tok) * p.o_s[1];
-      if (tok < Tlen) {
-        *reinterpret_cast<uint32_t*>(op) = o_st[0][0];
-        *reinterpret_cast<uint32_t*>(op + 8) = o_st[0][1];
-      }
-      if (tok + 8 < Tlen) {
-        *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1]) = o_st[1][0];
-        *reinterpret_cast<uint32_t*>(op + 8 * p.o_s[1] + 8) = o_st[1][1];
-      }
+      const int tok = (NT - 1) * BT;
+      if (tok + (lane >> 1) < Tlen) *reinterpret_cast<uint4*>(ob + static_cast<int64_t>(tok) * p.o_s[1]) = lds_u32x4(ost_get);
     }
 
     if (!failed && p.ht != nullptr) {
@@ -364,25 +372,26 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     for (int n = max(0, issued - K2M_STAGES); n < issued; ++n)
       mbar_wait_bounded(full0 + (n % K2M_STAGES) * 8, (n / K2M_STAGES) & 1, nullptr);
   }
+  if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
 }
 
-template <int CW, bool STATE_ONLY, int MINB, bool ORD = false>
+template <int CW, bool STATE_ONLY, int MINB, bool ORD = false, int K2M_STAGES = 4>
 static cudaError_t launch_k2m_t(const K2Params& p, int nblocks, cudaStream_t stream) {
-  constexpr int smem_bytes = K2mSmem<CW>::TOTAL;
+  constexpr int smem_bytes = K2mSmem<CW, K2M_STAGES>::TOTAL;
   static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD, K2M_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes > ONE_CTA_SMEM ? smem_bytes : ONE_CTA_SMEM);
     if (e != cudaSuccess) return e;
     // K1's carve-out: CTAs of this kernel move onto an SM while K1 still leaves it (and two of them fit)
-    e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD, K2M_STAGES>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_dep(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
+  return launch_dep(kda_k2m_kernel<CW, STATE_ONLY, MINB, ORD, K2M_STAGES>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
 }
 
 template <int CW, bool STATE_ONLY>
@@ -396,6 +405,8 @@ static cudaError_t launch_k2m_c(const K2Params& p, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (8 / CW);
+  if constexpr (CW == 4 && !STATE_ONLY)
+    if (p.progress != nullptr) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
   if (CW == 4 && nblocks > sms[dev]) return launch_k2m_t<CW, STATE_ONLY, 2>(p, nblocks, stream);
   if constexpr (CW == 4 && !STATE_ONLY)   // the tail of a tensor-memory launch
     if (p.by_length) return launch_k2m_t<4, false, 1, true>(p, nblocks, stream);

@@ -54,7 +54,7 @@ struct K1Params {
   // K2 beside K1 (null = K2 starts after K1): items run time-major, and the finished items of every
   // window of chunks (all chains) are counted in progress[window]
   int* progress;
-  int ctas_per_sm;         // cap on the resident K1 CTAs per SM (0 = as many as fit)
+  int n_sms, k2_sms, k2_sm_ctas;   // SMs of the device, how many of them K2 runs on, and how many K1 CTAs stay on those
   FastDiv div_b, div_win;  // divide by B and by the items of a window
 };
 

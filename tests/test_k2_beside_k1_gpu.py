@@ -66,6 +66,42 @@ def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
 
 
+# K2 on SMs of its own: the 8-row form with four consumer warps, the 16-row form in place of the 8-row one and as chosen, the
+# tensor-memory form with two CTAs per SM and with one; both sides of the lines between them, partial last chunks.  Decays
+# that leave much of the state, so that every step matters to the last bit.
+@pytest.mark.parametrize("B,T,H", [
+    (1, 1991, 19), (1, 1657, 23), (1, 4267, 24), (1, 3185, 32), (1, 3201, 32), (2, 1531, 19), (1, 1530, 42), (1, 1521, 43),
+    (1, 8180, 88), (1, 8180, 89), (1, 8177, 103), (1, 1500, 104), (1, 531, 123), (1, 531, 124)])
+def test_beside_equals_after_where_k2_has_sms_of_its_own(cuda_device, B, T, H):
+    d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.3), cuda_device)
+    d["g"] = (d["g"].float() - 4.0).bfloat16()
+    ref = _after(d, B, T, H, cuda_device)
+    for _ in range(2):
+        got = _whole(d, B, T, H, cuda_device)
+        assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+# one chunk, fewer chunks than stages of the record ring, more; a partial last chunk
+@pytest.mark.parametrize("T", [5, 16, 33, 64, 100, 1003])
+@pytest.mark.parametrize("k_first", [False, True])
+def test_both_register_forms_give_the_same_bits(cuda_device, T, k_first):
+    B, H = 2, 3
+    d = to_device(O.make_inputs(B, T, H, seed0=T, h0_std=0.3), cuda_device)
+    d["g"] = (d["g"].float() - 4.0).bfloat16()
+    flags = api._flags(True, True, True) | (_lib.FLAG_STATE_K_FIRST if k_first else 0)
+    lib, st, got = _lib.load(), api._stream_handle(), []
+    for variant, splits in ((1, (4, 8, 16)), (3, (2, 4, 8))):
+        for vsplit in splits:
+            o, ht, ws = _buffers(B, T, H, cuda_device)
+            a = _args(d, o, ht, ws, flags=flags)
+            a.k2_variant, a.k2_vsplit = variant, vsplit
+            api._check(lib.kda_fwd(ctypes.byref(a), st))
+            assert api.check_device_status(ws) == 0
+            got.append((o, ht))
+    for o, ht in got[1:]:
+        assert torch.equal(o, got[0][0]) and torch.equal(ht, got[0][1])
+
+
 # K1 beside K2 is compiled for either gate type and centring, with all three of gate, l2-norm and sigmoid in the kernel, with
 # none of them (general centring only), and with the flags deciding (some of them, or debug outputs): all ten instances, in
 # front of either form of K2
