@@ -171,10 +171,11 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // warps wait for the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA
 // is already running.  On k2_sms of the SMs only k2_sm_ctas of K1's CTAs stay (k1_stays), and K2's CTAs fit nowhere else.
 // Which of it pays, measured on B200 as the whole forward in us, K2 after K1 against beside it unless said otherwise:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on K2's SMs: B1 T32768 H16 1,028 /
-//     987, T8192 H16 266.5 / 259.1, H8 236 / 226.  With one K1 CTA there K1 is the longer part (T32768 H16 1,329).
-//   Up to 23 of 148 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H19 337 / 296, H22
-//     351 / 293, T2500 H19 113 / 110, H23 117 / 115.  Beyond, K1 has too few SMs left: T8192 H24 360 / 363, T2500 H25 121 / 134.
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on every SM: B1 T32768 H16 1,028 /
+//     987, T8192 H16 266.5 / 259.1, H8 236 / 226.  With four on the SMs that K2 leaves free T131072 H16 3,727 against 3,704, B2
+//     T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
+//   Up to 23 of 148 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H19 337 / 277, H22
+//     351 / 290, T2500 H19 113 / 110, H23 117 / 115.  Beyond, K1 has too few SMs left: T8192 H24 360 / 363, T2500 H25 121 / 134.
 //   From there to 42 of 148 chains: the 16-row form, whose bits are the same, on SMs of its own (2 per chain), at chunk counts
 //     that make up for its longer step: T8192 H24 360 / 352, H32 397 / 355, H37 418 / 393, H38 511 / 410, H40 519 / 447; T4096
 //     H23 184 / 189, H25 189 / 189, H28 195 / 189, H34 208 / 192, H38 256 / 209, H42 265 / 248; T2048 H32 109 / 109, H40 137 /
@@ -201,7 +202,7 @@ Beside beside_plan(const KdaFwdArgs* a) {
   const bool automatic = a->k2_variant == 0 && a->k2_vsplit == 0;
   long long k2_sms = 0;
   if (r.variant == 1 && r.vsplit >= 8 && chains * r.vsplit <= r.sms) {
-    k2_sms = chains * r.vsplit; r.k2_sm_ctas = 2;
+    k2_sms = r.sms; r.k2_sm_ctas = 2;
   } else if (automatic && r.variant == 1 && chains * 32 <= 5LL * r.sms) {
     k2_sms = chains * 4;
   } else if (automatic && ((r.variant == 1 && chains * nt >= 6400) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 96))) {
@@ -237,6 +238,12 @@ Beside beside_plan(const KdaFwdArgs* a) {
   const long long by_round = ((r.k2_sm_ctas == 0 ? 1 : 2) * round + chains - 1) / chains;
   r.win = static_cast<int>(by_count > by_round ? by_count : by_round);
   return r;
+}
+
+// 2^g may be factored as 2^(g-g_mid) * 2^(g_mid) only while no factor can underflow:
+// 16 tokens * |lower_bound| * RCP_LN2 must stay inside the fp32 exponent range.
+bool fast_exp(const KdaFwdArgs* a) {
+  return (a->flags & KDA_FLAG_GATE_IN_KERNEL) && (16.0f * -a->lower_bound * kda::RCP_LN2 <= 120.0f);
 }
 
 int do_k1(const KdaFwdArgs* a, cudaStream_t st, const Beside& side = Beside{}) {
@@ -275,9 +282,6 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, const Beside& side = Beside{}) {
     p.div_b.set(static_cast<uint32_t>(p.B));
     p.div_win.set(static_cast<uint32_t>(side.win) * p.B * p.H);
   }
-  // 2^g may be factored as 2^(g-g_mid) * 2^(g_mid) only while no factor can underflow:
-  // 16 tokens * |lower_bound| * RCP_LN2 must stay inside the fp32 exponent range.
-  const bool fast_exp = (a->flags & KDA_FLAG_GATE_IN_KERNEL) && (16.0f * -a->lower_bound * kda::RCP_LN2 <= 120.0f);
   // The four tensor maps depend only on the input pointers, sizes and strides: a loop that calls with
   // the same buffers (a serving loop, a benchmark) re-uses the maps of its previous call.
   struct MapKey {
@@ -306,7 +310,7 @@ int do_k1(const KdaFwdArgs* a, cudaStream_t st, const Beside& side = Beside{}) {
     last_maps[0] = p.tm_q; last_maps[1] = p.tm_k; last_maps[2] = p.tm_v; last_maps[3] = p.tm_g;
     have_maps = true;
   }
-  e = kda::launch_k1(p, a->g_dtype == KDA_G_BF16, fast_exp, st);
+  e = kda::launch_k1(p, a->g_dtype == KDA_G_BF16, fast_exp(a), st);
   if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: K1 launch failed: %s", cudaGetErrorString(e));
   ++g_launches;
   return KDA_OK;
@@ -331,6 +335,8 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   if (side.win > 0) {
     p.progress = status_ptr(a) + kda::HDR_PROGRESS;
     p.win_chunks = side.win;
+    // two CTAs of a K1 with general centring leave 101 KB; K2 on its own SMs has all of it
+    p.long_ring = side.k2_sm_ctas == 0 || fast_exp(a);
   }
   p.pair_mode = (state_only && zero_u == 2) ? 1 : 0;
   if (a->n_seqs > 0) {

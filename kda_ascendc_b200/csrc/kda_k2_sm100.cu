@@ -27,7 +27,7 @@
 // One warp executes its chain in program order: 43 MMAs of 8 cycles, 20 movmatrix of 5.5, 34 ldmatrix, and the waits
 // between the dependent parts.  Loads are interleaved with the MMA sequences so that their latency is covered: P1
 // carries this step's kg fragment loads and the decay of hT; P2 carries the next step's [w;qg] / decay / u loads and P3.
-// A step takes 0.38 us with one or two consumer warps per CTA and 0.49 with four (T8192 H32 K2 250 us), where the operand
+// A step takes 0.34 to 0.35 us with one or two consumer warps per CTA and 0.47 with four (T8192 H32 K2 242 us), where the operand
 // fragments of four warps keep the SM's shared-memory pipe busy.  Measured without gain: the fragments copied into
 // tensor memory once per SM (tcgen05.cp) and read by tcgen05.ld, 0.79 us: a copy stalls the SM's mma.sync while it runs.
 //
@@ -41,14 +41,14 @@
 
 namespace kda {
 
-constexpr int K2_STAGES = 4;
-
+// STAGES: 4, and beside K1, which holds up the records now and then, 6 (with four consumer warps, on SMs of their own, 8):
+// whole forward T131072 H16 3,756 -> 3,704 us, B2 T4096 H8 131.4 -> 129.0, T8192 H19 296 -> 277, H22 293 -> 290
 // UT = 8-column u tiles a warp reads per step (its NVT row tiles; one in the transform-pair mode)
-template <int CW, int UT>
+template <int CW, int UT, int STAGES>
 struct K2Smem {
   static constexpr int STAGE = REC_SHARED_BYTES + CW * UT * REC_U_TILE_BYTES;
-  static constexpr int BARS = K2_STAGES * STAGE;               // full[S], empty[S]
-  static constexpr int FLAG = BARS + 2 * K2_STAGES * 8;        // abort flag, issued count
+  static constexpr int BARS = STAGES * STAGE;               // full[S], empty[S]
+  static constexpr int FLAG = BARS + 2 * STAGES * 8;        // abort flag, issued count
   static constexpr int TOTAL = FLAG + 16;
 };
 
@@ -59,12 +59,12 @@ struct K2Smem {
 // The states leave as [chains][2][128][128].
 // ORD: packed sequences, longest first (an instantiation of its own: the plain one steps 10 % slower with the
 // order compiled in, T8192 H32 418 -> 460 us).
-template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false>
+template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false, int K2_STAGES = 4>
 __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params p) {
   static_assert(!PAIR || (STATE_ONLY && NVT == 2), "the pair mode is a state-only pass over two tiles");
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int RT = PAIR ? 1 : NVT;    // distinct 8-row tiles per warp
-  using SM = K2Smem<CW, RT>;
+  using SM = K2Smem<CW, RT, K2_STAGES>;
   constexpr int VCOLS = CW * RT * 8;    // state rows (v) per CTA
   constexpr int NV = D / VCOLS;         // CTAs per (batch, head)
   const int tid = threadIdx.x;
@@ -226,21 +226,24 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
 
     // A step is two straight runs of instructions around one branch (the slow path of the wait for the next record),
     // which is what the compiler schedules well: the last step, which has no next record to wait for and to load from, is an
-    // instantiation of its own, the output stores are predicated and the shared-memory loads are pinned.  K2 alone (us), with
-    // conditions around them, with the loads made in the last step too (out of a stage that no copy has filled), and now:
-    // T8192 H32 262, 249.5, 249; T4096 H8 -, 98.8, 94.6; T16 H32 4.7, 4.9, 4.2 (whole forward 9.3, 10.3, 9.3); state-only
-    // T8192 H32 203, 198, 184; T4096 H8 -, 84.4, 71.2; transform pairs T8192 H32 278, 254.5, 257.5.
+    // instantiation of its own, the output stores are predicated and the shared-memory loads are pinned.  The stage goes
+    // round as an address and a parity carried from step to step; worked out from n instead, a step takes 6 % longer, except in
+    // the transform pairs, where the compiler does better with n.  K2 alone (us), before the address was carried and v_new and
+    // o were summed in pairs, and now: T8192 H32 249 / 242, H8 185 / 172, T4096 H8 96.8 / 90.7; state-only T8192 H32 183 / 181, H8 148 /
+    // 146; transform pairs T8192 H16 181 / 177, H32 258 / 260 (276 with the address carried, 282 with paired sums).
     __nv_bfloat16* o_at = STATE_ONLY ? nullptr : ob + static_cast<int64_t>(gq) * p.o_s[1];
     const int64_t o_step = BT * p.o_s[1], o_8 = 8 * p.o_s[1];
     int left = Tlen;
+    uint32_t at = sbase, at_bar = full0, at_ph = 0;   // the chunk's stage, its full barrier and that barrier's parity
     auto step = [&](auto more_c, int n) {
       constexpr bool MORE = decltype(more_c)::value;   // chunk n + 1 exists
-      const int s = n % K2_STAGES;
-      const uint32_t sp = sbase + s * SM::STAGE;
-      const uint32_t t2 = sp + a2_lane;
-      const int s1 = (n + 1) % K2_STAGES;
-      const uint32_t sp1 = sbase + s1 * SM::STAGE;
-      const uint32_t t1n = sp1 + a1_lane;
+      const int s = n % K2_STAGES, s1 = (n + 1) % K2_STAGES;
+      const bool wrap = at == sbase + (K2_STAGES - 1) * SM::STAGE;
+      const uint32_t sp = PAIR ? sbase + s * SM::STAGE : at, bar = PAIR ? full0 + s * 8 : at_bar;
+      const uint32_t sp1 = PAIR ? sbase + s1 * SM::STAGE : wrap ? sbase : at + SM::STAGE;
+      const uint32_t bar1 = PAIR ? full0 + s1 * 8 : wrap ? full0 : at_bar + 8;
+      const uint32_t ph1 = PAIR ? ((n + 1) / K2_STAGES) & 1 : wrap ? at_ph ^ 1 : at_ph;
+      const uint32_t t2 = sp + a2_lane, t1n = sp1 + a1_lane;
 
       // B fragments of bf16(hT) (pre-chunk state): accumulator fragment -> pack -> 8x8 transpose
       uint32_t bh[8][NVT][2];
@@ -280,7 +283,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         }
       }
       // probed here and looked at when the answer is needed: a probe and the vote on it take 126 cycles
-      const bool next_ready = MORE ? mbar_test_wait(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1) : true;
+      const bool next_ready = MORE ? mbar_test_wait(bar1, ph1) : true;
       uint32_t ah3[4], al3[4];
       if (!STATE_ONLY) {
         ldsm_x4(sp + a3_off, ah3[0], ah3[1], ah3[2], ah3[3]);
@@ -292,8 +295,15 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
 #pragma unroll
       for (int nv = 0; nv < NVT; ++nv) {
         uint32_t h01, l01, h23, l23;
+        if constexpr (PAIR) {
+        const float x0 = u[nv].x - (pw[0][nv][0] + pw[1][nv][0]), x1 = u[nv].y - (pw[0][nv][1] + pw[1][nv][1]);
+        const float x2 = u[nv].z - (pw[0][nv][2] + pw[1][nv][2]), x3 = u[nv].w - (pw[0][nv][3] + pw[1][nv][3]);
+        split_pack(x0, x1, h01, l01);
+        split_pack(x2, x3, h23, l23);
+        } else {
         split_pack_diff(make_float2(u[nv].x, u[nv].y), &pw[0][nv][0], &pw[1][nv][0], h01, l01);
         split_pack_diff(make_float2(u[nv].z, u[nv].w), &pw[0][nv][2], &pw[1][nv][2], h23, l23);
+        }
         bvh[nv][0] = movmatrix_t(h01); bvh[nv][1] = movmatrix_t(h23);
         bvl[nv][0] = movmatrix_t(l01); bvl[nv][1] = movmatrix_t(l23);
       }
@@ -307,9 +317,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         asm volatile("" ::"r"(landed) : "memory");
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(empty0 + s * 8);
+      if (lane == 0) mbar_arrive(bar + K2_STAGES * 8);
       if (MORE && !__all_sync(0xffffffffu, next_ready)) {
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(full0 + s1 * 8, ((n + 1) / K2_STAGES) & 1, sAbort))) {
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar1, ph1, sAbort))) {
           if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2_FULL_TIMEOUT); }
           failed = true;
           return;
@@ -371,34 +381,16 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         for (int nv = 0; nv < NVT; ++nv)
           u[nv] = (use_u && !(PAIR && nv == 0)) ? lds_f32x4(sp1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
                                                 : make_float4(0, 0, 0, 0);
+        if (!PAIR) { at = sp1; at_bar = bar1; at_ph = ph1; }
       }
     };
-    // The same walk in three spellings, because the compiler's schedule of a step hangs on the loop around it.  T4096, us per
-    // CTA split in 4 / 8 / 16, in the spelling of pairs, of states, of outputs: outputs 127.7 / 98.9 / 97.0, 128.7 / 96.8 /
-    // 94.8, 127.5 / 96.8 / 94.8; states 108 / 91.3 / 84.6, 94.7 / 78.3 / 72.2, 107.8 / 90.9 / 85.0; pairs 132 / 115 / 119,
-    // 137 / 115 / 122, 134 / 120 / 117.  With `&& !failed` as the loop's condition: outputs 144 / 113 / 109.
+    // (With `&& !failed` as the loop's condition the compiler's schedule of a step is 10 to 15 % longer.)
     if (!failed) {
-      if constexpr (PAIR) {
-        int n = 0;
-        for (int todo = NT - 1; todo > 0; --todo, ++n) {
-          step(std::true_type{}, n);
-          if (failed) break;
-        }
-        if (!failed) step(std::false_type{}, NT - 1);
-      } else if constexpr (STATE_ONLY) {
-        int n = 0;
-        for (; n + 1 < NT; ++n) {
-          step(std::true_type{}, n);
-          if (failed) break;
-        }
-        if (n + 1 >= NT) step(std::false_type{}, n);
-      } else {
-        for (int n = 0; n + 1 < NT; ++n) {
-          step(std::true_type{}, n);
-          if (failed) break;
-        }
-        if (!failed) step(std::false_type{}, NT - 1);
+      for (int n = 0; n + 1 < NT; ++n) {
+        step(std::true_type{}, n);
+        if (failed) break;
       }
+      if (!failed) step(std::false_type{}, NT - 1);
     }
 
     if (!failed && (p.ht != nullptr || (PAIR && p.push_on))) {
@@ -441,31 +433,36 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
   if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
 }
 
-template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false>
+template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false, int K2_STAGES = 4>
 static cudaError_t launch_k2_t(const K2Params& p, cudaStream_t stream) {
   constexpr int RT = PAIR ? 1 : NVT;
-  constexpr int smem_bytes = K2Smem<CW, RT>::TOTAL;
+  constexpr int smem_bytes = K2Smem<CW, RT, K2_STAGES>::TOTAL;
   static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD>,
+    cudaError_t e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD, K2_STAGES>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes > ONE_CTA_SMEM ? smem_bytes : ONE_CTA_SMEM);
     if (e != cudaSuccess) return e;
     // the carve-out of K1, so that an SM can hold CTAs of both
-    e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD>, cudaFuncAttributePreferredSharedMemoryCarveout,
+    e = cudaFuncSetAttribute(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD, K2_STAGES>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (D / (CW * RT * 8));
-  return launch_dep(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
+  return launch_dep(kda_k2_kernel<CW, NVT, STATE_ONLY, PAIR, ORD, K2_STAGES>, nblocks, (CW + 1) * 32, k2_smem(p, smem_bytes), stream, p.pdl, p);
 }
 
 cudaError_t launch_k2n(const K2Params& p, int vsplit, int ntile, bool state_only, cudaStream_t stream) {
   // vsplit CTAs per head, ntile 8-row tiles per warp  =>  16 / (vsplit * ntile) consumer warps per CTA
   // (at most 4: a fifth warp is the producer, and CTAs of more than 8 warps lose registers per thread)
+  if (p.long_ring && !state_only && ntile == 1) {
+    if (vsplit == 4) return launch_k2_t<4, 1, false, false, false, 8>(p, stream);
+    if (vsplit == 8) return launch_k2_t<2, 1, false, false, false, 6>(p, stream);
+    if (vsplit == 16) return launch_k2_t<1, 1, false, false, false, 6>(p, stream);
+  }
 #define KDA_K2_CASE(VS, NT_, CW_)                                                                  \
   if (vsplit == VS && ntile == NT_)                                                                \
     return state_only ? launch_k2_t<CW_, NT_, true>(p, stream)                                     \

@@ -406,7 +406,7 @@ static cudaError_t launch_k2m_c(const K2Params& p, cudaStream_t stream) {
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (8 / CW);
   if constexpr (CW == 4 && !STATE_ONLY)
-    if (p.progress != nullptr) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
+    if (p.long_ring) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
   if (CW == 4 && nblocks > sms[dev]) return launch_k2m_t<CW, STATE_ONLY, 2>(p, nblocks, stream);
   if constexpr (CW == 4 && !STATE_ONLY)   // the tail of a tensor-memory launch
     if (p.by_length) return launch_k2m_t<4, false, 1, true>(p, nblocks, stream);
