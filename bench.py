@@ -69,7 +69,7 @@ K2_FLOPS_PER_CHUNK = 1638400.0
 # reported only for that shape and only while the record layout it was captured with is current.
 NCU_TRAFFIC = dict(shape=(1, 8192, 32), source="profiles/kda_k1_k2_B1_T8192_H32.md",
                    record=dict(REC_W=0, REC_QG=2048, REC_HALF=4096, REC_KGH=8192, REC_KGL=12288, REC_AQK=16384, REC_AQL=16640,
-                               REC_DEC=17408, REC_U=17920, REC_BYTES=26112),
+                               REC_DEC=17408, REC_XBH=17920, REC_XBL=18432, REC_DEC2=18944, REC_V=19456, REC_USED_BYTES=23552),
                    bytes={"kda_k1": 642.58e6, "kda_k2": 488.83e6})
 
 

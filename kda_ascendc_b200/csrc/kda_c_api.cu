@@ -172,7 +172,7 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // is already running.  On k2_sms of the SMs only k2_sm_ctas of K1's CTAs stay (k1_stays), and K2's CTAs fit nowhere else.
 // Which of it pays, measured on B200 as the whole forward in us, K2 after K1 against beside it unless said otherwise:
 //   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on every SM: B1 T32768 H16 1,028 /
-//     987, T8192 H16 266.5 / 259.1, H8 236 / 226.  With four on the SMs that K2 leaves free T131072 H16 3,727 against 3,704, B2
+//     987, T8192 H16 266.5 / 259.1, H8 236 / 226 (an earlier K1).  With four on the SMs that K2 leaves free T131072 H16 3,727 against 3,704, B2
 //     T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
 //   Up to 23 of 148 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H19 337 / 277, H22
 //     351 / 290, T2500 H19 113 / 110, H23 117 / 115.  Beyond, K1 has too few SMs left: T8192 H24 360 / 363, T2500 H25 121 / 134.
@@ -335,8 +335,8 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   if (side.win > 0) {
     p.progress = status_ptr(a) + kda::HDR_PROGRESS;
     p.win_chunks = side.win;
-    // two CTAs of a K1 with general centring leave 101 KB; K2 on its own SMs has all of it
-    p.long_ring = side.k2_sm_ctas == 0 || fast_exp(a);
+    // two CTAs of K1 leave K2 126 KB of an SM, 8 KB less with an fp32 gate, 17 with general centring
+    p.long_ring = side.k2_sm_ctas == 0 ? 8 : 6 - (a->g_dtype == KDA_G_FP32) - !fast_exp(a);
   }
   p.pair_mode = (state_only && zero_u == 2) ? 1 : 0;
   if (a->n_seqs > 0) {

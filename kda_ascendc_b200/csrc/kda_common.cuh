@@ -8,18 +8,21 @@
 // stage is one bulk (TMA) copy.
 //
 //   offset  bytes  contents
-//   0       8192   w, qg     bf16, two halves of 64 k: [half][w, qg][16 tok][64 k], the eight 16-byte units of a
+//   0       8192   -w, qg    bf16, two halves of 64 k: [half][-w, qg][16 tok][64 k], the eight 16-byte units of a
 //                            128-byte row XOR-permuted by the row index (wq_off)
 //   8192    4096   kg_h      bf16 [2 token halves][128 k][8 tok] \ hi/lo split of khat * 2^(g_last - g),
 //   12288   4096   kg_l      bf16 [2][128][8]                    / transposed (kg_off)
 //   16384   1024   Aqk       bf16 [2 column halves][hi, lo][16 i][8 j]: hi/lo split of the scaled lower triangle
 //                            incl. diagonal (aq_off)
 //   17408   512    dec       fp32 [128]      = 2^(g_last)
-//   17920   8192   u         fp32, accumulator-fragment order [16 column tile][32 lane][4]:
-//                            lane (g = lane/4, t = lane%4) holds u[tok g][v], u[tok g][v+1],
-//                            u[tok g+8][v], u[tok g+8][v+1] with v = 8*tile + 2t
+//   17920   512    Xb_h      bf16 [2 column halves][16 i][8 j] \ hi/lo split of X diag(beta), X = (I + Akk)^-1
+//   18432   512    Xb_l      bf16 [2][16][8]                   / (xb_off)
+//   18944   512    dec       fp32 again, in the order in which the 8-row K2's lanes read it (dec_lane_off)
+//   19456   4096   v         bf16 [2 halves of 64 columns][16 tok][64], 16-byte units permuted as in w (v_off)
+// (23,552 of the 26,112 bytes)
 //
-// with qg = bf16(qhat * 2^g).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
+// with qg = bf16(qhat * 2^g).  u = X diag(beta) v is not stored: K2 adds it up from Xb and v, which is exact in bf16, on
+// the accumulator of -w h (4 KiB less to write and to read, and K1 does not touch v at all).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
 // operand as it stands: [w; qg] is a 32-row K-major operand in the 128-byte swizzle of tcgen05 (8-row groups 1024
 // bytes apart), kg^T and Aqk are 8x8 core matrices of 128 contiguous bytes (K-major without swizzle).  tcgen05.mma
 // reads them by descriptor, and every 8x8 matrix of an ldmatrix is free of bank conflicts, most of them at
@@ -42,9 +45,13 @@ constexpr int REC_KGL = 12288;
 constexpr int REC_AQK = 16384;   // hi; lo at REC_AQL
 constexpr int REC_AQL = 16640;
 constexpr int REC_DEC = 17408;
-constexpr int REC_U = 17920;
-constexpr int REC_SHARED_BYTES = 17920;  // everything every V-slice needs
-constexpr int REC_U_TILE_BYTES = 512;    // one 8-column tile of u
+constexpr int REC_XBH = 17920;
+constexpr int REC_XBL = 18432;
+constexpr int REC_DEC2 = 18944;
+constexpr int REC_V = 19456;             // 64 columns of v at REC_V + half * REC_V_HALF
+constexpr int REC_V_HALF = 2048;
+constexpr int REC_SHARED_BYTES = 19456;  // everything every V-slice needs
+constexpr int REC_USED_BYTES = 23552;
 constexpr int REC_BYTES = 26112;
 constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the workspace
 // Header words: 0 = status; HDR_K1_STATUS = K1's own code, which no later kernel overwrites (K2 waits for K1, so a K1
@@ -91,6 +98,17 @@ __device__ __forceinline__ uint32_t kg_off(int tok, int k) {
 }
 __device__ __forceinline__ uint32_t aq_off(int i, int j) {
   return static_cast<uint32_t>((j >> 3) * 512 + i * 16 + (j & 7) * 2);
+}
+
+__device__ __forceinline__ uint32_t xb_off(int i, int j) {
+  return static_cast<uint32_t>((j >> 3) * 256 + i * 16 + (j & 7) * 2);
+}
+__device__ __forceinline__ uint32_t v_off(int tok, int v) {
+  return static_cast<uint32_t>((v >> 6) * REC_V_HALF + tok * 128 + (((((v >> 3) & 7) ^ (tok & 7)) << 4) | ((v & 7) << 1)));
+}
+// lane (g = lane / 4) of the 8-row K2 holds k = 16 m + g and 16 m + 8 + g, m = 0..7: four 16-byte loads
+__device__ __forceinline__ uint32_t dec_lane_off(int k) {
+  return static_cast<uint32_t>((k >> 5) * 128 + (k & 7) * 16 + ((k >> 3) & 3) * 4);
 }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -409,10 +427,10 @@ __device__ __forceinline__ void split_pack2(float2 x, uint32_t& hi, uint32_t& lo
   const float2 r = __ffma2_rn(make_float2(bf16_lo_to_f32(hi), bf16_hi_to_f32(hi)), make_float2(-1.f, -1.f), x);
   lo = pack_bf16(r.x, r.y);
 }
-// u - (a + b) of two neighbours of an accumulator fragment, as a hi/lo pair
-__device__ __forceinline__ void split_pack_diff(float2 u, const float* a, const float* b, uint32_t& hi, uint32_t& lo) {
+// u + (a + b) of two neighbours of an accumulator fragment, as a hi/lo pair
+__device__ __forceinline__ void split_pack_sum(const float* u, const float* a, const float* b, uint32_t& hi, uint32_t& lo) {
   const float2 s = __fadd2_rn(make_float2(a[0], a[1]), make_float2(b[0], b[1]));
-  split_pack2(__fadd2_rn(u, make_float2(-s.x, -s.y)), hi, lo);
+  split_pack2(__fadd2_rn(make_float2(u[0], u[1]), s), hi, lo);
 }
 __device__ __forceinline__ float rcpf(float x) {
   float y;

@@ -11,7 +11,8 @@
 //      with gm = g - g[centre]; tensor-core MMAs on hi/lo bf16 splits of the fp32 operands
 //      (three partial products, fp32 accumulate => ~2^-16 relative, "fp32-like")
 //   3. X = (I + Akk)^-1 by forward substitution, fp32, one lane per column of X
-//   4. w = X (khat beta 2^g)   (bf16 out),   u = X (v beta)   (fp32 out, split-bf16 MMAs)
+//   4. w = X (khat beta 2^g)   (bf16 out);   u = X diag(beta) v is left to K2 as its two factors: X diag(beta) as a
+//      hi/lo bf16 pair, and v as it came
 // and additionally pre-computes what the reference's Triton K2 re-derives every step
 // (src/kda_bt16/kernels.py:255-259,271,286-287): qg = bf16(qhat 2^g),
 // kg = khat 2^(g_last-g) as a hi/lo bf16 pair, dec = 2^g_last -- the arrangement of
@@ -21,9 +22,12 @@
 // (d, head, token, batch) built from the caller's strides, so head-shard and segment views
 // need no copy; rows past T are zero-filled by the copy) that complete on one mbarrier; as soon as
 // a chunk's inputs have been consumed the copies of the CTA's next chunk are issued into the
-// same tiles, so the ~2.5 us load latency hides behind the rest of the chunk.  Of the
-// 26,112-byte chunk record (kda_common.cuh) qg, the kg / Aqk / dec part and w leave by five
-// bulk stores; u is stored straight from the accumulator fragments (512 contiguous bytes per warp).
+// same tiles, so the ~2.5 us load latency hides behind the rest of the chunk.  v is only passed on: its two 64-column boxes
+// arrive, swizzled by the copy, where the record's part with kg, Aqk, dec, Xb and v is put together.  That part, qg and w leave
+// by five bulk stores.  With u worked out here and stored as fp32 from the accumulator fragments K1 alone took 147.5 us, now
+// 132.7 (T8192 H32; H96 426 -> 383, in a row of calls at the power limit 468 -> 410; the prepared batch 276 -> 257).
+// khat beta 2^g is rounded to bf16 with beta in it, as ever: without, where gates are near zero khat 2^g rounds back to
+// khat more often than not, and the state's error against 64 bits grows by 1 % (gates of -8: 1.283e-3 -> 1.298e-3).
 #include "kda_common.cuh"
 #include "kda_kernels.h"
 
@@ -31,15 +35,19 @@ namespace kda {
 
 // shared-memory map (bytes): four CTAs of the production variant (bf16 gate, FAST_EXP) per SM
 constexpr int S_QG = 0;                               // two halves of 2048 bytes -> the record's qg parts
-constexpr int S_KGH = 4096, S_KGL = 8192;             // -> record[8192, 16384)
-constexpr int S_AQK = 12288, S_AQL = S_AQK + (REC_AQL - REC_AQK), S_DEC = 13312;   // -> record[16384, 17920)
-constexpr int S_L = 13824;                            // fp32 [16][16], -Akk
-constexpr int S_XH = 14848, S_XL = 15360;             // bf16 [16][16] hi / lo of (I+Akk)^-1
-constexpr int S_GRAM = 15872;
+// as in the record from REC_KGH on (kg, Aqk, dec, Xb, dec again, v): one bulk store
+constexpr int S_KGH = 4096, S_KGL = S_KGH + (REC_KGL - REC_KGH);
+constexpr int S_AQK = S_KGH + (REC_AQK - REC_KGH), S_AQL = S_KGH + (REC_AQL - REC_KGH), S_DEC = S_KGH + (REC_DEC - REC_KGH);
+constexpr int S_XBH = S_KGH + (REC_XBH - REC_KGH), S_XBL = S_KGH + (REC_XBL - REC_KGH), S_DEC2 = S_KGH + (REC_DEC2 - REC_KGH);
+constexpr int S_V = S_KGH + (REC_V - REC_KGH);
+static_assert(S_V % 1024 == 0, "the copies of v swizzle within 1024 bytes");
+constexpr int S_L = S_KGH + (REC_USED_BYTES - REC_KGH);   // fp32 [16][16], -Akk
+constexpr int S_XH = S_L, S_XL = S_L + (REC_XBL - REC_XBH);   // bf16 hi / lo of (I+Akk)^-1 in the layout of Xb, over -Akk
+constexpr int S_GRAM = S_L + 1024;
 constexpr int S_QGH = S_GRAM, S_QGL = S_GRAM + 4096, S_KQH = S_GRAM + 8192, S_KQL = S_GRAM + 12288,
               S_KNH = S_GRAM + 16384, S_KNL = S_GRAM + 20480;   // KN tiles only without FAST_EXP
-// once the Grams are done their A tiles hold the B operands of w and u
-constexpr int S_KBH = S_GRAM, S_VBH = S_GRAM + 4096, S_VBL = S_GRAM + 8192;
+// once the Grams are done their A tiles hold the B operand of w
+constexpr int S_KBH = S_GRAM;
 constexpr int S_WST = S_GRAM + 12288;   // staging tile of w (the fourth Gram tile slot), -> the record's w parts
 
 // element (r, c) of a staged w or qg tile: the record's layout with the two halves back to back
@@ -50,14 +58,15 @@ __device__ __forceinline__ uint32_t stage_off(int r, int c) {
 template <bool G_BF16, bool FAST_EXP>
 struct K1Smem {
   static constexpr int IN = S_GRAM + (FAST_EXP ? 16384 : 24576);
-  static constexpr int Q = IN, K = IN + 4096, V = IN + 8192, G = IN + 12288;
+  static constexpr int Q = IN, K = IN + 4096, G = IN + 8192;
   static constexpr int G_BYTES = G_BF16 ? 4096 : 8192;
   static constexpr int SMALL = G + G_BYTES;
   static constexpr int BETA = SMALL;          // fp32 [2][16] activated beta + [2] exp(A_log): this item / next item
   static constexpr int TOT = BETA + 144;      // fp32 [2][128]: column sums of the gate over rows 0..7 and rows 8..15
   static constexpr int GMID = TOT + 1024;     // fp32 [128] g[mid] (not needed with FAST_EXP)
   static constexpr int MBAR = GMID + (FAST_EXP ? 0 : 512);
-  static constexpr int FLAG = MBAR + 8;   // a wait gave up; the item after the next one (beside K2)
+  static constexpr int MBAR_V = MBAR + 8;
+  static constexpr int FLAG = MBAR_V + 8;   // a wait gave up; the item after the next one (beside K2)
   static constexpr int TOTAL = FLAG + 8;
 };
 
@@ -106,8 +115,8 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // beside the 8-row form both fit (T32768 H16 988 and 990, B2 T4096 H8 135.1 and 135.6).
 // FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel; FORM_NONE: all
 // three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags decide.  Against
-// FORM_ANY for the same call: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs prepared by the caller (B8 T2037
-// H32 with 8 q/k heads) 294 -> 274; kda_fwd T8192 H96 881 -> 849, the prepared batch 474 -> 454.
+// FORM_ANY for the same call, with u still worked out here: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs
+// prepared by the caller (B8 T2037 H32 with 8 q/k heads) 294 -> 274.
 enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
 //
 // Beside K2 the work is handed out item by item, and not every SM does the same share of it: on k2_sms of the SMs (spread
@@ -140,7 +149,7 @@ template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_constant__ K1Params p) {
   extern __shared__ __align__(1024) uint8_t smem[];
   using SM = K1Smem<G_BF16, FAST_EXP>;
-  constexpr int S_Q = SM::Q, S_K = SM::K, S_V = SM::V, S_G = SM::G;
+  constexpr int S_Q = SM::Q, S_K = SM::K, S_G = SM::G;
   constexpr uint32_t ROW_BYTES = D * 2;
   constexpr uint32_t G_ROW_BYTES = G_BF16 ? D * 2 : D * 4;
   const int tid = threadIdx.x;
@@ -150,7 +159,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   const int n_items = (p.chunk_table != nullptr ? p.n_chunks : p.B * p.NT) * p.H;
 
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t mbar = sbase + SM::MBAR;
+  const uint32_t mbar = sbase + SM::MBAR, mbar_v = sbase + SM::MBAR_V;
   float* sL = reinterpret_cast<float*>(smem + S_L);
   float* sBetaAll = reinterpret_cast<float*>(smem + SM::BETA);   // [2][16], then expA[2] at +32
   float* sTot = reinterpret_cast<float*>(smem + SM::TOT);
@@ -168,6 +177,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
 
   if (tid == 0) {
     mbar_init(mbar, 1);
+    mbar_init(mbar_v, 1);
     sFlag[0] = 0;   // a wait gave up
     fence_mbar_init();
     if (BESIDE) sFlag[1] = k1_stays(p) ? atomicAdd(p.progress - HDR_PROGRESS + HDR_TICKET, 2) : n_items;
@@ -179,12 +189,17 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   // towards the transaction bytes.
   auto issue_loads = [&](const K1Item& w) {
     if (tid == 0) {
-      mbar_arrive_expect_tx(mbar, BT * (3 * ROW_BYTES + G_ROW_BYTES));
+      mbar_arrive_expect_tx(mbar, BT * (2 * ROW_BYTES + G_ROW_BYTES));
       tma_load_4d(sbase + S_Q, &p.tm_q, 0, w.hq, w.t0, w.b, mbar);
       tma_load_4d(sbase + S_K, &p.tm_k, 0, w.hq, w.t0, w.b, mbar);
-      tma_load_4d(sbase + S_V, &p.tm_v, 0, w.h, w.t0, w.b, mbar);
       tma_load_4d(sbase + S_G, &p.tm_g, 0, w.h, w.t0, w.b, mbar);
     }
+  };
+  // thread 0: v goes straight into the record's part that leaves last, once that tile is free
+  auto issue_v = [&](const K1Item& w) {
+    mbar_arrive_expect_tx(mbar_v, BT * ROW_BYTES);
+    tma_load_4d(sbase + S_V, &p.tm_v, 0, w.h, w.t0, w.b, mbar_v);
+    tma_load_4d(sbase + S_V + REC_V_HALF, &p.tm_v, 64, w.h, w.t0, w.b, mbar_v);
   };
   // per-item parameters, fetched one item ahead so that their global-load latency is hidden
   struct Par { float a_log, bias0, bias1, beta; };
@@ -306,7 +321,6 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         const uint4 z = make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4*>(smem + S_Q + i * 16) = z;
         *reinterpret_cast<uint4*>(smem + S_K + i * 16) = z;
-        *reinterpret_cast<uint4*>(smem + S_V + i * 16) = z;
         *reinterpret_cast<uint4*>(smem + S_G + i * (G_BF16 ? 16 : 32)) = z;
         if (!G_BF16) *reinterpret_cast<uint4*>(smem + S_G + i * 32 + 16) = z;
       }
@@ -323,6 +337,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         atomicExch(p.status, ST_K1_LOAD_TIMEOUT);
         p.status[HDR_K1_STATUS] = ST_K1_LOAD_TIMEOUT;
         mbar_wait_bounded(mbar, it & 1, nullptr);
+        bulk_wait_read_all();
       }
       __syncthreads();
       return;
@@ -337,7 +352,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     // in (-11, 0).  FAST_EXP (16*|lower_bound|*RCP_LN2 <= 120, e.g. the production -5): the
     // LAST row, where 2^(g_last-g) <= 1 is exactly K2's kg operand, so the Grams reuse the kg
     // tiles as their B operand and 2^g = 2^(g-g_last) * 2^g_last costs no third exponential.
-    uint32_t kbh[8], vbh[8], vbl[8];
+    uint32_t kbh[8];
     float2 dec2;
     {
       float2 gv[8];
@@ -375,7 +390,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         if (!FAST_EXP && rh == (mid >> 3)) *reinterpret_cast<float2*>(sGmid + c0) = gm;
         // the previous item's bulk stores must have read the qg / kg / Aqk / dec tiles before the
         // operand loop below rewrites them; by now they have had two phases to do so
-        if (tid == 0) drain_stores();
+        if (tid == 0) { drain_stores(); issue_v(cur); }
         __syncthreads();
         const float2 t0 = *reinterpret_cast<const float2*>(sTot + c0);
         const float2 t1 = *reinterpret_cast<const float2*>(sTot1 + c0);
@@ -395,11 +410,16 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         for (int i = 0; i < 8; ++i) gv[i] = ld_g(min(r0 + i, nvalid - 1));
         gmid = ld_g(min(BT / 2, nvalid - 1));
         glast = ld_g(nvalid - 1);
-        if (tid == 0) drain_stores();   // as above
+        if (tid == 0) { drain_stores(); issue_v(cur); }   // as above
         __syncthreads();
       }
       dec2 = make_float2(ex2f(glast.x), ex2f(glast.y));
-      if (rh == 1) *reinterpret_cast<float2*>(smem + S_DEC + c0 * 4) = dec2;
+      if (rh == 1) {
+        *reinterpret_cast<float2*>(smem + S_DEC + c0 * 4) = dec2;
+      } else {
+        *reinterpret_cast<float*>(smem + S_DEC2 + dec_lane_off(c0)) = dec2.x;
+        *reinterpret_cast<float*>(smem + S_DEC2 + dec_lane_off(c0 + 1)) = dec2.y;
+      }
 
       if (FORM == FORM_ANY && p.g_out != nullptr) {
 #pragma unroll
@@ -421,10 +441,8 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
           const uint32_t off = swz_off(r, c0);
           const uint32_t qp = *reinterpret_cast<const uint32_t*>(smem + S_Q + (r * D + c0) * 2);
           const uint32_t kp = *reinterpret_cast<const uint32_t*>(smem + S_K + (r * D + c0) * 2);
-          const uint32_t vp = *reinterpret_cast<const uint32_t*>(smem + S_V + (r * D + c0) * 2);
           const float2 qn = make_float2(bf16_lo_to_f32(qp), bf16_hi_to_f32(qp));   // already normalised
           const float2 kn = make_float2(bf16_lo_to_f32(kp), bf16_hi_to_f32(kp));
-          const float br = sBeta[r];
           const float2 d = __fadd2_rn(gv[i], ncentre);                  // g - centre
           const float2 e = make_float2(ex2f(d.x), ex2f(d.y));           // 2^(g - centre)
           const float2 en = make_float2(ex2f(-d.x), ex2f(-d.y));        // 2^(centre - g)
@@ -449,9 +467,9 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
           kg2[ii] = __fmul2_rn(kn, ekg);
           const float2 qgo = __fmul2_rn(qn, eg);
           *reinterpret_cast<uint32_t*>(smem + S_QG + stage_off(r, c0)) = pack_bf16(qgo.x, qgo.y);
+          const float br = sBeta[r];
           const float2 kbv = __fmul2_rn(__fmul2_rn(kn, make_float2(br, br)), eg);
           kbh[i] = pack_bf16(kbv.x, kbv.y);
-          split_pack2(__fmul2_rn(make_float2(bf16_lo_to_f32(vp), bf16_hi_to_f32(vp)), make_float2(br, br)), vbh[i], vbl[i]);
         }
         split_pack(kg2[0].x, kg2[1].x, kgh[0][i2], kgl[0][i2]);
         split_pack(kg2[0].y, kg2[1].y, kgh[1][i2], kgl[1][i2]);
@@ -470,7 +488,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       put(S_KGH, kgh);
       put(S_KGL, kgl);
     }
-    __syncthreads();  // every thread has read its q/k/v/g elements: the input tiles are free
+    __syncthreads();  // every thread has read its q/k/g elements: the input tiles are free
 
     // ---- prefetch: the next item's inputs go into the same tiles while this one finishes ----
     if (has_next) {
@@ -539,25 +557,24 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     }
     __syncthreads();   // Grams done: their A tiles are free, -Akk is visible
 
-    // B operands of w and u take the place of the Gram A tiles
+    // the B operand of w takes the place of a Gram A tile
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const uint32_t off = swz_off(r0 + i, c0);
       *reinterpret_cast<uint32_t*>(smem + S_KBH + off) = kbh[i];
-      *reinterpret_cast<uint32_t*>(smem + S_VBH + off) = vbh[i];
-      *reinterpret_cast<uint32_t*>(smem + S_VBL + off) = vbl[i];
     }
 
     // next item's scalar parameters (warp 1, while warp 0 solves)
     if (has_next) publish_params(par_next, nxt.nvalid, (it + 1) & 1);
 
-    // ---- phase D: X = (I + L)^-1, lane j of warp 0 owns column j ---------------
+    // ---- phase D: X = (I + L)^-1, lanes j and 16 + j of warp 0 own column j (the latter go on with X diag(beta)) ----
     // Column sweep (right-looking): once x[m] is final, every later row takes its update, so the
     // dependent chain is 16 FMAs long; -L is read four columns at a time.
-    if (warp == 0 && lane < 16) {
+    if (warp == 0) {
+      const int col = lane & 15;
       float x[BT];
 #pragma unroll
-      for (int i = 0; i < BT; ++i) x[i] = (i == lane) ? 1.f : 0.f;
+      for (int i = 0; i < BT; ++i) x[i] = (i == col) ? 1.f : 0.f;
 #pragma unroll
       for (int mb = 0; mb < 4; ++mb) {
 #pragma unroll
@@ -569,66 +586,70 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
             if (mb * 4 + mm < i) x[i] = fmaf(lv[mm], x[mb * 4 + mm], x[i]);
         }
       }
+      __syncwarp();   // -Akk has been read by all lanes: X takes its place
+      const float by = lane < 16 ? 1.f : sBeta[col];
+      const uint32_t x_at = (lane < 16 ? S_XH : S_XBH) + xb_off(0, col);
+      static_assert(S_XL - S_XH == S_XBL - S_XBH, "hi to lo");
 #pragma unroll
       for (int i = 0; i < BT; ++i) {
-        const float hi = bf16_round(x[i]);
-        *reinterpret_cast<unsigned short*>(smem + S_XH + (i * 16 + lane) * 2) = bf16_bits(hi);
-        *reinterpret_cast<unsigned short*>(smem + S_XL + (i * 16 + lane) * 2) = bf16_bits(x[i] - hi);
+        const float xb = x[i] * by, hi = bf16_round(xb);
+        *reinterpret_cast<unsigned short*>(smem + x_at + i * 16) = bf16_bits(hi);
+        *reinterpret_cast<unsigned short*>(smem + x_at + i * 16 + (S_XL - S_XH)) = bf16_bits(xb - hi);
       }
       if (FORM == FORM_ANY && p.ainv_out != nullptr) {
 #pragma unroll
         for (int i = 0; i < BT; ++i)
-          if (i < nvalid) p.ainv_out[((static_cast<size_t>(b) * p.T + t0 + i) * p.H + h) * BT + lane] = x[i];
+          if (i < nvalid && lane < 16) p.ainv_out[((static_cast<size_t>(b) * p.T + t0 + i) * p.H + h) * BT + lane] = x[i];
       }
     }
-    fence_proxy_async();   // qg / kg / Aqk / dec tiles were written with plain stores
+    // packed sequences: v behind the last token of a sequence, as for the other inputs above
+    if (!BESIDE && p.chunk_table != nullptr && nvalid < BT) {
+      if (!mbar_wait_bounded(mbar_v, it & 1, sFlag)) *sFlag = 1;
+#pragma unroll 1
+      for (int i = nvalid * 16 + tid; *sFlag == 0 && i < BT * 16; i += 128)   // 16-byte units
+        *reinterpret_cast<uint4*>(smem + S_V + (i & 1) * REC_V_HALF + (i >> 1) * 16) = make_uint4(0, 0, 0, 0);
+    }
+    fence_proxy_async();   // qg / kg / Aqk / dec / Xb tiles were written with plain stores
     __syncthreads();
 
     // the finished tiles leave while phase E runs
     if (tid == 0) {
+      // v was asked for two phases ago; if it does not come, the CTA leaves at the start of the next item
+      if (!mbar_wait_bounded(mbar_v, it & 1, nullptr)) {
+        *sFlag = 1;
+        atomicExch(p.status, ST_K1_LOAD_TIMEOUT);
+        p.status[HDR_K1_STATUS] = ST_K1_LOAD_TIMEOUT;
+      }
       bulk_s2g(rec + REC_QG, sbase + S_QG, TILE_BYTES / 2);
       bulk_s2g(rec + REC_QG + REC_HALF, sbase + S_QG + TILE_BYTES / 2, TILE_BYTES / 2);
-      bulk_s2g(rec + REC_KGH, sbase + S_KGH, REC_U - REC_KGH);
+      bulk_s2g(rec + REC_KGH, sbase + S_KGH, REC_USED_BYTES - REC_KGH);
       bulk_commit();
     }
 
-    // ---- phase E: u = X (v beta) (fp32-like, three split MMAs), w = X (khat beta 2^g) (bf16),
-    //      u stored to the record straight from the accumulator fragments, w staged for a bulk store ----
+    // ---- phase E: -w = -X (khat beta 2^g) (bf16), staged for a bulk store ----
     {
       // X as A operand (row-major [M=i][K=m]), hi and lo parts
       uint32_t xah[4], xal[4];
       {
-        const int row2 = (lane & 7) + ((lane >> 3) & 1) * 8, col2 = (lane >> 4) * 8;
-        ldsm_x4(sbase + S_XH + (row2 * 16 + col2) * 2, xah[0], xah[1], xah[2], xah[3]);
-        ldsm_x4(sbase + S_XL + (row2 * 16 + col2) * 2, xal[0], xal[1], xal[2], xal[3]);
+        const uint32_t x_at = sbase + xb_off((lane & 7) + ((lane >> 3) & 1) * 8, (lane >> 4) * 8);
+        ldsm_x4(x_at + S_XH, xah[0], xah[1], xah[2], xah[3]);
+        ldsm_x4(x_at + S_XL, xal[0], xal[1], xal[2], xal[3]);
       }
       // B operands come from [tok][col] tiles through transposing ldmatrix; one x4 covers 16 columns
       const int btok = (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll
       for (int ni = 0; ni < 2; ++ni) {
         const int n0 = warp * 32 + ni * 16;
-        const int ccol = n0 + (lane >> 4) * 8;
-        uint32_t bvh[4], bvl[4], bk[4];
-        ldsm_x4_t(sbase + S_VBH + swz_off(btok, ccol), bvh[0], bvh[1], bvh[2], bvh[3]);
-        ldsm_x4_t(sbase + S_VBL + swz_off(btok, ccol), bvl[0], bvl[1], bvl[2], bvl[3]);
-        ldsm_x4_t(sbase + S_KBH + swz_off(btok, ccol), bk[0], bk[1], bk[2], bk[3]);
+        uint32_t bk[4];
+        ldsm_x4_t(sbase + S_KBH + swz_off(btok, n0 + (lane >> 4) * 8), bk[0], bk[1], bk[2], bk[3]);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-          // u tile: tokens x 8 value columns, stored as the raw accumulator fragment (K2 reads it back
-          // into the same fragment): [column tile][lane][4]
-          float acc[4] = {0, 0, 0, 0}, accl[4] = {0, 0, 0, 0};
-          mma_bf16(acc, xah, bvh[2 * j], bvh[2 * j + 1]);
-          mma_bf16(accl, xal, bvh[2 * j], bvh[2 * j + 1]);
-          mma_bf16(accl, xah, bvl[2 * j], bvl[2 * j + 1]);
-          const int vtile = (n0 >> 3) + j;
-          *reinterpret_cast<float4*>(rec + REC_U + (vtile * 32 + lane) * 16) =
-              make_float4(acc[0] + accl[0], acc[1] + accl[1], acc[2] + accl[2], acc[3] + accl[3]);
           float accw[4] = {0, 0, 0, 0};
           mma_bf16(accw, xah, bk[2 * j], bk[2 * j + 1]);
           mma_bf16(accw, xal, bk[2 * j], bk[2 * j + 1]);
           const int kc = n0 + j * 8 + tq * 2;
-          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq, kc)) = pack_bf16(accw[0], accw[1]);
-          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq + 8, kc)) = pack_bf16(accw[2], accw[3]);
+          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq, kc)) = pack_bf16(-accw[0], -accw[1]);
+          *reinterpret_cast<uint32_t*>(smem + S_WST + stage_off(gq + 8, kc)) = pack_bf16(-accw[2], -accw[3]);
         }
       }
     }
@@ -642,10 +663,9 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
       rep_win = cur.win;
       rep_done = done;
       done = 0;
-      fence_proxy_async_all();   // u left by plain stores, K2 reads it with bulk copies
     }
     if (BESIDE && tid == 0) sFlag[1] = ticket;
-    __syncthreads();   // also orders phase E's reads of X / KB / VB before the next item rewrites them
+    __syncthreads();   // also orders phase E's reads of Xb / KB before the next item rewrites them
     if (tid == 0) {
       bulk_s2g(rec + REC_W, sbase + S_WST, TILE_BYTES / 2);
       bulk_s2g(rec + REC_W + REC_HALF, sbase + S_WST + TILE_BYTES / 2, TILE_BYTES / 2);
@@ -654,7 +674,10 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     cur = nxt;
     par = par_next;
   }
-  if (tid == 0) drain_stores();
+  if (tid == 0) {
+    if (*sFlag == 0) drain_stores();
+    else bulk_wait_read_all();   // v of the last item did not come: no window is reported
+  }
 }
 
 template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
@@ -726,10 +749,12 @@ cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what) {
                              static_cast<cuuint64_t>(t.s[0]) * t.es};
     for (int i = 0; i < 3; ++i)
       if (dims[i + 1] == 1) strides[i] = static_cast<cuuint64_t>(D) * t.es;
-    const cuuint32_t box[4] = {static_cast<cuuint32_t>(D), 1, static_cast<cuuint32_t>(BT), 1};
+    // v arrives in two boxes of 64 columns, in the 128-byte swizzle of its place in the record
+    const bool is_v = t.m == &p.tm_v;
+    const cuuint32_t box[4] = {static_cast<cuuint32_t>(is_v ? D / 2 : D), 1, static_cast<cuuint32_t>(BT), 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = enc(t.m, t.dt, 4, const_cast<void*>(t.ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     is_v ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { *what = t.name; return cudaErrorInvalidValue; }
   }
   return cudaSuccess;

@@ -4,13 +4,15 @@
 // arithmetic is the recurrence of the reference's torch chunk implementation
 // (tests/test_torch_reference.py:175-194), V-first state h[V][K]:
 //   v_new = u - w h^T ;  o = scale (qg h^T) + Aqk v_new ;  h = h diag(dec) + v_new^T kg
+// The record holds -w, and u as its factors: u = Xb v.
 //
 // The recurrence is independent per state row v (v_new[:, v], o[:, v] and h[v, :] only use
 // row v), so V is the dimension that is spread over warps.  It is mapped to the MMA *N*
 // dimension, whose granularity is 8: a warp owns NVT tiles of 8 rows of h and keeps them,
 // transposed, in registers for the whole sequence:  hT[k][v], fp32, m16n8 accumulator
 // fragments (8 k-tiles of 16).  Per chunk, per warp:
-//   P1: [v_new | o] = [w ; qg] hT       M = 16+16 tokens, N = 8 v, K = 128   (16 MMAs / tile)
+//   P1: [-w hT | o] = [-w ; qg] hT      M = 16+16 tokens, N = 8 v, K = 128   (16 MMAs / tile)
+//   u = Xb v                            M = 16 tokens,    N = 8 v, K = 16    (2 MMAs, hi and lo of Xb)
 //   P2: hT += kg^T v_new                M = 128 k,        N = 8 v, K = 16    (3 x 8 MMAs)
 //   P3: o += Aqk v_new                  M = 16 tokens,    N = 8 v, K = 16    (3 MMAs)
 // A operands ([w;qg], kg^T, Aqk) are state independent and come from the chunk record in
@@ -24,10 +26,10 @@
 // with v_new and Aqk (the intra-chunk term dominates o); P1 uses plain bf16 operands.
 // The result does not depend on how the rows are distributed over warps and CTAs.
 //
-// One warp executes its chain in program order: 43 MMAs of 8 cycles, 20 movmatrix of 5.5, 34 ldmatrix, and the waits
+// One warp executes its chain in program order: 45 MMAs of 8 cycles, 20 movmatrix of 5.5, 37 ldmatrix, and the waits
 // between the dependent parts.  Loads are interleaved with the MMA sequences so that their latency is covered: P1
-// carries this step's kg fragment loads and the decay of hT; P2 carries the next step's [w;qg] / decay / u loads and P3.
-// A step takes 0.34 to 0.35 us with one or two consumer warps per CTA and 0.47 with four (T8192 H32 K2 242 us), where the operand
+// carries this step's kg fragment loads and the decay of hT; P2 carries the next step's [w;qg] / decay loads and P3.
+// A step takes 0.34 to 0.35 us with one or two consumer warps per CTA and 0.45 with four (T8192 H32 K2 230 us), where the operand
 // fragments of four warps keep the SM's shared-memory pipe busy.  Measured without gain: the fragments copied into
 // tensor memory once per SM (tcgen05.cp) and read by tcgen05.ld, 0.79 us: a copy stalls the SM's mma.sync while it runs.
 //
@@ -43,10 +45,9 @@ namespace kda {
 
 // STAGES: 4, and beside K1, which holds up the records now and then, 6 (with four consumer warps, on SMs of their own, 8):
 // whole forward T131072 H16 3,756 -> 3,704 us, B2 T4096 H8 131.4 -> 129.0, T8192 H19 296 -> 277, H22 293 -> 290
-// UT = 8-column u tiles a warp reads per step (its NVT row tiles; one in the transform-pair mode)
-template <int CW, int UT, int STAGES>
+template <int STAGES>
 struct K2Smem {
-  static constexpr int STAGE = REC_SHARED_BYTES + CW * UT * REC_U_TILE_BYTES;
+  static constexpr int STAGE = REC_SHARED_BYTES + REC_V_HALF;   // a CTA's columns of v lie in one half
   static constexpr int BARS = STAGES * STAGE;               // full[S], empty[S]
   static constexpr int FLAG = BARS + 2 * STAGES * 8;        // abort flag, issued count
   static constexpr int TOTAL = FLAG + 16;
@@ -64,7 +65,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
   static_assert(!PAIR || (STATE_ONLY && NVT == 2), "the pair mode is a state-only pass over two tiles");
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr int RT = PAIR ? 1 : NVT;    // distinct 8-row tiles per warp
-  using SM = K2Smem<CW, RT, K2_STAGES>;
+  using SM = K2Smem<K2_STAGES>;
   constexpr int VCOLS = CW * RT * 8;    // state rows (v) per CTA
   constexpr int NV = D / VCOLS;         // CTAs per (batch, head)
   const int tid = threadIdx.x;
@@ -132,8 +133,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         const uint32_t dst = sbase + s * SM::STAGE;
         mbar_arrive_expect_tx(full0 + s * 8, SM::STAGE);
         bulk_g2s(dst, rec, REC_SHARED_BYTES, full0 + s * 8);
-        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_U + vs * (CW * RT * REC_U_TILE_BYTES),
-                 CW * RT * REC_U_TILE_BYTES, full0 + s * 8);
+        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_V + (vs * VCOLS >> 6) * REC_V_HALF, REC_V_HALF, full0 + s * 8);
         *sIssued = n + 1;
       }
     }
@@ -193,14 +193,43 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     const uint32_t a2_lane = kg_off((mi >> 1) * 8, (mi & 1) * 8 + r8);                 // kg^T: rows k, cols tok
     const uint32_t a3_off = REC_AQK + aq_off(r8 + (mi & 1) * 8, (mi >> 1) * 8);        // Aqk: rows i, cols j
     auto wq_at = [](uint32_t base, int ks) { return (base ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF; };
-    const uint32_t u_off = REC_SHARED_BYTES + warp * (RT * REC_U_TILE_BYTES) + lane * 16;
+    const uint32_t x_off = REC_XBH + xb_off(r8 + (mi & 1) * 8, (mi >> 1) * 8);         // Xb: rows i, cols j
+    auto v_at = [&](int nv) { return REC_SHARED_BYTES + v_off(lane & 15, (v0 + nv * 8) & 63); };   // v: rows tok, 8 columns
     __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + v0 + tq * 2;
     const bool use_u = PAIR || (pair_rt ? plane == 1 : !(STATE_ONLY && p.zero_u));
 
     uint32_t aw[8][4], aq[8][4];     // A fragments of w and qg (one per 16-wide k-step)
     float dk[8][2];                  // decay of the rows k = 16m+gq and 16m+gq+8
-    float4 u[NVT];
+    float u[NVT][4];                 // Xb v
     float oa[NVT][4];                // output tile
+
+    uint32_t xh[4], xl[4], bu[RT][2];
+    auto load_xv = [&](uint32_t sp) {
+      ldsm_x4(sp + x_off, xh[0], xh[1], xh[2], xh[3]);
+      ldsm_x4(sp + x_off + (REC_XBL - REC_XBH), xl[0], xl[1], xl[2], xl[3]);
+#pragma unroll
+      for (int nv = 0; nv < RT; ++nv) ldsm_x2_t(sp + v_at(nv), bu[nv][0], bu[nv][1]);
+    };
+    auto make_u = [&]() {
+#pragma unroll
+      for (int nv = 0; nv < NVT; ++nv) {
+        float (&acc)[4] = u[nv];
+        if (PAIR && nv == 0) {
+          acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
+          continue;
+        }
+        mma_bf16_z(acc, xh, bu[PAIR ? 0 : nv][0], bu[PAIR ? 0 : nv][1]);
+        mma_bf16_v(acc, xl, bu[PAIR ? 0 : nv][0], bu[PAIR ? 0 : nv][1]);
+        if (STATE_ONLY && !PAIR) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[e] = use_u ? acc[e] : 0.f;
+        }
+      }
+    };
+    auto load_dec = [&](uint32_t sp, int j) {
+      const float4 d = lds_f32x4(sp + REC_DEC2 + j * 128 + gq * 16);
+      dk[2 * j][0] = d.x; dk[2 * j][1] = d.y; dk[2 * j + 1][0] = d.z; dk[2 * j + 1][1] = d.w;
+    };
 
     bool failed = false;
     if (!h0_ok) {
@@ -215,13 +244,11 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_W, aw[ks][0], aw[ks][1], aw[ks][2], aw[ks][3]);
         if (!STATE_ONLY)
           ldsm_x4(wq_at(sbase + a1_lane, ks) + REC_QG, aq[ks][0], aq[ks][1], aq[ks][2], aq[ks][3]);
-        dk[ks][0] = *reinterpret_cast<const float*>(smem + REC_DEC + (ks * 16 + gq) * 4);
-        dk[ks][1] = *reinterpret_cast<const float*>(smem + REC_DEC + (ks * 16 + gq + 8) * 4);
       }
 #pragma unroll
-      for (int nv = 0; nv < NVT; ++nv)
-        u[nv] = (use_u && !(PAIR && nv == 0)) ? *reinterpret_cast<const float4*>(smem + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
-                                              : make_float4(0, 0, 0, 0);
+      for (int j = 0; j < 4; ++j) load_dec(sbase, j);
+      load_xv(sbase);
+      if (STATE_ONLY) make_u();
     }
 
     // A step is two straight runs of instructions around one branch (the slow path of the wait for the next record),
@@ -229,8 +256,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
     // instantiation of its own, the output stores are predicated and the shared-memory loads are pinned.  The stage goes
     // round as an address and a parity carried from step to step; worked out from n instead, a step takes 6 % longer, except in
     // the transform pairs, where the compiler does better with n.  K2 alone (us), before the address was carried and v_new and
-    // o were summed in pairs, and now: T8192 H32 249 / 242, H8 185 / 172, T4096 H8 96.8 / 90.7; state-only T8192 H32 183 / 181, H8 148 /
-    // 146; transform pairs T8192 H16 181 / 177, H32 258 / 260 (276 with the address carried, 282 with paired sums).
+    // o were summed in pairs, after that, and now that u is worked out here and the decay comes in four loads instead of 16:
+    // T8192 H32 249 / 242 / 230, H8 185 / 172 / 173, T4096 H8 96.8 / 90.7 / 91.0; state-only T8192 H32 183 / 181 / 185, H8 148 /
+    // 146 / 150; transform pairs T8192 H16 181 / 177 / 183, H32 258 / 260 / 263.
     __nv_bfloat16* o_at = STATE_ONLY ? nullptr : ob + static_cast<int64_t>(gq) * p.o_s[1];
     const int64_t o_step = BT * p.o_s[1], o_8 = 8 * p.o_s[1];
     int left = Tlen;
@@ -282,6 +310,9 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
           hT[ks][nv][0] = lo.x; hT[ks][nv][1] = lo.y; hT[ks][nv][2] = hi.x; hT[ks][nv][3] = hi.y;
         }
       }
+      // u under the last products of P1 (T8192 H32 K2 230 us; at the end of the step before 237).  Without outputs there is
+      // less to hide it under: at the end of the step before, its operands earlier still (state-only T8192 H8 150; here 152)
+      if (!STATE_ONLY) make_u();
       // probed here and looked at when the answer is needed: a probe and the vote on it take 126 cycles
       const bool next_ready = MORE ? mbar_test_wait(bar1, ph1) : true;
       uint32_t ah3[4], al3[4];
@@ -295,15 +326,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
 #pragma unroll
       for (int nv = 0; nv < NVT; ++nv) {
         uint32_t h01, l01, h23, l23;
-        if constexpr (PAIR) {
-        const float x0 = u[nv].x - (pw[0][nv][0] + pw[1][nv][0]), x1 = u[nv].y - (pw[0][nv][1] + pw[1][nv][1]);
-        const float x2 = u[nv].z - (pw[0][nv][2] + pw[1][nv][2]), x3 = u[nv].w - (pw[0][nv][3] + pw[1][nv][3]);
-        split_pack(x0, x1, h01, l01);
-        split_pack(x2, x3, h23, l23);
-        } else {
-        split_pack_diff(make_float2(u[nv].x, u[nv].y), &pw[0][nv][0], &pw[1][nv][0], h01, l01);
-        split_pack_diff(make_float2(u[nv].z, u[nv].w), &pw[0][nv][2], &pw[1][nv][2], h23, l23);
-        }
+        split_pack_sum(&u[nv][0], &pw[0][nv][0], &pw[1][nv][0], h01, l01);
+        split_pack_sum(&u[nv][2], &pw[0][nv][2], &pw[1][nv][2], h23, l23);
         bvh[nv][0] = movmatrix_t(h01); bvh[nv][1] = movmatrix_t(h23);
         bvl[nv][0] = movmatrix_t(l01); bvl[nv][1] = movmatrix_t(l23);
       }
@@ -339,10 +363,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
       for (int m = 0; m < 8; ++m) {
 #pragma unroll
         for (int nv = 0; nv < NVT; ++nv) mma_bf16_v(hT[m][nv], kgh[m], bvl[nv][0], bvl[nv][1]);
-        if (MORE) {
-          dk[m][0] = lds_f32(sp1 + REC_DEC + (m * 16 + gq) * 4);
-          dk[m][1] = lds_f32(sp1 + REC_DEC + (m * 16 + gq + 8) * 4);
-        }
+        if (MORE && (m & 1)) load_dec(sp1, m >> 1);
+        if (MORE && STATE_ONLY && m == 4) load_xv(sp1);
       }
 #pragma unroll
       for (int m = 0; m < 8; ++m) {
@@ -377,20 +399,27 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
         left -= BT;
       }
       if (MORE) {
-#pragma unroll
-        for (int nv = 0; nv < NVT; ++nv)
-          u[nv] = (use_u && !(PAIR && nv == 0)) ? lds_f32x4(sp1 + u_off + (PAIR ? 0 : nv) * REC_U_TILE_BYTES)
-                                                : make_float4(0, 0, 0, 0);
+        if (!STATE_ONLY) load_xv(sp1);
+        else make_u();
         if (!PAIR) { at = sp1; at_bar = bar1; at_ph = ph1; }
       }
     };
     // (With `&& !failed` as the loop's condition the compiler's schedule of a step is 10 to 15 % longer.)
     if (!failed) {
-      for (int n = 0; n + 1 < NT; ++n) {
-        step(std::true_type{}, n);
-        if (failed) break;
+      if constexpr (PAIR) {   // (the compiler's schedule of a step: T8192 H32 264 us, 272 in the other spelling)
+        int n = 0;
+        for (; n + 1 < NT; ++n) {
+          step(std::true_type{}, n);
+          if (failed) break;
+        }
+        if (n + 1 >= NT) step(std::false_type{}, n);
+      } else {
+        for (int n = 0; n + 1 < NT; ++n) {
+          step(std::true_type{}, n);
+          if (failed) break;
+        }
+        if (!failed) step(std::false_type{}, NT - 1);
       }
-      if (!failed) step(std::false_type{}, NT - 1);
     }
 
     if (!failed && (p.ht != nullptr || (PAIR && p.push_on))) {
@@ -436,7 +465,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
 template <int CW, int NVT, bool STATE_ONLY, bool PAIR = false, bool ORD = false, int K2_STAGES = 4>
 static cudaError_t launch_k2_t(const K2Params& p, cudaStream_t stream) {
   constexpr int RT = PAIR ? 1 : NVT;
-  constexpr int smem_bytes = K2Smem<CW, RT, K2_STAGES>::TOTAL;
+  constexpr int smem_bytes = K2Smem<K2_STAGES>::TOTAL;
   static std::atomic<bool> configured[64];   // set after the attributes, also for other threads
   int dev = 0;
   cudaGetDevice(&dev);
@@ -458,10 +487,10 @@ static cudaError_t launch_k2_t(const K2Params& p, cudaStream_t stream) {
 cudaError_t launch_k2n(const K2Params& p, int vsplit, int ntile, bool state_only, cudaStream_t stream) {
   // vsplit CTAs per head, ntile 8-row tiles per warp  =>  16 / (vsplit * ntile) consumer warps per CTA
   // (at most 4: a fifth warp is the producer, and CTAs of more than 8 warps lose registers per thread)
-  if (p.long_ring && !state_only && ntile == 1) {
-    if (vsplit == 4) return launch_k2_t<4, 1, false, false, false, 8>(p, stream);
-    if (vsplit == 8) return launch_k2_t<2, 1, false, false, false, 6>(p, stream);
-    if (vsplit == 16) return launch_k2_t<1, 1, false, false, false, 6>(p, stream);
+  if (p.long_ring > 4 && !state_only && ntile == 1) {
+    if (vsplit == 4 && p.long_ring == 8) return launch_k2_t<4, 1, false, false, false, 8>(p, stream);
+    if (vsplit == 8) return p.long_ring > 5 ? launch_k2_t<2, 1, false, false, false, 6>(p, stream) : launch_k2_t<2, 1, false, false, false, 5>(p, stream);
+    if (vsplit == 16) return p.long_ring > 5 ? launch_k2_t<1, 1, false, false, false, 6>(p, stream) : launch_k2_t<1, 1, false, false, false, 5>(p, stream);
   }
 #define KDA_K2_CASE(VS, NT_, CW_)                                                                  \
   if (vsplit == VS && ntile == NT_)                                                                \

@@ -55,7 +55,7 @@ constexpr int ST_K2_XCHG_TIMEOUT = 4;
 
 template <int CW>
 struct K2LSmem {
-  static constexpr int STAGE = REC_SHARED_BYTES + CW * REC_U_TILE_BYTES;
+  static constexpr int STAGE = REC_SHARED_BYTES + REC_V_HALF;   // a CTA's columns of v lie in one half
   static constexpr int XG = K2L_STAGES * STAGE;                 // 2 x {C tile, A' tile}, 512 B each
   static constexpr int BARS = XG + 2 * 1024;                    // full[S], empty[S], xbar[2]
   static constexpr int FLAG = BARS + (2 * K2L_STAGES + 2) * 8;  // abort flag, issued count
@@ -125,8 +125,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
         const uint32_t dst = sbase + s * SM::STAGE;
         mbar_arrive_expect_tx(full0 + s * 8, SM::STAGE);
         bulk_g2s(dst, rec, REC_SHARED_BYTES, full0 + s * 8);
-        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_U + vs * (CW * REC_U_TILE_BYTES), CW * REC_U_TILE_BYTES,
-                 full0 + s * 8);
+        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_V + (vs * VCOLS >> 6) * REC_V_HALF, REC_V_HALF, full0 + s * 8);
         *sIssued = n + 1;
         if (++s == S) { s = 0; ++round; }
       }
@@ -162,7 +161,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
     const uint32_t aq_lane = aq_off(a1_row, a1_col);                                   // Aqk: rows i, cols j
     const uint32_t a3_off = (a1_row * 16 + a1_col) * 2;                                // exchange tiles: rows i, cols j
     auto wq_at = [](uint32_t base, int ks) { return (base ^ ((ks & 3) << 5)) + (ks >> 2) * REC_HALF; };
-    const uint32_t u_off = REC_SHARED_BYTES + warp * REC_U_TILE_BYTES + lane * 16;
+    const uint32_t x_off = REC_XBH + xb_off(a1_row, a1_col);                           // Xb: rows i, cols j
+    const uint32_t v_at = REC_SHARED_BYTES + v_off(lane & 15, v0 & 63);                // v: rows tok, this warp's 8 columns
     // this warp's cross-Gram tiles: tile t -> part (0 = w -> C, 1 = qg -> A'), half of the 16 kg rows
     const int tile0 = warp * TPW;
     const bool has_tile = tile0 < NTILES;
@@ -176,6 +176,17 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
     }
     __nv_bfloat16* const ob = STATE_ONLY ? nullptr : p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2] + v0 + tq * 2;
     const bool use_u = !(STATE_ONLY && p.zero_u);
+    // u = Xb v of the chunk in a stage, as an accumulator fragment
+    auto load_u = [&](uint32_t sp) {
+      float acc[4];
+      uint32_t x[4], b0, b1;
+      ldsm_x2_t(sp + v_at, b0, b1);
+      ldsm_x4(sp + x_off, x[0], x[1], x[2], x[3]);
+      mma_bf16_z(acc, x, b0, b1);
+      ldsm_x4(sp + x_off + (REC_XBL - REC_XBH), x[0], x[1], x[2], x[3]);
+      mma_bf16_v(acc, x, b0, b1);
+      return use_u ? make_float4(acc[0], acc[1], acc[2], acc[3]) : make_float4(0, 0, 0, 0);
+    };
 
     bool failed = false;
     auto give_up = [&](int code) {
@@ -228,10 +239,10 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
           }
         }
       }
-      const float4 u0 = use_u ? *reinterpret_cast<const float4*>(smem + u_off) : make_float4(0, 0, 0, 0);
+      const float4 u0 = load_u(sbase);
       uint32_t h01, l01, h23, l23;
-      split_pack(u0.x - (pw[0][0] + pw[1][0]), u0.y - (pw[0][1] + pw[1][1]), h01, l01);
-      split_pack(u0.z - (pw[0][2] + pw[1][2]), u0.w - (pw[0][3] + pw[1][3]), h23, l23);
+      split_pack(u0.x + (pw[0][0] + pw[1][0]), u0.y + (pw[0][1] + pw[1][1]), h01, l01);   // (the record holds -w)
+      split_pack(u0.z + (pw[0][2] + pw[1][2]), u0.w + (pw[0][3] + pw[1][3]), h23, l23);
       bvh[0] = movmatrix_t(h01); bvh[1] = movmatrix_t(h23);
       bvl[0] = movmatrix_t(l01); bvl[1] = movmatrix_t(l23);
 #pragma unroll
@@ -253,7 +264,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
       constexpr bool MORE2 = decltype(more2_c)::value;   // chunk n+2 exists
       const uint32_t sp0 = sbase + s0 * SM::STAGE, sp1 = sbase + s1 * SM::STAGE, sp2 = sbase + s2 * SM::STAGE;
       const uint8_t* spg0 = smem + s0 * SM::STAGE;
-      const uint8_t* spg1 = smem + s1 * SM::STAGE;
       const uint32_t t0k = sp0 + a2_lane, t1a = sp1 + a1_lane, t2a = sp2 + a1_lane;
       const int xb = (n + 1) & 1;   // exchange buffer of [C ; A']_{n+1}; that of chunk n+2 is xb ^ 1
 
@@ -311,7 +321,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
         if (xb) xph1 ^= 1; else xph0 ^= 1;
         ldsm_x4(sbase + SM::XG + xb * 1024 + a3_off, cfw[0], cfw[1], cfw[2], cfw[3]);
         if (!STATE_ONLY) ldsm_x4(sbase + SM::XG + xb * 1024 + 512 + a3_off, cfq[0], cfq[1], cfq[2], cfq[3]);
-        if (use_u) un = *reinterpret_cast<const float4*>(spg1 + u_off);
+        un = load_u(sp1);
       }
 
       // decay of the fp32 state, and B fragments of its bf16 snapshot X_n (accumulator fragment ->
@@ -408,8 +418,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2la_kernel(const K2Para
       // V_{n+1} and the products of chunk n+1 for the next step
       if (MORE) {
         uint32_t h01, l01, h23, l23;
-        split_pack((un.x - pwn[1][0]) - pwn[0][0], (un.y - pwn[1][1]) - pwn[0][1], h01, l01);
-        split_pack((un.z - pwn[1][2]) - pwn[0][2], (un.w - pwn[1][3]) - pwn[0][3], h23, l23);
+        split_pack((un.x + pwn[1][0]) + pwn[0][0], (un.y + pwn[1][1]) + pwn[0][1], h01, l01);
+        split_pack((un.z + pwn[1][2]) + pwn[0][2], (un.w + pwn[1][3]) + pwn[0][3], h23, l23);
         bvh[0] = movmatrix_t(h01); bvh[1] = movmatrix_t(h23);
         bvl[0] = movmatrix_t(l01); bvl[1] = movmatrix_t(l23);
         if (!STATE_ONLY) {

@@ -2,7 +2,8 @@
 //
 // Same recurrence as kda_k2_sm100.cu (reference: src/kda_bt16/kernels.py:187-302,
 // tests/test_torch_reference.py:175-194), evaluated in the transposed form
-//   P1: [v_new^T | o^T] = h [w^T | qg^T]    (M = 16 rows v, N = 16+16 tokens, K = 128)  32 MMAs
+//   P1: [-h w^T | o^T] = h [-w^T | qg^T]    (M = 16 rows v, N = 16+16 tokens, K = 128)  32 MMAs
+//   u^T = v^T Xb^T                          (M = 16 rows v, N = 16 tokens, K = 16)      4 MMAs
 //   P2: h += v_new^T kg                     (M = 16 rows v, N = 128 k, K = 16 tokens)  3 x 16 MMAs
 //   P3: o^T += v_new^T Aqk^T                (M = 16 rows v, N = 16 tokens, K = 16)     6 MMAs
 // The state tile h[16 v][128 k] lives in registers as fp32 accumulator fragments; the
@@ -10,7 +11,7 @@
 // so bf16(h) and v_new feed the next product by a register pack alone.  The shared operands
 // (w, qg, kg, Aqk) are the B side here: a B fragment is half the size of an A fragment, so this
 // organisation reads half as many shared-memory bytes per MMA as the "n8" one, at the price of
-// a chain twice as long per warp (86 MMAs per step).  Per state row it needs fewer instructions
+// a chain twice as long per warp (90 MMAs per step).  Per state row it needs fewer instructions
 // (no transposes, operand loads shared by 16 rows), which makes it the better choice once
 // there are more 8-row tiles than SM sub-partitions (more than about 37 (batch, head) chains).
 //
@@ -24,7 +25,8 @@
 // probed a pass ahead, so that one condition (the slow path of that wait) cuts a step behind the store of the previous
 // output.  P1's sums run over even and odd k-steps apart, as in the 8-row form, so that both forms give the same bits (T8192
 // H32 298 -> 303 us).  K2 alone with conditions around the loads and now: T4096 H64 201 -> 172 us, T2048 H32 CTA-split in four 90 -> 79,
-// state-only T4096 H64 157 -> 130; one chunk, H32 in four 4.8 -> 4.4.  Producer warp, stage ring, bounded waits: as in kda_k2_sm100.cu.
+// state-only T4096 H64 157 -> 130; one chunk, H32 in four 4.8 -> 4.4.  u from eight 4-byte loads of the record and from
+// three ldmatrix and four MMAs, now: T4096 H64 167 -> 162, state-only 130 -> 122, T8192 H32 298 -> 288.  Producer warp, stage ring, bounded waits: as in kda_k2_sm100.cu.
 #include <type_traits>
 
 #include "kda_common.cuh"
@@ -34,8 +36,8 @@ namespace kda {
 
 // STAGES: 8 on an SM of its own beside K1, which holds up the records now and then (T8192 H32 363 -> 355 us); else 4
 template <int CW, int STAGES>
-struct K2mSmem {
-  static constexpr int STAGE = REC_SHARED_BYTES + CW * 2 * REC_U_TILE_BYTES;   // 16 rows = two 8-column u tiles
+struct K2mSmem {   // a CTA's columns of v lie in one half
+  static constexpr int STAGE = REC_SHARED_BYTES + REC_V_HALF;
   static constexpr int BARS = STAGES * STAGE;
   static constexpr int FLAG = BARS + 2 * STAGES * 8;
   static constexpr int OST = FLAG + 16;              // a warp's output tile: [16 tok][16 v] bf16
@@ -114,8 +116,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         const uint32_t dst = sbase + s * SM::STAGE;
         mbar_arrive_expect_tx(full0 + s * 8, SM::STAGE);
         bulk_g2s(dst, rec, REC_SHARED_BYTES, full0 + s * 8);
-        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_U + vs * (CW * 2 * REC_U_TILE_BYTES), CW * 2 * REC_U_TILE_BYTES,
-                 full0 + s * 8);
+        bulk_g2s(dst + REC_SHARED_BYTES, rec + REC_V + (vs * CW * 16 >> 6) * REC_V_HALF, REC_V_HALF, full0 + s * 8);
         *sIssued = n + 1;
       }
     }
@@ -163,9 +164,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     const uint32_t b1_lane = wq_off(r8 + (mi >> 1) * 8, (mi & 1) * 8);
     const uint32_t b2_lane = kg_off((mi & 1) * 8, (mi >> 1) * 8 + r8);               // kg: [N=k][K=tok]
     const uint32_t b3_off = REC_AQK + aq_off((mi >> 1) * 8 + r8, (mi & 1) * 8);      // Aqk: [N=i][K=j]
-    // u^T fragment of this warp out of the record's [8-column tile][lane][4] blocks (see kda_common.cuh):
-    // element (v = vrow0 + gq + 8a, tok = 2tq + j + 8c)  ->  tile 2*warp + a, lane (2tq+j)*4 + gq/2, slot 2c + gq%2
-    const uint32_t u_off = REC_SHARED_BYTES + (warp * 2) * REC_U_TILE_BYTES + ((tq * 2) * 4 + (gq >> 1)) * 16 + (gq & 1) * 4;
+    const uint32_t x_off = REC_XBH + xb_off((mi >> 1) * 8 + r8, (mi & 1) * 8);       // Xb: [N=i][K=j]
+    const uint32_t v_lane = REC_SHARED_BYTES + v_off((mi >> 1) * 8 + r8, (vrow0 + (mi & 1) * 8) & 63);   // v: rows tok, through .trans
     // the output tile: the 16-byte units of tokens 4..7 and 12..15 swapped, so that eight rows of either unit lie in different banks
     auto ost_at = [&](int tok, int unit) { return sbase + SM::OST + warp * 512 + tok * 32 + ((unit ^ ((tok >> 2) & 1)) << 4); };
     const uint32_t ost_put = ost_at((mi >> 1) * 8 + r8, mi & 1), ost_get = ost_at(lane >> 1, lane & 1);
@@ -175,18 +175,25 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
     // rolling B fragments of P1: two k-steps ahead
     uint32_t bw[2][4], bq[2][4];
-    float ut[2][4];             // u^T fragment: [token tile c][e]: e = 2a + j
+    float ut[2][4];             // u^T = v^T Xb^T, [token tile]
+    uint32_t av[4], xh[4], xl[4];
     float2 dec[16];             // decay of the columns k = 8nt + 2tq, +1 (loaded one step ahead)
 
-    auto load_u = [&](uint32_t spg) {
+    auto load_xv = [&](uint32_t sp) {
+      ldsm_x4_t(sp + v_lane, av[0], av[1], av[2], av[3]);
+      ldsm_x4(sp + x_off, xh[0], xh[1], xh[2], xh[3]);
+      ldsm_x4(sp + x_off + (REC_XBL - REC_XBH), xl[0], xl[1], xl[2], xl[3]);
+    };
+    auto make_u = [&]() {
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+      for (int c = 0; c < 2; ++c) {
+        mma_bf16_z(ut[c], av, xh[2 * c], xh[2 * c + 1]);
+        mma_bf16_v(ut[c], av, xl[2 * c], xl[2 * c + 1]);
+        if (STATE_ONLY) {
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int j = 0; j < 2; ++j)
-            ut[c][a * 2 + j] = use_u ? lds_f32(spg + u_off + a * REC_U_TILE_BYTES + j * 64 + c * 8)
-                                     : 0.f;
+          for (int e = 0; e < 4; ++e) ut[c][e] = use_u ? ut[c][e] : 0.f;
+        }
+      }
     };
     auto load_dec = [&](uint32_t spg, int nt0, int nt1) {
 #pragma unroll
@@ -208,7 +215,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     } else {
       load_b1(sbase, 0, 0);
       load_b1(sbase, 1, 1);
-      load_u(sbase);
+      load_xv(sbase);
+      make_u();
       load_dec(sbase, 0, 16);
     }
 
@@ -263,7 +271,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
       // v_new^T (fp32, accumulator layout: rows v, cols tok) and its hi/lo A fragments
       uint32_t avh[4], avl[4];
-      auto vn = [&](int c, int e) { return ut[c][e] - (pw[0][c][e] + pw[1][c][e]); };
+      auto vn = [&](int c, int e) { return ut[c][e] + (pw[0][c][e] + pw[1][c][e]); };
       split_pack(vn(0, 0), vn(0, 1), avh[0], avl[0]);
       split_pack(vn(0, 2), vn(0, 3), avh[1], avl[1]);
       split_pack(vn(1, 0), vn(1, 1), avh[2], avl[2]);
@@ -330,7 +338,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
         if (MORE) {
           if (np == 4) { load_b1(sp1, 0, 0); load_dec(sp1, 0, 6); }
           if (np == 5) { load_b1(sp1, 1, 1); load_dec(sp1, 6, 12); }
-          if (np == 6) { load_u(sp1); load_dec(sp1, 12, 16); }
+          if (np == 6) { load_xv(sp1); load_dec(sp1, 12, 16); }
+          if (np == 7) make_u();
         }
       }
 
@@ -406,7 +415,7 @@ static cudaError_t launch_k2m_c(const K2Params& p, cudaStream_t stream) {
   }
   const int nblocks = (p.n_chains > 0 ? p.n_chains : (p.seq_table != nullptr ? p.n_seqs : p.B) * p.H) * (8 / CW);
   if constexpr (CW == 4 && !STATE_ONLY)
-    if (p.long_ring) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
+    if (p.long_ring == 8) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
   if (CW == 4 && nblocks > sms[dev]) return launch_k2m_t<CW, STATE_ONLY, 2>(p, nblocks, stream);
   if constexpr (CW == 4 && !STATE_ONLY)   // the tail of a tensor-memory launch
     if (p.by_length) return launch_k2m_t<4, false, 1, true>(p, nblocks, stream);

@@ -6,13 +6,17 @@
 //   v_new = u - w h^T ;  o = scale (qg h^T) + Aqk v_new ;  h = h diag(dec) + v_new^T kg
 // One CTA owns ALL 128 state rows of one (batch, head): the fp32 state lives in tensor memory
 // (128 lanes = rows v, 128 columns = k) for the whole sequence.  Per chunk:
-//   P1  D1[v][32]  = bf16(h)[v][:] . [w ; qg]^T          8 x tcgen05.mma M128 N32 K16   (A from TMEM)
-//   E1  v_new = u - D1[:, 0:16]  ->  hi/lo bf16 pair back into TMEM          (256 threads)
+//   P1  D1[v][32]  = bf16(h)[v][:] . [-w ; qg]^T         8 x tcgen05.mma M128 N32 K16   (A from TMEM)
+//   P0  D1[v][0:16] += v^T[v][:] . Xb^T  (= u)            2 x M128 N16 K16   (A from shared memory, v as it lies)
+//   E1  v_new = D1[:, 0:16]  ->  hi/lo bf16 pair back into TMEM              (256 threads)
 //   P2  h[v][:]   += v_new^T[v][:] . kg                   3 x M128 N128 K16 (hi.hi, lo.hi, hi.lo)
 //   P3  D3[v][16]  = v_new^T[v][:] . Aqk^T                3 x M128 N16 K16
 //   E2  read h, write bf16(h) (next P1's A operand) and h * dec(next chunk); o = scale D1[:, 16:32] + D3
 // The record's tiles are tensor-core operands as they stand (kda_common.cuh): one bulk copy per chunk, no second
 // pass over them.
+//
+// P0 goes last, so that the sum over k is not rounded at the size of u again and again; first (under the state pass of the
+// step before) it is no faster.  With u read by the element-wise warps: B8 T2048 H32 185 -> 176 us, T8192 H96 447 -> 446.
 //
 // A step is a chain of hand-overs: eight MMAs, commit and wait about 190 cycles, P2 300, a TMEM load 140, the state pass
 // 600.  One CTA alone on its SM takes 0.88 us per step (the 8-row mma.sync form 0.37 to 0.49), two resident ones 1.55
@@ -34,7 +38,8 @@ namespace {
 constexpr int KT_STAGES = 3;
 constexpr int KT_EPI_WARPS = 8;
 constexpr int KT_THREADS = (KT_EPI_WARPS + 2) * 32;
-constexpr int T_STAGE = (REC_BYTES + 1023) / 1024 * 1024;   // a record as it is (1024-byte aligned: the swizzled atoms need it)
+constexpr int T_STAGE = REC_USED_BYTES;   // a record as it is
+static_assert(T_STAGE % 1024 == 0 && REC_V % 1024 == 0, "the swizzled atoms are 1024-byte aligned");
 constexpr int T_BARS = KT_STAGES * T_STAGE;
 // The state snapshot reaches the MMA thread in KT_PG column groups, so that the first k-steps of the
 // next P1 are issued while the element-wise warps still convert the rest of the state.
@@ -114,8 +119,8 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
           gate += p.win_chunks;
         }
         if (n >= KT_STAGES && !mbar_wait_bounded(empty(s), ((n / KT_STAGES) - 1) & 1, sAbort)) { give_up(); break; }
-        mbar_arrive_expect_tx(full(s), REC_BYTES);
-        bulk_g2s(sbase + s * T_STAGE, p.rec + (rec_first + n) * REC_BYTES, REC_BYTES, full(s));
+        mbar_arrive_expect_tx(full(s), REC_USED_BYTES);
+        bulk_g2s(sbase + s * T_STAGE, p.rec + (rec_first + n) * REC_BYTES, REC_USED_BYTES, full(s));
         *sIssued = n + 1;
       }
     }
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   } else if (warp == KT_EPI_WARPS + 1) {
     // ------------------------------ MMA issuer ------------------------------
     // The whole warp walks the loop, so that the descriptors stay in uniform registers; one lane issues.
-    constexpr uint32_t ID_P1 = instr_desc(128, 32), ID_P2 = instr_desc(128, 128), ID_P3 = instr_desc(128, 16);
+    constexpr uint32_t ID_P0 = instr_desc(128, 16) | INSTR_A_MN_MAJOR, ID_P1 = instr_desc(128, 32), ID_P2 = instr_desc(128, 128), ID_P3 = instr_desc(128, 16);
     auto wait = [&](uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, sAbort)) != 0; };
     int s = 0;
     uint32_t ph = 0;
@@ -147,7 +152,12 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
                 umma_ts(tbase + C_D1, tbase + C_AS + ks * 8, dwq + static_cast<uint64_t>((hf * REC_HALF + cc * 32) >> 4), ID_P1,
                         !(cc == 0 && hf == 0));
               }
-            if (q == KT_PG - 1) umma_commit(bar_p1);
+            if (q == KT_PG - 1) {
+              const uint64_t dv = smem_desc(st + REC_V, REC_V_HALF, 1024, 2);
+              umma_ss(tbase + C_D1, dv, smem_desc(st + REC_XBL, 256, 128, 0), ID_P0, 1);
+              umma_ss(tbase + C_D1, dv, smem_desc(st + REC_XBH, 256, 128, 0), ID_P0, 1);
+              umma_commit(bar_p1);
+            }
           }
           __syncwarp();
         }
@@ -172,10 +182,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   } else {
     // ------------------------------ element-wise warps ----------------------
     const int quad = warp & 3, half = warp >> 2;
-    const int v = quad * 32 + lane;                       // state row = TMEM lane
     const uint32_t tl = tbase + (static_cast<uint32_t>(quad * 32) << 16);
-    // u[tok = 8 half + j][v] in the record's fragment order
-    const uint32_t u_off = REC_U + (v >> 3) * 512 + ((v & 7) >> 1) * 16 + (half * 2 + (v & 1)) * 4;
     bool ok = true;
 
     // initial state: TMEM <- h0 * dec(chunk 0); bf16(h0) as the first A operand
@@ -225,19 +232,10 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
       give_up();
     }
 
-    float oq[8], o3[8], uv[8];
+    float oq[8], o3[8];
     uint32_t aq[8];
     __nv_bfloat16* const orow = p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2];
 
-    // State-independent operands of chunk n1: this thread's eight u values.  Runs while the tensor core works.
-    auto prepare = [&](int n1) -> bool {
-      const int s1 = n1 % KT_STAGES;
-      if (!mbar_wait_bounded(full(s1), (n1 / KT_STAGES) & 1, sAbort)) return false;
-      const uint8_t* stg = smem + s1 * T_STAGE;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) uv[j] = *reinterpret_cast<const float*>(stg + u_off + j * 64);
-      return true;
-    };
     // o[tok][v] = scale * (qg h^T) + Aqk v_new of chunk nd, from the registers filled by its E2: a warp's 8 tokens
     // x 32 rows are transposed through its own 512 bytes, so that every thread stores 16 contiguous bytes of a
     // token row and no warp waits for another.  Against whole 256-byte rows, which take a barrier over the eight
@@ -255,12 +253,11 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
             *reinterpret_cast<const uint4*>(buf + row * 64 + seg * 16);
     };
 
-    if (ok) ok = prepare(0);
     for (int n = 0; n < NT && ok; ++n) {
       const int s = n % KT_STAGES;
       const bool more = n + 1 < NT;
 
-      // ---- E1: v_new = u - w h^T for this thread's row and eight tokens ----
+      // ---- E1: v_new for this thread's row and eight tokens ----
       if (!mbar_wait_bounded(bar_p1, n & 1, sAbort)) { ok = false; break; }
       tc_fence_after();
       {
@@ -273,7 +270,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
         uint32_t vh[4], vl[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c)
-          split_pack(uv[2 * c] - __uint_as_float(d1[2 * c]), uv[2 * c + 1] - __uint_as_float(d1[2 * c + 1]), vh[c], vl[c]);
+          split_pack(__uint_as_float(d1[2 * c]), __uint_as_float(d1[2 * c + 1]), vh[c], vl[c]);
         tmem_st4(tl + C_VH + half * 4, vh);
         tmem_st4(tl + C_VL + half * 4, vl);
         tc_wait_st();
@@ -282,15 +279,15 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_v);
 
-      // while P2 runs: the next chunk's operands
+      // while P2 runs: the next chunk's record (its decay)
 #pragma unroll
       for (int j = 0; j < 8; ++j) oq[j] = __uint_as_float(aq[j]);
-      if (more && !prepare(n + 1)) { ok = false; break; }
+      if (more && !mbar_wait_bounded(full((n + 1) % KT_STAGES), ((n + 1) / KT_STAGES) & 1, sAbort)) { ok = false; break; }
 
       // ---- E2: after P2 / P3 ----
       if (!mbar_wait_bounded(bar_p2, n & 1, sAbort)) { ok = false; break; }
       tc_fence_after();
-      // dec of the next chunk (its stage was waited for in prepare)
+      // dec of the next chunk (its stage was waited for above)
       const float* decn = reinterpret_cast<const float*>(smem + ((n + 1) % KT_STAGES) * T_STAGE + REC_DEC) + half * 64;
       // the TMEM loads of the state are issued one 16-column step ahead of their use
       uint32_t sr[2][16];

@@ -101,7 +101,7 @@ struct K2Params {
   int pdl;
   const int* progress;
   int win_chunks;
-  int long_ring;     // register forms beside K1: more stages of records (where K1 leaves the shared memory for them)
+  int long_ring;     // register forms beside K1: the stages of records that K1 leaves the shared memory for
   int one_per_sm;    // no SM may take two CTAs of the launch (there are enough SMs, but K1 leaves them one by one)
 };
 

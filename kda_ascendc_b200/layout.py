@@ -14,7 +14,8 @@ CHUNK = 16
 D = 128
 REC_BYTES = 26112
 WS_HEADER_BYTES = 256
-REC_W, REC_QG, REC_KGH, REC_KGL, REC_AQK, REC_AQL, REC_DEC, REC_U = 0, 2048, 8192, 12288, 16384, 16640, 17408, 17920
+REC_W, REC_QG, REC_KGH, REC_KGL, REC_AQK, REC_AQL, REC_DEC = 0, 2048, 8192, 12288, 16384, 16640, 17408
+REC_XBH, REC_XBL, REC_DEC2, REC_V, REC_USED_BYTES = 17920, 18432, 18944, 19456, 23552
 REC_HALF = 4096   # from a 64-column half of w / qg to the other
 
 
@@ -61,8 +62,21 @@ def _aq_index(device) -> torch.Tensor:
     return (j >> 3) * 512 + i * 16 + ((j & 7) << 1)
 
 
+def _xb_index(device) -> torch.Tensor:
+    """Byte offset of element (i, j) of the hi (or lo) part of X diag(beta)."""
+    i = torch.arange(CHUNK, device=device)[:, None]
+    j = torch.arange(CHUNK, device=device)[None, :]
+    return (j >> 3) * 256 + i * 16 + ((j & 7) << 1)
+
+
+def _dec2_index(device) -> torch.Tensor:
+    """Position (in fp32 elements) of element k of the decay's second copy."""
+    k = torch.arange(D, device=device)
+    return (k >> 5) * 32 + (k & 7) * 4 + ((k >> 3) & 3)
+
+
 def _u_index(device) -> torch.Tensor:
-    """Position (in fp32 elements) of u[tok][v] inside the fragment-ordered u block."""
+    """Position (in fp32 elements) of u[tok][v] in the accumulator fragments of an 8-row K2: [column tile][lane][4]."""
     tok = torch.arange(CHUNK, device=device)[:, None]
     v = torch.arange(D, device=device)[None, :]
     tile, vr = v // 8, v % 8
@@ -74,7 +88,7 @@ def _u_index(device) -> torch.Tensor:
 def unpack_records(workspace: torch.Tensor, B: int, T: int, H: int) -> dict:
     """Decode the chunk records of a finished K1 pass.
 
-    Returns ``w, qg`` (bf16), ``kg, u`` (fp32; kg = hi + lo), ``Aqk`` (fp32 = hi + lo, ``[B,T,H,16]``)
+    Returns ``w, qg`` (bf16), ``kg, u`` (fp32; kg = hi + lo, u = X diag(beta) v of what the record holds), ``Aqk`` (fp32 = hi + lo, ``[B,T,H,16]``)
     in the public token layout (rows past ``T`` dropped) and ``dec`` fp32 ``[B,H,NT,128]``.
     """
     nt = (T + CHUNK - 1) // CHUNK
@@ -91,10 +105,11 @@ def unpack_records(workspace: torch.Tensor, B: int, T: int, H: int) -> dict:
         y = x.view(B, H, nt, CHUNK, n).permute(0, 2, 3, 1, 4).reshape(B, nt * CHUNK, H, n)
         return y[:, :T].contiguous()
 
-    uT = rec[:, REC_U:REC_U + 8192].contiguous().view(torch.float32)[:, _u_index(dev)].view(c, CHUNK, D)
-    wq, kg, aq = _wq_index(dev), _kg_index(dev), _aq_index(dev)
+    wq, kg, aq, xb = _wq_index(dev), _kg_index(dev), _aq_index(dev), _xb_index(dev)
+    v = elements(REC_V, 2 * _swizzle_index(dev).view(CHUNK, D)).float()
+    u = (elements(REC_XBH, xb).double() + elements(REC_XBL, xb).double()) @ v.double()
     aqk = elements(REC_AQK, aq).float() + elements(REC_AQL, aq).float()
     dec = rec[:, REC_DEC:REC_DEC + 512].contiguous().view(torch.float32).view(B, H, nt, D)
-    return dict(w=to_public(elements(REC_W, wq)), qg=to_public(elements(REC_QG, wq)),
+    return dict(w=to_public(-elements(REC_W, wq)), qg=to_public(elements(REC_QG, wq)),
                 kg=to_public(elements(REC_KGH, kg).float() + elements(REC_KGL, kg).float()),
-                u=to_public(uT), Aqk=to_public(aqk), dec=dec)
+                u=to_public(u.float()), Aqk=to_public(aqk), dec=dec)
