@@ -91,6 +91,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   __syncthreads();
 
   const uint8_t* rec_bh = p.rec + rec_first * REC_BYTES;
+  grid_dep_launch();
 
   if (warp == CW) {
     // ------------------------------ producer -------------------------------

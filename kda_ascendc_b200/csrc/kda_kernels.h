@@ -110,7 +110,10 @@ struct K2Params {
 constexpr int ONE_CTA_SMEM = 116 * 1024;
 inline int k2_smem(const K2Params& p, int need) { return p.one_per_sm && need < ONE_CTA_SMEM ? ONE_CTA_SMEM : need; }
 
-// One launch, with or without the programmatic stream serialization attribute.
+// One launch, with or without the programmatic stream serialization attribute.  K1 and the token recurrence are launched
+// with it: their CTAs take the places that the last kernel's leave, wait for its end and start at once.  Calls one after
+// the other, us, before and now: one-token recurrence B1 H32 5.3 / 4.6, B8 8.2 / 6.6, four tokens B16 19.3 / 17.6; B2 T1024 H4
+// forward 32.6 / 30.5.
 template <typename Kernel, typename Params>
 cudaError_t launch_dep(Kernel kernel, int grid, int block, int smem_bytes, cudaStream_t stream, int pdl, const Params& p) {
   cudaLaunchConfig_t cfg = {};

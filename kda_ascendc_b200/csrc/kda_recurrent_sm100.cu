@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(REC_WARPS * 32, 6) kda_recurrent_kernel(const 
   const int k0 = lane * 4;                             // first state column of this lane
   constexpr int SH = 4 - Log2<ROWS>::v;                // lanes that end up with one sum of a token: 1 << SH
 
+  grid_dep_start();
   float4 s[ROWS];
   constexpr int PIECE = (ROWS % 4 == 0) ? 4 : 2;   // floats per access along v in the K-first layout
   if (p.h0 != nullptr && p.k_first) {
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(128, 7) kda_recurrent_kfirst_kernel(const Recu
   const int v0 = slice * 32 + vq * 4;   // first state column of this thread
   const int k0 = kg * 8;                // first state row of this thread
 
+  grid_dep_start();
   float4 s[8];
   if (p.h0 != nullptr) {
     const float* h0 = p.h0 + (static_cast<size_t>(bh) * D + k0) * D + v0;
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(128, G_BF16 ? 7 : 6) kda_recurrent_kfirst_one_
   const int v0 = slice * 32 + vq * 4;   // first state column of this thread
   const int k0 = kg * 8;                // first state row of this thread
 
+  grid_dep_start();
   float4 s[8];
   if (p.h0 != nullptr) {
     const float* h0 = p.h0 + (static_cast<size_t>(bh) * D + k0) * D + v0;
@@ -466,14 +469,11 @@ __global__ void __launch_bounds__(128, G_BF16 ? 7 : 6) kda_recurrent_kfirst_one_
 template <int ROWS>
 cudaError_t launch_rows(const RecurrentParams& p, bool g_bf16, cudaStream_t stream) {
   const int grid = p.B * p.H * (D / (ROWS * REC_WARPS));
-  if (p.T == 1) {
-    if (g_bf16) kda_recurrent_kernel<ROWS, true, true><<<grid, REC_WARPS * 32, 0, stream>>>(p);
-    else kda_recurrent_kernel<ROWS, false, true><<<grid, REC_WARPS * 32, 0, stream>>>(p);
-  } else {
-    if (g_bf16) kda_recurrent_kernel<ROWS, true, false><<<grid, REC_WARPS * 32, 0, stream>>>(p);
-    else kda_recurrent_kernel<ROWS, false, false><<<grid, REC_WARPS * 32, 0, stream>>>(p);
-  }
-  return cudaGetLastError();
+  if (p.T == 1)
+    return g_bf16 ? launch_dep(kda_recurrent_kernel<ROWS, true, true>, grid, REC_WARPS * 32, 0, stream, 1, p)
+                  : launch_dep(kda_recurrent_kernel<ROWS, false, true>, grid, REC_WARPS * 32, 0, stream, 1, p);
+  return g_bf16 ? launch_dep(kda_recurrent_kernel<ROWS, true, false>, grid, REC_WARPS * 32, 0, stream, 1, p)
+                : launch_dep(kda_recurrent_kernel<ROWS, false, false>, grid, REC_WARPS * 32, 0, stream, 1, p);
 }
 }  // namespace
 
@@ -485,14 +485,11 @@ cudaError_t launch_recurrent(const RecurrentParams& p, bool g_bf16, int sms, cud
     // four CTAs per head with the lanes along v; with fewer heads the calls are latency-bound and the
     // row-per-warp kernel's strided state accesses cost nothing measurable
     const int grid = static_cast<int>(bh) * 4;
-    if (p.T == 1) {
-      if (g_bf16) kda_recurrent_kfirst_one_kernel<true><<<grid, 128, 0, stream>>>(p);
-      else kda_recurrent_kfirst_one_kernel<false><<<grid, 128, 0, stream>>>(p);
-    } else {
-      if (g_bf16) kda_recurrent_kfirst_kernel<true><<<grid, 128, 0, stream>>>(p);
-      else kda_recurrent_kfirst_kernel<false><<<grid, 128, 0, stream>>>(p);
-    }
-    return cudaGetLastError();
+    if (p.T == 1)
+      return g_bf16 ? launch_dep(kda_recurrent_kfirst_one_kernel<true>, grid, 128, 0, stream, 1, p)
+                    : launch_dep(kda_recurrent_kfirst_one_kernel<false>, grid, 128, 0, stream, 1, p);
+    return g_bf16 ? launch_dep(kda_recurrent_kfirst_kernel<true>, grid, 128, 0, stream, 1, p)
+                  : launch_dep(kda_recurrent_kfirst_kernel<false>, grid, 128, 0, stream, 1, p);
   }
   if (bh * 4 >= 2LL * sms) return launch_rows<8>(p, g_bf16, stream);
   if (bh * 8 >= 2LL * sms) return launch_rows<4>(p, g_bf16, stream);

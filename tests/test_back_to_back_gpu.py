@@ -1,0 +1,70 @@
+"""Calls one after the other without a wait on the host: each starts ahead of the end of the one before and must not read
+what that one still writes."""
+import pytest
+import torch
+
+import kda_ascendc_b200 as K
+from oracle import kda_oracle as O
+from tests.conftest import to_device
+
+pytestmark = pytest.mark.gpu
+FLAGS = dict(use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True, output_final_state=True)
+
+
+def _inputs(B, T, H, dev):
+    d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.3), dev)
+    d["g"] = (d["g"].float() - 4.0).bfloat16()     # decays that leave much of the state
+    return d
+
+
+def _piece(d, a, b):
+    return [d[n][:, a:b].contiguous() for n in ("q", "k", "v", "g", "beta")]
+
+
+# 8-row, 16-row and tensor-memory K2, one to six chunks a call: every call's initial state is the final state of the one before
+@pytest.mark.parametrize("B,H,piece", [(1, 32, 16), (1, 2, 96), (2, 30, 32), (5, 32, 64)])
+def test_pieces_of_a_sequence(cuda_device, B, H, piece):
+    n = 24
+    d = _inputs(B, n * piece, H, cuda_device)
+    kw = dict(scale=d["scale"], lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"], **FLAGS)
+    pieces = [_piece(d, i * piece, (i + 1) * piece) for i in range(n)]
+
+    def walk(wait):
+        h, os = d["initial_state"], []
+        for x in pieces:
+            o, h = K.kda_bt16_fwd(*x, initial_state=h, **kw)
+            if wait:
+                torch.cuda.synchronize()
+            os.append(o)
+        return torch.cat(os, 1), h
+
+    want = walk(True)
+    for _ in range(5):
+        got = walk(False)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("B,T,k_first", [(1, 1, False), (64, 1, False), (64, 1, True), (16, 4, False), (16, 4, True)])
+def test_decode_steps_behind_a_forward(cuda_device, B, T, k_first):
+    """A forward, then steps on its final state in place; inputs made on the stream right before each call."""
+    H, n = 16, 12
+    d = _inputs(B, 32 + n * T, H, cuda_device)
+    kw = dict(scale=d["scale"], lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"], state_v_first=not k_first)
+    h0 = d["initial_state"].transpose(-1, -2).contiguous() if k_first else d["initial_state"]
+
+    def walk(wait):
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        _, h = K.kda_bt16_fwd(*_piece(d, 0, 32), initial_state=h0, **kw, **FLAGS)
+        sync()
+        os = []
+        for i in range(n):
+            x = _piece(d, 32 + i * T, 32 + (i + 1) * T)
+            sync()
+            os.append(K.kda_recurrent_fwd(*x, initial_state=h, inplace_state=True, **kw)[0])
+            sync()
+        return torch.cat(os, 1), h
+
+    want = walk(True)
+    for _ in range(5):
+        got = walk(False)
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
