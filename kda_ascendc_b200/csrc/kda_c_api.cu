@@ -172,21 +172,21 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // is already running.  On k2_sms of the SMs only k2_sm_ctas of K1's CTAs stay (k1_stays), and K2's CTAs fit nowhere else.
 // Which of it pays, measured on B200 as the whole forward in us, K2 after K1 against beside it unless said otherwise:
 //   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on every SM: B1 T32768 H16 1,028 /
-//     987, T8192 H16 266.5 / 259.1, H8 236 / 226 (an earlier K1).  With four on the SMs that K2 leaves free T131072 H16 3,727 against 3,704, B2
-//     T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
-//   Up to 23 of 148 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H19 337 / 277, H22
-//     351 / 290, T2500 H19 113 / 110, H23 117 / 115.  Beyond, K1 has too few SMs left: T8192 H24 360 / 363, T2500 H25 121 / 134.
-//   From there to 42 of 148 chains: the 16-row form, whose bits are the same, on SMs of its own (2 per chain), at chunk counts
-//     that make up for its longer step: T8192 H24 360 / 352, H32 397 / 355, H37 418 / 393, H38 511 / 410, H40 519 / 447; T4096
-//     H23 184 / 189, H25 189 / 189, H28 195 / 189, H34 208 / 192, H38 256 / 209, H42 265 / 248; T2048 H32 109 / 109, H40 137 /
-//     126, H42 138 / 136; T2500 H25 121 / 126, H30 127 / 129; T1600 H38 109 / 97, H42 112 / 112, H43 113 / 117; T1100 H37 67 /
-//     74, H40 80 / 78, H42 81 / 83.  With a K1 CTA beside K2's: T8192 H32 403.
-//   Tensor-memory form with one CTA per SM and two K1 CTAs there (a K1 of 112 registers: see there), four on the other SMs,
-//     against two everywhere up to 111 chains and after K1 beyond: T8192 H96 850 / 721, T4096 H75 371 / 337, H111 493 / 442, T1024
-//     H75 105 / 104, H96 123 / 115, H111 134 / 124; T1024 H120 142 / 135, T4096 H120 504 / 493, H128 524 / 521, H136 545 / 560.
-//   The same form, two CTAs per SM on SMs of their own, where its step for two (1.36 us) and K1 on the others take the same
-//     time, and long chains: against the line above T8192 H88 689 / 690, H96 721 / 701, H104 782 / 780, H111 839 / 857, T2048
-//     H96 198 / 199, T512 H96 68.6 / 75.4.
+//     987, T8192 H16 266.5 / 259.1, H8 236 / 226 (an earlier K1).  With four on the SMs that K2 leaves free T131072 H16 3,727
+//     against 3,704, B2 T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
+//   Up to SMs / 6 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H23 326 / 283, H24
+//     330 / 312, T2500 H23 107 / 102, H24 110.5 / 109.9.  Beyond, K1 has too few SMs left: H25 335 / 347, T2500 111 / 119.
+//   From there to 42 of 148 chains: the 16-row form, whose bits are the same, on SMs of its own (2 per chain).  Where the 8-row
+//     form is the choice, at chunk counts that make up for the longer step (0.66 us against 0.45 and K1's time): T8192 H25 335 /
+//     341, H26 339 / 341, H32 397 / 341, T2500 H28 115 / 120, H32 119 / 121, H37 126 / 122, T1600 H32 82 / 85, H37 83 / 86.
+//     Where the 16-row form is the choice anyway: T2500 H40 154 / 136, H42 155 / 148, H44 159 / 163, T1600 H40 101 / 93, H42 102 /
+//     101, H44 106 / 111, T8192 H43 492 / 460.  With a K1 CTA beside K2's: T8192 H32 403 against 363.
+//   Tensor-memory form with one CTA per SM and two K1 CTAs there (a K1 of 112 registers: see there), four on the other SMs:
+//     T1024 H75 108 / 101, H96 121 / 109, H123 136 / 127, H136 143 / 139, H148 149 / 152; T8192 H75 754 / 636, H96 834 / 686,
+//     H123 942 / 867, H136 998 / 969, H148 1,046 / 1,082.
+//   The same form, two CTAs per SM on SMs of their own, where its step for two (1.27 us) and K1 on the others take about the
+//     same time, and long chains: against the line above T8192 H75 636 / 639, H88 672 / 655, H96 686 / 651, H104 716 / 705, H111
+//     769 / 772; T1024 H88 106 / 108, H96 109 / 107, H111 115 / 120.
 struct Beside {
   int win;                       // chunks per window; 0 = K2 starts after K1
   int variant, vsplit;           // K2's form: pick_split's, or one with the same bits
@@ -203,13 +203,13 @@ Beside beside_plan(const KdaFwdArgs* a) {
   long long k2_sms = 0;
   if (r.variant == 1 && r.vsplit >= 8 && chains * r.vsplit <= r.sms) {
     k2_sms = r.sms; r.k2_sm_ctas = 2;
-  } else if (automatic && r.variant == 1 && chains * 32 <= 5LL * r.sms) {
+  } else if (automatic && r.variant == 1 && chains * 6 <= r.sms) {
     k2_sms = chains * 4;
-  } else if (automatic && ((r.variant == 1 && chains * nt >= 6400) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 96))) {
+  } else if (automatic && ((r.variant == 1 && (chains * 6 - r.sms) * nt >= 7500) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 96))) {
     k2_sms = chains * 2; r.variant = 3; r.vsplit = 2;
-  } else if (r.variant == 4 && chains * 5 > 3LL * r.sms && chains * 10 <= 7LL * r.sms && nt >= 512) {
+  } else if (r.variant == 4 && chains * 11 > 6LL * r.sms && chains * 10 <= 7LL * r.sms && nt >= 256) {
     k2_sms = (chains + 1) / 2;
-  } else if (r.variant == 4 && chains * 6 <= 5LL * r.sms) {
+  } else if (r.variant == 4 && chains * 14 <= 13LL * r.sms) {
     k2_sms = chains; r.k2_sm_ctas = 2;
   } else {
     return r;
