@@ -482,8 +482,9 @@ int kda_fwd(const KdaFwdArgs* a, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const Beside side = beside_plan(a);
   if (side.win > 0) {   // the window counters must be zero before either kernel starts
-    cudaError_t e = cudaMemsetAsync(a->workspace, 0, kda::WS_HEADER_BYTES, st);
+    cudaError_t e = kda::launch_clear_header(status_ptr(a), st);
     if (e != cudaSuccess) return fail(KDA_ERR_CUDA, "kda: header clear failed: %s", cudaGetErrorString(e));
+    ++g_launches;
   }
   if (int rc = do_k1(a, st, side)) return rc;
   return do_k2(a, false, 0, st, nullptr, nullptr, true, side);

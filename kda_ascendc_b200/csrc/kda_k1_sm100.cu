@@ -166,7 +166,6 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   float* sGmid = reinterpret_cast<float*>(smem + SM::GMID);
   float* sTot1 = sTot + D;
   volatile int* sFlag = reinterpret_cast<volatile int*>(smem + SM::FLAG);
-  if (BESIDE) grid_dep_launch();   // K2 may run beside this kernel
 
   const bool use_gate = FORM == FORM_ANY ? (p.flags & 1u) != 0 : FORM == FORM_ALL;
   const bool use_l2 = FORM == FORM_ANY ? (p.flags & 2u) != 0 : FORM == FORM_ALL;
@@ -179,14 +178,14 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     mbar_init(mbar_v, 1);
     sFlag[0] = 0;   // a wait gave up
     fence_mbar_init();
-    if (!BESIDE) grid_dep_wait();   // (beside K2 this is an ordinary launch) the barrier holds the rest of the CTA
+    grid_dep_wait();   // the barrier holds the rest of the CTA
     if (!BESIDE && blockIdx.x == 0) *reinterpret_cast<int2*>(p.status) = make_int2(ST_OK, ST_OK);
     if (BESIDE) sFlag[1] = k1_stays(p) ? atomicAdd(p.progress - HDR_PROGRESS + HDR_TICKET, 2) : n_items;
   }
   __syncthreads();
-  // K2 may be set up beside this kernel.  Not before this kernel's own wait: K2 reads the initial state, and the table of
-  // packed sequences, without waiting for more than this.
-  if (!BESIDE) grid_dep_launch();
+  // K2 may be set up, or run, beside this kernel.  Not before this kernel's own wait: K2 reads the initial state, and the table
+  // of packed sequences, without waiting for more than this.
+  grid_dep_launch();
 
   // issue the input copies of one work item: one tiled TMA box (16 tokens x 128) per tensor.
   // The box may reach past T in the last chunk; those rows arrive as zeros and still count
@@ -684,6 +683,17 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
   }
 }
 
+// Clears the header for a K1 with K2 beside it: starts ahead of the end of the call before, and K1 ahead of this one's end.
+__global__ void kda_clear_header_kernel(int* header) {
+  grid_dep_wait();
+  header[threadIdx.x] = 0;
+  grid_dep_launch();
+}
+
+cudaError_t launch_clear_header(int* header, cudaStream_t stream) {
+  return launch_dep(kda_clear_header_kernel, 1, WS_HEADER_BYTES / 4, 0, stream, 1, header);
+}
+
 template <bool G_BF16, bool FAST_EXP, bool BESIDE, K1Form FORM>
 static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   constexpr int smem_bytes = K1Smem<G_BF16, FAST_EXP>::TOTAL;
@@ -712,7 +722,7 @@ static cudaError_t launch_k1_t(const K1Params& p, cudaStream_t stream) {
   const long long n_items = (p.chunk_table != nullptr ? static_cast<long long>(p.n_chunks) : static_cast<long long>(p.B) * p.NT) * p.H;
   const int cap = (res >> 8) * (res & 255);   // persistent: one CTA per slot
   const int grid = static_cast<int>(n_items < cap ? n_items : cap);
-  return launch_dep(kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, FORM>, grid, 128, smem_bytes, stream, !BESIDE, p);
+  return launch_dep(kda_k1_kernel<G_BF16, FAST_EXP, BESIDE, FORM>, grid, 128, smem_bytes, stream, 1, p);
 }
 
 namespace {

@@ -130,6 +130,7 @@ cudaError_t launch_dep(Kernel kernel, int grid, int block, int smem_bytes, cudaS
 }
 
 cudaError_t launch_k1(const K1Params& p, bool g_bf16, bool fast_exp, cudaStream_t stream);
+cudaError_t launch_clear_header(int* header, cudaStream_t stream);
 // Fills the four tensor maps of p from its pointers, sizes and strides (host, no device work).
 cudaError_t k1_encode_tensor_maps(K1Params& p, bool g_bf16, const char** what);
 // Two organisations of K2 (same arithmetic, bit-identical results within one organisation):
