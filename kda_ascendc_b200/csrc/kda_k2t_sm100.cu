@@ -20,7 +20,7 @@
 //
 // A step is a chain of hand-overs: eight MMAs, commit and wait about 190 cycles, P2 300, a TMEM load 140, the state pass
 // 600.  One CTA alone on its SM takes 0.88 us per step (the 8-row mma.sync form 0.37 to 0.49), two resident ones 1.55
-// together (256 of the 512 TMEM columns, 88 KB of shared memory each): the form pays once there are enough chains.
+// together (256 of the 512 TMEM columns, 100 KB of shared memory each): the form pays once there are enough chains.
 // Every tcgen05 instruction is issued behind elect.sync (see elect_one) by a warp that walks the loop as a whole.  K2
 // alone with the instructions behind lane == 0 and records loaded by tiled copies, and now: T8192 H96 606 -> 447 us,
 // B8 T1024 H32 110.5 -> 98.6.
@@ -35,7 +35,9 @@ namespace kda {
 
 namespace {
 
-constexpr int KT_STAGES = 3;
+// Four stages, given back by a commit behind P3: K2 alone T8192 H96 447 -> 432 us (three and by an element-wise warp at the end of
+// its state pass before; two: 689), the forward, K1 beside it, 654 -> 633.  Two CTAs of five do not fit an SM.
+constexpr int KT_STAGES = 4;
 constexpr int KT_EPI_WARPS = 8;
 constexpr int KT_THREADS = (KT_EPI_WARPS + 2) * 32;
 constexpr int T_STAGE = REC_USED_BYTES;   // a record as it is
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
         umma_ts(tbase + C_D3, tbase + C_VL, dah, ID_P3, 1);
         umma_ts(tbase + C_D3, tbase + C_VH, dal, ID_P3, 1);
         umma_commit(bar_p3);
+        umma_commit(empty(s));   // the products are the last to read the stage: its decay was read in the step before
       }
       __syncwarp();
       if (++s == KT_STAGES) { s = 0; ph ^= 1; }
@@ -255,7 +258,6 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     };
 
     for (int n = 0; n < NT && ok; ++n) {
-      const int s = n % KT_STAGES;
       const bool more = n + 1 < NT;
 
       // ---- E1: v_new for this thread's row and eight tokens ----
@@ -330,7 +332,6 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
       // Aqk v_new of this chunk (P3 was committed after P2; it must leave TMEM before the next P3)
       if (!mbar_wait_bounded(bar_p3, n & 1, sAbort)) { ok = false; break; }
       tc_fence_after();
-      if (tid == 0) mbar_arrive(empty(s));   // every operand of this stage has been consumed
       {
         uint32_t c3[8];
         tmem_ld8(tl + C_D3 + half * 8, c3);
