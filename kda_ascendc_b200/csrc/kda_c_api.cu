@@ -1,5 +1,6 @@
 // C-ABI layer of libkda_b200.so: argument checks, workspace arithmetic, stage launches.
 // Interface and the reference entry points it stands in for: include/kda_b200.h.
+#include <algorithm>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -434,7 +435,32 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     // chunks, H16: 420 us in their own order, 435 by length; of 8 to 13 chunks 701 and 709, of 29 1,240 and 1,040).
     const long long mean_steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : 0;
     p.by_length = a->n_seqs > 1 && a->n_seqs <= kda::MAX_SORTED_SEQS && bh > sms && bh <= 4LL * sms * mean_steps;
-    if (a->k2_variant == 0 && bh > 2LL * sms && tail > 0 && tail * 2 <= sms) {
+    // A sequence much longer than the others: its chains go on alone when the rest is done, at 1.3 us per step while their SM
+    // has a second CTA and 0.85 without, against 0.56 in the 16-row form.  So the longest sequences, on at most half of the
+    // SMs, run there, in front of and beside the tensor-memory launch (which starts when K1 has ended, about 2 us later
+    // than without), if they are long: more steps than 0.9 x the chunks of all chains per SM, which take 0.67 us each in pairs,
+    // and than 1.5 x the mean.  The lengths are on the device: either kernel leaves out what the other does.  Whole forward, us,
+    // without / with, log-normal lengths (sigma 1): 24 sequences of 16,411 tokens H32 487 / 467, 40 of 30,000 H8 297 / 245, 20 of
+    // 20,000 H8 290 / 227, 10 of 12,000 H16 286 / 227, 8 of 24,000 H32 802 / 741, 6 of 20,000 H32 652 / 637, 9 of 14,000 H16 396 /
+    // 317, 12 of 30,000 H8 419 / 339.  Where no sequence is long: 64 of 32,000 H32 879 / 880, 12 of 8,000 H32 238 / 240,
+    // 16 x 1,024 H32 441 / 443, 32 x 500 H16 238 / 240, 5 x 2,000 H32 314 / 317; shorter ones do not pay for the launch (8 x 520 H32
+    // 126 / 128).  On all SMs instead of half of them 6 of 20,000 H32 takes 692; with 1.25 x the mean 4 x 2,500 H32 304 / 356.
+    const long long items = static_cast<long long>(a->n_chunks) * a->H;
+    const int long_max = static_cast<int>(std::min<long long>(a->n_seqs - 1, sms / (4LL * a->H)));
+    if (a->k2_variant == 0 && (p.by_length || bh <= sms) && a->n_seqs <= kda::MAX_SORTED_SEQS && long_max > 0 && items >= 64LL * sms) {
+      p.by_length = 1;
+      p.long_max = long_max;
+      p.long_len = static_cast<int>(std::max(9 * items / (10LL * sms), 3LL * a->n_chunks / (2LL * a->n_seqs))) + 1;
+      p.n_chains = long_max * a->H;
+      p.one_per_sm = 1;
+      e = kda::launch_k2m(p, 2, false, st);
+      if (e == cudaSuccess) {
+        ++g_launches;
+        p.n_chains = p.one_per_sm = 0;
+        p.pdl = 1;
+        e = kda::launch_k2t(p, st);
+      }
+    } else if (a->k2_variant == 0 && bh > 2LL * sms && tail > 0 && tail * 2 <= sms) {
       p.chain0 = 0;
       p.n_chains = static_cast<int>(bh - tail);
       e = kda::launch_k2t(p, st);

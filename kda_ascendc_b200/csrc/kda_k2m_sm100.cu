@@ -71,6 +71,10 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
     tok0 = e.x; NT = e.y; Tlen = e.w;
     rec_first = static_cast<size_t>(e.z) + static_cast<size_t>(h) * NT;
     b = 0;
+    if (ORD && NT < p.long_len) {   // left to the tensor-memory form, which takes the end of K1 from this kernel
+      grid_dep_wait();
+      return;
+    }
   }
 
   const uint32_t sbase = smem_u32(smem);
@@ -91,12 +95,13 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   __syncthreads();
 
   const uint8_t* rec_bh = p.rec + rec_first * REC_BYTES;
-  grid_dep_launch();
+  if (!ORD || p.long_len == 0) grid_dep_launch();
 
   if (warp == CW) {
     // ------------------------------ producer -------------------------------
     if (lane == 0) {
       if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      if (ORD && p.long_len > 0) grid_dep_launch();
       int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
         const int s = n % K2M_STAGES;

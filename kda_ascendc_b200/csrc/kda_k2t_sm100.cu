@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     tok0 = e.x; NT = e.y; Tlen = e.w;
     rec_first = static_cast<size_t>(e.z) + static_cast<size_t>(h) * NT;
     b = 0;
+    if (p.long_len > 0 && NT >= p.long_len && (blockIdx.x + p.chain0) / p.H < p.long_max) return;   // in the 16-row form
   }
 
   const uint32_t sbase = smem_u32(smem);
@@ -110,7 +111,8 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   if (warp == KT_EPI_WARPS) {
     // ------------------------------ producer -------------------------------
     if (elect_one()) {
-      if (p.progress == nullptr) grid_dep_wait();   // K1's records; everything above ran under K1's tail
+      // K1's records; everything above ran under K1's tail.  Behind a 16-row launch for the long sequences K1 has ended.
+      if (p.progress == nullptr && p.long_len == 0) grid_dep_wait();
       int gate = 0;                                 // beside K1: the first chunk of the next window
       for (int n = 0; n < NT; ++n) {
         const int s = n % KT_STAGES;
@@ -385,7 +387,7 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   __syncthreads();
   if (warp == KT_EPI_WARPS + 1)
     tmem_dealloc(tbase, C_TOTAL);
-  if (p.progress != nullptr) grid_dep_wait();   // this grid ends after K1
+  if (p.progress != nullptr || (p.long_len > 0 && blockIdx.x == gridDim.x - 1)) grid_dep_wait();   // this grid ends after K1, or the 16-row launch
 }
 
 }  // namespace

@@ -80,6 +80,9 @@ struct K2Params {
   const int4* seq_table;
   int n_seqs;
   int by_length;     // packed: chains are taken longest sequence first (n_seqs <= MAX_SORTED_SEQS)
+  // packed, longest first: of the first long_max sequences those of long_len chunks or more run in the 16-row form, launched
+  // in front of the tensor-memory form, which leaves them out (0: none)
+  int long_len, long_max;
   // a launch may cover a sub-range of the (batch, head) chains: first chain and count (0 = all)
   int chain0, n_chains;
   // Transform-pair pass of a sequence split over peer memory (the 8-row pair form only): the (M, Q) tiles
