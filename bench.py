@@ -70,7 +70,7 @@ K2_FLOPS_PER_CHUNK = 1638400.0
 NCU_TRAFFIC = dict(shape=(1, 8192, 32), source="profiles/kda_k1_k2_B1_T8192_H32.md",
                    record=dict(REC_W=0, REC_QG=2048, REC_HALF=4096, REC_KGH=8192, REC_KGL=12288, REC_AQK=16384, REC_AQL=16640,
                                REC_DEC=17408, REC_XBH=17920, REC_XBL=18432, REC_DEC2=18944, REC_V=19456, REC_USED_BYTES=23552),
-                   bytes={"kda_k1": 642.58e6, "kda_k2": 488.83e6})
+                   bytes={"kda_k1": 602.40e6, "kda_k2": 445.85e6})
 
 
 def merge_exchange_marks(names, values):
@@ -374,7 +374,9 @@ def run_gpu_arm(steps, warmup, n_gpus, kernels_only=False):
     # encoding and the launch itself, about 6 us, would otherwise sit inside K1's interval).
     k1_ms, k2_ms = [], []
     ev = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(steps)]
-    assert lib.kda_fwd(ctypes.byref(args), stream) == 0, _lib.last_error()   # keeps the GPU busy while the first pair is queued
+    for _ in range(2):   # untimed: the stage calls may run other kernels than the whole forward, and the GPU is kept busy while the first pair is queued
+        assert lib.kda_fwd_k1(ctypes.byref(args), stream) == 0, _lib.last_error()
+        assert lib.kda_fwd_k2(ctypes.byref(args), stream) == 0, _lib.last_error()
     for e in ev:
         e[0].record()
         assert lib.kda_fwd_k1(ctypes.byref(args), stream) == 0, _lib.last_error()
@@ -419,7 +421,9 @@ def run_gpu_arm(steps, warmup, n_gpus, kernels_only=False):
         launches_heads = steps * lib.kda_last_launch_count()
         hk1, hk2 = [], []
         evh = [[torch.cuda.Event(enable_timing=True) for _ in range(3)] for _ in range(min(steps, 10))]
-        fwd_heads()                       # keeps the GPU busy while the first pair is queued (as above)
+        for _ in range(2):                # untimed (as above)
+            assert lib.kda_fwd_k1(ctypes.byref(args_h), stream) == 0, _lib.last_error()
+            assert lib.kda_fwd_k2(ctypes.byref(args_h), stream) == 0, _lib.last_error()
         for e in evh:
             e[0].record()
             assert lib.kda_fwd_k1(ctypes.byref(args_h), stream) == 0, _lib.last_error()
