@@ -417,8 +417,8 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   if (variant == 4) {
     // Tail wave.  The tensor-memory form holds two chains per SM at once; when the chains left over
     // after the full waves are at most half as many as SMs, they run faster in an mma.sync form
-    // (8-row for at most SMs/4 chains, 0.49 us per step; 16-row: two CTAs per chain, one per SM, 0.65 us
-    // per step; against 0.9 for a lone tensor-memory CTA), launched behind the full waves, at every length that the
+    // (8-row for at most SMs/4 chains, 0.45 us per step; 16-row: two CTAs per chain, one per SM, 0.56 us
+    // per step; against 0.84 for a lone tensor-memory CTA), launched behind the full waves, at every length that the
     // tensor-memory form is chosen for.  kda_fwd in us, no tail / 16-row / 8-row, 296 chains and so many more x chunks:
     // 9 x 4 45.5 / 43.4 / 41.3, 9 x 64 335 / 325 / 306; 37 x 4 47.3 / 45.0 / 45.2, 37 x 64 353 / 342 / 331; 38 x 4 47.9 /
     // 45.3 / 47.4, 38 x 64 353 / 343 / 363; 74 x 4 49.7 / 47.7 / 50.5, 74 x 64 374 / 365 / 389; 75 x 4 50.7 / 52.6,

@@ -19,7 +19,7 @@
 // step before) it is no faster.  With u read by the element-wise warps: B8 T2048 H32 185 -> 176 us, T8192 H96 447 -> 446.
 //
 // A step is a chain of hand-overs: eight MMAs, commit and wait about 190 cycles, P2 300, a TMEM load 140, the state pass
-// 600.  One CTA alone on its SM takes 0.88 us per step (the 8-row mma.sync form 0.37 to 0.49), two resident ones 1.55
+// 600.  One CTA alone on its SM takes 0.84 us per step (the 8-row mma.sync form 0.34 to 0.45), two resident ones 1.34
 // together (256 of the 512 TMEM columns, 100 KB of shared memory each): the form pays once there are enough chains.
 // Every tcgen05 instruction is issued behind elect.sync (see elect_one) by a warp that walks the loop as a whole.  K2
 // alone with the instructions behind lane == 0 and records loaded by tiled copies, and now: T8192 H96 606 -> 447 us,
