@@ -21,7 +21,8 @@
 // the decay row and the kg(hi) fragments; P2's first two passes carry kg(lo), its last pass the
 // next step's first fragments; the output tile is transposed through 512 bytes of a warp's own
 // (stmatrix) and leaves one step late, 16 bytes a lane, as whole 32-byte sectors (four 4-byte stores behind movmatrix before:
-// K2 alone T4096 H64 172 -> 167 us, the forward T8192 H32 with K2 on SMs of its own 381 -> 363).  The last step, which has no next record, is an instantiation of its own, and the next record's barrier is
+// K2 alone T4096 H64 172 -> 167 us, the forward T8192 H32 with K2 on SMs of its own 381 -> 363), through a pointer that is carried
+// along (worked out from the chunk number in front of every step: 162 instead of 155, 342 instead of 327).  The last step, which has no next record, is an instantiation of its own, and the next record's barrier is
 // probed a pass ahead, so that one condition (the slow path of that wait) cuts a step behind the store of the previous
 // output.  P1's sums run over even and odd k-steps apart, as in the 8-row form, so that both forms give the same bits (T8192
 // H32 298 -> 303 us).  K2 alone with conditions around the loads and now: T4096 H64 201 -> 172 us, T2048 H32 CTA-split in four 90 -> 79,
@@ -226,6 +227,8 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       load_dec(sbase, 0, 16);
     }
 
+    __nv_bfloat16* o_at = ob;   // of the previous chunk
+    const int64_t o_step = STATE_ONLY ? 0 : BT * p.o_s[1];
     auto step = [&](auto more_c, int n) {
       constexpr bool MORE = decltype(more_c)::value;   // chunk n + 1 exists
       const int s = n % K2M_STAGES;
@@ -234,8 +237,10 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
       const uint32_t sp1 = sbase + s1 * SM::STAGE;
 
       // the previous step's output tile (always a full chunk): 16 bytes of a token row per lane
-      if (!STATE_ONLY && n > 0)
-        *reinterpret_cast<uint4*>(ob + static_cast<int64_t>((n - 1) * BT) * p.o_s[1]) = lds_u32x4(ost_get);
+      if (!STATE_ONLY && n > 0) {
+        *reinterpret_cast<uint4*>(o_at) = lds_u32x4(ost_get);
+        o_at += o_step;
+      }
 
       // P1 with the A fragments of bf16(h) packed on the fly; carries the decay of the fp32 state,
       // its own rolling B loads and the kg(hi) fragments of this step
@@ -362,7 +367,7 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
 
     // the last chunk's output tile (it may be a partial chunk)
     if (!STATE_ONLY && !failed) {
-      const int tok = (NT - 1) * BT;
+      const int tok = (NT - 1) * BT;   // (not by o_at: kept alive so far it costs the steps 2 %)
       if (tok + (lane >> 1) < Tlen) *reinterpret_cast<uint4*>(ob + static_cast<int64_t>(tok) * p.o_s[1]) = lds_u32x4(ost_get);
     }
 
