@@ -176,12 +176,13 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 //     987, T8192 H16 266.5 / 259.1, H8 236 / 226 (an earlier K1).  With four on the SMs that K2 leaves free T131072 H16 3,727
 //     against 3,704, B2 T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
 //   Up to SMs / 6 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H23 326 / 283, H24
-//     330 / 312, T2500 H23 107 / 102, H24 110.5 / 109.9.  Beyond, K1 has too few SMs left: H25 335 / 347, T2500 111 / 119.
+//     330 / 309, T4096 H24 172 / 164, T2500 H23 107 / 102. Beyond, K1 has too few SMs left: T4096 H25 173 / 181.
 //   From there to 42 of 148 chains: the 16-row form, whose bits are the same, on SMs of its own (2 per chain).  Where the 8-row
-//     form is the choice, at chunk counts that make up for the longer step (0.66 us against 0.45 and K1's time): T8192 H25 335 /
-//     341, H26 339 / 341, H32 397 / 341, T2500 H28 115 / 120, H32 119 / 121, H37 126 / 122, T1600 H32 82 / 85, H37 83 / 86.
-//     Where the 16-row form is the choice anyway: T2500 H40 154 / 136, H42 155 / 148, H44 159 / 163, T1600 H40 101 / 93, H42 102 /
-//     101, H44 106 / 111, T8192 H43 492 / 460.  With a K1 CTA beside K2's: T8192 H32 403 against 363.
+//     form is the choice, at chunk counts that make up for the longer step (0.61 us against 0.45 and K1's time): T8192 H25 335 /
+//     322, H32 362 / 326, H37 380 / 346; T4096 H25 173 / 171, H28 178 / 172, H32 186 / 174; T2500 H25 110 / 113, H26 110 / 113, H28 115 /
+//     113, H32 120 / 114; T1600 H28 77 / 79, H30 78 / 80, H32 80.6 / 80.1, H37 83 / 82.  Where the 16-row form is the choice anyway:
+//     T8192 H38 461 / 362, H42 477 / 435, H44 483 / 477; T1200 H38 75 / 68, H42 78.6 / 78.3, H43 79.4 / 80.5, H44 79 / 84.  With a K1
+//     CTA beside K2's: T8192 H32 403 against 363.
 //   Tensor-memory form with one CTA per SM and two K1 CTAs there (a K1 of 112 registers: see there), four on the other SMs:
 //     T1024 H75 108 / 101, H96 121 / 109, H123 136 / 127, H136 143 / 139, H148 149 / 152; T8192 H75 754 / 636, H96 834 / 686,
 //     H123 942 / 867, H136 998 / 969, H148 1,046 / 1,082.
@@ -206,7 +207,7 @@ Beside beside_plan(const KdaFwdArgs* a) {
     k2_sms = r.sms; r.k2_sm_ctas = 2;
   } else if (automatic && r.variant == 1 && chains * 6 <= r.sms) {
     k2_sms = chains * 4;
-  } else if (automatic && ((r.variant == 1 && (chains * 6 - r.sms) * nt >= 7500) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 96))) {
+  } else if (automatic && ((r.variant == 1 && (chains * 15 - 2LL * r.sms) * nt >= 18750) || (r.variant == 3 && chains * 7 <= 2LL * r.sms && nt >= 72))) {
     k2_sms = chains * 2; r.variant = 3; r.vsplit = 2;
   } else if (r.variant == 4 && chains * 11 > 6LL * r.sms && chains * 10 <= 7LL * r.sms && nt >= 256) {
     k2_sms = (chains + 1) / 2;

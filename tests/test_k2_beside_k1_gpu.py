@@ -70,7 +70,7 @@ def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
 # tensor-memory form with two CTAs per SM and with one; both sides of the lines between them, partial last chunks.  Decays
 # that leave much of the state, so that every step matters to the last bit.
 @pytest.mark.parametrize("B,T,H", [
-    (1, 1991, 19), (1, 1570, 24), (1, 2705, 32), (1, 2721, 32), (2, 1531, 19), (1, 1530, 42), (1, 1521, 43),
+    (1, 1991, 19), (1, 1570, 24), (1, 1616, 32), (1, 1630, 32), (1, 1157, 37), (2, 1531, 19), (1, 1530, 42), (1, 1521, 43),
     (1, 4085, 80), (1, 4085, 81), (1, 4067, 103), (1, 4090, 103), (1, 1500, 104), (1, 531, 137), (1, 531, 138)])
 def test_beside_equals_after_where_k2_has_sms_of_its_own(cuda_device, B, T, H):
     d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.3), cuda_device)
