@@ -240,7 +240,10 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
 
     float oq[8], o3[8];
     uint32_t aq[8];
-    __nv_bfloat16* const orow = p.o + b * p.o_s[0] + tok0 * p.o_s[1] + h * p.o_s[2];
+    // this thread's 16 bytes of a chunk's outputs: token 8 half + lane / 4, rows 32 quad + 8 (lane % 4)
+    __nv_bfloat16* o_at = p.o + b * p.o_s[0] + (tok0 + half * 8 + (lane >> 2)) * p.o_s[1] + h * p.o_s[2] + quad * 32 + (lane & 3) * 8;
+    const int64_t o_step = BT * p.o_s[1];
+    int left = Tlen - half * 8 - (lane >> 2);
 
     // o[tok][v] = scale * (qg h^T) + Aqk v_new of chunk nd, from the registers filled by its E2: a warp's 8 tokens
     // x 32 rows are transposed through its own 512 bytes, so that every thread stores 16 contiguous bytes of a
@@ -252,11 +255,9 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
       for (int j = 0; j < 8; ++j)
         *reinterpret_cast<__nv_bfloat16*>(buf + j * 64 + lane * 2) = __float2bfloat16(fmaf(p.scale, oq[j], o3[j]));
       __syncwarp();
-      const int row = lane >> 2, seg = lane & 3;
-      const int tok = nd * BT + half * 8 + row;
-      if (tok < Tlen)
-        *reinterpret_cast<uint4*>(orow + static_cast<int64_t>(tok) * p.o_s[1] + quad * 32 + seg * 8) =
-            *reinterpret_cast<const uint4*>(buf + row * 64 + seg * 16);
+      if (left > 0) *reinterpret_cast<uint4*>(o_at) = *reinterpret_cast<const uint4*>(buf + lane * 16);
+      o_at += o_step;
+      left -= BT;
     };
 
     for (int n = 0; n < NT && ok; ++n) {
