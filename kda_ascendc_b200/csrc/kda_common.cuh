@@ -217,13 +217,6 @@ __device__ __forceinline__ bool flag_wait_bounded(const int* flag, int epoch) {
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// At the start of a kernel that is launched ahead of the end of whatever runs before it in the stream, and lets the next
-// one start in the same way: nothing of global memory is touched before the wait.
-__device__ __forceinline__ void grid_dep_start() {
-  grid_dep_launch();
-  grid_dep_wait();
-}
-
 // fence between the generic and the async proxy for every state space (the plain form above covers
 // shared memory only): global memory written with plain stores and read by bulk copies, or the reverse
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }

@@ -108,7 +108,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, 1) kda_k2_kernel(const K2Params
   __syncthreads();
 
   const uint8_t* rec_bh = p.rec + rec_first * REC_BYTES;
-  grid_dep_launch();
 
   if (warp == CW) {
     // ------------------------------ producer -------------------------------

@@ -96,7 +96,6 @@ __global__ void __launch_bounds__((CW + 1) * 32, MINB) kda_k2m_kernel(const K2Pa
   __syncthreads();
 
   const uint8_t* rec_bh = p.rec + rec_first * REC_BYTES;
-  if (!ORD || p.long_len == 0) grid_dep_launch();
 
   if (warp == CW) {
     // ------------------------------ producer -------------------------------

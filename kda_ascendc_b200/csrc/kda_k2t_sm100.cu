@@ -102,7 +102,6 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = __shfl_sync(0xffffffffu, *slot, 0);
-  grid_dep_launch();
 
   auto give_up = [&]() {
     if (*sAbort == 0) { *sAbort = 1; atomicExch(p.status, ST_K2T_TIMEOUT); }

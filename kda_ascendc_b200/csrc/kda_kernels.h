@@ -114,9 +114,11 @@ constexpr int ONE_CTA_SMEM = 116 * 1024;
 inline int k2_smem(const K2Params& p, int need) { return p.one_per_sm && need < ONE_CTA_SMEM ? ONE_CTA_SMEM : need; }
 
 // One launch, with or without the programmatic stream serialization attribute.  K1 and the token recurrence are launched
-// with it: their CTAs take the places that the last kernel's leave, wait for its end and start at once.  Calls one after
-// the other, us, before and now: one-token recurrence B1 H32 5.3 / 4.6, B8 8.2 / 6.6, four tokens B16 19.3 / 17.6; B2 T1024 H4
-// forward 32.6 / 30.5.
+// with it behind whatever runs before them.  K2 and the recurrence do not let the next kernel start before their end: its
+// launch is under way by then all the same, and CTAs that only wait took room and cost more than their early start gave.  Calls
+// one after the other, us, ordinary launches / with the attribute / and with an early start: one-token recurrence B8 H32 8.2 /
+// 6.4 / 6.6, B64 43.7 / 42.3 / 43.9, four tokens B16 20.5 / 18.7 / 19.1; forward T16 H32 9.3 / 7.5 / 8.2, T100 H32 13.2 / 11.3 / 13.0, T64
+// H150 23.0 / 21.6 / 22.9, B2 T1024 H4 32.8 / 30.0 / 30.6.
 template <typename Kernel, typename Params>
 cudaError_t launch_dep(Kernel kernel, int grid, int block, int smem_bytes, cudaStream_t stream, int pdl, const Params& p) {
   cudaLaunchConfig_t cfg = {};

@@ -129,7 +129,10 @@ __global__ void __launch_bounds__(REC_WARPS * 32, 6) kda_recurrent_kernel(const 
   const int k0 = lane * 4;                             // first state column of this lane
   constexpr int SH = 4 - Log2<ROWS>::v;                // lanes that end up with one sum of a token: 1 << SH
 
-  grid_dep_start();
+  // Launched ahead of the end of whatever runs before it in the stream; nothing of global memory is touched before this.  It
+  // does not let the next kernel start in turn: one that starts with this one's last wave, or behind its loads, and not at its end
+  // takes places that this one's loads could use (in place of 42.3 us 43.9 and 44.5, B64 H32).
+  grid_dep_wait();
   float4 s[ROWS];
   constexpr int PIECE = (ROWS % 4 == 0) ? 4 : 2;   // floats per access along v in the K-first layout
   if (p.h0 != nullptr && p.k_first) {
@@ -265,7 +268,7 @@ __global__ void __launch_bounds__(128, 7) kda_recurrent_kfirst_kernel(const Recu
   const int v0 = slice * 32 + vq * 4;   // first state column of this thread
   const int k0 = kg * 8;                // first state row of this thread
 
-  grid_dep_start();
+  grid_dep_wait();
   float4 s[8];
   if (p.h0 != nullptr) {
     const float* h0 = p.h0 + (static_cast<size_t>(bh) * D + k0) * D + v0;
@@ -360,7 +363,7 @@ __global__ void __launch_bounds__(128, G_BF16 ? 7 : 6) kda_recurrent_kfirst_one_
   const int v0 = slice * 32 + vq * 4;   // first state column of this thread
   const int k0 = kg * 8;                // first state row of this thread
 
-  grid_dep_start();
+  grid_dep_wait();
   float4 s[8];
   if (p.h0 != nullptr) {
     const float* h0 = p.h0 + (static_cast<size_t>(bh) * D + k0) * D + v0;
