@@ -418,7 +418,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
   if (variant == 4) {
     // Tail wave.  The tensor-memory form holds two chains per SM at once; when the chains left over
     // after the full waves are at most half as many as SMs, they run faster in an mma.sync form
-    // (8-row for at most SMs/4 chains, 0.45 us per step; 16-row: two CTAs per chain, one per SM, 0.56 us
+    // (8-row for at most SMs/4 chains, 0.45 us per step; 16-row: two CTAs per chain, one per SM, 0.53 us
     // per step; against 0.84 for a lone tensor-memory CTA), launched behind the full waves, at every length that the
     // tensor-memory form is chosen for.  kda_fwd in us, no tail / 16-row / 8-row, 296 chains and so many more x chunks:
     // 9 x 4 45.5 / 43.4 / 41.3, 9 x 64 335 / 325 / 306; 37 x 4 47.3 / 45.0 / 45.2, 37 x 64 353 / 342 / 331; 38 x 4 47.9 /
@@ -437,7 +437,7 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     const long long mean_steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : 0;
     p.by_length = a->n_seqs > 1 && a->n_seqs <= kda::MAX_SORTED_SEQS && bh > sms && bh <= 4LL * sms * mean_steps;
     // A sequence much longer than the others: its chains go on alone when the rest is done, at 1.3 us per step while their SM
-    // has a second CTA and 0.85 without, against 0.56 in the 16-row form.  So the longest sequences, on at most half of the
+    // has a second CTA and 0.85 without, against 0.53 in the 16-row form.  So the longest sequences, on at most half of the
     // SMs, run there, in front of and beside the tensor-memory launch (which starts when K1 has ended, about 2 us later
     // than without), if they are long: more steps than 0.9 x the chunks of all chains per SM, which take 0.67 us each in pairs,
     // and than 1.5 x the mean.  The lengths are on the device: either kernel leaves out what the other does.  Whole forward, us,
