@@ -118,14 +118,14 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // FORM_ANY for the same call, with u still worked out here: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs
 // prepared by the caller (B8 T2037 H32 with 8 q/k heads) 294 -> 274.
 enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
-//
+
 // Beside K2 the work is handed out item by item, and not every SM does the same share of it: on k2_sms of the SMs (spread
 // evenly) only the first k2_sm_ctas CTAs of this kernel stay, and K2's CTAs, which find no room on the others, are placed
 // there.  The first ones, by the warp slots they run in, so that the registers and the shared memory that become free lie together:
 // with two other CTAs staying (as they came) a tensor-memory K2 found no room on some SMs until K1 ended (T8192 H96
 // 720 -> 1,200 us).  Those that leave wait until the whole grid has started, so that no later CTA takes their place,
-// and until somebody stays.  Where that takes longer than 20 us they stay too: all this decides about speed only, whoever
-// stays takes items until none is left.
+// and stay too where that takes longer than 20 us, or where fewer than half of those that should stay do so (another stream's
+// kernels hold the first warp slots): all this decides about speed only, whoever stays takes items until none is left.
 __device__ __forceinline__ bool k1_stays(const K1Params& p) {
   uint32_t sm, slot;
   asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
@@ -140,7 +140,11 @@ __device__ __forceinline__ bool k1_stays(const K1Params& p) {
   do {
     int n;
     asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(n) : "l"(arrived) : "memory");
-    if ((n & (STAYS - 1)) == static_cast<int>(gridDim.x) && n >= STAYS) return false;
+    if ((n & (STAYS - 1)) == static_cast<int>(gridDim.x)) {
+      const int per_sm = static_cast<int>(gridDim.x) / p.n_sms;
+      const int wanted = (p.n_sms - p.k2_sms) * per_sm + p.k2_sms * min(p.k2_sm_ctas, per_sm);
+      return n / STAYS * 2 < wanted;
+    }
   } while (globaltimer_ns() - t0 < 20000ull);
   return true;
 }

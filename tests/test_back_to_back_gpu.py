@@ -68,3 +68,22 @@ def test_decode_steps_behind_a_forward(cuda_device, B, T, k_first):
     for _ in range(5):
         got = walk(False)
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("B,T,H", [(2, 2400, 8), (1, 1991, 19), (1, 1700, 40), (1, 600, 96), (1, 4085, 88)])
+def test_two_streams_at_once(cuda_device, B, T, H):
+    """Forwards whose K2 runs beside K1 on two streams: each finds the other's CTAs on the SMs that it counted on."""
+    runs = []
+    for seed in range(2):
+        d = _inputs(B, T + 16 * seed, H, cuda_device)
+        plan = K.ForwardPlan(d["q"], d["k"], d["v"], d["g"], d["beta"], scale=d["scale"], initial_state=d["initial_state"],
+                             lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"])
+        plan.run()
+        torch.cuda.synchronize()
+        runs.append((plan, torch.cuda.Stream(), plan.o.clone(), plan.final_state.clone()))
+    for _ in range(8):
+        for plan, stream, _, _ in runs:
+            plan.run(stream.cuda_stream)
+    torch.cuda.synchronize()
+    for plan, _, o, ht in runs:
+        assert torch.equal(plan.o, o) and torch.equal(plan.final_state, ht)
