@@ -55,6 +55,13 @@ bool row_aligned(const void* p, const int64_t s[3], int elem_bytes) {
   return true;
 }
 
+// The fp32 parameters that are read one float at a time: views of larger buffers, so no more than their own alignment is asked for.
+bool params_aligned(const KdaFwdArgs* a, bool gate) {
+  uintptr_t at = reinterpret_cast<uintptr_t>(a->beta);
+  if (gate) at |= reinterpret_cast<uintptr_t>(a->A_log) | reinterpret_cast<uintptr_t>(a->dt_bias);
+  return at % sizeof(float) == 0;
+}
+
 int check_k1(const KdaFwdArgs* a) {
   if (int rc = check_common(a)) return rc;
   if (!a->q || !a->k || !a->v || !a->g || !a->beta)
@@ -68,6 +75,10 @@ int check_k1(const KdaFwdArgs* a) {
   if (!row_aligned(a->q, a->q_stride, 2) || !row_aligned(a->k, a->k_stride, 2) || !row_aligned(a->v, a->v_stride, 2) ||
       !row_aligned(a->g, a->g_stride, a->g_dtype == KDA_G_BF16 ? 2 : 4))
     return fail(KDA_ERR_INVALID_ARG, "kda: q/k/v/g rows must start on 16-byte boundaries%s", "");
+  if (!params_aligned(a, (a->flags & KDA_FLAG_GATE_IN_KERNEL) != 0))
+    return fail(KDA_ERR_INVALID_ARG, "kda: beta, A_log and dt_bias must be 4-byte aligned%s", "");
+  if (reinterpret_cast<uintptr_t>(a->g_out) % 8 != 0 || reinterpret_cast<uintptr_t>(a->ainv_out) % 4 != 0)
+    return fail(KDA_ERR_INVALID_ARG, "kda: g_out must be 8-byte and ainv_out 4-byte aligned%s", "");
   // an expanded view (stride 0 on a dimension larger than 1) cannot be described to the TMA unit
   const int hq = a->Hq > 0 ? a->Hq : a->H;
   const struct { const int64_t* s; int heads; const char* name; } views[4] = {
@@ -569,6 +580,8 @@ int kda_recurrent_fwd(const KdaFwdArgs* a, void* stream) {
   if (!row_aligned(a->q, a->q_stride, 2) || !row_aligned(a->k, a->k_stride, 2) || !row_aligned(a->v, a->v_stride, 2) ||
       !row_aligned(a->g, a->g_stride, a->g_dtype == KDA_G_BF16 ? 2 : 4) || !row_aligned(a->o, a->o_stride, 2))
     return fail(KDA_ERR_INVALID_ARG, "kda: q/k/v/g/o rows must start on 16-byte boundaries%s", "");
+  if (!params_aligned(a, true))
+    return fail(KDA_ERR_INVALID_ARG, "kda: beta, A_log and dt_bias must be 4-byte aligned%s", "");
   for (const void* ptr : {static_cast<const void*>(a->h0), static_cast<const void*>(a->ht), static_cast<const void*>(a->dt_bias)})
     if (ptr != nullptr && reinterpret_cast<uintptr_t>(ptr) % 16 != 0)
       return fail(KDA_ERR_INVALID_ARG, "kda: h0, ht and dt_bias must be 16-byte aligned%s", "");

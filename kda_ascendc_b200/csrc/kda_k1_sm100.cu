@@ -113,9 +113,9 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
 // start before K1 ends.  kda_fwd, with 128 registers and with 112: T8192 H96 1,223 and 849 us, T2048 H80 303 and 201;
 // beside the 8-row form both fit (T32768 H16 988 and 990, B2 T4096 H8 135.1 and 135.6).
-// FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel; FORM_NONE: all
-// three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags decide.  Against
-// FORM_ANY for the same call, with u still worked out here: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs
+// FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel, dt_bias at an 8-byte
+// boundary; FORM_NONE: all three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags
+// decide.  Against FORM_ANY for the same call, with u still worked out here: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs
 // prepared by the caller (B8 T2037 H32 with 8 q/k heads) 294 -> 274.
 enum K1Form { FORM_ANY, FORM_ALL, FORM_NONE };
 
@@ -215,8 +215,13 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     q.a_log = use_gate ? ldg_pinned(p.A_log + w.h) : 0.f;
     q.bias0 = q.bias1 = 0.f;
     if (use_gate && p.dt_bias != nullptr) {
-      const float2 bb = ldg_pinned2(p.dt_bias + w.h * D + c0);
-      q.bias0 = bb.x; q.bias1 = bb.y;
+      if (FORM == FORM_ALL) {   // at an 8-byte boundary: see the choice of the instance
+        const float2 bb = ldg_pinned2(p.dt_bias + w.h * D + c0);
+        q.bias0 = bb.x; q.bias1 = bb.y;
+      } else {
+        q.bias0 = ldg_pinned(p.dt_bias + w.h * D + c0);
+        q.bias1 = ldg_pinned(p.dt_bias + w.h * D + c0 + 1);
+      }
     }
     q.beta = 0.f;   // held by threads 32..47 (warp 1), one token each
     if (tid >= 32 && tid < 48 && tid - 32 < w.nvalid)
@@ -781,10 +786,13 @@ template <bool G_BF16, bool BESIDE>
 static cudaError_t launch_k1_b(const K1Params& p, bool fast_exp, cudaStream_t stream) {
   const uint32_t in_kernel = p.flags & 7u;
   const bool debug = p.g_out != nullptr || p.ainv_out != nullptr;
+  // dt_bias may be a view that starts at any float of a larger buffer.  FORM_ALL reads it two floats at a time (one at a time
+  // costs it 0.2 %: T8192 H96 719.7 -> 721.2 us, T100 H32 11.16 -> 11.22), the others by single floats.
+  const bool all = in_kernel == 7u && !debug && reinterpret_cast<uintptr_t>(p.dt_bias) % sizeof(float2) == 0;
   if (fast_exp)
-    return in_kernel == 7u && !debug ? launch_k1_t<G_BF16, true, BESIDE, FORM_ALL>(p, stream)
-                                     : launch_k1_t<G_BF16, true, BESIDE, FORM_ANY>(p, stream);
-  if (in_kernel == 7u && !debug) return launch_k1_t<G_BF16, false, BESIDE, FORM_ALL>(p, stream);
+    return all ? launch_k1_t<G_BF16, true, BESIDE, FORM_ALL>(p, stream)
+               : launch_k1_t<G_BF16, true, BESIDE, FORM_ANY>(p, stream);
+  if (all) return launch_k1_t<G_BF16, false, BESIDE, FORM_ALL>(p, stream);
   if (in_kernel == 0u && !debug) return launch_k1_t<G_BF16, false, BESIDE, FORM_NONE>(p, stream);
   return launch_k1_t<G_BF16, false, BESIDE, FORM_ANY>(p, stream);
 }

@@ -142,3 +142,25 @@ def test_forms_that_cannot_wait_for_their_entry_state_are_refused(cuda_device, H
     torch.cuda.synchronize()
     assert rc == UNSUPPORTED and "wait" in _lib.last_error()
     assert c.o.isnan().all()
+
+
+# K1 alone in front of K2 and beside it, the general centring (its other instances), packed sequences
+@pytest.mark.parametrize("B,T,H,lower_bound,cu", [(1, 33, 2, -5.0, None), (2, 2400, 8, -5.0, None), (1, 100, 3, -8.0, None),
+                                                  (1, 50, 2, -5.0, [0, 17, 50])])
+def test_gate_parameters_may_be_views_at_any_float(cuda_device, B, T, H, lower_bound, cu):
+    d = _inputs(cuda_device, B, T, H, seed=T)
+    h0 = None if cu else d["h0"]
+
+    def run(beta, A_log, dt_bias):
+        return K.kda_bt16_fwd(d["q"], d["k"], d["v"], d["g"], beta, initial_state=h0, output_final_state=True,
+                              use_qk_l2norm_in_kernel=True, use_gate_in_kernel=True, use_beta_sigmoid_in_kernel=True,
+                              lower_bound=lower_bound, A_log=A_log, dt_bias=dt_bias, cu_seqlens=cu)
+
+    want = run(d["beta"], d["A_log"], d["dt_bias"])
+    for shift in (1, 2, 3):
+        views = []
+        for n in ("beta", "A_log", "dt_bias"):
+            flat = torch.full((d[n].numel() + shift,), float("nan"), device=cuda_device)
+            flat[shift:] = d[n].flatten()
+            views.append(flat[shift:].view(d[n].shape))
+        assert _same(run(*views), want)

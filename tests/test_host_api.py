@@ -87,6 +87,28 @@ def test_c_abi_rejects_bad_arguments_without_a_gpu():
     assert lib.kda_fwd(None, None) == -1
 
 
+def test_misaligned_parameters_are_refused_before_any_launch():
+    lib = _lib.load()
+
+    def refused(fn, words, **ptrs):
+        a = _lib.KdaFwdArgs()
+        a.B, a.T, a.H, a.flags, a.lower_bound = 1, 16, 1, 7, -5.0
+        for name in ("q", "k", "v", "g", "beta", "A_log", "dt_bias", "h0", "o", "ht", "workspace"):
+            setattr(a, name, 1 << 20)
+        for name in ("q_stride", "k_stride", "v_stride", "g_stride", "o_stride"):
+            setattr(a, name, (ctypes.c_int64 * 3)(2048, 128, 128))
+        for name, at in ptrs.items():
+            setattr(a, name, at)
+        return fn(ctypes.byref(a), None) == -1 and words in _lib.last_error()
+
+    for fn in (lib.kda_fwd, lib.kda_fwd_k1, lib.kda_recurrent_fwd):
+        for name in ("beta", "A_log", "dt_bias"):
+            assert refused(fn, "4-byte", **{name: (1 << 20) + 2})
+    for fn in (lib.kda_fwd, lib.kda_fwd_k1):
+        assert refused(fn, "g_out", g_out=(1 << 20) + 4) and refused(fn, "ainv_out", ainv_out=(1 << 20) + 2)
+    assert refused(lib.kda_recurrent_fwd, "16-byte", dt_bias=(1 << 20) + 4)
+
+
 def test_reference_validation_messages():
     q, k, v, g, beta = _mk()
     with pytest.raises(ValueError, match="q must be contiguous"):
