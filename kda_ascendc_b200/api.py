@@ -33,6 +33,8 @@ HEAD_DIM = 128
 REC_BYTES = 26112
 WS_HEADER_BYTES = 256
 
+# Scratch that outlives a call: none.  The header of a workspace holds the work tickets and counters of one forward, so calls
+# on several streams, from several threads or out of captured graphs must not meet in one.
 _WORKSPACE_CACHE: dict[tuple, torch.Tensor] = {}
 _LAST_PROFILE: dict[str, object] = {}
 RECURRENT_MAX_TOKENS = 4   # kda_recurrent_fwd hands longer calls to the chunk kernels
@@ -219,16 +221,8 @@ def k2_choice(B: int, T: int, H: int, *, state_only: bool = False, n_seqs: int =
     return K2_FORMS[var.value], vs.value
 
 
-def _get_workspace(device, B, T, H, reuse: bool) -> torch.Tensor:
-    nbytes = workspace_bytes(B, T, H)
-    if reuse:
-        key = (device, B, T, H)
-        ws = _WORKSPACE_CACHE.get(key)
-        if ws is None:
-            ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-            _WORKSPACE_CACHE[key] = ws
-        return ws
-    return torch.empty(nbytes, dtype=torch.uint8, device=device)
+def _get_workspace(device, B, T, H) -> torch.Tensor:
+    return torch.empty(workspace_bytes(B, T, H), dtype=torch.uint8, device=device)
 
 
 def _varlen_tables(cu_seqlens, T: int, H: int, device):
@@ -270,8 +264,7 @@ def _flags(use_gate, use_l2, use_beta_sigmoid) -> int:
 
 def _forward(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
              use_gate_in_kernel, use_beta_sigmoid_in_kernel, lower_bound, A_log, dt_bias, state_v_first,
-             return_intermediates=False, reuse_workspace=False, k2_vsplit=0, k2_variant=0, workspace=None,
-             cu_seqlens=None):
+             return_intermediates=False, k2_vsplit=0, k2_variant=0, workspace=None, cu_seqlens=None):
     """Allocate, launch K1 + K2 on the current stream, return (o, ht[, intermediates])."""
     lib = _lib.load()
     B, T, _, K = q.shape
@@ -284,7 +277,7 @@ def _forward(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_
         tables = _varlen_tables(cu_seqlens, T, H, dev)
         n_states, ws_tokens = tables[0], BT * tables[1]
     ht = torch.empty((n_states, H, HEAD_DIM, HEAD_DIM), dtype=torch.float32, device=dev) if output_final_state else None
-    ws = workspace if workspace is not None else _get_workspace(dev, B, ws_tokens, H, reuse_workspace)
+    ws = workspace if workspace is not None else _get_workspace(dev, B, ws_tokens, H)
     g_out = ainv = None
     if return_intermediates:
         g_out = torch.empty((B, T, H, HEAD_DIM), dtype=torch.float32, device=dev)
@@ -369,7 +362,7 @@ def kda_recurrent_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_f
     # The line was drawn for an earlier token kernel; with this one calls of five and six tokens would be faster
     # token by token as well (K-first B1 T6: 8.0 / 7.8).
     chunked = T > RECURRENT_MAX_TOKENS
-    ws = _get_workspace(dev, B, T, H, False) if chunked else None   # calls on several streams share no scratch
+    ws = _get_workspace(dev, B, T, H) if chunked else None   # calls on several streams share no scratch
     args = make_args(q, k, v, g, beta, scale=scale, lower_bound=lower_bound, A_log=A_log, dt_bias=dt_bias,
                      h0=initial_state, o=o, ht=ht, workspace=ws,
                      flags=_flags(True, True, True) | (0 if state_v_first else _lib.FLAG_STATE_K_FIRST))
@@ -479,7 +472,8 @@ def kda_bt16_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_final_
 
     ``use_fused_kernel`` is accepted for signature compatibility: the reference's
     single-kernel variant computes the same function, and this build has one device path.
-    ``reuse_workspace`` caches only the internal scratch per shape (never the outputs).
+    So is ``reuse_workspace``: the scratch of every call comes from PyTorch's caching allocator, which
+    gives a stream's next call the block of its last one, and nothing is shared between streams.
 
     ``cu_seqlens`` (not in the reference, which lists variable-length input as future work,
     ``README.md:509``; the convention is that of ``chunk_kda`` in flash-linear-attention): packed
@@ -487,13 +481,12 @@ def kda_bt16_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_final_
     chunked from its own first token, ``initial_state`` / the returned state are
     ``[n_seqs, H, 128, 128]``.
     """
-    if not reuse_workspace:
-        res = _lib.host().chunk(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
-                                use_gate_in_kernel, use_beta_sigmoid_in_kernel, safe_gate, lower_bound, A_log, dt_bias,
-                                state_v_first, cu_seqlens, False)
-        if res is not None:
-            _count_chunk()
-            return res
+    res = _lib.host().chunk(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
+                            use_gate_in_kernel, use_beta_sigmoid_in_kernel, safe_gate, lower_bound, A_log, dt_bias,
+                            state_v_first, cu_seqlens, False)
+    if res is not None:
+        _count_chunk()
+        return res
     n_states = None
     if cu_seqlens is not None:
         if q.ndim == 4 and q.shape[0] != 1:
@@ -506,7 +499,7 @@ def kda_bt16_fwd(q, k, v, g, beta, scale=None, initial_state=None, output_final_
         scale = q.shape[-1] ** -0.5
     return _forward(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel,
                     use_gate_in_kernel, use_beta_sigmoid_in_kernel, lower_bound, A_log, dt_bias, state_v_first,
-                    reuse_workspace=reuse_workspace, cu_seqlens=cu_seqlens)
+                    cu_seqlens=cu_seqlens)
 
 
 def kda_bt16_debug(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False,

@@ -1,9 +1,12 @@
 """Calls one after the other without a wait on the host: each starts ahead of the end of the one before and must not read
 what that one still writes."""
+import threading
+
 import pytest
 import torch
 
 import kda_ascendc_b200 as K
+from kda_ascendc_b200 import api
 from oracle import kda_oracle as O
 from tests.conftest import to_device
 
@@ -87,3 +90,35 @@ def test_two_streams_at_once(cuda_device, B, T, H):
     torch.cuda.synchronize()
     for plan, _, o, ht in runs:
         assert torch.equal(plan.o, o) and torch.equal(plan.final_state, ht)
+
+
+def test_reused_workspaces_are_not_shared_by_streams(cuda_device):
+    """reuse_workspace=True with one shape on two streams, from two threads: K2 beside K1 and after it."""
+    for B, T, H in ((2, 2400, 8), (1, 100, 32), (1, 1616, 32)):
+        d = [_inputs(B, T, H, cuda_device) for _ in range(2)]
+        d[1]["v"] = d[1]["v"] * -0.5
+
+        def fwd(x):
+            return K.kda_bt16_fwd(x["q"], x["k"], x["v"], x["g"], x["beta"], scale=x["scale"], initial_state=x["initial_state"],
+                                  lower_bound=x["lower_bound"], A_log=x["A_log"], dt_bias=x["dt_bias"], reuse_workspace=True, **FLAGS)
+
+        want = [fwd(x) for x in d]
+        assert not api._WORKSPACE_CACHE
+        torch.cuda.synchronize()
+        got, streams = [[], []], [torch.cuda.Stream() for _ in d]
+
+        def walk(i):
+            with torch.cuda.stream(streams[i]):
+                for _ in range(8):
+                    got[i].append(fwd(d[i]))
+
+        threads = [threading.Thread(target=walk, args=(i,)) for i in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        for i in range(2):
+            assert len(got[i]) == 8
+            for o, ht in got[i]:
+                assert torch.equal(o, want[i][0]) and torch.equal(ht, want[i][1])
