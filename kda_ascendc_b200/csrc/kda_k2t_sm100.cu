@@ -383,6 +383,10 @@ __global__ void __launch_bounds__(KT_THREADS, 2) kda_k2t_kernel(const __grid_con
     const int issued = *sIssued;
     for (int n = max(0, issued - KT_STAGES); n < issued; ++n)
       mbar_wait_bounded(full(n % KT_STAGES), (n / KT_STAGES) & 1, nullptr);
+  } else if (*sAbort == 0 && tid < KT_STAGES && tid < NT) {
+    // the last stages' way back: an arrival that nobody waits for could still be under way when the shared memory goes
+    // (left out behind a comparison in the issuing loop instead: K2 alone T8192 H96 430.5 -> 432.4 us)
+    mbar_wait_bounded(empty(tid), ((NT - 1 - tid) / KT_STAGES) & 1, nullptr);
   }
   __syncthreads();
   if (warp == KT_EPI_WARPS + 1)

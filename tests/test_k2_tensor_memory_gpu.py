@@ -137,3 +137,17 @@ def test_any_lengths_longest_first(n, lo, hi, H):
     o3, ht3 = _run(inp, 3, cu=cu)
     assert (o - o3).abs().max().item() <= 2.5e-4       # one bf16 step of |o| <= 0.06, as above
     assert (ht - ht3).abs().max().item() <= 2e-5
+
+
+def test_any_number_of_chunks_around_the_stages():
+    """One chunk to more than twice the four stages: every length gives the bits of the longest one's first chunks."""
+    inp = O.make_inputs(2, 16 * 9 - 3, 3, seed0=29, regime="carry", h0_std=0.3)
+    want, _ = _run(inp, 4)
+    for n in range(1, 9):
+        part = {k: v[:, :16 * n].contiguous() if k in ("q", "k", "v", "g", "beta") else v for k, v in inp.items()}
+        for _ in range(2):
+            o, ht = _run(part, 4)
+            assert torch.equal(o, want[:, :16 * n])
+        rest = {k: v[:, 16 * n:].contiguous() if k in ("q", "k", "v", "g", "beta") else v for k, v in inp.items()}
+        o, _ = _run(dict(rest, initial_state=ht.cpu()), 4)
+        assert torch.equal(o, want[:, 16 * n:])
