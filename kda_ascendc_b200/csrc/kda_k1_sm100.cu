@@ -308,7 +308,8 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     }
   };
 
-  for (int it = 0; id < n_items; ++it, id = id_next, id_next = BESIDE ? sFlag[1] : id_next + static_cast<int>(gridDim.x)) {
+  int it = 0;
+  for (; id < n_items; ++it, id = id_next, id_next = BESIDE ? sFlag[1] : id_next + static_cast<int>(gridDim.x)) {
     const int b = cur.b, h = cur.h, t0 = cur.t0, nvalid = cur.nvalid;
     uint8_t* rec = p.rec + cur.rec_idx * REC_BYTES;
     const bool has_next = id_next < n_items;
@@ -351,6 +352,7 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
         atomicExch(p.status, ST_K1_LOAD_TIMEOUT);
         p.status[HDR_K1_STATUS] = ST_K1_LOAD_TIMEOUT;
         mbar_wait_bounded(mbar, it & 1, nullptr);
+        mbar_wait_bounded(mbar_v, (it + 1) & 1, nullptr);   // of the item before
         bulk_wait_read_all();
       }
       __syncthreads();
@@ -618,7 +620,11 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     }
     // packed sequences: v behind the last token of a sequence, as for the other inputs above
     if (!BESIDE && p.chunk_table != nullptr && nvalid < BT) {
-      if (!mbar_wait_bounded(mbar_v, it & 1, sFlag)) *sFlag = 1;
+      if (!mbar_wait_bounded(mbar_v, it & 1, sFlag)) {   // reported here: for thread 0 it may yet come
+        *sFlag = 1;
+        atomicExch(p.status, ST_K1_LOAD_TIMEOUT);
+        p.status[HDR_K1_STATUS] = ST_K1_LOAD_TIMEOUT;
+      }
 #pragma unroll 1
       for (int i = nvalid * 16 + tid; *sFlag == 0 && i < BT * 16; i += 128)   // 16-byte units
         *reinterpret_cast<uint4*>(smem + S_V + (i & 1) * REC_V_HALF + (i >> 1) * 16) = make_uint4(0, 0, 0, 0);
@@ -689,8 +695,12 @@ __global__ void __maxnreg__(BESIDE ? 112 : 128) kda_k1_kernel(const __grid_const
     par = par_next;
   }
   if (tid == 0) {
-    if (*sFlag == 0) drain_stores();
-    else bulk_wait_read_all();   // v of the last item did not come: no window is reported
+    if (*sFlag == 0) {
+      drain_stores();
+    } else {   // v of the last item did not come: no window is reported
+      mbar_wait_bounded(mbar_v, (it + 1) & 1, nullptr);
+      bulk_wait_read_all();
+    }
   }
 }
 
