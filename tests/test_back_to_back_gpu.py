@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import kda_ascendc_b200 as K
-from kda_ascendc_b200 import api
+from kda_ascendc_b200 import _lib, api
 from oracle import kda_oracle as O
 from tests.conftest import to_device
 
@@ -82,6 +82,8 @@ def test_two_streams_at_once(cuda_device, B, T, H):
         plan = K.ForwardPlan(d["q"], d["k"], d["v"], d["g"], d["beta"], scale=d["scale"], initial_state=d["initial_state"],
                              lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"])
         plan.run()
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:   # clear, K1 and K2: beside
+            assert _lib.load().kda_last_launch_count() == 3
         torch.cuda.synchronize()
         runs.append((plan, torch.cuda.Stream(), plan.o.clone(), plan.final_state.clone()))
     for _ in range(8):
@@ -122,3 +124,96 @@ def test_reused_workspaces_are_not_shared_by_streams(cuda_device):
             assert len(got[i]) == 8
             for o, ht in got[i]:
                 assert torch.equal(o, want[i][0]) and torch.equal(ht, want[i][1])
+
+
+# some sequences long enough for the 16-row launch in front of the tensor-memory one, few of each, and none
+@pytest.mark.parametrize("H,chunks", [(16, [300] + [40] * 9), (8, [20] * 12 + [400, 380, 360, 340, 320, 17]), (16, [60] * 11)])
+def test_packed_calls_back_to_back_and_on_two_streams(cuda_device, H, chunks):
+    cu, n = [0], len(chunks)
+    for i, c in enumerate(chunks):
+        cu.append(cu[-1] + 16 * c - (i * 5) % 16)
+    d = _inputs(1, cu[-1], H, cuda_device)
+    gen = torch.Generator(cuda_device).manual_seed(3)
+    h0 = torch.randn(n, H, 128, 128, device=cuda_device, generator=gen) * 0.3
+    kw = dict(scale=d["scale"], lower_bound=d["lower_bound"], A_log=d["A_log"], dt_bias=d["dt_bias"], **FLAGS)
+
+    def fwd(v, h):
+        return K.kda_bt16_fwd(d["q"], d["k"], v, d["g"], d["beta"], initial_state=h, cu_seqlens=cu, **kw)
+
+    fwd(d["v"], h0)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:   # K1, 16-row, tensor-memory
+        assert _lib.load().kda_last_launch_count() == 3
+
+    def walk(sign, wait):   # every call's initial states are the final states of the one before, its values made right before it
+        h, os = h0, []
+        for i in range(4):
+            o, h = fwd(d["v"] * (sign * (i + 1)), h)
+            if wait:
+                torch.cuda.synchronize()
+            os.append(o)
+        return os, h
+
+    want = [walk(sign, True) for sign in (1.0, -0.5)]
+    streams = [torch.cuda.Stream() for _ in want]
+    torch.cuda.synchronize()
+    got = [walk(1.0, False)]
+    for stream, sign in zip(streams, (1.0, -0.5)):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            got.append(walk(sign, False))
+    torch.cuda.synchronize()
+    for g, w in zip(got, (want[0], *want)):
+        assert all(torch.equal(a, b) for a, b in zip(g[0], w[0])) and torch.equal(g[1], w[1])
+
+
+# K1 after K2's set-up only, beside K2 in either register form and in tensor memory
+@pytest.mark.parametrize("B,T,H", [(1, 100, 32), (2, 2400, 8), (1, 1630, 32), (1, 600, 96)])
+@pytest.mark.parametrize("front", ["memset", "copy", "event", "join"])
+def test_captured_forward_and_decode_steps_behind_any_node(cuda_device, B, T, H, front):
+    """A graph in which the node in front of the forward is a memset, a copy, an event of another stream or a join of two
+    streams, and token steps on the forward's final state come behind it; replayed on changing values."""
+    d = _inputs(B, T + 2, H, cuda_device)
+    x = [t.clone() for t in _piece(d, 0, T)]
+    src = x[2].clone()
+    toks = [_piece(d, T + i, T + i + 1) for i in range(2)]
+    plan = K.ForwardPlan(*x, scale=d["scale"], initial_state=d["initial_state"], lower_bound=d["lower_bound"], A_log=d["A_log"],
+                         dt_bias=d["dt_bias"])
+    steps = [K.RecurrentPlan(*t, plan.final_state, scale=d["scale"], lower_bound=d["lower_bound"], A_log=d["A_log"],
+                             dt_bias=d["dt_bias"]) for t in toks]
+    v, outs = x[2], [torch.empty_like(steps[0].o) for _ in steps]
+
+    def body(main, other):
+        if front in ("memset", "copy"):
+            v.zero_() if front == "memset" else v.copy_(src)
+        else:
+            if other is not None:
+                other.wait_stream(main)
+            with torch.cuda.stream(main if other is None else other):
+                v.copy_(src)
+                v.mul_(-0.5)
+            y = src * 2 if front == "join" else None   # a kernel on this stream too
+            if other is not None:
+                main.wait_stream(other)
+            if y is not None:
+                v.add_(y)
+        plan.run()
+        for s, o in zip(steps, outs):
+            s.step()
+            o.copy_(s.o)
+
+    body(torch.cuda.current_stream(), None)
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        body(torch.cuda.current_stream(), torch.cuda.Stream())
+    for i in range(3):
+        src.mul_(-0.75)
+        torch.cuda.synchronize()
+        v.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        got = [t.clone() for t in (plan.o, plan.final_state, *outs)]
+        body(torch.cuda.current_stream(), None)
+        assert all(t.isfinite().all() for t in got)
+        assert all(torch.equal(a, b) for a, b in zip(got, (plan.o, plan.final_state, *outs)))
+    del graph

@@ -38,22 +38,32 @@ def _after(d, B, T, H, dev, **kw):
     return o, ht
 
 
-def _whole(d, B, T, H, dev, **kw):
+def _whole(d, B, T, H, dev, launches=None, **kw):
     o, ht, ws = _buffers(B, T, H, dev)
     a = _args(d, o, ht, ws, **kw)
     api._check(_lib.load().kda_fwd(ctypes.byref(a), api._stream_handle()))
+    if launches is not None and _sms() == 148:   # the lines between the forms are in SMs
+        assert _lib.load().kda_last_launch_count() == launches
     assert api.check_device_status(ws) == 0
     return o, ht
 
 
-# 8-row form (chains x 8 <= SMs) and tensor-memory form (up to three quarters of the SMs), on both sides of the
+def _sms():
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+AFTER, BESIDE = 2, 3   # launches of a forward: K1 and K2, and beside K1 the kernel that clears the header
+
+
+# 8-row form (chains x 8 <= SMs) and tensor-memory form (up to 13/14 of the SMs), on both sides of the
 # rule's line of 16 items per SM and of its line in chains; whole and partial last windows and chunks
-@pytest.mark.parametrize("B,T,H,lower_bound,prepared", [
-    (1, 4736, 8, -5.0, False), (1, 4720, 8, -5.0, False), (2, 2353, 8, -5.0, False), (1, 40001, 1, -5.0, False),
-    (3, 9000, 6, -5.0, False), (2, 2400, 8, -8.0, False), (2, 2400, 8, -5.0, True), (1, 16 * 121 + 5, 18, -5.0, False),
-    (1, 531, 75, -5.0, False), (1, 1024, 96, -5.0, False), (3, 1003, 37, -5.0, False), (1, 530, 112, -5.0, False),
-    (1, 20, 96, -5.0, False)])
-def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
+@pytest.mark.parametrize("B,T,H,lower_bound,prepared,launches", [
+    (1, 4736, 8, -5.0, False, BESIDE), (1, 4720, 8, -5.0, False, AFTER), (2, 2353, 8, -5.0, False, BESIDE),
+    (1, 40001, 1, -5.0, False, BESIDE), (3, 9000, 6, -5.0, False, BESIDE), (2, 2400, 8, -8.0, False, BESIDE),
+    (2, 2400, 8, -5.0, True, BESIDE), (1, 16 * 121 + 5, 18, -5.0, False, AFTER), (1, 531, 75, -5.0, False, BESIDE),
+    (1, 1024, 96, -5.0, False, BESIDE), (3, 1003, 37, -5.0, False, BESIDE), (1, 530, 112, -5.0, False, BESIDE),
+    (1, 20, 96, -5.0, False, AFTER)])
+def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared, launches):
     d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.05), cuda_device)
     d["lower_bound"] = lower_bound
     if prepared:   # what a caller that normalises and sums the gate itself hands over
@@ -62,23 +72,36 @@ def test_beside_equals_after(cuda_device, B, T, H, lower_bound, prepared):
         d["beta"] = d["beta"].sigmoid()
     ref = _after(d, B, T, H, cuda_device, prepared=prepared)
     for _ in range(3):
-        got = _whole(d, B, T, H, cuda_device, prepared=prepared)
+        got = _whole(d, B, T, H, cuda_device, launches, prepared=prepared)
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
 
 
 # K2 on SMs of its own: the 8-row form with four consumer warps, the 16-row form in place of the 8-row one and as chosen, the
 # tensor-memory form with two CTAs per SM and with one; both sides of the lines between them, partial last chunks.  Decays
 # that leave much of the state, so that every step matters to the last bit.
-@pytest.mark.parametrize("B,T,H", [
-    (1, 1991, 19), (1, 1570, 24), (1, 1616, 32), (1, 1630, 32), (1, 1157, 37), (2, 1531, 19), (1, 1530, 42), (1, 1521, 43),
-    (1, 4085, 80), (1, 4085, 81), (1, 4067, 103), (1, 4090, 103), (1, 1500, 104), (1, 531, 137), (1, 531, 138)])
-def test_beside_equals_after_where_k2_has_sms_of_its_own(cuda_device, B, T, H):
+@pytest.mark.parametrize("B,T,H,launches", [
+    (1, 1991, 19, BESIDE), (1, 1570, 24, BESIDE), (1, 1616, 32, AFTER), (1, 1630, 32, BESIDE), (1, 1157, 37, BESIDE),
+    (2, 1531, 19, BESIDE), (1, 1530, 42, BESIDE), (1, 1521, 43, AFTER), (1, 4085, 80, BESIDE), (1, 4085, 81, BESIDE),
+    (1, 4067, 103, BESIDE), (1, 4090, 103, BESIDE), (1, 1500, 104, BESIDE), (1, 531, 137, BESIDE), (1, 531, 138, AFTER)])
+def test_beside_equals_after_where_k2_has_sms_of_its_own(cuda_device, B, T, H, launches):
     d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.3), cuda_device)
     d["g"] = (d["g"].float() - 4.0).bfloat16()
     ref = _after(d, B, T, H, cuda_device)
     for _ in range(2):
-        got = _whole(d, B, T, H, cuda_device)
+        got = _whole(d, B, T, H, cuda_device, launches)
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+# the 8-row, the 16-row (in place of the 8-row and as chosen) and the tensor-memory form on SMs of their own
+@pytest.mark.parametrize("B,T,H", [(1, 1991, 19), (1, 1630, 32), (2, 1531, 19), (1, 4085, 81)])
+@pytest.mark.parametrize("g32,k_first", [(True, False), (False, True), (True, True)])
+def test_either_gate_type_and_state_order_where_k2_has_sms_of_its_own(cuda_device, B, T, H, g32, k_first):
+    d = to_device(O.make_inputs(B, T, H, seed0=T + H, h0_std=0.3), cuda_device)
+    d["g"] = (d["g"].float() - 4.0).to(torch.float32 if g32 else torch.bfloat16)
+    flags = api._flags(True, True, True) | (_lib.FLAG_STATE_K_FIRST if k_first else 0)
+    ref = _after(d, B, T, H, cuda_device, flags=flags)
+    got = _whole(d, B, T, H, cuda_device, BESIDE, flags=flags)
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
 
 
 # one chunk, fewer chunks than stages of the record ring, more; a partial last chunk
@@ -157,8 +180,8 @@ def test_captured_forward_follows_its_inputs(cuda_device, B, T, H):
         assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
 
 
-# the 8-row form (full barrier: 2) and the tensor-memory form (any of its waits: 4)
-@pytest.mark.parametrize("B,T,H,own", [(1, 4736, 8, 2), (1, 600, 96, 4)])
+# the 8-row and the 16-row form (full barrier: 2) and the tensor-memory form (any of its waits: 4)
+@pytest.mark.parametrize("B,T,H,own", [(1, 4736, 8, 2), (1, 600, 96, 4), (1, 1991, 19, 2), (1, 1630, 32, 2), (1, 1530, 42, 2)])
 @pytest.mark.parametrize("k1_status", [0, 1])
 def test_window_wait_runs_out(cuda_device, B, T, H, own, k1_status):
     """K2 on window counters that nothing counts up: it gives up after its limit, the outputs are left alone and the
