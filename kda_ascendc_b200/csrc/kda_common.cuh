@@ -19,10 +19,10 @@
 //   18432   512    Xb_l      bf16 [2][16][8]                   / (xb_off)
 //   18944   512    dec       fp32 again, in the order in which the 8-row K2's lanes read it (dec_lane_off)
 //   19456   4096   v         bf16 [2 halves of 64 columns][16 tok][64], 16-byte units permuted as in w (v_off)
-// (23,552 of the 26,112 bytes)
+// (23,552 of the 26,112 bytes; a record that held u as fp32 used them all)
 //
 // with qg = bf16(qhat * 2^g).  u = X diag(beta) v is not stored: K2 adds it up from Xb and v, which is exact in bf16, on
-// the accumulator of -w h (4 KiB less to write and to read, and K1 does not touch v at all).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
+// the accumulator of -w h (2.5 KiB less to write and to read, and K1 computes nothing with v).  After a plain bulk copy into shared memory (1024-byte aligned) every part is a tensor-core
 // operand as it stands: [w; qg] is a 32-row K-major operand in the 128-byte swizzle of tcgen05 (8-row groups 1024
 // bytes apart), kg^T and Aqk are 8x8 core matrices of 128 contiguous bytes (K-major without swizzle).  tcgen05.mma
 // reads them by descriptor, and every 8x8 matrix of an ldmatrix is free of bank conflicts, most of them at
@@ -52,6 +52,8 @@ constexpr int REC_V = 19456;             // 64 columns of v at REC_V + half * RE
 constexpr int REC_V_HALF = 2048;
 constexpr int REC_SHARED_BYTES = 19456;  // everything every V-slice needs
 constexpr int REC_USED_BYTES = 23552;
+// From record to record.  kda_fwd_workspace_bytes and the problems that the fixed scratch holds follow from it, and callers have
+// sized their buffers by it; records 23,552 bytes apart take the same time (T8192 H32 327.8 us either way, H96 634, T65536 H16 1,731).
 constexpr int REC_BYTES = 26112;
 constexpr int WS_HEADER_BYTES = 256;     // status block at the start of the workspace
 // Header words: 0 = status; HDR_K1_STATUS = K1's own code, which no later kernel overwrites (K2 waits for K1, so a K1
@@ -179,15 +181,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
   }
 }
 
-// Bounded busy-poll for waits that are expected to last a few dozen cycles (a partner warp
-// on another SM sub-partition): polls with the non-blocking test_wait, same limits.
-__device__ __forceinline__ bool mbar_spin_bounded(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-#pragma unroll 1
-  for (int i = 0; i < 4096; ++i)
-    if (mbar_test_wait(bar, parity)) return true;
-  return mbar_wait_bounded(bar, parity, abort_flag);
-}
-
 // ---- flags between GPUs (peer memory) ------------------------------------------
 // A flag is an int32 epoch counter in the waiting GPU's own memory; a peer raises it with a
 // system-scope release store after its data stores, the owner polls it with system-scope acquire
@@ -297,12 +290,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst_smem, const void* tmap,
           "r"(dst_smem), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
-// the same box, only pulled into L2 (no shared-memory destination, nothing to wait for)
-__device__ __forceinline__ void tma_prefetch_l2_4d(const void* tmap, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(tmap), "r"(c0), "r"(c1),
-               "r"(c2), "r"(c3)
-               : "memory");
-}
 __device__ __forceinline__ void bulk_s2g(void* dst, uint32_t src_smem, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src_smem), "r"(bytes)
                : "memory");
@@ -312,11 +299,6 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 
 // ---- shared-memory loads pinned where they are written ------------------------------
-__device__ __forceinline__ float lds_f32(uint32_t addr) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-  return v;
-}
 __device__ __forceinline__ float2 lds_f32x2(uint32_t addr) {
   float2 v;
   asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
