@@ -183,8 +183,9 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 // warps wait for the window of the record they load next.  K2 waits for K1 only, and starts when every K1 CTA
 // is already running.  On k2_sms of the SMs only k2_sm_ctas of K1's CTAs stay (k1_stays), and K2's CTAs fit nowhere else.
 // Which of it pays, measured on B200 as the whole forward in us, K2 after K1 against beside it unless said otherwise:
-//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on every SM: B1 T32768 H16 1,028 /
-//     987, T8192 H16 266.5 / 259.1, H8 236 / 226 (an earlier K1).  With four on the SMs that K2 leaves free T131072 H16 3,727
+//   8-row form with one or two consumer warps per CTA (chains x 8 <= SMs), two K1 CTAs on every SM: B1 T131072 H16 3,705 / 3,438,
+//     T32768 H16 935 / 872, T8192 H16 241 / 227, H12 225 / 214, H8 204.7 / 201.2, B2 T4096 H8 123.8 / 120.4; near the line of 16
+//     items per SM it costs up to 1 %: T5000 H8 127.4 / 128.1, T2600 H16 80.9 / 81.5, T2400 H18 77.3 / 78.3.  With four on the SMs that K2 leaves free T131072 H16 3,727
 //     against 3,704, B2 T4096 H8 129.6 / 129.0; with one on K2's SMs K1 is the longer part (T32768 H16 1,329).
 //   Up to SMs / 6 chains: the 8-row form with four consumer warps on SMs of its own (4 per chain): T8192 H23 326 / 283, H24
 //     330 / 309, T4096 H24 172 / 164, T2500 H23 107 / 102. Beyond, K1 has too few SMs left: T4096 H25 173 / 181.
@@ -199,7 +200,10 @@ Span span_of(const void* ptr, const int64_t s[3], const KdaFwdArgs* a, int heads
 //     H123 942 / 867, H136 998 / 969, H148 1,046 / 1,082.
 //   The same form, two CTAs per SM on SMs of their own, where its step for two (1.27 us) and K1 on the others take about the
 //     same time, and long chains: against the line above T8192 H75 636 / 639, H88 672 / 655, H96 686 / 651, H104 716 / 705, H111
-//     769 / 772; T1024 H88 106 / 108, H96 109 / 107, H111 115 / 120.
+//     769 / 772; T1024 H88 106 / 108, H96 109 / 107, H111 115 / 120.  The line in chunks, 64 / 128 / 192 / 256: H81 100 and 108 / 173
+//     and 174 / 249 and 248 / 339 and 329, H88 102 and 106 / 179 and 178 / 263 and 257 / 353 and 344, H96 106 and 109 / 187 and 185 / 278 and
+//     274 / 362 and 358; with the most chains, where K1 on the SMs left is the longer part, it comes later: H100 equal at 256, H103
+//     387 and 393 there.
 struct Beside {
   int win;                       // chunks per window; 0 = K2 starts after K1
   int variant, vsplit;           // K2's form: pick_split's, or one with the same bits
@@ -364,7 +368,9 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     // that K1 leaves.  Whole forward on B200, ordinary launch against this one: B1 T100 H32 17.0 -> 14.9 us, T512
     // H32 35.6 -> 35.1, T1024 H8 41.3 -> 38.4, B8 T2048 H32 512 -> 507.  Not the 8-row form with four consumer
     // warps per CTA on more than 32 chunks: in the order in which K1 leaves the SMs its CTAs step slower than
-    // in the order of an ordinary launch (T2048 H32 113.0 -> 115.2, T8192 H32 415 -> 420, H24 379 -> 386).
+    // in the order of an ordinary launch.  Of the calls that still run after K1 and reach this line that holds for the longest only
+    // (T2500 H26 110.2 -> 112.5, T4096 H25 171.5 -> 171.7, T1600 H28 76.2 -> 76.3, T1540 H24 70.0 -> 70.2); shorter ones would be faster
+    // started ahead: T1600 H30 76.2 -> 75.3, T1200 H32 61.6 -> 59.2, T1000 H24 47.6 -> 46.9, T800 H37 45.4 -> 43.0, T544 H20 28.8 -> 26.7.
     const long long steps = a->n_seqs > 0 ? a->n_chunks / a->n_seqs : p.NT;
     // Nor packed sequences of more than eight chunks in the mean in the 16-row form on more CTAs than SMs: the long
     // chains of unequal lengths then run on beside others of the launch.  3 to 64 sequences of log-normal lengths
@@ -451,12 +457,15 @@ int do_k2(const KdaFwdArgs* a, bool state_only, int zero_u, cudaStream_t st, con
     // has a second CTA and 0.85 without, against 0.53 in the 16-row form.  So the longest sequences, on at most half of the
     // SMs, run there, in front of and beside the tensor-memory launch (which starts when K1 has ended, about 2 us later
     // than without), if they are long: more steps than 0.9 x the chunks of all chains per SM, which take 0.67 us each in pairs,
-    // and than 1.5 x the mean.  The lengths are on the device: either kernel leaves out what the other does.  Whole forward, us,
-    // without / with, log-normal lengths (sigma 1): 24 sequences of 16,411 tokens H32 487 / 467, 40 of 30,000 H8 297 / 245, 20 of
-    // 20,000 H8 290 / 227, 10 of 12,000 H16 286 / 227, 8 of 24,000 H32 802 / 741, 6 of 20,000 H32 652 / 637, 9 of 14,000 H16 396 /
-    // 317, 12 of 30,000 H8 419 / 339.  Where no sequence is long: 64 of 32,000 H32 879 / 880, 12 of 8,000 H32 238 / 240,
-    // 16 x 1,024 H32 441 / 443, 32 x 500 H16 238 / 240, 5 x 2,000 H32 314 / 317; shorter ones do not pay for the launch (8 x 520 H32
-    // 126 / 128).  On all SMs instead of half of them 6 of 20,000 H32 takes 692; with 1.25 x the mean 4 x 2,500 H32 304 / 356.
+    // and than 1.5 x the mean.  The lengths are on the device: either kernel leaves out what the other does.  Whole forward on one
+    // set of buffers, us, without / with, log-normal lengths (sigma 1): 24 sequences of 16,411 tokens H32 525 / 519 (as one call among
+    // others on changing buffers 536 / 534), 16 of 20,000 H32 636 / 630, 8 of 24,000 H32 780 / 763, 6 of 20,000 H32 774 / 657, 30 of
+    // 24,000 H16 388 / 379, 40 of 28,000 H8 306 / 228, 64 of 32,000 H8 470 / 366.  Where no sequence is long, or hardly, the launch costs
+    // up to 1.6 %: 16 x 1,024 H32 494 / 501, 32 x 500 H16 258 / 262, 5 x 2,000 H32 329 / 331, 64 x 500 H32 1,001 / 1,007, 48 of 32,000 H16
+    // 495 / 503; shorter ones do not pay for it (8 x 520 H32 126 / 128).  The factor at 0.8 / 0.9 / 1.0: 24 of 16,411 H32 517 / 519 / 542 and
+    // with other lengths 516 / 514 / 510, 16 of 20,000 H32 621 / 630 / 659, 6 of 20,000 639 / 657 / 663, 30 of 24,000 H16 373 / 379 / 402, 40
+    // of 28,000 H8 228 / 228 / 233.  On all SMs instead of half of them 6 of 20,000 H32 took 692 in place of 653; with 1.25 x the mean
+    // 4 x 2,500 H32 356 in place of 304.
     const long long items = static_cast<long long>(a->n_chunks) * a->H;
     const int long_max = static_cast<int>(std::min<long long>(a->n_seqs - 1, sms / (4LL * a->H)));
     if (a->k2_variant == 0 && (p.by_length || bh <= sms) && a->n_seqs <= kda::MAX_SORTED_SEQS && long_max > 0 && items >= 64LL * sms) {

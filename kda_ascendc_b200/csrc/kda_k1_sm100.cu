@@ -18,13 +18,15 @@
 // kg = khat 2^(g_last-g) as a hi/lo bf16 pair, dec = 2^g_last -- the arrangement of
 // the reference's Ascend pipeline (python/kda_ascendc_v1/api.py:890-897).
 //
-// Data movement: the four 16x128 input tiles arrive by tiled TMA copies (4-D tensor maps over
+// Data movement: the 16x128 input tiles arrive by tiled TMA copies (4-D tensor maps over
 // (d, head, token, batch) built from the caller's strides, so head-shard and segment views
-// need no copy; rows past T are zero-filled by the copy) that complete on one mbarrier; as soon as
-// a chunk's inputs have been consumed the copies of the CTA's next chunk are issued into the
-// same tiles, so the ~2.5 us load latency hides behind the rest of the chunk.  v is only passed on: its two 64-column boxes
-// arrive, swizzled by the copy, where the record's part with kg, Aqk, dec, Xb and v is put together.  That part, qg and w leave
-// by five bulk stores.  With u worked out here and stored as fp32 from the accumulator fragments K1 alone took 147.5 us, now
+// need no copy; rows past T are zero-filled by the copy).  Those of q, k and g complete on one mbarrier; as soon as
+// a chunk's have been consumed the copies of the CTA's next chunk are issued into the
+// same tiles, so the ~2.5 us load latency hides behind the rest of the chunk.  v is only passed on (of packed sequences, with the
+// rows behind a sequence's end cleared): its two 64-column boxes, with a barrier of their own, arrive, swizzled by the copy, where
+// the record's part with kg, Aqk, dec, Xb and v is put together.  They are asked for within their own item, once the stores of the
+// item before have left that place (the first item's at once with the rest: T100 H32 11.3 -> 11.5 us), and waited for two phases
+// later.  That part, qg and w leave by five bulk stores.  With u worked out here and stored as fp32 from the accumulator fragments K1 alone took 147.5 us, now
 // 132.7 (T8192 H32; H96 426 -> 383, in a row of calls at the power limit 468 -> 410; the prepared batch 276 -> 257).
 // khat beta 2^g is rounded to bf16 with beta in it, as ever: without, where gates are near zero khat 2^g rounds back to
 // khat more often than not, and the state's error against 64 bits grows by 1 % (gates of -8: 1.283e-3 -> 1.298e-3).
@@ -111,8 +113,9 @@ __device__ __forceinline__ K1Item k1_item(const K1Params& p, int id) {
 // BESIDE: K2 runs beside this kernel (time-major items, finished items counted per window).  Registers: four CTAs per
 // SM need 128 a thread or fewer.  Beside K2, two CTAs share every SM sub-partition's 16,384 registers with up to three
 // warps of the tensor-memory K2 (96 a thread): 2 x 32 x 112 + 3 x 32 x 96 is all of them, and with more K2 does not
-// start before K1 ends.  kda_fwd, with 128 registers and with 112: T8192 H96 1,223 and 849 us, T2048 H80 303 and 201;
-// beside the 8-row form both fit (T32768 H16 988 and 990, B2 T4096 H8 135.1 and 135.6).
+// start before K1 ends.  kda_fwd, with 128 registers and with 112: T2048 H80 262 and 172 us, T1024 H120 173 and 120.
+// Beside the other forms, and a tensor-memory K2 on SMs of its own, either fits: T32768 H16 871 and 872, B2 T4096 H8 119.9 and
+// 120.2, T8192 H32 326 and 325, H96 623 and 628, H24 302 and 308.
 // FORM: what is known when the kernel is compiled.  FORM_ALL: gate, l2-norm and beta sigmoid in the kernel, dt_bias at an 8-byte
 // boundary; FORM_NONE: all three done by the caller (then FAST_EXP is false); neither with debug outputs.  FORM_ANY: the flags
 // decide.  Against FORM_ANY for the same call, with u still worked out here: K1 alone T8192 H32 156.4 -> 147.8 us, H96 445 -> 427, inputs

@@ -427,7 +427,7 @@ static cudaError_t launch_k2m_c(const K2Params& p, cudaStream_t stream) {
   if constexpr (CW == 4 && !STATE_ONLY)
     if (p.long_ring == 8) return launch_k2m_t<4, false, 1, false, 8>(p, nblocks, stream);
   if (CW == 4 && nblocks > sms[dev]) return launch_k2m_t<CW, STATE_ONLY, 2>(p, nblocks, stream);
-  if constexpr (CW == 4 && !STATE_ONLY)   // the tail of a tensor-memory launch
+  if constexpr (CW == 4 && !STATE_ONLY)   // packed: the tail of a tensor-memory launch, or the long sequences in front of one
     if (p.by_length) return launch_k2m_t<4, false, 1, true>(p, nblocks, stream);
   return launch_k2m_t<CW, STATE_ONLY, 1>(p, nblocks, stream);
 }

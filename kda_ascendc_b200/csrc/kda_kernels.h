@@ -115,7 +115,10 @@ inline int k2_smem(const K2Params& p, int need) { return p.one_per_sm && need < 
 
 // One launch, with or without the programmatic stream serialization attribute.  K1 and the token recurrence are launched
 // with it behind whatever runs before them.  K2 and the recurrence do not let the next kernel start before their end: its
-// launch is under way by then all the same, and CTAs that only wait took room and cost more than their early start gave.  Calls
+// launch is under way by then all the same, and CTAs that only wait took room and cost more than their early start gave.  One
+// exception: the 16-row K2 of the long ones of packed sequences, beside which the tensor-memory K2 of the others is to run.  Its
+// CTAs let that start, or leave, only behind their own wait for K1, so the tensor-memory K2 reads records without waiting, and
+// the last of its CTAs waits for the 16-row launch, so that the call's last kernel ends last.  Calls
 // one after the other, us, ordinary launches / with the attribute / and with an early start: one-token recurrence B8 H32 8.2 /
 // 6.4 / 6.6, B64 43.7 / 42.3 / 43.9, four tokens B16 20.5 / 18.7 / 19.1; forward T16 H32 9.3 / 7.5 / 8.2, T100 H32 13.2 / 11.3 / 13.0, T64
 // H150 23.0 / 21.6 / 22.9, B2 T1024 H4 32.8 / 30.0 / 30.6.
